@@ -247,7 +247,7 @@ struct gls_ctx {
     uint64_t pins_total = 0;
     std::vector<uint8_t> driven;             // net driven by a gate output
     std::vector<uint32_t> ext_inputs;        // nets read by gates and driven by no gate
-    DevBuf meta, arcs, ndel, lut, slut;
+    DevBuf meta, arcs, ndel, lut, slut, fast;
     std::vector<LevelScratch *> lsc;         // level work spaces ([0]: sequential runs)
     uint32_t seg_cap = 0;                    // segment-table size new work spaces get
     uint64_t scr_cap = 0;                    // stack words new work spaces get

@@ -87,6 +87,17 @@ struct NetDelay {
     uint32_t d[8];
 };
 
+// What the gate kernels' fast step needs of a gate output with at most three
+// input nets, where every input net has its arcs (or none has any), all its
+// delays are below 2^16 - 1 and known inputs give known outputs.
+struct FastRec {
+    uint32_t d[6];   // per input net: delays of a rising, a falling input edge, as rise | fall << 16
+    uint32_t tt;     // output (bit) for input values 0 / 1: bit sum(value(net j) << 2j)
+    uint32_t usable; // 0: the general step only
+};
+static_assert(sizeof(FastRec) == 32, "FastRec is read as two 16-byte words");
+constexpr uint32_t kFastDelayMax = 0xFFFEu;
+
 // CheckDelay (src/simulate.cpp:1178-1201) as a function of (pre, cur)
 __host__ __device__ constexpr int sense_of(uint32_t pre, uint32_t cur)
 {
@@ -179,6 +190,7 @@ struct LevelArgs {
     const DrvMeta *meta;
     const uint4 *slut;          // per driver with at most 3 input nets: truth table over its input nets' values,
                                 // 2 bits per entry, entry = sum(value(net j) << 2j) (64 entries in 128 bits)
+    const uint4 *fast;          // per driver: its FastRec as two 16-byte words
     const ArcDev *arcs;
     const NetDelay *ndel;
     const uint8_t *lut;

@@ -514,7 +514,10 @@ __device__ __forceinline__ uint32_t sel4(const uint4 &q, uint32_t k)
 // the variant; 64-bit windows always run variant 0.
 constexpr uint32_t kSimBlock = 128;
 constexpr int kSimV256 = 1, kSimVWide = 2;
-template <int kV> constexpr uint32_t sim_block() { return (kV & kSimV256) ? 256u : kSimBlock; }
+template <int kV, int M> __host__ __device__ constexpr uint32_t sim_block()
+{
+    return (kV & kSimV256) ? 256u : kSimBlock;
+}
 #ifndef GLS_READER_W3
 #define GLS_READER_W3 1   // events per reader chunk in the wider gate kernels
 #endif
@@ -726,6 +729,16 @@ __device__ __forceinline__ void cut_at(const Wd *__restrict__ pool, const uint64
     }
 }
 
+// The time of cut sk alone (0 < sk < S), as cut_at computes it.
+__device__ __forceinline__ uint32_t cut_time(const uint32_t *__restrict__ pool, int sec, uint64_t poff, uint64_t soff,
+                                             uint32_t plen, uint32_t slen, uint32_t sk, uint32_t S)
+{
+    if (sec < 0) return ev_time(pool[poff + mul_div(sk, plen, S)]);
+    uint32_t ip, is;
+    const uint32_t r = mul_div(sk, plen + slen, S);
+    return rank_time2(pool + poff, plen, pool + soff, slen, r, mul_div(r, plen, plen + slen), ip, is);
+}
+
 template <int M, class Wd, bool kWideChunk>
 __device__ void sim_segment(const WinDev &w, const LevelArgs &a, const DrvMeta &md, uint32_t s,
                             uint32_t S, uint32_t seg_id, uint64_t scr, const uint4 sl)
@@ -841,6 +854,228 @@ __device__ void sim_segment(const WinDev &w, const LevelArgs &a, const DrvMeta &
     reinterpret_cast<SegRecT<Wd> *>(w.segs)[seg_id] = r;
 }
 
+// the word at q where `go`, else kInf, without a branch
+__device__ __forceinline__ uint32_t ld_if(const uint32_t *q, bool go)
+{
+    uint32_t v;
+    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\tmov.u32 %0, 0xFFFFFFFF;\n\t@p ld.global.nc.u32 %0, [%1];\n\t}"
+        : "=r"(v) : "l"(q), "r"((uint32_t)go));
+    return v;
+}
+
+// Reader of one change list a word at a time: the head and the event after
+// it in registers, kInf behind the list's end.  Moving on is branch-free, so
+// that lanes whose lists move at different steps stay together.  (More
+// events held ahead measured no faster: 79.6 ms of gate kernels with one and
+// with two for 2-input gates, 80.9 with three and two.)
+struct ListReader {
+    uint32_t h, n;
+    const uint32_t *q;   // the event after n
+    uint32_t qe;         // low word of the list's end (a list is shorter than 2^30 events)
+
+    __device__ __forceinline__ void start(const uint32_t *x, uint32_t b, uint32_t len)
+    {
+        h = ld_if(x + b, b < len);
+        n = ld_if(x + b + 1, b + 1 < len);
+        q = x + min(b + 2, len);
+        qe = (uint32_t)(uintptr_t)(x + len);
+    }
+    __device__ __forceinline__ void advance(bool go)
+    {
+        const bool more = go && (uint32_t)(uintptr_t)q != qe;
+        h = go ? n : h;
+        asm("{\n\t.reg .pred p, r;\n\tsetp.ne.u32 p, %2, 0;\n\tsetp.ne.u32 r, %3, 0;\n\t@p mov.u32 %0, 0xFFFFFFFF;\n\t"
+            "@r ld.global.nc.u32 %0, [%1];\n\t}"
+            : "+r"(n) : "l"(q), "r"((uint32_t)go), "r"((uint32_t)more));
+        q += more ? 1 : 0;
+    }
+};
+
+// One time segment of a gate output with at most three input nets, 32-bit
+// words.  Steps whose input values are all 0 or 1 before and after (nearly
+// all of them: X and Z leave a net with its first real event) take the fast
+// step; any other step, and every step of a gate output whose FastRec is
+// not usable, takes the general one.
+//
+// What bounds it: instruction issue.  A lane walks its own segment, so a
+// warp issues both the step and, on nearly every iteration, the output
+// change of some lane.  The fast step therefore keeps everything in
+// registers and is branch-free but for the rare pops: the truth table is one
+// word shifted by the input state, the delays of all input nets are packed
+// (rise, fall) pairs whose 16-bit minimum is one instruction, the end of the
+// segment is a time (so no list needs an end position beyond its own end),
+// the entry below the stack top is kept so that an inertial pop rarely reads
+// the stack back, and the range check of output times is made once per
+// segment (a delay is below 2^16).  Measured against the walk with inner
+// branches and delay-table loads (sim_segment): the 3-input kernel of the
+// 100,000-cell, 6-level large-configuration case 460 -> 301 us and 350 -> 183
+// M warp instructions at 14 -> 25 active lanes, the 2-input one 320 -> 277 us
+// and 205 -> 119 M; the 2 M cell design over 5,000 cycles 97.2 -> 79.6 ms of
+// gate kernels.
+template <int M>
+__device__ __forceinline__ void sim_segment2(const WinDev &w, const LevelArgs &a, uint32_t drv, uint32_t s, uint32_t S,
+                                             uint32_t seg_id, uint64_t scr)
+{
+    const uint32_t *__restrict__ pw = w.pool;
+    const DrvMeta *__restrict__ mdp = a.meta + drv;
+    const int m = mdp->m;   // M, or 0 in the 1-input class
+    uint64_t off[M];
+    uint32_t len[M];
+    int piv = 0, sec = -1;   // the longest input list and the longest of the others
+    uint32_t plen = 0, slen = 0;
+#pragma unroll
+    for (int j = 0; j < M; ++j) {
+        len[j] = 0; off[j] = 0;
+        if (j < m) {
+            const uint32_t net = mdp->net[j];
+            off[j] = w.net_off[net];
+            len[j] = w.net_len[net];
+            if (len[j] > plen) { sec = piv; slen = plen; plen = len[j]; piv = j; }
+            else if (sec < 0 || len[j] > slen) { sec = j; slen = len[j]; }
+        }
+    }
+    if (m < 2) sec = -1;
+    uint64_t poff = 0, soff = 0;
+#pragma unroll
+    for (int j = 0; j < M; ++j) {
+        if (j == piv) poff = off[j];
+        if (j == sec) soff = off[j];
+    }
+    // the segment's first events (cut s) and its end time (cut s + 1)
+    uint32_t cb[M];
+#pragma unroll
+    for (int j = 0; j < M; ++j) cb[j] = 0;
+    if (s > 0) cut_at<M>(pw, off, len, m, piv, sec, poff, soff, plen, slen, s, S, cb);
+    uint32_t tmax, tend;   // latest event time of the segment; words at or above tend lie behind it
+    if (s + 1 < S) {
+        tmax = cut_time(pw, sec, poff, soff, plen, slen, s + 1, S);
+        tend = tmax << 2;
+    } else {
+        tmax = 0;
+#pragma unroll
+        for (int j = 0; j < M; ++j)
+            if (len[j]) tmax = max(tmax, ev_time(pw[off[j] + len[j] - 1]));
+        tend = kInf;
+    }
+    const uint4 f0 = __ldg(a.fast + 2ull * drv), f1 = __ldg(a.fast + 2ull * drv + 1);
+    const uint32_t dp[3] = {f0.x, f0.z, f1.x}, dn[3] = {f0.y, f0.w, f1.y};
+    const uint32_t tt = f1.z;
+    // input values, 2 bits per net; 0x15 bits of `mixed` mark nets at X or Z
+    uint32_t curp = 0x15u, region = s;
+    bool before = false;
+    ListReader rd[M];
+#pragma unroll
+    for (int j = 0; j < M; ++j) {
+        const uint32_t b = cb[j];
+        region += b;
+        const uint32_t *x = pw + off[j];
+        if (b > 0) {
+            curp = (curp & ~(3u << (2 * j))) | (ev_val(x[b - 1]) << (2 * j));
+            before = true;
+        }
+        rd[j].start(x, b, len[j]);
+    }
+    constexpr uint32_t kBits = M == 1 ? 0x1u : (M == 2 ? 0x5u : 0x15u);
+    // a gate output without a usable FastRec, or times too close to the
+    // largest one, take the general step throughout
+    const uint32_t never = (f1.w != 0u && tmax <= kMaxTime - 0x10000u) ? 0u : kBits;
+    uint32_t mixed = ((curp ^ (curp >> 1)) & kBits) | never;
+    // Every step consumes an event and pushes at most one entry, so a
+    // segment's stack ends within the gate output's scratch.
+    uint32_t *ot = w.scratch + scr + region;
+    uint32_t cnt = 0;
+    // top of the stack and the entry below it (kInf: not at hand).  With no
+    // entry left the top reads as (0, X): below every later candidate, and
+    // different from 0 and 1.
+    uint32_t top = EvW<uint32_t>::word(0, kVX), below = kInf;
+    if (s == 0) { ot[0] = top; cnt = 1; }
+    uint32_t fprev = kVX;
+    if (before) fprev = slut_get<M>(__ldg(a.slut + drv), curp);
+    uint32_t minw = kInf;   // smallest candidate time << 2
+    for (;;) {
+        uint32_t mk = rd[0].h | 3u;
+#pragma unroll
+        for (int j = 1; j < M; ++j) mk = min(mk, rd[j].h | 3u);
+        if (mk >= tend) break;
+        const uint32_t lastp = curp;
+        bool ch[M];
+#pragma unroll
+        for (int j = 0; j < M; ++j) {
+            ch[j] = (rd[j].h | 3u) == mk;
+            const uint32_t cj = (curp & ~(3u << (2 * j))) | ((rd[j].h << (2 * j)) & (3u << (2 * j)));
+            curp = ch[j] ? cj : curp;
+            rd[j].advance(ch[j]);
+        }
+        const uint32_t mixed0 = mixed;
+        mixed = ((curp ^ (curp >> 1)) & kBits) | never;
+        if ((mixed | mixed0) == 0u) {
+            const uint32_t F = ((tt >> (curp & kBits)) & 1u) ? kV1 : kV0;
+            const bool chg = F != fprev;
+            fprev = F;
+            const uint32_t fall = lastp & ~curp;
+            uint32_t r[3] = {kInf, kInf, kInf};
+#pragma unroll
+            for (int j = 0; j < M; ++j) r[j] = ch[j] ? ((fall & (1u << (2 * j))) ? dn[j] : dp[j]) : kInf;
+            const uint32_t d2 = M == 1 ? r[0] : (M == 2 ? __vminu2(r[0], r[1]) : __vimin3_u16x2(r[0], r[1], r[2]));
+            const uint32_t d = F ? (d2 & 0xFFFFu) : (d2 >> 16);
+            const uint32_t lo = (mk ^ 3u) + (d << 2);
+            minw = chg ? min(minw, lo) : minw;
+            // inertial update, src/simulate.cpp:991-1009.  Both states of a
+            // fast step are known, so it is not the first: lo > 0, and the
+            // bottom (0, X) is never popped.
+            if (chg && top >= lo) {
+                do {
+                    --cnt;
+                    if (below != kInf) top = below;
+                    else top = cnt > 0 ? ot[cnt - 1] : EvW<uint32_t>::word(0, kVX);
+                    below = kInf;
+                } while (top >= lo);
+            }
+            const bool push = chg && ((top ^ F) & 3u) != 0u;
+            if (push) ot[cnt] = lo | F;
+            below = push ? top : below;
+            top = push ? lo | F : top;
+            cnt += push ? 1u : 0u;
+            continue;
+        }
+        // general step
+        const uint32_t F = slut_get<M>(__ldg(a.slut + drv), curp);
+        if (F == fprev) continue;
+        const uint32_t so1 = (kSense1Tab >> (2 * (fprev * 4 + F))) & 3u;
+        fprev = F;
+        uint32_t chg = 0;
+#pragma unroll
+        for (int j = 0; j < M; ++j) chg |= ch[j] ? 1u << j : 0u;
+        const uint32_t d = (mdp->flags & kFlagRegular)
+                               ? regular_delay<M>(a.ndel + mdp->dt_off, chg, so1, curp, lastp, a.def_delay)
+                               : select_delay(a.arcs + mdp->arc_off, mdp->n_arcs, chg, (int)so1 + 1, curp, lastp,
+                                              a.def_delay);
+        const uint64_t o64 = (uint64_t)ev_time(mk) + d;
+        if (o64 > kMaxTime) { atomicOr(w.err, kErrTime); break; }
+        const uint32_t lo = (uint32_t)o64 << 2;
+        minw = min(minw, lo);
+        int popped_v = -1;
+        while (cnt > 0 && top >= lo) {
+            if (s == 0 && cnt == 1) { popped_v = (int)ev_val(top); cnt = 0; break; }
+            --cnt;
+            top = cnt > 0 ? ot[cnt - 1] : EvW<uint32_t>::word(0, kVX);
+            below = kInf;
+        }
+        const int prevv = cnt > 0 ? (int)ev_val(top) : popped_v;
+        if (prevv != (int)F) {
+            below = kInf;
+            top = lo | F;
+            ot[cnt++] = top;
+        } else if (cnt == 0) {
+            atomicOr(w.err, kErrEmptied);
+            break;
+        }
+    }
+    SegRec r;
+    r.region = region; r.cnt = cnt; r.min_o = minw == kInf ? kInf : minw >> 2; r.last = top;
+    w.segs[seg_id] = r;
+}
+
 // Segments of all windows of a launch form one index space: s_pre[k] is
 // the first index of window k.
 // skip_err leaves out windows whose error flag is set; only kernels during
@@ -898,10 +1133,11 @@ template <int M, bool kBatch, class Wd, int kV>
 #ifndef GLS_SIM1_BLOCKS
 #define GLS_SIM1_BLOCKS GLS_SIM2_BLOCKS   // resident blocks per SM the 1-input gate kernel is compiled for
 #endif
-__global__ void __launch_bounds__(sim_block<kV>(), (M == 1 ? GLS_SIM1_BLOCKS : (M == 2 ? GLS_SIM2_BLOCKS : (M == 3 ? GLS_SIM3_BLOCKS : 4))) /
-                                                    ((kV & kSimV256) ? 2 : 1))
+__global__ void __launch_bounds__(sim_block<kV, M>(), (M == 1 ? GLS_SIM1_BLOCKS : (M == 2 ? GLS_SIM2_BLOCKS : (M == 3 ? GLS_SIM3_BLOCKS : 4))) /
+                                                    (sim_block<kV, M>() / kSimBlock))
     k_sim(const WinSet<kBatch> ws, LevelArgs a, uint32_t d0, uint32_t d1)
 {
+    constexpr bool kFast = M <= 3 && std::is_same<Wd, uint32_t>::value && !(kV & kSimVWide);
     __shared__ uint32_t s_next;
     __shared__ uint32_t s_pre[kBatch ? kMaxWave + 1 : 2];
     __shared__ uint32_t sm32[32];
@@ -970,9 +1206,13 @@ __global__ void __launch_bounds__(sim_block<kV>(), (M == 1 ? GLS_SIM1_BLOCKS : (
         if (!kBatch) s_hint = i;
         const uint32_t sb = w.seg_base[i];
         const uint32_t S = w.seg_base[i + 1] - sb;
-        const DrvMeta md = a.meta[a.lo + i];
-        const uint4 sl = M <= 3 ? __ldg(a.slut + a.lo + i) : make_uint4(0, 0, 0, 0);
-        sim_segment<M, Wd, (kV & kSimVWide) != 0>(w, a, md, g - sb, S, g, w.scr[i], sl);
+        if constexpr (kFast) {
+            sim_segment2<M>(w, a, a.lo + i, g - sb, S, g, w.scr[i]);
+        } else {
+            const DrvMeta md = a.meta[a.lo + i];
+            const uint4 sl = M <= 3 ? __ldg(a.slut + a.lo + i) : make_uint4(0, 0, 0, 0);
+            sim_segment<M, Wd, (kV & kSimVWide) != 0>(w, a, md, g - sb, S, g, w.scr[i], sl);
+        }
     }
 }
 
@@ -1860,15 +2100,16 @@ static void sim_thread(const WS &ws, const LevelArgs &a, int cls, uint32_t d0, u
                        cudaStream_t st)
 {
     constexpr bool B = std::is_same<WS, WinSet<true>>::value;
-    constexpr uint32_t bs = sim_block<kV>();
-    const int per_sm = (cls == 0 ? GLS_SIM1_BLOCKS : (cls == 1 ? GLS_SIM2_BLOCKS : (cls == 2 ? GLS_SIM3_BLOCKS : 4))) /
-                       ((kV & kSimV256) ? 2 : 1);
-    const int grid = sm_count * per_sm;
+    auto go = [&](auto mt, int per_sm) {   // per_sm: resident 128-thread blocks
+        constexpr int M = decltype(mt)::value;
+        constexpr uint32_t bs = sim_block<kV, M>();
+        k_sim<M, B, Wd, kV><<<sm_count * per_sm / (bs / kSimBlock), bs, 0, st>>>(ws, a, d0, d1);
+    };
     switch (cls) {
-    case 0: k_sim<1, B, Wd, kV><<<grid, bs, 0, st>>>(ws, a, d0, d1); break;
-    case 1: k_sim<2, B, Wd, kV><<<grid, bs, 0, st>>>(ws, a, d0, d1); break;
-    case 2: k_sim<3, B, Wd, kV><<<grid, bs, 0, st>>>(ws, a, d0, d1); break;
-    default: k_sim<kMaxSlots, B, Wd, kV><<<grid, bs, 0, st>>>(ws, a, d0, d1); break;
+    case 0: go(std::integral_constant<int, 1>(), GLS_SIM1_BLOCKS); break;
+    case 1: go(std::integral_constant<int, 2>(), GLS_SIM2_BLOCKS); break;
+    case 2: go(std::integral_constant<int, 3>(), GLS_SIM3_BLOCKS); break;
+    default: go(std::integral_constant<int, kMaxSlots>(), 4); break;
     }
 }
 
