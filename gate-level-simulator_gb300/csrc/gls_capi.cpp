@@ -70,6 +70,7 @@ void ctx_level_args(const gls_ctx *ctx, LevelArgs *a)
     a->wave_e = nullptr;
     a->wide = 0;
     a->plan_part = 0;
+    a->level = 0;
 }
 
 namespace {
@@ -160,6 +161,8 @@ extern "C" int gls_create(const gls_opts *opts, gls_ctx **out)
     if (const char *v = getenv("GLS_SIM_CONCURRENT")) ctx->concurrent = strtoul(v, nullptr, 0) != 0;
     if (const char *v = getenv("GLS_SIM_PIPELINE")) ctx->pipeline = strtoul(v, nullptr, 0) != 0;
     if (const char *v = getenv("GLS_PLAN_OVERLAP")) ctx->plan_overlap = strtoul(v, nullptr, 0) != 0;
+    if (const char *v = getenv("GLS_GATE")) ctx->gate_kernel = strtoul(v, nullptr, 0) != 0;
+    if (const char *v = getenv("GLS_GATE_THREADS")) ctx->gate_threads = (uint32_t)strtoul(v, nullptr, 0);
     if (const char *v = getenv("GLS_COPY_LANES")) ctx->copy_lanes = (uint32_t)strtoul(v, nullptr, 0);
     uint32_t per_sm = 128;
     if (const char *v = getenv("GLS_SIM_WARP_SEGS")) per_sm = std::max(1u, (uint32_t)strtoul(v, nullptr, 0));
@@ -177,6 +180,7 @@ static void free_window(Window *w)
     w->init_off.release(); w->init_len.release(); w->saif.release(); w->small.release();
     w->stim_dev.release();
     w->dwin.release();
+    w->lvl.release();
     w->h_words.release(); w->h_off.release(); w->h_len.release();
     delete w;
 }
@@ -591,6 +595,12 @@ static double pool_scale(const gls_ctx *ctx, const Window *w)
     return avg * (double)ctx->pins_total;
 }
 
+// about the fan-in events of one gate output
+static double gate_events_est(const gls_ctx *ctx, const Window *w)
+{
+    return ctx->n_drv ? 2.5 * pool_scale(ctx, w) / ctx->n_drv : 0.0;
+}
+
 // the pool a window is given: its estimate, raised to what earlier windows
 // of this netlist needed (unless the caller fixed the size)
 static uint64_t projected_cap(const gls_ctx *ctx, const Window *w)
@@ -619,6 +629,7 @@ static int upload_window(gls_ctx *ctx, Window *w, bool sync = true)
     CK(take_buf(ctx, w->init_len, n * 4), "alloc init_len");
     CK(w->saif.ensure(n * 24), "alloc saif");
     CK(w->small.ensure(256), "alloc counters");
+    CK(w->lvl.ensure((ctx->drv_level_start.size()) * sizeof(LevelCtr)), "alloc level counters");
     CK(take_buf(ctx, w->stim_dev, w->stim_nets.size() * 4 + 16), "alloc stim nets");
     if (w->stim_events)
         CK(cudaMemcpyAsync(w->pool.p, w->h_words.p, w->stim_events * wb, cudaMemcpyHostToDevice, ctx->stream),
@@ -821,6 +832,7 @@ static WinDev make_windev(gls_ctx *ctx, Window *w, const LevelScratch &ls, int p
     d.segs = ls.segs.as<SegRec>();   // SegRecT<WideWord> records in a window of 64-bit words
     d.copies = ls.copies.as<CopyRec>();
     d.scratch = ls.scratch.as<uint32_t>();
+    d.lvl = w->lvl.as<LevelCtr>();
     d.scr_cap = ls.scr_cap * 4 / w->word_bytes();   // the stacks are sized in 32-bit words
     d.cap = w->cap;
     d.seg_cap = ls.seg_cap;
@@ -854,9 +866,36 @@ static int reset_window(gls_ctx *ctx, Window *w)
     CK(cudaMemcpyAsync(w->net_off.p, w->init_off.p, n * 8, cudaMemcpyDeviceToDevice, ctx->stream), "reset offsets");
     CK(cudaMemcpyAsync(w->net_len.p, w->init_len.p, n * 4, cudaMemcpyDeviceToDevice, ctx->stream), "reset lengths");
     CK(cudaMemsetAsync(w->saif.p, 0xFF, n * 24, ctx->stream), "reset saif");
+    CK(cudaMemsetAsync(w->lvl.p, 0, ctx->drv_level_start.size() * sizeof(LevelCtr), ctx->stream), "reset level counters");
     unsigned long long small[8] = {w->stim_events + ctx->pool_gap, 0, 0, 0, 0, 0, 0, 0};
     CK(cudaMemcpyAsync(w->small.p, small, sizeof small, cudaMemcpyHostToDevice, ctx->stream), "reset counters");
     return GLS_OK;
+}
+
+// Whether a run's levels go through k_gate: 32-bit words and the default
+// thread-per-segment schedule.
+static bool gate_path(const gls_ctx *ctx, const LevelArgs &a, bool)
+{
+    return ctx->gate_kernel && !a.wide && a.warp_mask == 0 && a.sim_variant == 0 && a.bal_weight <= 0.f;
+}
+
+// k_gate's threads (and so time segments) per gate output, for a level of
+// `outs` gate outputs of about `est` fan-in events each.  Fewer, longer
+// segments spend less on cut searches and linking; more of them even out the
+// level's end and fill the GPU where the level is narrow.  Measured (device
+// ms, threads 32 / 64 / 128 / 256 / 512): 16,667 outputs of 5,300 events a
+// level 102 / 88 / 82 / 96 / 138; 3,333 of 9,600 38 / 24 / 16.7 / 14.9 /
+// 17.8; 800 of 2,900 5.1 / 3.0 / 2.0 / 1.8 / 2.3; 100 of 670 .53 / .40 / .34
+// / .34 / .34; 26,700 of 1,200 25.1 / 29.1 / 27.6 / 40 / 73.  So: at least 24
+// estimated events a thread; while one and a half rounds of blocks take the
+// whole level, six.
+static uint32_t gate_block(const gls_ctx *ctx, uint64_t outs, double est)
+{
+    if (ctx->gate_threads) return std::min(kGateMaxThreads, std::max(32u, ctx->gate_threads & ~31u));
+    uint32_t t = 32;
+    while (t < 256 && est >= 2.0 * 24 * t) t *= 2;
+    while (t < 256 && outs * t * 2 <= (uint64_t)ctx->sm_count * 1536 && est >= 2.0 * 6 * t) t *= 2;
+    return t;
 }
 
 // The launches of a run of nwin windows: stimulus SAIF, then per level the
@@ -865,7 +904,7 @@ static int reset_window(gls_ctx *ctx, Window *w)
 // whose per-gate-output tables serve levels of parity p.  With `prof` the
 // kernel classes are bracketed with events (not during stream capture).
 static int enqueue_levels(gls_ctx *ctx, const WinDev *const dw[2], const WinDev *const h[2], uint32_t nwin,
-                          uint32_t max_stim, bool prof, uint32_t *launches, bool w64 = false)
+                          uint32_t max_stim, bool prof, uint32_t *launches, bool w64, double est)
 {
     LevelArgs a;
     ctx_level_args(ctx, &a);
@@ -903,6 +942,32 @@ static int enqueue_levels(gls_ctx *ctx, const WinDev *const dw[2], const WinDev 
     ++*launches;
     if (prof) prof_mark(ctx);
     const size_t nlev = ctx->drv_level_start.size() - 1;
+    if (gate_path(ctx, a, prof)) {
+        for (size_t L = 0; L < nlev; ++L) {
+            a.lo = ctx->drv_level_start[L];
+            a.hi = ctx->drv_level_start[L + 1];
+            a.level = (uint32_t)L;
+            if (a.hi == a.lo) continue;
+            if (learned) {
+                PresizeArgs pa;
+                ctx_presize_args(ctx, &pa);
+                pa.wv = dw[0];
+                pa.nwin = nwin;
+                pa.lo = a.lo;
+                pa.n = a.hi - a.lo;
+                launch_presize(pa, true, ctx->stream);
+                ++*launches;
+            }
+            if (prof) prof_mark(ctx);
+            launch_gate(dw[0], *h[0], nwin, a, &ctx->cls_start[(kClasses + 1) * L],
+                        gate_block(ctx, (uint64_t)(a.hi - a.lo) * nwin, est), ctx->sm_count, ctx->stream, launches);
+            if (prof) prof_mark(ctx);
+            if (prof) prof_mark(ctx);
+        }
+        if (overlap_ok && !learned) CK(cudaStreamWaitEvent(ctx->stream, ctx->stim_join, 0), "stim join wait");
+        CK(cudaGetLastError(), "kernel launch");
+        return GLS_OK;
+    }
     if (nwin > 1) {
         // per level, the wave's fan-in events per class: segments are cut to
         // one size across the windows of the wave
@@ -1047,7 +1112,7 @@ static int enqueue_window(gls_ctx *ctx, Window *w, uint32_t *launches)
     CK(cudaMemcpyAsync(w->dwin.p, d, sizeof d, cudaMemcpyHostToDevice, ctx->stream), "upload window descriptor");
     const WinDev *dw[2] = {w->dwin.as<WinDev>(), w->dwin.as<WinDev>() + 1};
     const WinDev *hp[2] = {&d[0], &d[1]};
-    return enqueue_levels(ctx, dw, hp, 1, d[0].n_stim, true, launches, w->w64);
+    return enqueue_levels(ctx, dw, hp, 1, d[0].n_stim, true, launches, w->w64, gate_events_est(ctx, w));
 }
 
 // Totals of a run over its windows.
@@ -1271,6 +1336,7 @@ static int run_wave(gls_ctx *ctx, size_t w0, uint32_t nwin, const gls_batch_opts
 {
     WinDev *hw = ctx->hwave.as<WinDev>();
     uint32_t max_stim = 0;
+    double est = 0.0;
     for (uint32_t k = 0; k < nwin; ++k)
         CK(ctx->lsc[k]->ensure(ctx->max_width, ctx->seg_cap, ctx->scr_cap), "alloc level work spaces");
     for (uint32_t k = 0; k < nwin; ++k) {
@@ -1282,6 +1348,7 @@ static int run_wave(gls_ctx *ctx, size_t w0, uint32_t nwin, const gls_batch_opts
         hw[k] = make_windev(ctx, w, *ctx->lsc[k], 0);
         hw[kMaxWave + k] = make_windev(ctx, w, *ctx->lsc[k], 1);
         max_stim = std::max(max_stim, hw[k].n_stim);
+        est += gate_events_est(ctx, w) / nwin;
     }
     CK(cudaEventRecord(e0, ctx->stream), "event");
     for (int p = 0; p < 2; ++p)
@@ -1306,7 +1373,7 @@ static int run_wave(gls_ctx *ctx, size_t w0, uint32_t nwin, const gls_batch_opts
             cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
             int rc = GLS_OK;
             if (e == cudaSuccess) {
-                rc = enqueue_levels(ctx, dw, hp, nwin, max_stim, false, &l);
+                rc = enqueue_levels(ctx, dw, hp, nwin, max_stim, false, &l, false, est);
                 const cudaError_t e2 = cudaStreamEndCapture(ctx->stream, &g);
                 if (rc == GLS_OK && e2 != cudaSuccess) e = e2;
             }
@@ -1322,7 +1389,7 @@ static int run_wave(gls_ctx *ctx, size_t w0, uint32_t nwin, const gls_batch_opts
         acc.launches += l;
     } else {
         int rc = enqueue_levels(ctx, dw, hp, nwin, max_stim, false, &acc.launches,
-                                nwin == 1 && ctx->windows[w0]->w64);
+                                nwin == 1 && ctx->windows[w0]->w64, est);
         if (rc) return rc;
     }
     CK(cudaEventRecord(e1, ctx->stream), "event");

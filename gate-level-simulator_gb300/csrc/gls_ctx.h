@@ -201,6 +201,7 @@ struct Window {
     uint64_t cap = 0;
     DevBuf pool, net_off, net_len, init_off, init_len, saif, small, stim_dev;
     DevBuf dwin;                        // the window's WinDev on the device (sequential runs)
+    DevBuf lvl;                         // LevelCtr per level
     bool done = false;
     bool uploaded = false;              // device buffers hold this stimulus (uploaded when the window first runs)
     bool saif_only = false;             // pool released after a batched run: SAIF counts and lengths kept
@@ -235,6 +236,8 @@ struct gls_ctx {
     float bal_weight = 0.f;          // learned balance of segments in use (0: off)
     float bal_weight_on = 0.5f;      // its factor when GLS_SCHED_LEARNED_BALANCE is set (GLS_BALANCE_WEIGHT)
     bool pipeline = true;            // with concurrent classes: each class links and copies on its own stream
+    uint32_t gate_threads = 0;       // k_gate's block (GLS_GATE_THREADS; 0: by the level's width)
+    bool gate_kernel = true;         // levels run in one launch (GLS_GATE=0: the segment kernels)
     uint32_t copy_lanes = 8;         // lanes per segment of the copy kernel (GLS_COPY_LANES: 4, 8, 16, 32)
     int sm_count = 0;
     std::string err;

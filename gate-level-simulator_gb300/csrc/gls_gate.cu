@@ -1,0 +1,363 @@
+// k_gate: one level of gate outputs in one launch (32-bit event words).
+//
+// A block takes one gate output at a time: it cuts its fan-in timeline into
+// one time segment per thread, walks them, links the segments' stacks, places
+// the list in the event pool, copies it there and takes its SAIF integral.
+// Nothing but the finished list leaves the block, so a level needs no plan,
+// no segment tables and no launches in between.
+//
+// What bounds it: issue (60 %) and the integer pipe (67 %) on wide levels, the
+// chain of dependent loads of one gate output (its record, its lists' places,
+// the cut search, the walk) on narrow ones.  Against plan, three classes of
+// simulate, link and copy kernels with one thread per segment of a level-wide
+// segment list (device ms): 2,000 cells over 1,000 cycles .95 -> .34; 37,501
+// cells, 3,333 cycles 3.97 -> 1.80; 200,000 cells, 10,000 cycles 20.1 -> 14.9;
+// 2 M cells, 5,000 cycles 95.8 -> 84.  The segment search is made once per
+// segment instead of at both ends, the lanes of a warp walk the same gate
+// output, and link and copy find the stacks in L1 and L2.
+//
+// The stack contract of a segment and why the split is exact: see the head of
+// gls_kernels.cu.
+#include <cuda_runtime.h>
+#include <cstdint>
+#include "gls_device.cuh"
+
+namespace gls {
+
+namespace {
+
+constexpr int kMaxWarps = kGateMaxThreads / 32;
+
+struct GateSmem {
+    WinDev win;                  // wave of windows: the descriptor of the block's current window
+    uint32_t cw;                 // its number
+    uint32_t q;                  // the block's gate output, kInf: none left
+    uint32_t skip;               // its window has failed
+    unsigned long long ctr[4];   // gate events, output events, segments, fan-in events of the window at hand
+    uint32_t wmin[kMaxWarps];    // smallest candidate of every warp's segments
+    uint32_t wlast[kMaxWarps];   // value of the last kept entry of every warp's segments (4: none)
+    uint32_t wsum[kMaxWarps];    // kept entries
+    uint32_t s0[kMaxWarps], s1[kMaxWarps];
+    unsigned long long scr, dst; // the gate output's stacks in the scratch, its list in the pool
+    uint32_t ok;                 // the list has its place
+};
+
+// Per thread of the block, one time segment: shared arrays behind GateSmem.
+struct SegSmem {
+    uint32_t *tcut;   // time it starts at
+    uint32_t *src;    // its first kept entry, from the gate output's stacks on
+    uint32_t *n;      // entries kept
+    uint32_t *pos;    // their place in the list
+    uint32_t *pv;     // value before them
+};
+
+// fetch: thread 0 sets sm.q and sm.skip to the block's next gate output; called
+// where the wait for it overlaps others and every thread has read the present one.
+template <int M, class Fetch>
+__device__ __forceinline__ void run_gate(const WinDev &w, const LevelArgs &a, uint32_t i, GateSmem &sm,
+                                         const SegSmem &sg, Fetch fetch)
+{
+    const unsigned FULL = 0xffffffffu;
+    const uint32_t tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31u, wid = tid >> 5, nw = nthr >> 5;
+    const uint32_t drv = a.lo + i;
+    const DrvMeta *__restrict__ mdp = a.meta + drv;
+    const int m = mdp->m;
+    uint64_t off[M], poff = 0, soff = 0;
+    uint32_t len[M], plen = 0, slen = 0;
+    unsigned long long E = 0;
+    int piv = 0, sec = -1;   // the longest input list and the longest of the others
+#pragma unroll
+    for (int j = 0; j < M; ++j) {
+        len[j] = 0; off[j] = 0;
+        if (j < m) {
+            const uint32_t net = mdp->net[j];
+            off[j] = w.net_off[net];
+            len[j] = w.net_len[net];
+            E += len[j];
+            if (len[j] > plen) { sec = piv; slen = plen; plen = len[j]; piv = j; }
+            else if (sec < 0 || len[j] > slen) { sec = j; slen = len[j]; }
+        }
+    }
+    if (m < 2) sec = -1;
+#pragma unroll
+    for (int j = 0; j < M; ++j) {
+        if (j == piv) poff = off[j];
+        if (j == sec) soff = off[j];
+    }
+    // one segment per thread, none shorter than the smallest worth a search
+    unsigned long long seg = a.seg_events ? max(a.seg_events, 8u) : kGateMinSeg;
+    seg = max(seg, (E + nthr - 1) / nthr);
+    const uint32_t S = (uint32_t)max(1ull, (E + seg - 1) / seg);
+    if (tid == 0) {
+        const unsigned long long need = (E + S + 3) & ~3ull;
+        const unsigned long long at = atomicAdd(&w.lvl[a.level].scr, need);
+        sm.scr = at;
+        sm.ok = at + need <= w.scr_cap;
+        if (!sm.ok) atomicOr(w.err, kErrScratch);
+        sm.ctr[2] += S;
+        sm.ctr[3] += E;
+        if (mdp->flags & kFlagFirstOut)   // first output of its instance: count fan-in per pin
+            for (int p = 0; p < mdp->n_pins; ++p) sm.ctr[0] += w.net_len[mdp->net[(mdp->pin_slot >> (3 * p)) & 7u]];
+    }
+    // the segment's start; its end is the next thread's start
+    const bool mine = tid < S;
+    uint32_t cb[M], tcut = 0;
+#pragma unroll
+    for (int j = 0; j < M; ++j) cb[j] = 0;
+    if (mine && tid > 0)
+        tcut = cut_at<M>(w.pool, off, len, m, piv, sec, poff, soff, plen, slen, tid, S, cb);
+    if (mine) sg.tcut[tid] = tcut;
+    __syncthreads();
+    if (!sm.ok) {   // the same for the whole block
+        if (tid == 0) fetch();
+        return;
+    }
+    uint32_t *const scr = w.scratch + sm.scr;
+    uint32_t region = tid;
+    WalkOut o = {0, kInf, 0};
+    if (mine) {
+#pragma unroll
+        for (int j = 0; j < M; ++j) region += cb[j];
+        o = walk_segment<M>(w, a, drv, tid, off, len, cb, tid + 1 < S ? sg.tcut[tid + 1] : kInf, scr + region);
+    }
+    // later segments cut this one's stack at their smallest candidate
+    uint32_t x = o.minw;
+#pragma unroll
+    for (int k = 1; k < 32; k <<= 1) {
+        const uint32_t y = __shfl_down_sync(FULL, x, k);
+        if (lane + k < 32) x = min(x, y);
+    }
+    if (lane == 0) sm.wmin[wid] = x;
+    uint32_t later = __shfl_down_sync(FULL, x, 1);
+    if (lane == 31) later = kInf;
+    __syncthreads();
+    for (uint32_t k = wid + 1; k < nw; ++k) later = min(later, sm.wmin[k]);
+    const uint32_t *ot = scr + region;
+    uint32_t keep = o.cnt, firstv = 0, lastv = 0;
+    if (keep && later != kInf)
+        while (keep && ((keep == o.cnt ? o.top : ot[keep - 1]) | 3u) >= later) --keep;
+    if (keep) {
+        firstv = ev_val(ot[0]);
+        lastv = ev_val(keep == o.cnt ? o.top : ot[keep - 1]);
+    }
+    // an entry at a segment's bottom that repeats the last kept value before it goes
+    const unsigned bal = __ballot_sync(FULL, keep > 0);
+    const unsigned prior = bal & ((1u << lane) - 1u);
+    uint32_t vprev = __shfl_sync(FULL, lastv, prior ? 31 - __clz(prior) : 0);
+    const uint32_t vtop = __shfl_sync(FULL, lastv, bal ? 31 - __clz(bal) : 0);
+    if (lane == 0) sm.wlast[wid] = bal ? vtop : 4u;
+    __syncthreads();
+    if (!prior) {
+        vprev = kVX;
+        for (int k = (int)wid - 1; k >= 0; --k)
+            if (sm.wlast[k] < 4u) { vprev = sm.wlast[k]; break; }
+    }
+    const uint32_t drop = (tid > 0 && keep > 0 && firstv == vprev) ? 1u : 0u;
+    const uint32_t fin = keep - drop;
+    uint32_t inc = fin;
+#pragma unroll
+    for (int k = 1; k < 32; k <<= 1) {
+        const uint32_t y = __shfl_up_sync(FULL, inc, k);
+        if (lane >= k) inc += y;
+    }
+    if (lane == 31) sm.wsum[wid] = inc;
+    __syncthreads();
+    uint32_t pos = inc - fin, total = 0;
+    for (uint32_t k = 0; k < nw; ++k) {
+        if (k < wid) pos += sm.wsum[k];
+        total += sm.wsum[k];
+    }
+    if (mine) {
+        sg.src[tid] = region + drop;
+        sg.n[tid] = fin;
+        sg.pos[tid] = pos;
+        sg.pv[tid] = vprev;
+    }
+    if (tid == 0) {
+        // the list's place: reserved up front for its bound or its predicted
+        // length, or (exact placement, or a list longer than predicted) as long as it is
+        unsigned long long need = (total + 3ull) & ~3ull;
+        if (a.alloc_mode == kAllocBound) need = (E + 1 + 3) & ~3ull;
+        else if (a.alloc_mode == kAllocLearned) {
+            const unsigned long long res = min((E + 1 + 3) & ~3ull, ((unsigned long long)w.pred[i] + 3) & ~3ull);
+            if (total > res) {
+                atomicAdd(w.n_over, 1ull);
+                atomicAdd(w.top, res);   // the slot it outgrew
+            } else {
+                need = res;
+            }
+        }
+        fetch();
+        const unsigned long long st = atomicAdd(w.top, need);
+        sm.dst = st;
+        sm.ok = st + need <= w.cap;
+        if (!sm.ok) atomicOr(w.err, kErrPool);
+        else {
+            w.net_off[mdp->out_net] = st;
+            w.net_len[mdp->out_net] = total;
+        }
+        sm.ctr[1] += total;
+    }
+    __syncthreads();
+    if (!sm.ok) return;
+    // Copy, eight lanes a segment, with the SAIF integral: an entry at time t
+    // ends the hold of the value before it and starts its own, so class c's
+    // time is the sum of t over the entries after a value of class c minus
+    // the sum over those of class c, plus t_end for the last value's class.
+    // Times are window-relative and below 2^30: the sums wrap in 32 bits and
+    // are read back as signed.
+    constexpr uint32_t W = 8, U = 4;
+    const uint32_t sub = tid & (W - 1);
+    const RelClampT<uint32_t> rc(w.t_begin, w.t_end);
+    uint32_t s0 = 0, s1 = 0;
+    uint32_t *const dst = w.pool + sm.dst;
+    for (uint32_t b = wid * (32 / W); b < S; b += nthr / W) {   // a warp's four segments
+        const uint32_t k = b + (lane / W);
+        const uint32_t n = k < S ? sg.n[k] : 0u;
+        uint32_t nmax = n;
+        nmax = max(nmax, __shfl_xor_sync(FULL, nmax, 8));
+        nmax = max(nmax, __shfl_xor_sync(FULL, nmax, 16));
+        if (nmax == 0) continue;
+        const uint32_t *sp = scr + (k < S ? sg.src[k] : 0u);
+        uint32_t *dp = dst + (k < S ? sg.pos[k] : 0u);
+        uint32_t pv = k < S ? sg.pv[k] : 0u;
+        for (uint32_t e0 = 0; e0 < nmax; e0 += W * U) {
+            uint32_t wd[U];
+#pragma unroll
+            for (uint32_t u = 0; u < U; ++u) {
+                const uint32_t e = e0 + u * W + sub;
+                wd[u] = e < n ? sp[e] : 0u;
+            }
+#pragma unroll
+            for (uint32_t u = 0; u < U; ++u) {
+                const uint32_t e = e0 + u * W + sub;
+                uint32_t before = __shfl_up_sync(FULL, wd[u], 1, W);
+                if (sub == 0) before = pv;
+                pv = __shfl_sync(FULL, wd[u], W - 1, W);
+                if (e < n) {
+                    dp[e] = wd[u];
+                    const uint32_t t = rc(ev_time(wd[u])), c = ev_val(wd[u]), p = ev_val(before);
+                    s0 += (p == kV0 ? t : 0u) - (c == kV0 ? t : 0u);
+                    s1 += (p == kV1 ? t : 0u) - (c == kV1 ? t : 0u);
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 16; k > 0; k >>= 1) {
+        s0 += __shfl_xor_sync(FULL, s0, k);
+        s1 += __shfl_xor_sync(FULL, s1, k);
+    }
+    if (lane == 0) { sm.s0[wid] = s0; sm.s1[wid] = s1; }
+    __syncthreads();
+    if (tid == 0) {
+        uint32_t last = kVX;
+        s0 = s1 = 0;
+        for (uint32_t k = 0; k < nw; ++k) {
+            s0 += sm.s0[k];
+            s1 += sm.s1[k];
+            if (sm.wlast[k] < 4u) last = sm.wlast[k];
+        }
+        const unsigned long long D = w.t_end - w.t_begin;
+        const unsigned long long t0 = (unsigned long long)(long long)(int)s0 + (last == kV0 ? D : 0ull);
+        const unsigned long long t1 = (unsigned long long)(long long)(int)s1 + (last == kV1 ? D : 0ull);
+        unsigned long long *sf = w.saif + 3ull * mdp->out_net;
+        sf[0] = t0;
+        sf[1] = t1;
+        sf[2] = D - t0 - t1;
+    }
+}
+
+}  // namespace
+
+// Gate outputs [d0, d1) of the level of every window of the launch (kSix: the
+// class of four to six input nets, else the narrower ones; c1, c2: where the
+// 2- and 3-input ones start).  Blocks take gate outputs from the back, the
+// widest first, as they become free.
+template <bool kBatch, bool kSix>
+__global__ void __launch_bounds__(kGateMaxThreads, kSix ? 1 : 1024 / kGateMaxThreads)
+    k_gate(const WinSet<kBatch> ws, LevelArgs a, uint32_t d0, uint32_t d1, uint32_t c1, uint32_t c2)
+{
+    __shared__ GateSmem sm;
+    extern __shared__ uint32_t s_seg[];
+    const uint32_t nthr = blockDim.x;
+    const SegSmem sg = {s_seg, s_seg + nthr, s_seg + 2 * nthr, s_seg + 3 * nthr, s_seg + 4 * nthr};
+    const uint32_t n = d1 - d0, total = n * ws.size();
+    auto fetch = [&](uint32_t q) {   // thread 0
+        sm.q = q < total ? q : kInf;
+        if (q < total) sm.skip = *(volatile uint32_t *)ws.get(kBatch ? q / n : 0u).err != 0;
+    };
+    auto flush = [&]() {
+        const WinDev &w = ws.get(kBatch ? sm.cw : 0u);
+        for (int k = 0; k < 4; ++k) {
+            if (sm.ctr[k]) atomicAdd(&w.counters[k], sm.ctr[k]);
+            sm.ctr[k] = 0;
+        }
+    };
+    if (threadIdx.x == 0) {
+        sm.cw = kInf;
+        for (int k = 0; k < 4; ++k) sm.ctr[k] = 0;
+        fetch(blockIdx.x);   // the grid has at most one block per gate output
+    }
+    for (;;) {
+        __syncthreads();
+        const uint32_t q = sm.q;
+        if (q == kInf) break;
+        const bool skip = sm.skip != 0;
+        const uint32_t win = kBatch ? q / n : 0u;
+        if constexpr (kBatch) {
+            // the window's descriptor in shared memory, out of the way of the walks
+            const uint32_t cw = sm.cw;
+            __syncthreads();
+            if (win != cw) {
+                if (threadIdx.x == 0) {
+                    if (cw != kInf) flush();
+                    sm.cw = win;
+                }
+                const uint32_t *src = reinterpret_cast<const uint32_t *>(&ws.get(win));
+                uint32_t *d = reinterpret_cast<uint32_t *>(&sm.win);
+                for (uint32_t k = threadIdx.x; k < sizeof(WinDev) / 4; k += blockDim.x) d[k] = src[k];
+                __syncthreads();
+            }
+        }
+        auto next = [&]() { fetch(gridDim.x + atomicAdd(&ws.get(0).lvl[a.level].next[kSix ? 0 : 1], 1u)); };
+        if (skip) {
+            __syncthreads();   // sm.q is read
+            if (threadIdx.x == 0) next();
+            continue;
+        }
+        const uint32_t i = d1 - 1 - (kBatch ? q - win * n : q);
+        auto go = [&](const WinDev &w) {
+            if constexpr (kSix) {
+                run_gate<kMaxSlots>(w, a, i, sm, sg, next);
+            } else {
+                if (i >= c2) run_gate<3>(w, a, i, sm, sg, next);
+                else if (i >= c1) run_gate<2>(w, a, i, sm, sg, next);
+                else run_gate<1>(w, a, i, sm, sg, next);
+            }
+        };
+        if constexpr (kBatch) go(sm.win);
+        else go(ws.get(0));
+    }
+    if (threadIdx.x == 0 && (!kBatch || sm.cw != kInf)) flush();
+}
+
+void launch_gate(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelArgs &a, const uint32_t *cls,
+                 uint32_t threads, int sm_count, cudaStream_t st, uint32_t *launches)
+{
+    const uint32_t smem = threads * 5 * 4;
+    auto go = [&](auto six, uint32_t d0, uint32_t d1) {
+        constexpr bool kSix = decltype(six)::value;
+        if (d1 <= d0) return;
+        const uint64_t total = (uint64_t)(d1 - d0) * nwin;
+        const uint64_t room = (uint64_t)sm_count * ((kSix ? 512 : 1024) / threads);
+        const uint32_t grid = (uint32_t)(total < room ? total : room);
+        if (nwin == 1) k_gate<false, kSix><<<grid, threads, smem, st>>>(WinSet<false>{h}, a, d0, d1, cls[1], cls[2]);
+        else k_gate<true, kSix><<<grid, threads, smem, st>>>(WinSet<true>{dw, nwin}, a, d0, d1, cls[1], cls[2]);
+        ++*launches;
+    };
+    go(std::integral_constant<bool, true>(), cls[3], cls[4]);
+    go(std::integral_constant<bool, false>(), 0u, cls[3]);
+}
+
+}  // namespace gls

@@ -159,6 +159,11 @@ struct CopyRec {            // what k_copy does for one segment
     uint32_t out_net;       // the gate output's net
 };
 
+struct LevelCtr {           // k_gate: per window and level, cleared before the run
+    uint32_t next[2];           // gate outputs taken (4- to 6-input class, the others; window 0's counts)
+    unsigned long long scr;     // stack words handed out
+};
+
 struct WinDev {
     uint64_t *net_off;
     uint32_t *net_len;
@@ -178,6 +183,7 @@ struct WinDev {
     uint32_t *pred;             // per driver of the level: predicted slot length (learned mode)
     const uint32_t *stim_nets;  // nets the stimulus drives
     uint32_t *scratch;          // level scratch: segment stacks (event words)
+    LevelCtr *lvl;              // k_gate: counters of every level
     uint64_t cap;               // pool capacity (events)
     uint64_t scr_cap;           // scratch capacity (events)
     uint64_t t_begin, t_end;
@@ -206,6 +212,7 @@ struct LevelArgs {
     uint32_t wide;              // 1: the window holds 64-bit event words (one window per launch)
     uint32_t sim_variant;       // thread-per-segment gate kernel variant: bit 0 256-thread blocks, bit 1 wider loads
     float bal_weight;           // learned mode: segment work = fan-in events + bal_weight * predicted output events
+    uint32_t level;             // the level's number
     uint32_t plan_part;         // k_plan: 0 all of it; learned mode split in two: 1 segments and stacks
                                 // (slots left open), 2 slot placement from the predictions
 };
@@ -232,5 +239,13 @@ void launch_link(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelAr
                  cudaStream_t st);
 void launch_copy(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelArgs &a, uint32_t d0, uint32_t d1,
                  int sm_count, cudaStream_t st);
+
+// One level in one launch (32-bit words; a second one where gate outputs with
+// four to six input nets exist).  cls: the level's fan-in class starts
+// (kClasses + 1); threads per block: 32 .. kGateMaxThreads, a power of two.
+constexpr uint32_t kGateMaxThreads = 512;
+constexpr uint32_t kGateMinSeg = 16;   // fan-in events a time segment is worth a search
+void launch_gate(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelArgs &a, const uint32_t *cls,
+                 uint32_t threads, int sm_count, cudaStream_t st, uint32_t *launches);
 
 }  // namespace gls

@@ -1,0 +1,87 @@
+"""k_gate (one level in one launch, a block per gate output) at its edges,
+bit-exact against the oracle: every block size, list lengths around the
+smallest segment and around one segment per thread, gates of one to six
+input nets, stack and pool space that has to grow, waves of windows."""
+import numpy as np
+import pytest
+
+from cases import random_case, stimulus
+from gls import synth
+from gls.cells import LIBRARY
+from gls.levelize import assemble, default_arcs
+from gls.capi import ALLOC_EXACT
+from gpu_util import assert_same, gpu_run, simulator
+from oracle.runner import run_oracle
+
+pytestmark = pytest.mark.gpu
+CELLS = ["GEN_BUF_D1", "GEN_XOR2_D1", "GEN_AND2_D1", "GEN_MUX2_D1", "GEN_OAI21_D1"]
+
+
+def fan_design():
+    insts, nn = [], 3
+    for k, name in enumerate(CELLS * 2):
+        c = LIBRARY[name]
+        src = [0, 1, 2] if k < len(CELLS) else [3 + (k + p) % len(CELLS) for p in range(3)]
+        insts.append((name, src[:c.n_in], [nn], default_arcs(c, 3.0 + k, 7.0 + k)))
+        nn += 1
+    return assemble(insts, n_nets=nn)
+
+
+def even_lists(events):
+    return stimulus({net: [(0, 1)] + [(20 * e + 7 * net + 5, 3 if e % 2 else 0) for e in range(events)]
+                     for net in range(3)})
+
+
+@pytest.mark.parametrize("events", [0, 1, 7, 15, 16, 17, 255, 1023, 5000])
+@pytest.mark.parametrize("threads", [32, 64, 128, 256, 512])
+def test_block_sizes(threads, events, gpu, oracle_bin):
+    nl, st = fan_design(), even_lists(events)
+    t_end = 20 * events + 500
+    ow, osaif, _ = run_oracle(nl, st, 0, t_end)
+    gw, gs, _, _ = gpu_run(nl, st, 0, t_end, env={"GLS_GATE_THREADS": str(threads)})
+    assert_same(gw, gs, ow, osaif, f"{threads} threads, {events} events")
+
+
+@pytest.mark.parametrize("threads", [32, 512])
+@pytest.mark.parametrize("alloc", [0, 1])
+def test_against_the_segment_kernels(alloc, threads, gpu):
+    """A netlist with lists long enough for full blocks, in both paths; a pool
+    that has to grow on the way."""
+    cfg = synth.scaled(synth.CONFIGS["c1"], cells=900, cycles=2500, depth=12)
+    nl = synth.make_netlist(cfg, seed=5)
+    st = synth.make_stimulus(cfg, nl.ppi_nets, seed=6)
+    res = []
+    for env in ({"GLS_GATE": "0"}, {"GLS_GATE_THREADS": str(threads)}):
+        with simulator(env=env, alloc_mode=alloc, pool_events=200_000) as s:
+            s.load(nl)
+            w = s.add_window(st, 300, cfg.t_end - 700)
+            s.run()
+            assert s.stats()["overflow_retries"] > 0
+            res.append((s.saif(w), s.lengths(w), [s.waveform(int(n), w) for n in range(0, nl.n_nets, 37)]))
+    assert np.array_equal(res[0][0], res[1][0]) and np.array_equal(res[0][1], res[1][1])
+    for (t0, v0), (t1, v1) in zip(res[0][2], res[1][2]):
+        assert np.array_equal(t0, t1) and np.array_equal(v0, v1)
+
+
+@pytest.mark.parametrize("threads", [32, 256])
+def test_wave_with_uneven_windows(threads, gpu, oracle_bin):
+    """Windows of one wave from one event a list to thousands, gates of
+    up to six input nets."""
+    nl, _ = random_case(3, max_gates=16, max_in=6)
+    rng = np.random.default_rng(9)
+    wins = []
+    for events in (1, 3, 40, 900, 4000, 2):
+        d = {}
+        for net in nl.ppi_nets:
+            t = np.cumsum(rng.integers(1, 12, events)) if events else np.zeros(0, int)
+            d[int(net)] = list(zip(t.tolist(), rng.choice([0, 3, 1], events, p=[.49, .49, .02]).tolist()))
+        wins.append(stimulus(d))
+    with simulator(env={"GLS_GATE_THREADS": str(threads)}, alloc_mode=ALLOC_EXACT) as s:
+        s.load(nl)
+        ids = [s.add_window(st, 10, 60_000) for st in wins]
+        s.run_batched()
+        for wid, st in zip(ids, wins):
+            ow, osaif, _ = run_oracle(nl, st, 10, 60_000)
+            lens = s.lengths(wid)
+            gw = {n: s.waveform(n, wid) for n in range(nl.n_nets) if lens[n] != 2**32 - 1}
+            assert_same(gw, s.saif(wid), ow, osaif, f"wave window {wid}")
