@@ -71,6 +71,7 @@ void ctx_level_args(const gls_ctx *ctx, LevelArgs *a)
     a->wide = 0;
     a->plan_part = 0;
     a->level = 0;
+    a->n_nets = ctx->n_nets;
 }
 
 namespace {
@@ -624,9 +625,9 @@ static int upload_window(gls_ctx *ctx, Window *w, bool sync = true)
     if (w->pool.p && w->pool.bytes < w->cap * wb) w->pool.release();
     CK(take_buf(ctx, w->pool, w->cap * wb), "alloc event pool");
     CK(take_buf(ctx, w->net_off, n * 8), "alloc net_off");
-    CK(w->net_len.ensure(n * 4), "alloc net_len");
+    CK(w->net_len.ensure(n * 8), "alloc net_len");   // lengths, then the X times
     CK(take_buf(ctx, w->init_off, n * 8), "alloc init_off");
-    CK(take_buf(ctx, w->init_len, n * 4), "alloc init_len");
+    CK(take_buf(ctx, w->init_len, n * 8), "alloc init_len");
     CK(w->saif.ensure(n * 24), "alloc saif");
     CK(w->small.ensure(256), "alloc counters");
     CK(w->lvl.ensure((ctx->drv_level_start.size()) * sizeof(LevelCtr)), "alloc level counters");
@@ -634,17 +635,18 @@ static int upload_window(gls_ctx *ctx, Window *w, bool sync = true)
     if (w->stim_events)
         CK(cudaMemcpyAsync(w->pool.p, w->h_words.p, w->stim_events * wb, cudaMemcpyHostToDevice, ctx->stream),
            "upload stimulus");
-    if (!w->h_off.ensure(n * 8) || !w->h_len.ensure(n * 4)) return fail(ctx, GLS_ENOMEM, "pinned staging");
+    if (!w->h_off.ensure(n * 8) || !w->h_len.ensure(n * 8)) return fail(ctx, GLS_ENOMEM, "pinned staging");
     uint64_t *off = w->h_off.as<uint64_t>();
     uint32_t *len = w->h_len.as<uint32_t>();
     std::memset(off, 0, n * 8);
     std::memset(len, 0xFF, n * 4);
+    std::memset(len + n, 0, n * 4);   // k_stim_saif and the gate kernels fill it
     for (size_t k = 0; k < w->stim_nets.size(); ++k) {
         off[w->stim_nets[k]] = w->stim_off[k];
         len[w->stim_nets[k]] = w->stim_len[k];
     }
     CK(cudaMemcpyAsync(w->init_off.p, off, n * 8, cudaMemcpyHostToDevice, ctx->stream), "upload offsets");
-    CK(cudaMemcpyAsync(w->init_len.p, len, n * 4, cudaMemcpyHostToDevice, ctx->stream), "upload lengths");
+    CK(cudaMemcpyAsync(w->init_len.p, len, n * 8, cudaMemcpyHostToDevice, ctx->stream), "upload lengths");
     if (!w->stim_nets.empty())
         CK(cudaMemcpyAsync(w->stim_dev.p, w->stim_nets.data(), w->stim_nets.size() * 4, cudaMemcpyHostToDevice,
                            ctx->stream),
@@ -864,7 +866,7 @@ static int reset_window(gls_ctx *ctx, Window *w)
 {
     const uint64_t n = ctx->n_nets;
     CK(cudaMemcpyAsync(w->net_off.p, w->init_off.p, n * 8, cudaMemcpyDeviceToDevice, ctx->stream), "reset offsets");
-    CK(cudaMemcpyAsync(w->net_len.p, w->init_len.p, n * 4, cudaMemcpyDeviceToDevice, ctx->stream), "reset lengths");
+    CK(cudaMemcpyAsync(w->net_len.p, w->init_len.p, n * 8, cudaMemcpyDeviceToDevice, ctx->stream), "reset lengths");
     CK(cudaMemsetAsync(w->saif.p, 0xFF, n * 24, ctx->stream), "reset saif");
     CK(cudaMemsetAsync(w->lvl.p, 0, ctx->drv_level_start.size() * sizeof(LevelCtr), ctx->stream), "reset level counters");
     unsigned long long small[8] = {w->stim_events + ctx->pool_gap, 0, 0, 0, 0, 0, 0, 0};
@@ -874,7 +876,7 @@ static int reset_window(gls_ctx *ctx, Window *w)
 
 // Whether a run's levels go through k_gate: 32-bit words and the default
 // thread-per-segment schedule.
-static bool gate_path(const gls_ctx *ctx, const LevelArgs &a, bool)
+static bool gate_path(const gls_ctx *ctx, const LevelArgs &a)
 {
     return ctx->gate_kernel && !a.wide && a.warp_mask == 0 && a.sim_variant == 0 && a.bal_weight <= 0.f;
 }
@@ -891,8 +893,11 @@ static bool gate_path(const gls_ctx *ctx, const LevelArgs &a, bool)
 // whole level, six.
 static uint32_t gate_block(const gls_ctx *ctx, uint64_t outs, double est)
 {
-    if (ctx->gate_threads) return std::min(kGateMaxThreads, std::max(32u, ctx->gate_threads & ~31u));
     uint32_t t = 32;
+    if (ctx->gate_threads) {
+        while (t < kGateMaxThreads && t < ctx->gate_threads) t *= 2;
+        return t;
+    }
     while (t < 256 && est >= 2.0 * 24 * t) t *= 2;
     while (t < 256 && outs * t * 2 <= (uint64_t)ctx->sm_count * 1536 && est >= 2.0 * 6 * t) t *= 2;
     return t;
@@ -926,6 +931,7 @@ static int enqueue_levels(gls_ctx *ctx, const WinDev *const dw[2], const WinDev 
     // from the predictions: it keeps the plan whole, after the copies.)
     const bool learned = a.alloc_mode == kAllocLearned;
     const bool split = learned && ctx->bal_weight <= 0.f;
+    const bool gates = gate_path(ctx, a);
     const bool overlap_ok = ctx->concurrent && ctx->pipeline && ctx->plan_overlap && !(prof && ctx->opts.profile) &&
                             (!learned || split);
     if (prof) prof_mark(ctx);
@@ -934,15 +940,16 @@ static int enqueue_levels(gls_ctx *ctx, const WinDev *const dw[2], const WinDev 
         // writes their counts; learned mode's presize reads them)
         CK(cudaEventRecord(ctx->stim_fork, ctx->stream), "stim fork");
         CK(cudaStreamWaitEvent(ctx->stim_side, ctx->stim_fork, 0), "stim fork wait");
-        launch_stim_saif(dw[0], *h[0], nwin, max_stim, w64, ctx->stim_side);
+        launch_stim_saif(dw[0], *h[0], nwin, max_stim, w64, ctx->n_nets, ctx->stim_side);
         CK(cudaEventRecord(ctx->stim_join, ctx->stim_side), "stim join");
     } else {
-        launch_stim_saif(dw[0], *h[0], nwin, max_stim, w64, ctx->stream);
+        launch_stim_saif(dw[0], *h[0], nwin, max_stim, w64, ctx->n_nets, ctx->stream);
     }
     ++*launches;
     if (prof) prof_mark(ctx);
     const size_t nlev = ctx->drv_level_start.size() - 1;
-    if (gate_path(ctx, a, prof)) {
+    if (gates) {
+        bool stim_beside = overlap_ok && !learned;
         for (size_t L = 0; L < nlev; ++L) {
             a.lo = ctx->drv_level_start[L];
             a.hi = ctx->drv_level_start[L + 1];
@@ -960,11 +967,16 @@ static int enqueue_levels(gls_ctx *ctx, const WinDev *const dw[2], const WinDev 
             }
             if (prof) prof_mark(ctx);
             launch_gate(dw[0], *h[0], nwin, a, &ctx->cls_start[(kClasses + 1) * L],
-                        gate_block(ctx, (uint64_t)(a.hi - a.lo) * nwin, est), ctx->sm_count, ctx->stream, launches);
+                        gate_block(ctx, (uint64_t)(a.hi - a.lo) * nwin, est), !stim_beside, ctx->sm_count, ctx->stream,
+                        launches);
+            if (stim_beside) {   // the first level ran without the stimulus nets' X times
+                CK(cudaStreamWaitEvent(ctx->stream, ctx->stim_join, 0), "stim join wait");
+                stim_beside = false;
+            }
             if (prof) prof_mark(ctx);
             if (prof) prof_mark(ctx);
         }
-        if (overlap_ok && !learned) CK(cudaStreamWaitEvent(ctx->stream, ctx->stim_join, 0), "stim join wait");
+        if (stim_beside) CK(cudaStreamWaitEvent(ctx->stream, ctx->stim_join, 0), "stim join wait");
         CK(cudaGetLastError(), "kernel launch");
         return GLS_OK;
     }

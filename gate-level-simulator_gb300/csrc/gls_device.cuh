@@ -127,9 +127,10 @@ template <> struct WinSet<true> {
 // guess: gallop away from the guess, then bisect.  Event lists of one gate
 // share the clock, so a position scaled from another list is usually a few
 // events off.  Compares whole words: time >= key <=> word >= key << 2.
-template <class Wd>
-__device__ __forceinline__ uint32_t search_from(const Wd *__restrict__ x, uint32_t n, uint32_t key, uint32_t g)
+template <class P>
+__device__ __forceinline__ uint32_t search_from(P x, uint32_t n, uint32_t key, uint32_t g)
 {
+    using Wd = typename std::remove_cv<typename std::remove_reference<decltype(x[0])>::type>::type;
     if (n == 0) return 0;
     const Wd kw = (Wd)key << 2;
     if (g >= n) g = n - 1;
@@ -188,9 +189,9 @@ __device__ __forceinline__ uint32_t slut_get(const uint4 &t, uint32_t curp)
 // first events of X / Y at or after that time.  Equal times may sit in both
 // lists (not within one), so a cut at the returned time keeps every time's
 // events on one side.
-template <class Wd>
-__device__ __forceinline__ uint32_t rank_time2(const Wd *__restrict__ X, uint32_t nx, const Wd *__restrict__ Y,
-                                               uint32_t ny, uint32_t r, uint32_t g, uint32_t &ix, uint32_t &iy)
+template <class P>
+__device__ __forceinline__ uint32_t rank_time2(P X, uint32_t nx, P Y, uint32_t ny, uint32_t r, uint32_t g,
+                                               uint32_t &ix, uint32_t &iy)
 {
     // short(i): the first r merged events hold more than i events of X
     // (true for small i, false from the answer on)
@@ -330,12 +331,55 @@ struct ListReader {
     }
 };
 
+// A change list, or a stretch of one, in shared memory (its shared address).
+struct SmemList {
+    uint32_t at;
+    __device__ __forceinline__ uint32_t operator[](uint32_t i) const
+    {
+        uint32_t v;
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(at + 4 * i));
+        return v;
+    }
+    __device__ __forceinline__ void set(uint32_t i, uint32_t v) const
+    {
+        asm volatile("st.shared.u32 [%0], %1;" ::"r"(at + 4 * i), "r"(v) : "memory");
+    }
+};
+
+// Reader of a stretch in shared memory: two kInf words follow its last event.
+struct SmemReader {
+    uint32_t h, n;
+    uint32_t p;   // shared address of the head
+
+    __device__ __forceinline__ void start(SmemList x, uint32_t b)
+    {
+        p = x.at + 4 * b;
+        h = SmemList{p}[0];
+        n = SmemList{p}[1];
+    }
+    __device__ __forceinline__ void advance(bool go)
+    {
+        h = go ? n : h;
+        p += go ? 4u : 0u;
+        n = SmemList{p}[1];
+    }
+};
+
+// Where a segment's stack lies.
+struct GlobalStack {
+    uint32_t *x;
+    __device__ __forceinline__ uint32_t operator[](uint32_t i) const { return x[i]; }
+    __device__ __forceinline__ void set(uint32_t i, uint32_t v) const { x[i] = v; }
+};
+
 // The walk of one time segment of a gate output, 32-bit words: from the
-// segment's first event of every list (cb) to its end time, onto the stack at
-// ot.  Steps whose input values are all 0 or 1 before and after (nearly
-// all of them: X and Z leave a net with its first real event) take the fast
-// step; any other step, and every step of a gate output whose FastRec is
-// not usable, takes the general one.
+// segment's first event of every list (in rd, with the values before them in
+// curp; before: some list has one) to its end time tnext (kInf: the lists' end),
+// onto the stack ot.  tmax: no event of the segment is later.  Steps whose
+// input values are all 0 or 1 before and after (nearly all of them: X and Z
+// leave a net with its first real event) take the fast step; any other step,
+// and every step of a gate output whose FastRec is not usable, takes the
+// general one.
 //
 // What bounds it: instruction issue.  A lane walks its own segment, so a
 // warp issues both the step and, on nearly every iteration, the output
@@ -352,30 +396,51 @@ struct ListReader {
 // M warp instructions at 14 -> 25 active lanes, the 2-input one 320 -> 277 us
 // and 205 -> 119 M; the 2 M cell design over 5,000 cycles 97.2 -> 79.6 ms of
 // gate kernels.
+//
+// kTab: `tab` is the shared address of the gate output's step table (see
+// step_entry; aligned to its size).  clean: from the segment's start on, all
+// input values are known and the lists hold nothing but alternating 0 and 1;
+// then a step is one table read by the input state and the set of lists that
+// move, a third fewer instructions than the fast step, which reads values,
+// edges and delays for every list.
 struct WalkOut {
     uint32_t cnt;    // entries on the stack
-    uint32_t minw;   // smallest candidate time << 2 (kInf: no candidate)
+    uint32_t minw;   // word of the smallest candidate time (kInf: no candidate)
     uint32_t top;    // the stack's top entry (cnt > 0)
+    uint32_t xt;     // latest time an X or Z was pushed at (0: none but the first entry)
 };
+
+// Step table of a gate output with a usable FastRec: entry state << M | moves
+// (a bit per input net) holds delay << 2 | value of the output change, kInf
+// where the output stays.
 template <int M>
-__device__ __forceinline__ WalkOut walk_segment(const WinDev &w, const LevelArgs &a, uint32_t drv, uint32_t s,
-                                                const uint64_t (&off)[M], const uint32_t (&len)[M],
-                                                const uint32_t (&cb)[M], uint32_t tnext, uint32_t *ot)
+__device__ __forceinline__ uint32_t step_entry(const uint4 &f0, const uint4 &f1, uint32_t e)
 {
-    constexpr bool kFast = M <= 3;
-    const uint32_t *__restrict__ pw = w.pool;
-    const DrvMeta *__restrict__ mdp = a.meta + drv;
-    uint32_t tmax, tend;   // latest event time of the segment; words at or above tend lie behind it
-    if (tnext != kInf) {
-        tmax = tnext;
-        tend = tnext << 2;
-    } else {
-        tmax = 0;
+    const uint32_t dp[3] = {f0.x, f0.z, f1.x}, dn[3] = {f0.y, f0.w, f1.y};
+    const uint32_t mv = e & ((1u << M) - 1u), from = e >> M, to = from ^ mv;
+    auto out = [&](uint32_t x) { return (f1.z >> ((x & 1u) | (x & 2u) << 1 | (x & 4u) << 2)) & 1u; };
+    const uint32_t F = out(to);
+    if (mv == 0 || F == out(from)) return kInf;
+    uint32_t d = kInf;
 #pragma unroll
-        for (int j = 0; j < M; ++j)
-            if (len[j]) tmax = max(tmax, ev_time(pw[off[j] + len[j] - 1]));
-        tend = kInf;
-    }
+    for (int j = 0; j < M; ++j)
+        if ((mv >> j) & 1u) {
+            const uint32_t r = ((to >> j) & 1u) ? dp[j] : dn[j];
+            d = min(d, F ? r & 0xFFFFu : r >> 16);
+        }
+    return d << 2 | (F ? kV1 : kV0);
+}
+
+template <int M, bool kTab, class RD, class ST>
+__device__ __forceinline__ WalkOut walk_segment(const WinDev &w, const LevelArgs &a, uint32_t drv, uint32_t s,
+                                                RD (&rd)[M], uint32_t curp, bool before, uint32_t tnext,
+                                                uint32_t tmax, ST ot, uint32_t tab = 0, bool clean = false)
+{
+    static_assert(!kTab || M <= 3, "step tables are for up to three input nets");
+    constexpr bool kFast = M <= 3;
+    const DrvMeta *__restrict__ mdp = a.meta + drv;
+    // words at or above tend lie behind the segment
+    const uint32_t tend = tnext != kInf ? tnext << 2 : kInf;
     uint4 f0 = {0, 0, 0, 0}, f1 = {0, 0, 0, 0};
     if (kFast) {
         f0 = __ldg(a.fast + 2ull * drv);
@@ -383,24 +448,11 @@ __device__ __forceinline__ WalkOut walk_segment(const WinDev &w, const LevelArgs
     }
     const uint32_t dp[3] = {f0.x, f0.z, f1.x}, dn[3] = {f0.y, f0.w, f1.y};
     const uint32_t tt = f1.z;
-    // input values, 2 bits per net; 0x15 bits of `mixed` mark nets at X or Z
-    uint32_t curp = 0x555u & ((1u << (2 * M)) - 1u);
-    bool before = false;
-    ListReader rd[M];
-#pragma unroll
-    for (int j = 0; j < M; ++j) {
-        const uint32_t b = cb[j];
-        const uint32_t *x = pw + off[j];
-        if (b > 0) {
-            curp = (curp & ~(3u << (2 * j))) | (ev_val(x[b - 1]) << (2 * j));
-            before = true;
-        }
-        rd[j].start(x, b, len[j]);
-    }
     constexpr uint32_t kBits = 0x555u & ((1u << (2 * M)) - 1u);
     // a gate output without a usable FastRec, or times too close to the
     // largest one, take the general step throughout
     const uint32_t never = (kFast && f1.w != 0u && tmax <= kMaxTime - 0x10000u) ? 0u : kBits;
+    // input values are 2 bits per net; 0x15 bits of `mixed` mark nets at X or Z
     uint32_t mixed = ((curp ^ (curp >> 1)) & kBits) | never;
     // Every step consumes an event and pushes at most one entry, so a
     // segment's stack ends within the gate output's scratch.
@@ -409,19 +461,19 @@ __device__ __forceinline__ WalkOut walk_segment(const WinDev &w, const LevelArgs
     // entry left the top reads as (0, X): below every later candidate, and
     // different from 0 and 1.
     uint32_t top = EvW<uint32_t>::word(0, kVX), below = kInf;
-    if (s == 0) { ot[0] = top; cnt = 1; }
+    if (s == 0) { ot.set(0, top); cnt = 1; }
     uint32_t fprev = kVX;
     auto out_of = [&](uint32_t x) -> uint32_t {   // the general step's truth table
         if constexpr (kFast) return slut_get<M>(__ldg(a.slut + drv), x);
         else return __ldg(a.lut + mdp->lut_off + lut_index(x, *mdp));
     };
     if (before) fprev = out_of(curp);
-    uint32_t minw = kInf;   // smallest candidate time << 2
+    uint32_t minw = kInf, xt = 0;
     for (;;) {
         uint32_t mk = rd[0].h | 3u;
 #pragma unroll
         for (int j = 1; j < M; ++j) mk = min(mk, rd[j].h | 3u);
-        if (mk >= tend) break;
+        if (mk >= tend || (kTab && clean)) break;
         const uint32_t lastp = curp;
         bool ch[M];
 #pragma unroll
@@ -457,7 +509,7 @@ __device__ __forceinline__ WalkOut walk_segment(const WinDev &w, const LevelArgs
                 } while (top >= lo);
             }
             const bool push = chg && ((top ^ F) & 3u) != 0u;
-            if (push) ot[cnt] = lo | F;
+            if (push) ot.set(cnt, lo | F);
             below = push ? top : below;
             top = push ? lo | F : top;
             cnt += push ? 1u : 0u;
@@ -490,13 +542,52 @@ __device__ __forceinline__ WalkOut walk_segment(const WinDev &w, const LevelArgs
         if (prevv != (int)F) {
             below = kInf;
             top = lo | F;
-            ot[cnt++] = top;
+            ot.set(cnt++, top);
+            if (F == kVX || F == kVZ) xt = lo >> 2;
         } else if (cnt == 0) {
             atomicOr(w.err, kErrEmptied);
             break;
         }
     }
-    return {cnt, minw, top};
+    if constexpr (kTab) {
+        if (!clean) return {cnt, minw, top, xt};
+        uint32_t so = tab;   // the table row of the input state
+#pragma unroll
+        for (int j = 0; j < M; ++j) so += ((curp >> (2 * j)) & 1u) << (2 + M + j);
+        for (;;) {
+            uint32_t mk = rd[0].h | 3u;
+#pragma unroll
+            for (int j = 1; j < M; ++j) mk = min(mk, rd[j].h | 3u);
+            if (mk >= tend) break;
+            uint32_t x = so;
+#pragma unroll
+            for (int j = 0; j < M; ++j) {
+                const bool ch = (rd[j].h | 3u) == mk;
+                x |= ch ? 4u << j : 0u;
+                rd[j].advance(ch);
+            }
+            uint32_t st;
+            asm volatile("ld.shared.u32 %0, [%1];" : "=r"(st) : "r"(x));
+            so ^= (x ^ so) << M;
+            const bool chg = st != kInf;
+            const uint32_t nw = mk - 3u + st;   // the candidate's event word
+            minw = chg ? min(minw, nw) : minw;
+            if (chg && (top | 3u) >= nw) {   // times only: the bottom lies below every candidate
+                do {
+                    --cnt;
+                    if (below != kInf) top = below;
+                    else top = cnt > 0 ? ot[cnt - 1] : EvW<uint32_t>::word(0, kVX);
+                    below = kInf;
+                } while ((top | 3u) >= nw);
+            }
+            const bool put = chg && ((top ^ nw) & 3u) != 0u;
+            if (put) ot.set(cnt, nw);
+            below = put ? top : below;
+            top = put ? nw : top;
+            cnt += put ? 1u : 0u;
+        }
+    }
+    return {cnt, minw, top, xt};
 }
 
 }  // namespace gls

@@ -28,7 +28,8 @@ namespace {
 
 constexpr int kMaxWarps = kGateMaxThreads / 32;
 
-struct GateSmem {
+struct __align__(256) GateSmem {
+    uint32_t tab[64];            // the gate output's step table
     WinDev win;                  // wave of windows: the descriptor of the block's current window
     uint32_t cw;                 // its number
     uint32_t q;                  // the block's gate output, kInf: none left
@@ -40,6 +41,7 @@ struct GateSmem {
     uint32_t s0[kMaxWarps], s1[kMaxWarps];
     unsigned long long scr, dst; // the gate output's stacks in the scratch, its list in the pool
     uint32_t ok;                 // the list has its place
+    uint32_t xt;                 // latest X or Z of the list but its first entry
 };
 
 // Per thread of the block, one time segment: shared arrays behind GateSmem.
@@ -53,7 +55,7 @@ struct SegSmem {
 
 // fetch: thread 0 sets sm.q and sm.skip to the block's next gate output; called
 // where the wait for it overlaps others and every thread has read the present one.
-template <int M, class Fetch>
+template <int M, bool kTab, class Fetch>
 __device__ __forceinline__ void run_gate(const WinDev &w, const LevelArgs &a, uint32_t i, GateSmem &sm,
                                          const SegSmem &sg, Fetch fetch)
 {
@@ -65,6 +67,7 @@ __device__ __forceinline__ void run_gate(const WinDev &w, const LevelArgs &a, ui
     uint64_t off[M], poff = 0, soff = 0;
     uint32_t len[M], plen = 0, slen = 0;
     unsigned long long E = 0;
+    uint32_t xmax = 0;   // the latest X, Z or repeated value of the input lists
     int piv = 0, sec = -1;   // the longest input list and the longest of the others
 #pragma unroll
     for (int j = 0; j < M; ++j) {
@@ -74,6 +77,7 @@ __device__ __forceinline__ void run_gate(const WinDev &w, const LevelArgs &a, ui
             off[j] = w.net_off[net];
             len[j] = w.net_len[net];
             E += len[j];
+            if (kTab) xmax = max(xmax, w.net_len[a.n_nets + net]);
             if (len[j] > plen) { sec = piv; slen = plen; plen = len[j]; piv = j; }
             else if (sec < 0 || len[j] > slen) { sec = j; slen = len[j]; }
         }
@@ -99,6 +103,14 @@ __device__ __forceinline__ void run_gate(const WinDev &w, const LevelArgs &a, ui
         if (mdp->flags & kFlagFirstOut)   // first output of its instance: count fan-in per pin
             for (int p = 0; p < mdp->n_pins; ++p) sm.ctr[0] += w.net_len[mdp->net[(mdp->pin_slot >> (3 * p)) & 7u]];
     }
+    bool usable = false;   // the step table is
+    if constexpr (kTab) {
+        const uint4 f0 = __ldg(a.fast + 2ull * drv), f1 = __ldg(a.fast + 2ull * drv + 1);
+        usable = f1.w != 0u;
+        if (usable)
+            for (uint32_t e = tid; e < 1u << (2 * M); e += nthr) sm.tab[e] = step_entry<M>(f0, f1, e);
+    }
+    if (tid == 0) sm.xt = 0;
     // the segment's start; its end is the next thread's start
     const bool mine = tid < S;
     uint32_t cb[M], tcut = 0;
@@ -114,11 +126,40 @@ __device__ __forceinline__ void run_gate(const WinDev &w, const LevelArgs &a, ui
     }
     uint32_t *const scr = w.scratch + sm.scr;
     uint32_t region = tid;
-    WalkOut o = {0, kInf, 0};
+    WalkOut o = {0, kInf, 0, 0};
     if (mine) {
+        uint32_t curp = 0x555u & ((1u << (2 * M)) - 1u), tmax = 0;
+        bool before = false;
+        ListReader rd[M];
 #pragma unroll
-        for (int j = 0; j < M; ++j) region += cb[j];
-        o = walk_segment<M>(w, a, drv, tid, off, len, cb, tid + 1 < S ? sg.tcut[tid + 1] : kInf, scr + region);
+        for (int j = 0; j < M; ++j) {
+            const uint32_t *x = w.pool + off[j];
+            region += cb[j];
+            if (cb[j] > 0) {
+                curp = (curp & ~(3u << (2 * j))) | (ev_val(x[cb[j] - 1]) << (2 * j));
+                before = true;
+            }
+            rd[j].start(x, cb[j], len[j]);
+        }
+        const uint32_t tnext = tid + 1 < S ? sg.tcut[tid + 1] : kInf;
+        if (tnext != kInf) {
+            tmax = tnext;
+        } else {
+#pragma unroll
+            for (int j = 0; j < M; ++j)
+                if (len[j]) tmax = max(tmax, ev_time(w.pool[off[j] + len[j] - 1]));
+        }
+        // the step table serves a warp whose segments all start in known
+        // values, behind every X, Z and repeat: lanes of both kinds would
+        // walk one kind after the other
+        bool clean = false;
+        if constexpr (kTab) {
+            clean = usable && tmax <= kMaxTime - 0x10000u && tcut > xmax && ((curp ^ (curp >> 1)) & 0x15u) == 0u;
+            clean = __all_sync(__activemask(), clean);
+        }
+        o = walk_segment<M, kTab>(w, a, drv, tid, rd, curp, before, tnext, tmax, GlobalStack{scr + region},
+                                      (uint32_t)__cvta_generic_to_shared(sm.tab), clean);
+        if (o.xt) atomicMax(&sm.xt, o.xt);
     }
     // later segments cut this one's stack at their smallest candidate
     uint32_t x = o.minw;
@@ -195,6 +236,7 @@ __device__ __forceinline__ void run_gate(const WinDev &w, const LevelArgs &a, ui
         else {
             w.net_off[mdp->out_net] = st;
             w.net_len[mdp->out_net] = total;
+            w.net_len[a.n_nets + mdp->out_net] = sm.xt;
         }
         sm.ctr[1] += total;
     }
@@ -274,7 +316,7 @@ __device__ __forceinline__ void run_gate(const WinDev &w, const LevelArgs &a, ui
 // class of four to six input nets, else the narrower ones; c1, c2: where the
 // 2- and 3-input ones start).  Blocks take gate outputs from the back, the
 // widest first, as they become free.
-template <bool kBatch, bool kSix>
+template <bool kBatch, bool kSix, bool kTab>
 __global__ void __launch_bounds__(kGateMaxThreads, kSix ? 1 : 1024 / kGateMaxThreads)
     k_gate(const WinSet<kBatch> ws, LevelArgs a, uint32_t d0, uint32_t d1, uint32_t c1, uint32_t c2)
 {
@@ -294,6 +336,10 @@ __global__ void __launch_bounds__(kGateMaxThreads, kSix ? 1 : 1024 / kGateMaxThr
             sm.ctr[k] = 0;
         }
     };
+    // launched while the previous level's last blocks run: nothing it wrote is
+    // read before this; the next level's blocks may follow likewise
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (threadIdx.x == 0) {
         sm.cw = kInf;
         for (int k = 0; k < 4; ++k) sm.ctr[k] = 0;
@@ -329,11 +375,11 @@ __global__ void __launch_bounds__(kGateMaxThreads, kSix ? 1 : 1024 / kGateMaxThr
         const uint32_t i = d1 - 1 - (kBatch ? q - win * n : q);
         auto go = [&](const WinDev &w) {
             if constexpr (kSix) {
-                run_gate<kMaxSlots>(w, a, i, sm, sg, next);
+                run_gate<kMaxSlots, false>(w, a, i, sm, sg, next);
             } else {
-                if (i >= c2) run_gate<3>(w, a, i, sm, sg, next);
-                else if (i >= c1) run_gate<2>(w, a, i, sm, sg, next);
-                else run_gate<1>(w, a, i, sm, sg, next);
+                if (i >= c2) run_gate<3, kTab>(w, a, i, sm, sg, next);
+                else if (i >= c1) run_gate<2, kTab>(w, a, i, sm, sg, next);
+                else run_gate<1, kTab>(w, a, i, sm, sg, next);
             }
         };
         if constexpr (kBatch) go(sm.win);
@@ -343,21 +389,38 @@ __global__ void __launch_bounds__(kGateMaxThreads, kSix ? 1 : 1024 / kGateMaxThr
 }
 
 void launch_gate(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelArgs &a, const uint32_t *cls,
-                 uint32_t threads, int sm_count, cudaStream_t st, uint32_t *launches)
+                 uint32_t threads, bool table, int sm_count, cudaStream_t st, uint32_t *launches)
 {
     const uint32_t smem = threads * 5 * 4;
-    auto go = [&](auto six, uint32_t d0, uint32_t d1) {
-        constexpr bool kSix = decltype(six)::value;
+    auto go = [&](auto six, auto tab, uint32_t d0, uint32_t d1) {
+        constexpr bool kSix = decltype(six)::value, kTab = decltype(tab)::value;
         if (d1 <= d0) return;
         const uint64_t total = (uint64_t)(d1 - d0) * nwin;
-        const uint64_t room = (uint64_t)sm_count * ((kSix ? 512 : 1024) / threads);
+        const uint64_t room = (uint64_t)sm_count * ((kSix ? kGateMaxThreads : 1024) / threads);
         const uint32_t grid = (uint32_t)(total < room ? total : room);
-        if (nwin == 1) k_gate<false, kSix><<<grid, threads, smem, st>>>(WinSet<false>{h}, a, d0, d1, cls[1], cls[2]);
-        else k_gate<true, kSix><<<grid, threads, smem, st>>>(WinSet<true>{dw, nwin}, a, d0, d1, cls[1], cls[2]);
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t lc = {};
+        lc.gridDim = dim3(grid);
+        lc.blockDim = dim3(threads);
+        lc.dynamicSmemBytes = smem;
+        lc.stream = st;
+        lc.attrs = &at;
+        lc.numAttrs = 1;
+        if (nwin == 1)
+            cudaLaunchKernelEx(&lc, k_gate<false, kSix, kTab>, WinSet<false>{h}, a, d0, d1, cls[1], cls[2]);
+        else
+            cudaLaunchKernelEx(&lc, k_gate<true, kSix, kTab>, WinSet<true>{dw, nwin}, a, d0, d1, cls[1], cls[2]);
         ++*launches;
     };
-    go(std::integral_constant<bool, true>(), cls[3], cls[4]);
-    go(std::integral_constant<bool, false>(), 0u, cls[3]);
+    using T = std::integral_constant<bool, true>;
+    using F = std::integral_constant<bool, false>;
+    go(T(), F(), cls[3], cls[4]);
+    // the step table is for warps none of whose segments starts at X: in a
+    // block of one warp the first one does
+    if (table && threads > 32) go(F(), T(), 0u, cls[3]);
+    else go(F(), F(), 0u, cls[3]);
 }
 
 }  // namespace gls

@@ -166,7 +166,8 @@ struct LevelCtr {           // k_gate: per window and level, cleared before the 
 
 struct WinDev {
     uint64_t *net_off;
-    uint32_t *net_len;
+    uint32_t *net_len;          // n_nets lengths; k_gate: then, per net, the time after which its list holds
+                                // nothing but alternating 0 and 1
     uint32_t *pool;
     unsigned long long *saif;   // 3 per net
     unsigned long long *top;    // pool bump pointer (events)
@@ -213,6 +214,7 @@ struct LevelArgs {
     uint32_t sim_variant;       // thread-per-segment gate kernel variant: bit 0 256-thread blocks, bit 1 wider loads
     float bal_weight;           // learned mode: segment work = fan-in events + bal_weight * predicted output events
     uint32_t level;             // the level's number
+    uint32_t n_nets;
     uint32_t plan_part;         // k_plan: 0 all of it; learned mode split in two: 1 segments and stacks
                                 // (slots left open), 2 slot placement from the predictions
 };
@@ -226,7 +228,7 @@ __host__ __device__ inline int fanin_class(int m) { return m <= 1 ? 0 : (m == 2 
 
 // A launch covers nwin windows: `h` is window 0's descriptor on the host
 // (used when nwin == 1), `dw` the device array of all nwin descriptors.
-void launch_stim_saif(const WinDev *dw, const WinDev &h, uint32_t nwin, uint32_t max_stim, bool wide,
+void launch_stim_saif(const WinDev *dw, const WinDev &h, uint32_t nwin, uint32_t max_stim, bool wide, uint32_t n_nets,
                       cudaStream_t st);
 void launch_plan(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelArgs &a, cudaStream_t st);
 // a wave's fan-in events per class into a.wave_e (cleared before), so every
@@ -243,9 +245,9 @@ void launch_copy(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelAr
 // One level in one launch (32-bit words; a second one where gate outputs with
 // four to six input nets exist).  cls: the level's fan-in class starts
 // (kClasses + 1); threads per block: 32 .. kGateMaxThreads, a power of two.
-constexpr uint32_t kGateMaxThreads = 512;
+constexpr uint32_t kGateMaxThreads = 256;
 constexpr uint32_t kGateMinSeg = 16;   // fan-in events a time segment is worth a search
 void launch_gate(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelArgs &a, const uint32_t *cls,
-                 uint32_t threads, int sm_count, cudaStream_t st, uint32_t *launches);
+                 uint32_t threads, bool table, int sm_count, cudaStream_t st, uint32_t *launches);
 
 }  // namespace gls

@@ -637,7 +637,22 @@ __device__ __forceinline__ void sim_segment2(const WinDev &w, const LevelArgs &a
     uint32_t region = s;
 #pragma unroll
     for (int j = 0; j < M; ++j) region += cb[j];
-    const WalkOut o = walk_segment<M>(w, a, drv, s, off, len, cb, tnext, w.scratch + scr + region);
+    uint32_t curp = 0x555u & ((1u << (2 * M)) - 1u), tmax = 0;
+    bool before = false;
+    ListReader rd[M];
+#pragma unroll
+    for (int j = 0; j < M; ++j) {
+        const uint32_t *x = pw + off[j];
+        if (cb[j] > 0) {
+            curp = (curp & ~(3u << (2 * j))) | (ev_val(x[cb[j] - 1]) << (2 * j));
+            before = true;
+        }
+        if (len[j]) tmax = max(tmax, ev_time(x[len[j] - 1]));
+        rd[j].start(x, cb[j], len[j]);
+    }
+    if (tnext != kInf) tmax = tnext;
+    const WalkOut o = walk_segment<M, false>(w, a, drv, s, rd, curp, before, tnext, tmax,
+                                             GlobalStack{w.scratch + scr + region});
     SegRec r;
     r.region = region; r.cnt = o.cnt; r.min_o = o.minw == kInf ? kInf : o.minw >> 2; r.last = o.top;
     w.segs[seg_id] = r;
@@ -1565,9 +1580,11 @@ __global__ void __launch_bounds__(256, GLS_COPY_BLOCKS) k_copy(const WinSet<kBat
 }
 
 // ------------------------------------------------------- stimulus SAIF
-// one warp per stimulus net; blockIdx.y is the window
+// one warp per stimulus net; blockIdx.y is the window.  Beside the SAIF
+// counts, the time of the net's last X, Z or repeated value, after which it
+// only alternates between 0 and 1 (what k_gate's step table asks).
 template <bool kBatch, class Wd>
-__global__ void __launch_bounds__(256) k_stim_saif(const WinSet<kBatch> ws)
+__global__ void __launch_bounds__(256) k_stim_saif(const WinSet<kBatch> ws, uint32_t n_nets)
 {
     const WinDev &w = ws.get(blockIdx.y);
     const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1581,16 +1598,24 @@ __global__ void __launch_bounds__(256) k_stim_saif(const WinSet<kBatch> ws)
     P prev = 2u;   // before the first event: X from t_begin
     P acc[3] = {0, 0, 0};
     const Wd *pw = reinterpret_cast<const Wd *>(w.pool);
+    uint32_t xt = 0, vlast = 4;   // vlast: the value before this round
     for (uint32_t i0 = 0; i0 < len; i0 += 32) {
         const bool v = i0 + lane < len;
         const Wd word = v ? pw[off + i0 + lane] : Wd(0);
+        const uint32_t val = ev_val(word);
+        uint32_t vb = __shfl_up_sync(0xffffffffu, val, 1);
+        if (lane == 0) vb = vlast;
+        if (v && (val == kVX || val == kVZ || val == vb)) xt = ev_time(word);   // times increase
+        vlast = __shfl_sync(0xffffffffu, val, 31);
         integrate_group<32, Wd, P>(rc, word, v, len - i0, true, prev, acc);
     }
 #pragma unroll
     for (int k = 0; k < 3; ++k)
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) acc[k] += __shfl_down_sync(0xffffffffu, acc[k], o);
+    xt = __reduce_max_sync(0xffffffffu, xt);
     if (lane == 0) {
+        w.net_len[n_nets + net] = xt;
         // the last event holds until t_end
         unsigned long long tot[3] = {acc[0], acc[1], acc[2]};
         saif_add(tot, (int)(prev & 3u), w.t_end - (w.t_begin + (prev >> 2)));
@@ -1614,15 +1639,16 @@ __global__ void __launch_bounds__(256) k_stim_saif(const WinSet<kBatch> ws)
 
 // Windows of 64-bit event words (times past 2^30 - 2) run one at a time
 // through the thread-per-segment kernels: the host never batches them.
-void launch_stim_saif(const WinDev *dw, const WinDev &h, uint32_t nwin, uint32_t max_stim, bool wide, cudaStream_t st)
+void launch_stim_saif(const WinDev *dw, const WinDev &h, uint32_t nwin, uint32_t max_stim, bool wide, uint32_t n_nets,
+                      cudaStream_t st)
 {
     if (!max_stim || !nwin) return;
     const dim3 grid((uint32_t)(((uint64_t)max_stim * 32 + 255) / 256), nwin);
     if (wide) {
-        k_stim_saif<false, WideWord><<<grid, 256, 0, st>>>(WinSet<false>{h});
+        k_stim_saif<false, WideWord><<<grid, 256, 0, st>>>(WinSet<false>{h}, n_nets);
         return;
     }
-    GLS_DISPATCH(h, dw, nwin, (k_stim_saif<decltype(ws)::kIsBatch, uint32_t><<<grid, 256, 0, st>>>(ws)));
+    GLS_DISPATCH(h, dw, nwin, (k_stim_saif<decltype(ws)::kIsBatch, uint32_t><<<grid, 256, 0, st>>>(ws, n_nets)));
 }
 
 void launch_wave_events(const WinDev *dw, uint32_t nwin, const LevelArgs &a, cudaStream_t st)
