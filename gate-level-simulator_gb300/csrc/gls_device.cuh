@@ -2,6 +2,7 @@
 // readers, and the walk of one time segment.
 #pragma once
 #include <cuda_runtime.h>
+#include <cstddef>
 #include <cstdint>
 #include <type_traits>
 #include "gls_internal.h"
@@ -67,6 +68,12 @@ __device__ inline uint32_t select_delay(const ArcDev *__restrict__ arcs, int n_a
         any = true;
     }
     return any ? mn : defd;
+}
+
+static __device__ __noinline__ uint32_t select_delay_call(const ArcDev *__restrict__ arcs, int n_arcs, uint32_t chg, int so,
+                                                          uint32_t curp, uint32_t lastp, uint32_t defd)
+{
+    return select_delay(arcs, n_arcs, chg, so, curp, lastp, defd);
 }
 
 // Delay of an active step of a regular gate output: the smallest delay the
@@ -230,14 +237,26 @@ __device__ __forceinline__ uint32_t rank_time2(P X, uint32_t nx, P Y, uint32_t n
     return T;
 }
 
+template <class P>
+static __device__ __noinline__ uint32_t search_from_call(P x, uint32_t n, uint32_t key, uint32_t g)
+{
+    return search_from(x, n, key, g);
+}
+template <class P>
+static __device__ __noinline__ uint32_t rank_time2_call(P X, uint32_t nx, P Y, uint32_t ny, uint32_t r, uint32_t g,
+                                                        uint32_t &ix, uint32_t &iy)
+{
+    return rank_time2(X, nx, Y, ny, r, g, ix, iy);
+}
+
 // Cut sk of S (0 < sk < S) of a gate output's fan-in timeline: the time of
 // the event of rank sk * (plen + slen) / S in the merge of its two longest
 // input lists (piv, sec), so that those two (all of them for gates with two
 // input nets) split into segments of equal size; with one input net the
 // event of rank sk * plen / S of that list.  Returns that time; cut[j]
 // receives list j's first event at or after it.  The cut time does not
-// decrease with sk.
-template <int M, class Wd>
+// decrease with sk.  kCall: the searches are calls, not inlined (see k_gate).
+template <int M, bool kCall = false, class Wd>
 __device__ __forceinline__ uint32_t cut_at(const Wd *__restrict__ pool, const uint64_t (&off)[M],
                                        const uint32_t (&len)[M], int m, int piv, int sec, uint64_t poff, uint64_t soff,
                                        uint32_t plen, uint32_t slen, uint32_t sk, uint32_t S, uint32_t (&cut)[M])
@@ -245,15 +264,25 @@ __device__ __forceinline__ uint32_t cut_at(const Wd *__restrict__ pool, const ui
     uint32_t ip, is = 0, T;
     if (sec >= 0) {
         const uint32_t r = mul_div(sk, plen + slen, S);
-        T = rank_time2(pool + poff, plen, pool + soff, slen, r, mul_div(r, plen, plen + slen), ip, is);
+        const uint32_t g = mul_div(r, plen, plen + slen);
+        T = kCall ? rank_time2_call(pool + poff, plen, pool + soff, slen, r, g, ip, is)
+                  : rank_time2(pool + poff, plen, pool + soff, slen, r, g, ip, is);
     } else {
         ip = mul_div(sk, plen, S);
         T = ev_time(pool[poff + ip]);
     }
 #pragma unroll
     for (int j = 0; j < M; ++j) {
-        if (j < m)
-            cut[j] = j == piv ? ip : (j == sec ? is : search_from(pool + off[j], len[j], T, mul_div(ip, len[j], plen)));
+        if (j < m) {
+            if (j == piv) {
+                cut[j] = ip;
+            } else if (j == sec) {
+                cut[j] = is;
+            } else {
+                const uint32_t g = mul_div(ip, len[j], plen);
+                cut[j] = kCall ? search_from_call(pool + off[j], len[j], T, g) : search_from(pool + off[j], len[j], T, g);
+            }
+        }
     }
     return T;
 }
@@ -331,47 +360,6 @@ struct ListReader {
     }
 };
 
-// A change list, or a stretch of one, in shared memory (its shared address).
-struct SmemList {
-    uint32_t at;
-    __device__ __forceinline__ uint32_t operator[](uint32_t i) const
-    {
-        uint32_t v;
-        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(at + 4 * i));
-        return v;
-    }
-    __device__ __forceinline__ void set(uint32_t i, uint32_t v) const
-    {
-        asm volatile("st.shared.u32 [%0], %1;" ::"r"(at + 4 * i), "r"(v) : "memory");
-    }
-};
-
-// Reader of a stretch in shared memory: two kInf words follow its last event.
-struct SmemReader {
-    uint32_t h, n;
-    uint32_t p;   // shared address of the head
-
-    __device__ __forceinline__ void start(SmemList x, uint32_t b)
-    {
-        p = x.at + 4 * b;
-        h = SmemList{p}[0];
-        n = SmemList{p}[1];
-    }
-    __device__ __forceinline__ void advance(bool go)
-    {
-        h = go ? n : h;
-        p += go ? 4u : 0u;
-        n = SmemList{p}[1];
-    }
-};
-
-// Where a segment's stack lies.
-struct GlobalStack {
-    uint32_t *x;
-    __device__ __forceinline__ uint32_t operator[](uint32_t i) const { return x[i]; }
-    __device__ __forceinline__ void set(uint32_t i, uint32_t v) const { x[i] = v; }
-};
-
 // The walk of one time segment of a gate output, 32-bit words: from the
 // segment's first event of every list (in rd, with the values before them in
 // curp; before: some list has one) to its end time tnext (kInf: the lists' end),
@@ -431,13 +419,29 @@ __device__ __forceinline__ uint32_t step_entry(const uint4 &f0, const uint4 &f1,
     return d << 2 | (F ? kV1 : kV0);
 }
 
-template <int M, bool kTab, class RD, class ST>
-__device__ __forceinline__ WalkOut walk_segment(const WinDev &w, const LevelArgs &a, uint32_t drv, uint32_t s,
-                                                RD (&rd)[M], uint32_t curp, bool before, uint32_t tnext,
-                                                uint32_t tmax, ST ot, uint32_t tab = 0, bool clean = false)
+// What a gate output's walks read from shared memory (tab: its address).
+struct __align__(256) GateTab {
+    uint32_t step[64];   // the step table
+    uint32_t slut[4];    // the truth table (LevelArgs::slut)
+    uint32_t nd[24];     // its input nets' NetDelay entries (regular gate outputs)
+};
+__device__ __forceinline__ uint32_t lds32(uint32_t at)
 {
-    static_assert(!kTab || M <= 3, "step tables are for up to three input nets");
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(at));
+    return v;
+}
+
+// kSm: the general step reads the gate output's tables from shared memory too;
+// kCall: delays of irregular arcs by a call.
+template <int M, bool kTab, bool kSm, bool kCall>
+__device__ __forceinline__ WalkOut walk_segment(const WinDev &w, const LevelArgs &a, uint32_t drv, uint32_t s,
+                                                ListReader (&rd)[M], uint32_t curp, bool before, uint32_t tnext,
+                                                uint32_t tmax, uint32_t *ot, uint32_t tab = 0, bool clean = false)
+{
+    static_assert(!(kTab || kSm) || M <= 3, "the tables are for up to three input nets");
     constexpr bool kFast = M <= 3;
+    constexpr uint32_t kSlut = offsetof(GateTab, slut), kNd = offsetof(GateTab, nd);
     const DrvMeta *__restrict__ mdp = a.meta + drv;
     // words at or above tend lie behind the segment
     const uint32_t tend = tnext != kInf ? tnext << 2 : kInf;
@@ -461,13 +465,15 @@ __device__ __forceinline__ WalkOut walk_segment(const WinDev &w, const LevelArgs
     // entry left the top reads as (0, X): below every later candidate, and
     // different from 0 and 1.
     uint32_t top = EvW<uint32_t>::word(0, kVX), below = kInf;
-    if (s == 0) { ot.set(0, top); cnt = 1; }
+    if (s == 0) { ot[0] = top; cnt = 1; }
     uint32_t fprev = kVX;
     auto out_of = [&](uint32_t x) -> uint32_t {   // the general step's truth table
-        if constexpr (kFast) return slut_get<M>(__ldg(a.slut + drv), x);
+        if constexpr (kSm) return (lds32(tab + kSlut + (M == 3 ? (x >> 4) * 4 : 0u)) >> (2 * (x & 15u))) & 3u;
+        else if constexpr (kFast) return slut_get<M>(__ldg(a.slut + drv), x);
         else return __ldg(a.lut + mdp->lut_off + lut_index(x, *mdp));
     };
     if (before) fprev = out_of(curp);
+    const bool regular = mdp->flags & kFlagRegular;
     uint32_t minw = kInf, xt = 0;
     for (;;) {
         uint32_t mk = rd[0].h | 3u;
@@ -509,7 +515,7 @@ __device__ __forceinline__ WalkOut walk_segment(const WinDev &w, const LevelArgs
                 } while (top >= lo);
             }
             const bool push = chg && ((top ^ F) & 3u) != 0u;
-            if (push) ot.set(cnt, lo | F);
+            if (push) ot[cnt] = lo | F;
             below = push ? top : below;
             top = push ? lo | F : top;
             cnt += push ? 1u : 0u;
@@ -520,13 +526,23 @@ __device__ __forceinline__ WalkOut walk_segment(const WinDev &w, const LevelArgs
         if (F == fprev) continue;
         const uint32_t so1 = (kSense1Tab >> (2 * (fprev * 4 + F))) & 3u;
         fprev = F;
-        uint32_t chg = 0;
+        uint32_t d;
+        if (regular && kSm) {   // as regular_delay
+            d = kInf;
 #pragma unroll
-        for (int j = 0; j < M; ++j) chg |= ch[j] ? 1u << j : 0u;
-        const uint32_t d = (mdp->flags & kFlagRegular)
-                               ? regular_delay<M>(a.ndel + mdp->dt_off, chg, so1, curp, lastp, a.def_delay)
-                               : select_delay(a.arcs + mdp->arc_off, mdp->n_arcs, chg, (int)so1 + 1, curp, lastp,
-                                              a.def_delay);
+            for (int j = 0; j < M; ++j) {
+                const uint32_t neg = (kNegTab >> (slot_val(lastp, j) * 4 + slot_val(curp, j))) & 1u;
+                if (ch[j]) d = min(d, lds32(tab + kNd + (j * 8 + neg * 4 + so1) * 4));
+            }
+            d = d == kInf ? a.def_delay : d;
+        } else {
+            uint32_t chg = 0;
+#pragma unroll
+            for (int j = 0; j < M; ++j) chg |= ch[j] ? 1u << j : 0u;
+            d = regular ? regular_delay<M>(a.ndel + mdp->dt_off, chg, so1, curp, lastp, a.def_delay)
+                : kCall ? select_delay_call(a.arcs + mdp->arc_off, mdp->n_arcs, chg, (int)so1 + 1, curp, lastp, a.def_delay)
+                        : select_delay(a.arcs + mdp->arc_off, mdp->n_arcs, chg, (int)so1 + 1, curp, lastp, a.def_delay);
+        }
         const uint64_t o64 = (uint64_t)ev_time(mk) + d;
         if (o64 > kMaxTime) { atomicOr(w.err, kErrTime); break; }
         const uint32_t lo = (uint32_t)o64 << 2;
@@ -542,7 +558,7 @@ __device__ __forceinline__ WalkOut walk_segment(const WinDev &w, const LevelArgs
         if (prevv != (int)F) {
             below = kInf;
             top = lo | F;
-            ot.set(cnt++, top);
+            ot[cnt++] = top;
             if (F == kVX || F == kVZ) xt = lo >> 2;
         } else if (cnt == 0) {
             atomicOr(w.err, kErrEmptied);
@@ -566,8 +582,7 @@ __device__ __forceinline__ WalkOut walk_segment(const WinDev &w, const LevelArgs
                 x |= ch ? 4u << j : 0u;
                 rd[j].advance(ch);
             }
-            uint32_t st;
-            asm volatile("ld.shared.u32 %0, [%1];" : "=r"(st) : "r"(x));
+            const uint32_t st = lds32(x);
             so ^= (x ^ so) << M;
             const bool chg = st != kInf;
             const uint32_t nw = mk - 3u + st;   // the candidate's event word
@@ -581,7 +596,7 @@ __device__ __forceinline__ WalkOut walk_segment(const WinDev &w, const LevelArgs
                 } while ((top | 3u) >= nw);
             }
             const bool put = chg && ((top ^ nw) & 3u) != 0u;
-            if (put) ot.set(cnt, nw);
+            if (put) ot[cnt] = nw;
             below = put ? top : below;
             top = put ? nw : top;
             cnt += put ? 1u : 0u;

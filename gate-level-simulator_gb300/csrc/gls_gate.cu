@@ -28,8 +28,8 @@ namespace {
 
 constexpr int kMaxWarps = kGateMaxThreads / 32;
 
-struct __align__(256) GateSmem {
-    uint32_t tab[64];            // the gate output's step table
+struct GateSmem {
+    GateTab tab;                 // the gate output's tables
     WinDev win;                  // wave of windows: the descriptor of the block's current window
     uint32_t cw;                 // its number
     uint32_t q;                  // the block's gate output, kInf: none left
@@ -53,20 +53,33 @@ struct SegSmem {
     uint32_t *pv;     // value before them
 };
 
-// fetch: thread 0 sets sm.q and sm.skip to the block's next gate output; called
-// where the wait for it overlaps others and every thread has read the present one.
-template <int M, bool kTab, class Fetch>
-__device__ __forceinline__ void run_gate(const WinDev &w, const LevelArgs &a, uint32_t i, GateSmem &sm,
-                                         const SegSmem &sg, Fetch fetch)
+// The thread's part of a gate output after the walk.
+struct Walked {
+    WalkOut o;
+    uint32_t region;         // its stack among the gate output's
+    uint32_t S;              // segments of the gate output
+    unsigned long long E;    // fan-in events of the gate output
+};
+
+// Cut and walk gate output i of the level.
+template <int M, bool kTab>
+__device__ __forceinline__ Walked walk_gate(const WinDev &w, const LevelArgs &a, uint32_t i, GateSmem &sm,
+                                            const SegSmem &sg)
 {
-    const unsigned FULL = 0xffffffffu;
-    const uint32_t tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31u, wid = tid >> 5, nw = nthr >> 5;
+    const uint32_t tid = threadIdx.x, nthr = blockDim.x;
     const uint32_t drv = a.lo + i;
     const DrvMeta *__restrict__ mdp = a.meta + drv;
+    constexpr bool kSm = kTab;
+    uint4 f0 = {0, 0, 0, 0}, f1 = {0, 0, 0, 0};
+    if (kTab) {
+        f0 = __ldg(a.fast + 2ull * drv);
+        f1 = __ldg(a.fast + 2ull * drv + 1);
+    }
     const int m = mdp->m;
     uint64_t off[M], poff = 0, soff = 0;
     uint32_t len[M], plen = 0, slen = 0;
     unsigned long long E = 0;
+    uint32_t lmin = kInf;
     uint32_t xmax = 0;   // the latest X, Z or repeated value of the input lists
     int piv = 0, sec = -1;   // the longest input list and the longest of the others
 #pragma unroll
@@ -77,6 +90,7 @@ __device__ __forceinline__ void run_gate(const WinDev &w, const LevelArgs &a, ui
             off[j] = w.net_off[net];
             len[j] = w.net_len[net];
             E += len[j];
+            lmin = min(lmin, len[j]);
             if (kTab) xmax = max(xmax, w.net_len[a.n_nets + net]);
             if (len[j] > plen) { sec = piv; slen = plen; plen = len[j]; piv = j; }
             else if (sec < 0 || len[j] > slen) { sec = j; slen = len[j]; }
@@ -92,42 +106,44 @@ __device__ __forceinline__ void run_gate(const WinDev &w, const LevelArgs &a, ui
     unsigned long long seg = a.seg_events ? max(a.seg_events, 8u) : kGateMinSeg;
     seg = max(seg, (E + nthr - 1) / nthr);
     const uint32_t S = (uint32_t)max(1ull, (E + seg - 1) / seg);
-    if (tid == 0) {
-        const unsigned long long need = (E + S + 3) & ~3ull;
-        const unsigned long long at = atomicAdd(&w.lvl[a.level].scr, need);
-        sm.scr = at;
-        sm.ok = at + need <= w.scr_cap;
-        if (!sm.ok) atomicOr(w.err, kErrScratch);
-        sm.ctr[2] += S;
-        sm.ctr[3] += E;
-        if (mdp->flags & kFlagFirstOut)   // first output of its instance: count fan-in per pin
-            for (int p = 0; p < mdp->n_pins; ++p) sm.ctr[0] += w.net_len[mdp->net[(mdp->pin_slot >> (3 * p)) & 7u]];
+    const unsigned long long scr_need = (E + S + 3) & ~3ull;
+    unsigned long long scr_at = 0;   // thread 0; used once the cuts are found
+    if (tid == 0) scr_at = atomicAdd(&w.lvl[a.level].scr, scr_need);
+    const bool usable = kTab && f1.w != 0u;   // the step table is
+    uint32_t tabw = 0;   // a word of the tables, stored once the cuts are found
+    const uint32_t tk = nthr - 1 - tid;
+    if constexpr (kSm) {
+        if (tk < 4) tabw = __ldg(reinterpret_cast<const uint32_t *>(a.slut + drv) + tk);
+        else if (tk - 4 < 8 * (uint32_t)m && (mdp->flags & kFlagRegular)) tabw = __ldg(a.ndel[mdp->dt_off].d + (tk - 4));
     }
-    bool usable = false;   // the step table is
-    if constexpr (kTab) {
-        const uint4 f0 = __ldg(a.fast + 2ull * drv), f1 = __ldg(a.fast + 2ull * drv + 1);
-        usable = f1.w != 0u;
-        if (usable)
-            for (uint32_t e = tid; e < 1u << (2 * M); e += nthr) sm.tab[e] = step_entry<M>(f0, f1, e);
-    }
-    if (tid == 0) sm.xt = 0;
-    // the segment's start; its end is the next thread's start
+    // the segment's start; its end is the next thread's start.  With a step
+    // table the first warp's segments, which walk without it, are cut to half
+    // the others' length.
     const bool mine = tid < S;
+    const bool half = usable && S > 64 && lmin > 1;
+    const uint32_t sk = half && tid > 32 ? 2 * tid - 32 : tid, sn = half ? 2 * S - 32 : S;
     uint32_t cb[M], tcut = 0;
 #pragma unroll
     for (int j = 0; j < M; ++j) cb[j] = 0;
     if (mine && tid > 0)
-        tcut = cut_at<M>(w.pool, off, len, m, piv, sec, poff, soff, plen, slen, tid, S, cb);
+        tcut = cut_at<M, !kTab>(w.pool, off, len, m, piv, sec, poff, soff, plen, slen, sk, sn, cb);
     if (mine) sg.tcut[tid] = tcut;
-    __syncthreads();
-    if (!sm.ok) {   // the same for the whole block
-        if (tid == 0) fetch();
-        return;
+    if constexpr (kTab) {
+        if (usable)
+            for (uint32_t e = tid; e < 1u << (2 * M); e += nthr) sm.tab.step[e] = step_entry<M>(f0, f1, e);
     }
+    if (kSm && tk < 28) (&sm.tab.slut[0])[tk] = tabw;   // slut, then nd
+    if (tid == 0) {
+        sm.xt = 0;
+        sm.scr = scr_at;
+        sm.ok = scr_at + scr_need <= w.scr_cap;
+        if (!sm.ok) atomicOr(w.err, kErrScratch);
+    }
+    __syncthreads();
     uint32_t *const scr = w.scratch + sm.scr;
     uint32_t region = tid;
     WalkOut o = {0, kInf, 0, 0};
-    if (mine) {
+    if (mine && sm.ok) {
         uint32_t curp = 0x555u & ((1u << (2 * M)) - 1u), tmax = 0;
         bool before = false;
         ListReader rd[M];
@@ -157,10 +173,36 @@ __device__ __forceinline__ void run_gate(const WinDev &w, const LevelArgs &a, ui
             clean = usable && tmax <= kMaxTime - 0x10000u && tcut > xmax && ((curp ^ (curp >> 1)) & 0x15u) == 0u;
             clean = __all_sync(__activemask(), clean);
         }
-        o = walk_segment<M, kTab>(w, a, drv, tid, rd, curp, before, tnext, tmax, GlobalStack{scr + region},
-                                      (uint32_t)__cvta_generic_to_shared(sm.tab), clean);
+        o = walk_segment<M, kTab, kSm, !kTab>(w, a, drv, tid, rd, curp, before, tnext, tmax, scr + region,
+                                       (uint32_t)__cvta_generic_to_shared(&sm.tab), clean);
         if (o.xt) atomicMax(&sm.xt, o.xt);
     }
+    return {o, region, S, E};
+}
+
+// Link the walked segments' stacks, place the gate output's list and copy it.
+// fetch: thread 0 sets sm.q and sm.skip to the block's next gate output; called
+// where the wait for it overlaps others and every thread has read the present
+// one.
+template <class Fetch>
+__device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a, uint32_t i, GateSmem &sm,
+                                            const SegSmem &sg, const Walked &wk, Fetch fetch)
+{
+    const unsigned FULL = 0xffffffffu;
+    const uint32_t tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31u, wid = tid >> 5, nw = nthr >> 5;
+    const DrvMeta *__restrict__ mdp = a.meta + a.lo + i;
+    const WalkOut &o = wk.o;
+    const uint32_t region = wk.region, S = wk.S;
+    const unsigned long long E = wk.E;
+    const bool mine = tid < S;
+    if (!sm.ok) {   // no room for its stacks; the same for the whole block
+        __syncthreads();
+        if (tid == 0) fetch();
+        return;
+    }
+    uint32_t *const scr = w.scratch + sm.scr;
+    const uint32_t *ot = scr + region;
+    const uint32_t bottom = o.cnt ? ot[0] : 0u;   // on its way while the minima meet
     // later segments cut this one's stack at their smallest candidate
     uint32_t x = o.minw;
 #pragma unroll
@@ -173,12 +215,11 @@ __device__ __forceinline__ void run_gate(const WinDev &w, const LevelArgs &a, ui
     if (lane == 31) later = kInf;
     __syncthreads();
     for (uint32_t k = wid + 1; k < nw; ++k) later = min(later, sm.wmin[k]);
-    const uint32_t *ot = scr + region;
     uint32_t keep = o.cnt, firstv = 0, lastv = 0;
     if (keep && later != kInf)
         while (keep && ((keep == o.cnt ? o.top : ot[keep - 1]) | 3u) >= later) --keep;
     if (keep) {
-        firstv = ev_val(ot[0]);
+        firstv = ev_val(bottom);
         lastv = ev_val(keep == o.cnt ? o.top : ot[keep - 1]);
     }
     // an entry at a segment's bottom that repeats the last kept value before it goes
@@ -228,8 +269,8 @@ __device__ __forceinline__ void run_gate(const WinDev &w, const LevelArgs &a, ui
                 need = res;
             }
         }
-        fetch();
         const unsigned long long st = atomicAdd(w.top, need);
+        fetch();
         sm.dst = st;
         sm.ok = st + need <= w.cap;
         if (!sm.ok) atomicOr(w.err, kErrPool);
@@ -239,6 +280,13 @@ __device__ __forceinline__ void run_gate(const WinDev &w, const LevelArgs &a, ui
             w.net_len[a.n_nets + mdp->out_net] = sm.xt;
         }
         sm.ctr[1] += total;
+        sm.ctr[2] += S;
+        sm.ctr[3] += E;
+        if (mdp->flags & kFlagFirstOut) {   // first output of its instance: count fan-in per pin
+            if (mdp->flags & kFlagIdent) sm.ctr[0] += E;
+            else
+                for (int p = 0; p < mdp->n_pins; ++p) sm.ctr[0] += w.net_len[mdp->net[(mdp->pin_slot >> (3 * p)) & 7u]];
+        }
     }
     __syncthreads();
     if (!sm.ok) return;
@@ -247,7 +295,9 @@ __device__ __forceinline__ void run_gate(const WinDev &w, const LevelArgs &a, ui
     // time is the sum of t over the entries after a value of class c minus
     // the sum over those of class c, plus t_end for the last value's class.
     // Times are window-relative and below 2^30: the sums wrap in 32 bits and
-    // are read back as signed.
+    // are read back as signed.  (Four consecutive entries of the list a
+    // thread, found by bisection, and one 16-byte store: 75.1 ms instead of
+    // 74.4 on the 2 M cell design, 32.8 instead of 29.1 in waves.)
     constexpr uint32_t W = 8, U = 4;
     const uint32_t sub = tid & (W - 1);
     const RelClampT<uint32_t> rc(w.t_begin, w.t_end);
@@ -312,6 +362,13 @@ __device__ __forceinline__ void run_gate(const WinDev &w, const LevelArgs &a, ui
 
 }  // namespace
 
+// kTab = false is the kernel of one-warp blocks.  Their 32 warps on an SM run
+// all over it, and it is bound by instruction fetch (2.7 warps waiting for
+// instructions per issue): finish_gate is no template (three copies of it cost
+// 28.6 instead of 26.7 ms on 8 windows of 200,000 cells), and the cut searches
+// and irregular delays are calls (22.2 ms; on the 2 M cell design, whose
+// blocks of four warps run the other kernel, calls cost 75.8 instead of 73.9).
+//
 // Gate outputs [d0, d1) of the level of every window of the launch (kSix: the
 // class of four to six input nets, else the narrower ones; c1, c2: where the
 // 2- and 3-input ones start).  Blocks take gate outputs from the back, the
@@ -366,7 +423,7 @@ __global__ void __launch_bounds__(kGateMaxThreads, kSix ? 1 : 1024 / kGateMaxThr
                 __syncthreads();
             }
         }
-        auto next = [&]() { fetch(gridDim.x + atomicAdd(&ws.get(0).lvl[a.level].next[kSix ? 0 : 1], 1u)); };
+        auto next = [&]() { fetch(gridDim.x == total ? total : gridDim.x + atomicAdd(&ws.get(0).lvl[a.level].next[kSix ? 0 : 1], 1u)); };
         if (skip) {
             __syncthreads();   // sm.q is read
             if (threadIdx.x == 0) next();
@@ -374,13 +431,15 @@ __global__ void __launch_bounds__(kGateMaxThreads, kSix ? 1 : 1024 / kGateMaxThr
         }
         const uint32_t i = d1 - 1 - (kBatch ? q - win * n : q);
         auto go = [&](const WinDev &w) {
+            Walked wk;
             if constexpr (kSix) {
-                run_gate<kMaxSlots, false>(w, a, i, sm, sg, next);
+                wk = walk_gate<kMaxSlots, false>(w, a, i, sm, sg);
             } else {
-                if (i >= c2) run_gate<3, kTab>(w, a, i, sm, sg, next);
-                else if (i >= c1) run_gate<2, kTab>(w, a, i, sm, sg, next);
-                else run_gate<1, kTab>(w, a, i, sm, sg, next);
+                if (i >= c2) wk = walk_gate<3, kTab>(w, a, i, sm, sg);
+                else if (i >= c1) wk = walk_gate<2, kTab>(w, a, i, sm, sg);
+                else wk = walk_gate<1, kTab>(w, a, i, sm, sg);
             }
+            finish_gate(w, a, i, sm, sg, wk, next);
         };
         if constexpr (kBatch) go(sm.win);
         else go(ws.get(0));

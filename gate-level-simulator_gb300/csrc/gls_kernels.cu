@@ -651,8 +651,8 @@ __device__ __forceinline__ void sim_segment2(const WinDev &w, const LevelArgs &a
         rd[j].start(x, cb[j], len[j]);
     }
     if (tnext != kInf) tmax = tnext;
-    const WalkOut o = walk_segment<M, false>(w, a, drv, s, rd, curp, before, tnext, tmax,
-                                             GlobalStack{w.scratch + scr + region});
+    const WalkOut o = walk_segment<M, false, false, false>(w, a, drv, s, rd, curp, before, tnext, tmax,
+                                                    w.scratch + scr + region);
     SegRec r;
     r.region = region; r.cnt = o.cnt; r.min_o = o.minw == kInf ? kInf : o.minw >> 2; r.last = o.top;
     w.segs[seg_id] = r;
