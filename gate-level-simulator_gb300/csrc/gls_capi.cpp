@@ -831,7 +831,7 @@ static WinDev make_windev(gls_ctx *ctx, Window *w, const LevelScratch &ls, int p
     d.seg_base = (parity ? ls.seg_base1 : ls.seg_base).as<uint32_t>();
     d.slot = (parity ? ls.slot1 : ls.slot).as<uint64_t>();
     d.scr = (parity ? ls.scr1 : ls.scr).as<uint64_t>();
-    d.segs = ls.segs.as<SegRec>();   // SegRecT<WideWord> records in a window of 64-bit words
+    d.segs = ls.segs.as<SegRec>();
     d.copies = ls.copies.as<CopyRec>();
     d.scratch = ls.scratch.as<uint32_t>();
     d.lvl = w->lvl.as<LevelCtr>();
@@ -874,11 +874,11 @@ static int reset_window(gls_ctx *ctx, Window *w)
     return GLS_OK;
 }
 
-// Whether a run's levels go through k_gate: 32-bit words and the default
+// Whether a run's levels go through k_gate: 64-bit windows, and the default
 // thread-per-segment schedule.
 static bool gate_path(const gls_ctx *ctx, const LevelArgs &a)
 {
-    return ctx->gate_kernel && !a.wide && a.warp_mask == 0 && a.sim_variant == 0 && a.bal_weight <= 0.f;
+    return a.wide || (ctx->gate_kernel && a.warp_mask == 0 && a.sim_variant == 0 && a.bal_weight <= 0.f);
 }
 
 // k_gate's threads (and so time segments) per gate output, for a level of
@@ -913,11 +913,9 @@ static int enqueue_levels(gls_ctx *ctx, const WinDev *const dw[2], const WinDev 
 {
     LevelArgs a;
     ctx_level_args(ctx, &a);
-    if (w64) {   // a window of 64-bit words runs alone, through the thread-per-segment kernels
+    if (w64) {   // a window of 64-bit words runs alone, through k_gate
         if (nwin != 1) return fail(ctx, GLS_EINVAL, "64-bit event windows run one at a time");
         a.wide = 1;
-        a.warp_mask = 0;
-        a.sim_variant = 0;
     }
     // Overlapped levels: every class runs simulate, link and copy on its own
     // stream; the main stream plans the next level as soon as every class

@@ -168,8 +168,7 @@ struct LevelScratch {
             if (e == cudaSuccess) width = w;
         }
         if (e == cudaSuccess && segs_need > seg_cap) {
-            // room for the segment records of either event-word width
-            e = segs.ensure((size_t)segs_need * gls::kSegRecMax);
+            e = segs.ensure((size_t)segs_need * sizeof(gls::SegRec));
             if (e == cudaSuccess) e = copies.ensure((size_t)segs_need * sizeof(gls::CopyRec));
             if (e == cudaSuccess) seg_cap = segs_need;
         }
@@ -207,7 +206,7 @@ struct Window {
     bool saif_only = false;             // pool released after a batched run: SAIF counts and lengths kept
     // 64-bit event words: a stimulus time or a gate output past 2^30 - 2
     // (the pool, the stimulus staging and the level stacks hold 8 bytes per
-    // event; the window runs alone, through the thread-per-segment kernels)
+    // event; the window runs alone)
     bool w64 = false;
     uint64_t word_bytes() const { return w64 ? 8 : 4; }
 };

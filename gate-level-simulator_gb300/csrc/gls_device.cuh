@@ -323,25 +323,29 @@ template <> struct RelClampT<unsigned long long> {
         return min(max(x, lo), hi) - lo;
     }
 };
-// the word at q where `go`, else kInf, without a branch
-__device__ __forceinline__ uint32_t ld_if(const uint32_t *q, bool go)
-{
-    uint32_t v;
-    asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\tmov.u32 %0, 0xFFFFFFFF;\n\t@p ld.global.nc.u32 %0, [%1];\n\t}"
-        : "=r"(v) : "l"(q), "r"((uint32_t)go));
-    return v;
-}
+// the packed (relative time << 2 | value class) and the sums of a window's word type
+template <class Wd> using SaifP = typename std::conditional<std::is_same<Wd, uint32_t>::value, uint32_t,
+                                                            unsigned long long>::type;
 
 // Reader of one change list a word at a time: the head and the event after
-// it in registers, kInf behind the list's end.  Moving on is branch-free, so
+// it in registers, kInfW behind the list's end.  Moving on is branch-free, so
 // that lanes whose lists move at different steps stay together.  (More
-// events held ahead measured no faster: 79.6 ms of gate kernels with one and
-// with two for 2-input gates, 80.9 with three and two.)
-struct ListReader {
+// events held ahead measured no faster: moving a register waits for the load
+// that fills it.)
+template <class Wd> struct ListReader;
+template <>
+struct ListReader<uint32_t> {
     uint32_t h, n;
     const uint32_t *q;   // the event after n
     uint32_t qe;         // low word of the list's end (a list is shorter than 2^30 events)
 
+    static __device__ __forceinline__ uint32_t ld_if(const uint32_t *q, bool go)
+    {
+        uint32_t v;
+        asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\tmov.u32 %0, 0xFFFFFFFF;\n\t@p ld.global.nc.u32 %0, [%1];\n\t}"
+            : "=r"(v) : "l"(q), "r"((uint32_t)go));
+        return v;
+    }
     __device__ __forceinline__ void start(const uint32_t *x, uint32_t b, uint32_t len)
     {
         h = ld_if(x + b, b < len);
@@ -359,8 +363,37 @@ struct ListReader {
         q += more ? 1 : 0;
     }
 };
+template <>
+struct ListReader<WideWord> {   // a list of up to 2^32 events: its end is a whole address
+    WideWord h, n;
+    const WideWord *q, *qe;
 
-// The walk of one time segment of a gate output, 32-bit words: from the
+    static __device__ __forceinline__ WideWord ld_if(const WideWord *q, bool go)
+    {
+        WideWord v;
+        asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\tmov.u64 %0, -1;\n\t@p ld.global.nc.u64 %0, [%1];\n\t}"
+            : "=l"(v) : "l"(q), "r"((uint32_t)go));
+        return v;
+    }
+    __device__ __forceinline__ void start(const WideWord *x, uint32_t b, uint32_t len)
+    {
+        h = ld_if(x + b, b < len);
+        n = ld_if(x + b + 1, (uint64_t)b + 1 < len);
+        q = x + min((uint64_t)b + 2, (uint64_t)len);
+        qe = x + len;
+    }
+    __device__ __forceinline__ void advance(bool go)
+    {
+        const bool more = go && q != qe;
+        h = go ? n : h;
+        asm("{\n\t.reg .pred p, r;\n\tsetp.ne.u32 p, %2, 0;\n\tsetp.ne.u32 r, %3, 0;\n\t@p mov.u64 %0, -1;\n\t"
+            "@r ld.global.nc.u64 %0, [%1];\n\t}"
+            : "+l"(n) : "l"(q), "r"((uint32_t)go), "r"((uint32_t)more));
+        q += more ? 1 : 0;
+    }
+};
+
+// The walk of one time segment of a gate output: from the
 // segment's first event of every list (in rd, with the values before them in
 // curp; before: some list has one) to its end time tnext (kInf: the lists' end),
 // onto the stack ot.  tmax: no event of the segment is later.  Steps whose
@@ -391,10 +424,11 @@ struct ListReader {
 // then a step is one table read by the input state and the set of lists that
 // move, a third fewer instructions than the fast step, which reads values,
 // edges and delays for every list.
+template <class Wd>
 struct WalkOut {
     uint32_t cnt;    // entries on the stack
-    uint32_t minw;   // word of the smallest candidate time (kInf: no candidate)
-    uint32_t top;    // the stack's top entry (cnt > 0)
+    Wd minw;         // word of the smallest candidate time (kInfW: no candidate)
+    Wd top;          // the stack's top entry (cnt > 0)
     uint32_t xt;     // latest time an X or Z was pushed at (0: none but the first entry)
 };
 
@@ -434,17 +468,18 @@ __device__ __forceinline__ uint32_t lds32(uint32_t at)
 
 // kSm: the general step reads the gate output's tables from shared memory too;
 // kCall: delays of irregular arcs by a call.
-template <int M, bool kTab, bool kSm, bool kCall>
-__device__ __forceinline__ WalkOut walk_segment(const WinDev &w, const LevelArgs &a, uint32_t drv, uint32_t s,
-                                                ListReader (&rd)[M], uint32_t curp, bool before, uint32_t tnext,
-                                                uint32_t tmax, uint32_t *ot, uint32_t tab = 0, bool clean = false)
+template <int M, bool kTab, bool kSm, bool kCall, class Wd>
+__device__ __forceinline__ WalkOut<Wd> walk_segment(const WinDev &w, const LevelArgs &a, uint32_t drv, uint32_t s,
+                                                ListReader<Wd> (&rd)[M], uint32_t curp, bool before, uint32_t tnext,
+                                                uint32_t tmax, Wd *ot, uint32_t tab = 0, bool clean = false)
 {
     static_assert(!(kTab || kSm) || M <= 3, "the tables are for up to three input nets");
     constexpr bool kFast = M <= 3;
+    constexpr Wd kEnd = EvW<Wd>::kInfW;
     constexpr uint32_t kSlut = offsetof(GateTab, slut), kNd = offsetof(GateTab, nd);
     const DrvMeta *__restrict__ mdp = a.meta + drv;
     // words at or above tend lie behind the segment
-    const uint32_t tend = tnext != kInf ? tnext << 2 : kInf;
+    const Wd tend = tnext != kInf ? (Wd)tnext << 2 : kEnd;
     uint4 f0 = {0, 0, 0, 0}, f1 = {0, 0, 0, 0};
     if (kFast) {
         f0 = __ldg(a.fast + 2ull * drv);
@@ -455,16 +490,16 @@ __device__ __forceinline__ WalkOut walk_segment(const WinDev &w, const LevelArgs
     constexpr uint32_t kBits = 0x555u & ((1u << (2 * M)) - 1u);
     // a gate output without a usable FastRec, or times too close to the
     // largest one, take the general step throughout
-    const uint32_t never = (kFast && f1.w != 0u && tmax <= kMaxTime - 0x10000u) ? 0u : kBits;
+    const uint32_t never = (kFast && f1.w != 0u && tmax <= EvW<Wd>::kMax - 0x10000u) ? 0u : kBits;
     // input values are 2 bits per net; 0x15 bits of `mixed` mark nets at X or Z
     uint32_t mixed = ((curp ^ (curp >> 1)) & kBits) | never;
     // Every step consumes an event and pushes at most one entry, so a
     // segment's stack ends within the gate output's scratch.
     uint32_t cnt = 0;
-    // top of the stack and the entry below it (kInf: not at hand).  With no
+    // top of the stack and the entry below it (kEnd: not at hand).  With no
     // entry left the top reads as (0, X): below every later candidate, and
     // different from 0 and 1.
-    uint32_t top = EvW<uint32_t>::word(0, kVX), below = kInf;
+    Wd top = EvW<Wd>::word(0, kVX), below = kEnd;
     if (s == 0) { ot[0] = top; cnt = 1; }
     uint32_t fprev = kVX;
     auto out_of = [&](uint32_t x) -> uint32_t {   // the general step's truth table
@@ -474,18 +509,19 @@ __device__ __forceinline__ WalkOut walk_segment(const WinDev &w, const LevelArgs
     };
     if (before) fprev = out_of(curp);
     const bool regular = mdp->flags & kFlagRegular;
-    uint32_t minw = kInf, xt = 0;
+    Wd minw = kEnd;
+    uint32_t xt = 0;
     for (;;) {
-        uint32_t mk = rd[0].h | 3u;
+        Wd mk = rd[0].h | 3u;
 #pragma unroll
-        for (int j = 1; j < M; ++j) mk = min(mk, rd[j].h | 3u);
+        for (int j = 1; j < M; ++j) mk = min(mk, (Wd)(rd[j].h | 3u));
         if (mk >= tend || (kTab && clean)) break;
         const uint32_t lastp = curp;
         bool ch[M];
 #pragma unroll
         for (int j = 0; j < M; ++j) {
             ch[j] = (rd[j].h | 3u) == mk;
-            const uint32_t cj = (curp & ~(3u << (2 * j))) | ((rd[j].h << (2 * j)) & (3u << (2 * j)));
+            const uint32_t cj = (curp & ~(3u << (2 * j))) | (((uint32_t)rd[j].h << (2 * j)) & (3u << (2 * j)));
             curp = ch[j] ? cj : curp;
             rd[j].advance(ch[j]);
         }
@@ -501,7 +537,7 @@ __device__ __forceinline__ WalkOut walk_segment(const WinDev &w, const LevelArgs
             for (int j = 0; j < (M < 3 ? M : 3); ++j) r[j] = ch[j] ? ((fall & (1u << (2 * j))) ? dn[j] : dp[j]) : kInf;
             const uint32_t d2 = M == 1 ? r[0] : (M == 2 ? __vminu2(r[0], r[1]) : __vimin3_u16x2(r[0], r[1], r[2]));
             const uint32_t d = F ? (d2 & 0xFFFFu) : (d2 >> 16);
-            const uint32_t lo = (mk ^ 3u) + (d << 2);
+            const Wd lo = (mk ^ 3u) + (d << 2);
             minw = chg ? min(minw, lo) : minw;
             // inertial update, src/simulate.cpp:991-1009.  Both states of a
             // fast step are known, so it is not the first: lo > 0, and the
@@ -509,12 +545,12 @@ __device__ __forceinline__ WalkOut walk_segment(const WinDev &w, const LevelArgs
             if (chg && top >= lo) {
                 do {
                     --cnt;
-                    if (below != kInf) top = below;
-                    else top = cnt > 0 ? ot[cnt - 1] : EvW<uint32_t>::word(0, kVX);
-                    below = kInf;
+                    if (below != kEnd) top = below;
+                    else top = cnt > 0 ? ot[cnt - 1] : EvW<Wd>::word(0, kVX);
+                    below = kEnd;
                 } while (top >= lo);
             }
-            const bool push = chg && ((top ^ F) & 3u) != 0u;
+            const bool push = chg && (((uint32_t)top ^ F) & 3u) != 0u;
             if (push) ot[cnt] = lo | F;
             below = push ? top : below;
             top = push ? lo | F : top;
@@ -544,22 +580,22 @@ __device__ __forceinline__ WalkOut walk_segment(const WinDev &w, const LevelArgs
                         : select_delay(a.arcs + mdp->arc_off, mdp->n_arcs, chg, (int)so1 + 1, curp, lastp, a.def_delay);
         }
         const uint64_t o64 = (uint64_t)ev_time(mk) + d;
-        if (o64 > kMaxTime) { atomicOr(w.err, kErrTime); break; }
-        const uint32_t lo = (uint32_t)o64 << 2;
+        if (o64 > EvW<Wd>::kMax) { atomicOr(w.err, kErrTime); break; }
+        const Wd lo = (Wd)o64 << 2;
         minw = min(minw, lo);
         int popped_v = -1;
         while (cnt > 0 && top >= lo) {
             if (s == 0 && cnt == 1) { popped_v = (int)ev_val(top); cnt = 0; break; }
             --cnt;
-            top = cnt > 0 ? ot[cnt - 1] : EvW<uint32_t>::word(0, kVX);
-            below = kInf;
+            top = cnt > 0 ? ot[cnt - 1] : EvW<Wd>::word(0, kVX);
+            below = kEnd;
         }
         const int prevv = cnt > 0 ? (int)ev_val(top) : popped_v;
         if (prevv != (int)F) {
-            below = kInf;
+            below = kEnd;
             top = lo | F;
             ot[cnt++] = top;
-            if (F == kVX || F == kVZ) xt = lo >> 2;
+            if (F == kVX || F == kVZ) xt = (uint32_t)(lo >> 2);
         } else if (cnt == 0) {
             atomicOr(w.err, kErrEmptied);
             break;
@@ -571,9 +607,9 @@ __device__ __forceinline__ WalkOut walk_segment(const WinDev &w, const LevelArgs
 #pragma unroll
         for (int j = 0; j < M; ++j) so += ((curp >> (2 * j)) & 1u) << (2 + M + j);
         for (;;) {
-            uint32_t mk = rd[0].h | 3u;
+            Wd mk = rd[0].h | 3u;
 #pragma unroll
-            for (int j = 1; j < M; ++j) mk = min(mk, rd[j].h | 3u);
+            for (int j = 1; j < M; ++j) mk = min(mk, (Wd)(rd[j].h | 3u));
             if (mk >= tend) break;
             uint32_t x = so;
 #pragma unroll
@@ -585,17 +621,17 @@ __device__ __forceinline__ WalkOut walk_segment(const WinDev &w, const LevelArgs
             const uint32_t st = lds32(x);
             so ^= (x ^ so) << M;
             const bool chg = st != kInf;
-            const uint32_t nw = mk - 3u + st;   // the candidate's event word
+            const Wd nw = mk - 3u + st;   // the candidate's event word
             minw = chg ? min(minw, nw) : minw;
             if (chg && (top | 3u) >= nw) {   // times only: the bottom lies below every candidate
                 do {
                     --cnt;
-                    if (below != kInf) top = below;
-                    else top = cnt > 0 ? ot[cnt - 1] : EvW<uint32_t>::word(0, kVX);
-                    below = kInf;
+                    if (below != kEnd) top = below;
+                    else top = cnt > 0 ? ot[cnt - 1] : EvW<Wd>::word(0, kVX);
+                    below = kEnd;
                 } while ((top | 3u) >= nw);
             }
-            const bool put = chg && ((top ^ nw) & 3u) != 0u;
+            const bool put = chg && (((uint32_t)top ^ (uint32_t)nw) & 3u) != 0u;
             if (put) ot[cnt] = nw;
             below = put ? top : below;
             top = put ? nw : top;

@@ -1,4 +1,4 @@
-// k_gate: one level of gate outputs in one launch (32-bit event words).
+// k_gate: one level of gate outputs in one launch.
 //
 // A block takes one gate output at a time: it cuts its fan-in timeline into
 // one time segment per thread, walks them, links the segments' stacks, places
@@ -27,6 +27,8 @@ namespace gls {
 namespace {
 
 constexpr int kMaxWarps = kGateMaxThreads / 32;
+// threads per SM the narrow classes' kernel is compiled for
+template <class Wd> __host__ __device__ constexpr uint32_t gate_resident() { return sizeof(Wd) == 4 ? 1024u : 768u; }
 
 struct GateSmem {
     GateTab tab;                 // the gate output's tables
@@ -35,10 +37,10 @@ struct GateSmem {
     uint32_t q;                  // the block's gate output, kInf: none left
     uint32_t skip;               // its window has failed
     unsigned long long ctr[4];   // gate events, output events, segments, fan-in events of the window at hand
-    uint32_t wmin[kMaxWarps];    // smallest candidate of every warp's segments
+    WideWord wmin[kMaxWarps];    // smallest candidate of every warp's segments
     uint32_t wlast[kMaxWarps];   // value of the last kept entry of every warp's segments (4: none)
     uint32_t wsum[kMaxWarps];    // kept entries
-    uint32_t s0[kMaxWarps], s1[kMaxWarps];
+    WideWord s0[kMaxWarps], s1[kMaxWarps];
     unsigned long long scr, dst; // the gate output's stacks in the scratch, its list in the pool
     uint32_t ok;                 // the list has its place
     uint32_t xt;                 // latest X or Z of the list but its first entry
@@ -54,20 +56,22 @@ struct SegSmem {
 };
 
 // The thread's part of a gate output after the walk.
+template <class Wd>
 struct Walked {
-    WalkOut o;
+    WalkOut<Wd> o;
     uint32_t region;         // its stack among the gate output's
     uint32_t S;              // segments of the gate output
     unsigned long long E;    // fan-in events of the gate output
 };
 
 // Cut and walk gate output i of the level.
-template <int M, bool kTab>
-__device__ __forceinline__ Walked walk_gate(const WinDev &w, const LevelArgs &a, uint32_t i, GateSmem &sm,
+template <int M, bool kTab, class Wd>
+__device__ __forceinline__ Walked<Wd> walk_gate(const WinDev &w, const LevelArgs &a, uint32_t i, GateSmem &sm,
                                             const SegSmem &sg)
 {
     const uint32_t tid = threadIdx.x, nthr = blockDim.x;
     const uint32_t drv = a.lo + i;
+    const Wd *const pool = reinterpret_cast<const Wd *>(w.pool);
     const DrvMeta *__restrict__ mdp = a.meta + drv;
     constexpr bool kSm = kTab;
     uint4 f0 = {0, 0, 0, 0}, f1 = {0, 0, 0, 0};
@@ -126,7 +130,7 @@ __device__ __forceinline__ Walked walk_gate(const WinDev &w, const LevelArgs &a,
 #pragma unroll
     for (int j = 0; j < M; ++j) cb[j] = 0;
     if (mine && tid > 0)
-        tcut = cut_at<M, !kTab>(w.pool, off, len, m, piv, sec, poff, soff, plen, slen, sk, sn, cb);
+        tcut = cut_at<M, !kTab>(pool, off, len, m, piv, sec, poff, soff, plen, slen, sk, sn, cb);
     if (mine) sg.tcut[tid] = tcut;
     if constexpr (kTab) {
         if (usable)
@@ -140,16 +144,16 @@ __device__ __forceinline__ Walked walk_gate(const WinDev &w, const LevelArgs &a,
         if (!sm.ok) atomicOr(w.err, kErrScratch);
     }
     __syncthreads();
-    uint32_t *const scr = w.scratch + sm.scr;
+    Wd *const scr = reinterpret_cast<Wd *>(w.scratch) + sm.scr;
     uint32_t region = tid;
-    WalkOut o = {0, kInf, 0, 0};
+    WalkOut<Wd> o = {0, EvW<Wd>::kInfW, 0, 0};
     if (mine && sm.ok) {
         uint32_t curp = 0x555u & ((1u << (2 * M)) - 1u), tmax = 0;
         bool before = false;
-        ListReader rd[M];
+        ListReader<Wd> rd[M];
 #pragma unroll
         for (int j = 0; j < M; ++j) {
-            const uint32_t *x = w.pool + off[j];
+            const Wd *x = pool + off[j];
             region += cb[j];
             if (cb[j] > 0) {
                 curp = (curp & ~(3u << (2 * j))) | (ev_val(x[cb[j] - 1]) << (2 * j));
@@ -163,14 +167,14 @@ __device__ __forceinline__ Walked walk_gate(const WinDev &w, const LevelArgs &a,
         } else {
 #pragma unroll
             for (int j = 0; j < M; ++j)
-                if (len[j]) tmax = max(tmax, ev_time(w.pool[off[j] + len[j] - 1]));
+                if (len[j]) tmax = max(tmax, ev_time(pool[off[j] + len[j] - 1]));
         }
         // the step table serves a warp whose segments all start in known
         // values, behind every X, Z and repeat: lanes of both kinds would
         // walk one kind after the other
         bool clean = false;
         if constexpr (kTab) {
-            clean = usable && tmax <= kMaxTime - 0x10000u && tcut > xmax && ((curp ^ (curp >> 1)) & 0x15u) == 0u;
+            clean = usable && tmax <= EvW<Wd>::kMax - 0x10000u && tcut > xmax && ((curp ^ (curp >> 1)) & 0x15u) == 0u;
             clean = __all_sync(__activemask(), clean);
         }
         o = walk_segment<M, kTab, kSm, !kTab>(w, a, drv, tid, rd, curp, before, tnext, tmax, scr + region,
@@ -184,14 +188,14 @@ __device__ __forceinline__ Walked walk_gate(const WinDev &w, const LevelArgs &a,
 // fetch: thread 0 sets sm.q and sm.skip to the block's next gate output; called
 // where the wait for it overlaps others and every thread has read the present
 // one.
-template <class Fetch>
+template <class Wd, class Fetch>
 __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a, uint32_t i, GateSmem &sm,
-                                            const SegSmem &sg, const Walked &wk, Fetch fetch)
+                                            const SegSmem &sg, const Walked<Wd> &wk, Fetch fetch)
 {
     const unsigned FULL = 0xffffffffu;
     const uint32_t tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31u, wid = tid >> 5, nw = nthr >> 5;
     const DrvMeta *__restrict__ mdp = a.meta + a.lo + i;
-    const WalkOut &o = wk.o;
+    const WalkOut<Wd> &o = wk.o;
     const uint32_t region = wk.region, S = wk.S;
     const unsigned long long E = wk.E;
     const bool mine = tid < S;
@@ -200,23 +204,23 @@ __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a,
         if (tid == 0) fetch();
         return;
     }
-    uint32_t *const scr = w.scratch + sm.scr;
-    const uint32_t *ot = scr + region;
-    const uint32_t bottom = o.cnt ? ot[0] : 0u;   // on its way while the minima meet
+    Wd *const scr = reinterpret_cast<Wd *>(w.scratch) + sm.scr;
+    const Wd *ot = scr + region;
+    const Wd bottom = o.cnt ? ot[0] : Wd(0);   // on its way while the minima meet
     // later segments cut this one's stack at their smallest candidate
-    uint32_t x = o.minw;
+    Wd x = o.minw;
 #pragma unroll
     for (int k = 1; k < 32; k <<= 1) {
-        const uint32_t y = __shfl_down_sync(FULL, x, k);
+        const Wd y = __shfl_down_sync(FULL, x, k);
         if (lane + k < 32) x = min(x, y);
     }
     if (lane == 0) sm.wmin[wid] = x;
-    uint32_t later = __shfl_down_sync(FULL, x, 1);
-    if (lane == 31) later = kInf;
+    Wd later = __shfl_down_sync(FULL, x, 1);
+    if (lane == 31) later = EvW<Wd>::kInfW;
     __syncthreads();
-    for (uint32_t k = wid + 1; k < nw; ++k) later = min(later, sm.wmin[k]);
+    for (uint32_t k = wid + 1; k < nw; ++k) later = min(later, (Wd)sm.wmin[k]);
     uint32_t keep = o.cnt, firstv = 0, lastv = 0;
-    if (keep && later != kInf)
+    if (keep && later != EvW<Wd>::kInfW)
         while (keep && ((keep == o.cnt ? o.top : ot[keep - 1]) | 3u) >= later) --keep;
     if (keep) {
         firstv = ev_val(bottom);
@@ -300,9 +304,10 @@ __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a,
     // 74.4 on the 2 M cell design, 32.8 instead of 29.1 in waves.)
     constexpr uint32_t W = 8, U = 4;
     const uint32_t sub = tid & (W - 1);
-    const RelClampT<uint32_t> rc(w.t_begin, w.t_end);
-    uint32_t s0 = 0, s1 = 0;
-    uint32_t *const dst = w.pool + sm.dst;
+    using P = SaifP<Wd>;
+    const RelClampT<P> rc(w.t_begin, w.t_end);
+    P s0 = 0, s1 = 0;
+    Wd *const dst = reinterpret_cast<Wd *>(w.pool) + sm.dst;
     for (uint32_t b = wid * (32 / W); b < S; b += nthr / W) {   // a warp's four segments
         const uint32_t k = b + (lane / W);
         const uint32_t n = k < S ? sg.n[k] : 0u;
@@ -310,27 +315,28 @@ __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a,
         nmax = max(nmax, __shfl_xor_sync(FULL, nmax, 8));
         nmax = max(nmax, __shfl_xor_sync(FULL, nmax, 16));
         if (nmax == 0) continue;
-        const uint32_t *sp = scr + (k < S ? sg.src[k] : 0u);
-        uint32_t *dp = dst + (k < S ? sg.pos[k] : 0u);
+        const Wd *sp = scr + (k < S ? sg.src[k] : 0u);
+        Wd *dp = dst + (k < S ? sg.pos[k] : 0u);
         uint32_t pv = k < S ? sg.pv[k] : 0u;
         for (uint32_t e0 = 0; e0 < nmax; e0 += W * U) {
-            uint32_t wd[U];
+            Wd wd[U];
 #pragma unroll
             for (uint32_t u = 0; u < U; ++u) {
                 const uint32_t e = e0 + u * W + sub;
-                wd[u] = e < n ? sp[e] : 0u;
+                wd[u] = e < n ? sp[e] : Wd(0);
             }
 #pragma unroll
             for (uint32_t u = 0; u < U; ++u) {
                 const uint32_t e = e0 + u * W + sub;
-                uint32_t before = __shfl_up_sync(FULL, wd[u], 1, W);
+                uint32_t before = __shfl_up_sync(FULL, ev_val(wd[u]), 1, W);
                 if (sub == 0) before = pv;
-                pv = __shfl_sync(FULL, wd[u], W - 1, W);
+                pv = __shfl_sync(FULL, ev_val(wd[u]), W - 1, W);
                 if (e < n) {
                     dp[e] = wd[u];
-                    const uint32_t t = rc(ev_time(wd[u])), c = ev_val(wd[u]), p = ev_val(before);
-                    s0 += (p == kV0 ? t : 0u) - (c == kV0 ? t : 0u);
-                    s1 += (p == kV1 ? t : 0u) - (c == kV1 ? t : 0u);
+                    const P t = rc(ev_time(wd[u]));
+                    const uint32_t c = ev_val(wd[u]);
+                    s0 += (before == kV0 ? t : P(0)) - (c == kV0 ? t : P(0));
+                    s1 += (before == kV1 ? t : P(0)) - (c == kV1 ? t : P(0));
                 }
             }
         }
@@ -346,13 +352,14 @@ __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a,
         uint32_t last = kVX;
         s0 = s1 = 0;
         for (uint32_t k = 0; k < nw; ++k) {
-            s0 += sm.s0[k];
-            s1 += sm.s1[k];
+            s0 += (P)sm.s0[k];
+            s1 += (P)sm.s1[k];
             if (sm.wlast[k] < 4u) last = sm.wlast[k];
         }
+        using Sg = typename std::make_signed<P>::type;
         const unsigned long long D = w.t_end - w.t_begin;
-        const unsigned long long t0 = (unsigned long long)(long long)(int)s0 + (last == kV0 ? D : 0ull);
-        const unsigned long long t1 = (unsigned long long)(long long)(int)s1 + (last == kV1 ? D : 0ull);
+        const unsigned long long t0 = (unsigned long long)(long long)(Sg)s0 + (last == kV0 ? D : 0ull);
+        const unsigned long long t1 = (unsigned long long)(long long)(Sg)s1 + (last == kV1 ? D : 0ull);
         unsigned long long *sf = w.saif + 3ull * mdp->out_net;
         sf[0] = t0;
         sf[1] = t1;
@@ -373,8 +380,8 @@ __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a,
 // class of four to six input nets, else the narrower ones; c1, c2: where the
 // 2- and 3-input ones start).  Blocks take gate outputs from the back, the
 // widest first, as they become free.
-template <bool kBatch, bool kSix, bool kTab>
-__global__ void __launch_bounds__(kGateMaxThreads, kSix ? 1 : 1024 / kGateMaxThreads)
+template <bool kBatch, bool kSix, bool kTab, class Wd>
+__global__ void __launch_bounds__(kGateMaxThreads, kSix ? 1 : gate_resident<Wd>() / kGateMaxThreads)
     k_gate(const WinSet<kBatch> ws, LevelArgs a, uint32_t d0, uint32_t d1, uint32_t c1, uint32_t c2)
 {
     __shared__ GateSmem sm;
@@ -431,13 +438,13 @@ __global__ void __launch_bounds__(kGateMaxThreads, kSix ? 1 : 1024 / kGateMaxThr
         }
         const uint32_t i = d1 - 1 - (kBatch ? q - win * n : q);
         auto go = [&](const WinDev &w) {
-            Walked wk;
+            Walked<Wd> wk;
             if constexpr (kSix) {
-                wk = walk_gate<kMaxSlots, false>(w, a, i, sm, sg);
+                wk = walk_gate<kMaxSlots, false, Wd>(w, a, i, sm, sg);
             } else {
-                if (i >= c2) wk = walk_gate<3, kTab>(w, a, i, sm, sg);
-                else if (i >= c1) wk = walk_gate<2, kTab>(w, a, i, sm, sg);
-                else wk = walk_gate<1, kTab>(w, a, i, sm, sg);
+                if (i >= c2) wk = walk_gate<3, kTab, Wd>(w, a, i, sm, sg);
+                else if (i >= c1) wk = walk_gate<2, kTab, Wd>(w, a, i, sm, sg);
+                else wk = walk_gate<1, kTab, Wd>(w, a, i, sm, sg);
             }
             finish_gate(w, a, i, sm, sg, wk, next);
         };
@@ -455,7 +462,8 @@ void launch_gate(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelAr
         constexpr bool kSix = decltype(six)::value, kTab = decltype(tab)::value;
         if (d1 <= d0) return;
         const uint64_t total = (uint64_t)(d1 - d0) * nwin;
-        const uint64_t room = (uint64_t)sm_count * ((kSix ? kGateMaxThreads : 1024) / threads);
+        const uint64_t room =
+            (uint64_t)sm_count * ((kSix ? kGateMaxThreads : (a.wide ? gate_resident<WideWord>() : gate_resident<uint32_t>())) / threads);
         const uint32_t grid = (uint32_t)(total < room ? total : room);
         cudaLaunchAttribute at;
         at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -467,10 +475,12 @@ void launch_gate(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelAr
         lc.stream = st;
         lc.attrs = &at;
         lc.numAttrs = 1;
-        if (nwin == 1)
-            cudaLaunchKernelEx(&lc, k_gate<false, kSix, kTab>, WinSet<false>{h}, a, d0, d1, cls[1], cls[2]);
+        if (a.wide)   // one window per launch
+            cudaLaunchKernelEx(&lc, k_gate<false, kSix, kTab, WideWord>, WinSet<false>{h}, a, d0, d1, cls[1], cls[2]);
+        else if (nwin == 1)
+            cudaLaunchKernelEx(&lc, k_gate<false, kSix, kTab, uint32_t>, WinSet<false>{h}, a, d0, d1, cls[1], cls[2]);
         else
-            cudaLaunchKernelEx(&lc, k_gate<true, kSix, kTab>, WinSet<true>{dw, nwin}, a, d0, d1, cls[1], cls[2]);
+            cudaLaunchKernelEx(&lc, k_gate<true, kSix, kTab, uint32_t>, WinSet<true>{dw, nwin}, a, d0, d1, cls[1], cls[2]);
         ++*launches;
     };
     using T = std::integral_constant<bool, true>;

@@ -147,7 +147,6 @@ struct SegRecT {            // one time segment of one gate output
     Wd last;                // the stack's top entry (when cnt > 0): linking reads no scratch for it
 };
 using SegRec = SegRecT<uint32_t>;
-constexpr size_t kSegRecMax = sizeof(SegRecT<WideWord>);   // table entries are sized for either word
 
 struct CopyRec {            // what k_copy does for one segment
     uint64_t src;           // scratch index of the first kept entry
@@ -242,7 +241,7 @@ void launch_link(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelAr
 void launch_copy(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelArgs &a, uint32_t d0, uint32_t d1,
                  int sm_count, cudaStream_t st);
 
-// One level in one launch (32-bit words; a second one where gate outputs with
+// One level in one launch (a second one where gate outputs with
 // four to six input nets exist).  cls: the level's fan-in class starts
 // (kClasses + 1); threads per block: 32 .. kGateMaxThreads, a power of two.
 constexpr uint32_t kGateMaxThreads = 256;

@@ -355,7 +355,7 @@ __device__ __forceinline__ uint32_t sel4(const uint4 &q, uint32_t k)
 // the blocks, each balancing its segments over twice the warps).  Variants
 // with bit kSimVWide read twice the events per load (4 for 1- and 2-input
 // gates, 2 for wider ones: fewer loads, more registers).  The autotuner picks
-// the variant; 64-bit windows always run variant 0.
+// the variant.
 constexpr uint32_t kSimBlock = 128;
 constexpr int kSimV256 = 1, kSimVWide = 2;
 template <int kV, int M> __host__ __device__ constexpr uint32_t sim_block()
@@ -454,42 +454,13 @@ struct Reader<1> {
     }
 };
 
-// The same one-event reader for 64-bit words (windows with times past
-// 2^30 - 2); EvW<WideWord>::kInfW once exhausted.
-struct ReaderWide {
-    using C = WideWord;
-    const WideWord *q;
-    uint32_t left;
-    WideWord nt;
-
-    __device__ __forceinline__ WideWord first(const C *__restrict__ P, uint64_t off, uint32_t p0, uint32_t e0)
-    {
-        left = 0;
-        if (p0 >= e0) return EvW<WideWord>::kInfW;
-        const WideWord *x = P + off + p0;
-        const WideWord h = __ldg(x);
-        left = e0 - p0 - 1;
-        if (left) nt = __ldg(x + 1);
-        q = x + 2;
-        return h;
-    }
-    __device__ __forceinline__ WideWord next(const C *__restrict__)
-    {
-        if (!left) return EvW<WideWord>::kInfW;
-        const WideWord h = nt;
-        if (--left) nt = __ldg(q++);
-        return h;
-    }
-};
-
 template <int M, class Wd, bool kWideChunk>
 __device__ void sim_segment(const WinDev &w, const LevelArgs &a, const DrvMeta &md, uint32_t s,
                             uint32_t S, uint32_t seg_id, uint64_t scr, const uint4 sl)
 {
     constexpr bool kSlut = M <= 3;   // truth table in registers
     constexpr int kRW = (M >= 3 ? GLS_READER_W3 : GLS_READER_W2) * (kWideChunk ? 2 : 1);   // events per reader chunk
-    // 64-bit words (a window with times past 2^30 - 2) are read one at a time
-    using RD = typename std::conditional<std::is_same<Wd, uint32_t>::value, Reader<kRW>, ReaderWide>::type;
+    using RD = Reader<kRW>;
     using RC = typename RD::C;
     const RC *P = reinterpret_cast<const RC *>(w.pool);
     const Wd *pw = reinterpret_cast<const Wd *>(w.pool);
@@ -639,7 +610,7 @@ __device__ __forceinline__ void sim_segment2(const WinDev &w, const LevelArgs &a
     for (int j = 0; j < M; ++j) region += cb[j];
     uint32_t curp = 0x555u & ((1u << (2 * M)) - 1u), tmax = 0;
     bool before = false;
-    ListReader rd[M];
+    ListReader<uint32_t> rd[M];
 #pragma unroll
     for (int j = 0; j < M; ++j) {
         const uint32_t *x = pw + off[j];
@@ -651,7 +622,7 @@ __device__ __forceinline__ void sim_segment2(const WinDev &w, const LevelArgs &a
         rd[j].start(x, cb[j], len[j]);
     }
     if (tnext != kInf) tmax = tnext;
-    const WalkOut o = walk_segment<M, false, false, false>(w, a, drv, s, rd, curp, before, tnext, tmax,
+    const WalkOut<uint32_t> o = walk_segment<M, false, false, false>(w, a, drv, s, rd, curp, before, tnext, tmax,
                                                     w.scratch + scr + region);
     SegRec r;
     r.region = region; r.cnt = o.cnt; r.min_o = o.minw == kInf ? kInf : o.minw >> 2; r.last = o.top;
@@ -1430,9 +1401,6 @@ __global__ void __launch_bounds__(256, GLS_LINK_BLOCKS) k_link(const WinSet<kBat
     }
 }
 
-// the packed (relative time << 2 | value class) and the sums of a window's word type
-template <class Wd> using SaifP = typename std::conditional<std::is_same<Wd, uint32_t>::value, uint32_t,
-                                                            unsigned long long>::type;
 
 template <class P>
 __device__ __forceinline__ void saif_add32(P acc[3], P cls, P d)
@@ -1637,8 +1605,8 @@ __global__ void __launch_bounds__(256) k_stim_saif(const WinSet<kBatch> ws, uint
         }                                                        \
     } while (0)
 
-// Windows of 64-bit event words (times past 2^30 - 2) run one at a time
-// through the thread-per-segment kernels: the host never batches them.
+// Windows of 64-bit event words (times past 2^30 - 2) run one at a time, their
+// levels through k_gate: the host never batches them.
 void launch_stim_saif(const WinDev *dw, const WinDev &h, uint32_t nwin, uint32_t max_stim, bool wide, uint32_t n_nets,
                       cudaStream_t st)
 {
@@ -1708,10 +1676,6 @@ static void sim_kernels(const WS &ws, const LevelArgs &a, int cls, uint32_t d0, 
 void launch_sim(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelArgs &a, int cls, uint32_t d0, uint32_t d1,
                 int sm_count, cudaStream_t st)
 {
-    if (a.wide) {
-        sim_kernels<WideWord>(WinSet<false>{h}, a, cls, d0, d1, sm_count, st);
-        return;
-    }
     GLS_DISPATCH(h, dw, nwin, sim_kernels<uint32_t>(ws, a, cls, d0, d1, sm_count, st));
 }
 
@@ -1721,10 +1685,6 @@ void launch_link(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelAr
     const uint64_t warps = (uint64_t)(d1 - d0) * nwin;
     if (!warps) return;
     const uint32_t blocks = (uint32_t)((warps * 32 + 255) / 256);
-    if (a.wide) {
-        k_link<false, WideWord><<<blocks, 256, 0, st>>>(WinSet<false>{h}, a, d0, d1);
-        return;
-    }
     GLS_DISPATCH(h, dw, nwin, (k_link<decltype(ws)::kIsBatch, uint32_t><<<blocks, 256, 0, st>>>(ws, a, d0, d1)));
 }
 
@@ -1732,10 +1692,6 @@ void launch_copy(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelAr
                  int sm_count, cudaStream_t st)
 {
     const int grid = sm_count * 8;
-    if (a.wide) {   // 8 lanes move 64 bytes a step, as 16 lanes of 32-bit words do
-        k_copy<false, 8, WideWord><<<grid, 256, 0, st>>>(WinSet<false>{h}, a, d0, d1);
-        return;
-    }
     if (a.copy_lanes == 4) GLS_DISPATCH(h, dw, nwin, (k_copy<decltype(ws)::kIsBatch, 4, uint32_t><<<grid, 256, 0, st>>>(ws, a, d0, d1)));
     else if (a.copy_lanes == 8) GLS_DISPATCH(h, dw, nwin, (k_copy<decltype(ws)::kIsBatch, 8, uint32_t><<<grid, 256, 0, st>>>(ws, a, d0, d1)));
     else if (a.copy_lanes == 32) GLS_DISPATCH(h, dw, nwin, (k_copy<decltype(ws)::kIsBatch, 32, uint32_t><<<grid, 256, 0, st>>>(ws, a, d0, d1)));
