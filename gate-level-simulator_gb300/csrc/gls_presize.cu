@@ -366,159 +366,250 @@ void launch_presize(const PresizeArgs &a, bool tensor_cores, cudaStream_t st)
 }
 
 // ------------------------------------------------------------- training
-// C(i, j) = sum_k A(i, k) B(k, j) with A(i, k) = A[i * as0 + k * as1],
-// B(k, j) = B[k * bs0 + j * bs1] and row stride cs for C.  64 x 64 tiles,
-// 256 threads with 4 x 4 outputs each.  With several K splits
-// (gridDim.z) the partial sums are added into C with atomics (C cleared
-// first).  Epilogues: kEpiStore; kEpiBiasRelu stores z = acc + bias[j] in C
-// and max(z, 0) in C2; kEpiMask stores acc where mask(i, j) > 0, else 0.
-constexpr int kEpiStore = 0, kEpiBiasRelu = 1, kEpiMask = 2;
+// k_mlp_grad: loss and gradient over a minibatch in one launch.  A block takes
+// 64 rows at a time and keeps the weights and the rows' activations in shared
+// memory: both forward layers, the loss, and the backward products; its parts
+// of the weight gradients stay in registers over all its rows and reach the
+// gradient (cleared before) by one round of atomics.
+//
+// What bounds it: FP32 arithmetic, 114 kFLOP a row (8,192 rows: 14 us at the
+// peak rate).  Fifteen launches over activations in HBM, with 4 x 4 outputs a
+// thread, took 430 us a call.  Eight warps of eight rows each: a warp's lanes
+// share the row operand (broadcast reads), 4 columns a lane make 32 FMAs for
+// every three 16-byte reads; row strides of 4 more floats than a multiple of
+// 32 keep the 16-byte reads down a column free of bank conflicts.
+constexpr int kRows = 64;
+constexpr int kCopies = 8, kCopy = kParams + 1;   // a copy: the gradient and the loss sum
+constexpr int kLdX = kIn + 4, kLdH = kHid + 4;
+struct GradSmem {
+    float w1[kHid * kLdX], w2[kHid * kLdH];
+    float x[kRows * kLdX];
+    float h[kRows * kLdH];   // hidden layer 1, then its gradient
+    float d[kRows * kLdH];   // gradient at hidden layer 2
+};
 
-template <int EPI>
-__global__ void __launch_bounds__(256) k_gemm(int M, int N, int K, int kchunk, const float *__restrict__ A, long as0,
-                                              long as1, const float *__restrict__ B, long bs0, long bs1,
-                                              float *__restrict__ C, long cs, const float *__restrict__ bias,
-                                              const float *__restrict__ mask, float *__restrict__ C2)
+__device__ __forceinline__ float4 ld4(const float *p) { return *reinterpret_cast<const float4 *>(p); }
+__device__ __forceinline__ void fma4(float &acc, const float4 &a, const float4 &b)
 {
-    __shared__ float As[16][65], Bs[16][65];
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    const int i0 = blockIdx.y * 64, j0 = blockIdx.x * 64;
-    const int k0 = blockIdx.z * kchunk, k1 = min(K, k0 + kchunk);
-    float acc[4][4];
+    acc = fmaf(a.x, b.x, acc);
+    acc = fmaf(a.y, b.y, acc);
+    acc = fmaf(a.z, b.z, acc);
+    acc = fmaf(a.w, b.w, acc);
+}
+
+// rows first .. first + nb - 1 of the data, or (mul != 0) rows (mul * (first + i) + add) mod n
+__global__ void __launch_bounds__(256, 1) k_mlp_grad(int nb, uint64_t first, uint64_t mul, uint64_t add, uint64_t n,
+                                                     const float *__restrict__ X, const float *__restrict__ T,
+                                                     const float *__restrict__ P, float huber, float scale,
+                                                     float *__restrict__ G)
+{
+    extern __shared__ __align__(16) unsigned char s_raw[];
+    GradSmem &sm = *reinterpret_cast<GradSmem *>(s_raw);
+    const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5, r0 = ty * 8;
+    G += (blockIdx.x % kCopies) * kCopy;
+    for (int q = tid; q < kHid * kIn; q += 256) sm.w1[(q / kIn) * kLdX + q % kIn] = P[kOffW1 + q];
+    for (int q = tid; q < kHid * kHid; q += 256) sm.w2[(q / kHid) * kLdH + q % kHid] = P[kOffW2 + q];
+    float b1[4], b2[4], w3[4];   // columns tx + 32 c
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] = 0.f;
-    for (int kb = k0; kb < k1; kb += 16) {
-        for (int q = threadIdx.x; q < 1024; q += 256) {
-            const int ii = q >> 4, kk = q & 15, gi = i0 + ii, gk = kb + kk;
-            As[kk][ii] = (gi < M && gk < k1) ? A[(long)gi * as0 + (long)gk * as1] : 0.f;
-        }
-        for (int q = threadIdx.x; q < 1024; q += 256) {
-            const int kk = q >> 6, jj = q & 63, gk = kb + kk, gj = j0 + jj;
-            Bs[kk][jj] = (gk < k1 && gj < N) ? B[(long)gk * bs0 + (long)gj * bs1] : 0.f;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < 16; ++kk) {
-            float av[4], bv[4];
-#pragma unroll
-            for (int r = 0; r < 4; ++r) av[r] = As[kk][ty * 4 + r];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) bv[c] = Bs[kk][tx * 4 + c];
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(av[r], bv[c], acc[r][c]);
-        }
-        __syncthreads();
+    for (int c = 0; c < 4; ++c) {
+        b1[c] = P[kOffB1 + tx + 32 * c];
+        b2[c] = P[kOffB2 + tx + 32 * c];
+        w3[c] = P[kOffW3 + tx + 32 * c];
     }
+    const float b3 = P[kOffB3];
+    // this thread's part of the gradient: w2 rows u0 .. u0 + 7, columns k0 and
+    // 64 + k0 (4 each); w1 rows j0, columns x0 (4 each)
+    const int u0 = (tid >> 4) * 8, k0 = (tid & 15) * 4, j0 = (tid >> 3) * 4, x0 = (tid & 7) * 4;
+    float gw2[8][8] = {}, gw1[4][4] = {}, gw3[4] = {}, gb2[4] = {}, gb1[4] = {}, gb3 = 0.f, ls = 0.f;
+    const int tiles = (nb + kRows - 1) / kRows;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        __syncthreads();   // the weights are there; the tile before is done with x and h
+        const int base = tile * kRows;
+        for (int q = tid; q < kRows * kIn; q += 256) {
+            const int i = q / kIn, k = q % kIn;
+            float v = 0.f;
+            if (base + i < nb) {
+                const uint64_t at = first + base + i;
+                const uint64_t row = mul ? (uint64_t)(((unsigned __int128)mul * at + add) % n) : at;
+                v = X[row * kIn + k];
+            }
+            sm.x[i * kLdX + k] = v;
+        }
+        float t = 0.f;   // lanes 0 .. 7: the target of row r0 + lane
+        if (tx < 8 && base + r0 + tx < nb) {
+            const uint64_t at = first + base + r0 + tx;
+            t = T[mul ? (uint64_t)(((unsigned __int128)mul * at + add) % n) : at];
+        }
+        __syncthreads();
+        // forward, layer 1: rows r0 .. r0 + 7, columns tx + 32 c
+        float acc[8][4] = {};
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-        const int gi = i0 + ty * 4 + r;
-        if (gi >= M) continue;
+        for (int k = 0; k < kIn; k += 4) {
+            float4 bv[4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int gj = j0 + tx * 4 + c;
-            if (gj >= N) continue;
-            float *dst = C + (long)gi * cs + gj;
-            if (EPI == kEpiStore) {
-                if (gridDim.z > 1) atomicAdd(dst, acc[r][c]);
-                else *dst = acc[r][c];
-            } else if (EPI == kEpiBiasRelu) {
-                const float z = acc[r][c] + bias[gj];
-                *dst = z;
-                C2[(long)gi * cs + gj] = fmaxf(z, 0.f);
-            } else {
-                *dst = mask[(long)gi * cs + gj] > 0.f ? acc[r][c] : 0.f;
+            for (int c = 0; c < 4; ++c) bv[c] = ld4(&sm.w1[(tx + 32 * c) * kLdX + k]);
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const float4 av = ld4(&sm.x[(r0 + r) * kLdX + k]);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) fma4(acc[r][c], av, bv[c]);
             }
         }
-    }
-}
-
-// y[i] = b + sum_j H[i][j] w[j] (one warp per row)
-__global__ void __launch_bounds__(256) k_rowdot(int n, const float *__restrict__ H, const float *__restrict__ w,
-                                                const float *__restrict__ b, float *__restrict__ y)
-{
-    const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (row >= n) return;
-    float s = 0.f;
-    for (int j = lane; j < kHid; j += 32) s = fmaf(H[(long)row * kHid + j], w[j], s);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) y[row] = s + b[0];
-}
-
-// Huber loss on r = y - t: dy = scale * dloss/dy; the loss sum is added to *sum
-__global__ void __launch_bounds__(256) k_loss(int n, const float *__restrict__ y, const float *__restrict__ t,
-                                              float huber, float scale, float *__restrict__ dy, float *sum)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    float l = 0.f;
-    if (i < n) {
-        const float r = y[i] - t[i], ab = fabsf(r);
-        const bool in = ab <= huber;
-        l = in ? 0.5f * r * r : huber * (ab - 0.5f * huber);
-        dy[i] = scale * (in ? r : copysignf(huber, r));
+        for (int r = 0; r < 8; ++r)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                sm.h[(r0 + r) * kLdH + tx + 32 * c] = fmaxf(acc[r][c] + b1[c], 0.f);
+                acc[r][c] = 0.f;
+            }
+        __syncwarp();   // a warp reads its own rows only
+        // layer 2
+#pragma unroll 2
+        for (int k = 0; k < kHid; k += 4) {
+            float4 bv[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) bv[c] = ld4(&sm.w2[(tx + 32 * c) * kLdH + k]);
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const float4 av = ld4(&sm.h[(r0 + r) * kLdH + k]);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) fma4(acc[r][c], av, bv[c]);
+            }
+        }
+        // output, loss and the gradient at layer 2
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            float y = 0.f;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                acc[r][c] += b2[c];
+                y = fmaf(fmaxf(acc[r][c], 0.f), w3[c], y);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+            const float res = y + b3 - __shfl_sync(0xffffffffu, t, r), ab = fabsf(res);
+            const bool in = ab <= huber, valid = base + r0 + r < nb;
+            const float dy = valid ? scale * (in ? res : copysignf(huber, res)) : 0.f;
+            if (valid && tx == 0) {
+                ls += in ? 0.5f * res * res : huber * (ab - 0.5f * huber);
+                gb3 += dy;
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const float z = acc[r][c], dz = z > 0.f ? dy * w3[c] : 0.f;
+                gw3[c] = fmaf(fmaxf(z, 0.f), dy, gw3[c]);
+                gb2[c] += dz;
+                sm.d[(r0 + r) * kLdH + tx + 32 * c] = dz;
+                acc[r][c] = 0.f;
+            }
+        }
+        __syncthreads();
+        // gradient at layer 1: rows r0 .. r0 + 7, columns 4 tx + c
+#pragma unroll 2
+        for (int u = 0; u < kHid; u += 4) {
+            float4 bv[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) bv[q] = ld4(&sm.w2[(u + q) * kLdH + 4 * tx]);
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                const float4 av = ld4(&sm.d[(r0 + r) * kLdH + u]);
+                const float a4[4] = {av.x, av.y, av.z, av.w};
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    acc[r][0] = fmaf(a4[q], bv[q].x, acc[r][0]);
+                    acc[r][1] = fmaf(a4[q], bv[q].y, acc[r][1]);
+                    acc[r][2] = fmaf(a4[q], bv[q].z, acc[r][2]);
+                    acc[r][3] = fmaf(a4[q], bv[q].w, acc[r][3]);
+                }
+            }
+        }
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const float4 h = ld4(&sm.h[(r0 + r) * kLdH + 4 * tx]);
+            acc[r][0] = h.x > 0.f ? acc[r][0] : 0.f;
+            acc[r][1] = h.y > 0.f ? acc[r][1] : 0.f;
+            acc[r][2] = h.z > 0.f ? acc[r][2] : 0.f;
+            acc[r][3] = h.w > 0.f ? acc[r][3] : 0.f;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) gb1[c] += acc[r][c];
+        }
+        // weight gradient of layer 2
+#pragma unroll 2
+        for (int i = 0; i < kRows; ++i) {
+            const float4 da = ld4(&sm.d[i * kLdH + u0]), db = ld4(&sm.d[i * kLdH + u0 + 4]);
+            const float4 ha = ld4(&sm.h[i * kLdH + k0]), hb = ld4(&sm.h[i * kLdH + 64 + k0]);
+            const float dv[8] = {da.x, da.y, da.z, da.w, db.x, db.y, db.z, db.w};
+            const float hv[8] = {ha.x, ha.y, ha.z, ha.w, hb.x, hb.y, hb.z, hb.w};
+#pragma unroll
+            for (int p = 0; p < 8; ++p)
+#pragma unroll
+                for (int q = 0; q < 8; ++q) gw2[p][q] = fmaf(dv[p], hv[q], gw2[p][q]);
+        }
+        __syncthreads();   // hidden layer 1 is read
+#pragma unroll
+        for (int r = 0; r < 8; ++r)
+            *reinterpret_cast<float4 *>(&sm.h[(r0 + r) * kLdH + 4 * tx]) =
+                make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+        __syncthreads();
+        // weight gradient of layer 1
+#pragma unroll 4
+        for (int i = 0; i < kRows; ++i) {
+            const float4 d = ld4(&sm.h[i * kLdH + j0]), v = ld4(&sm.x[i * kLdX + x0]);
+            const float dv[4] = {d.x, d.y, d.z, d.w}, xv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int p = 0; p < 4; ++p)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) gw1[p][q] = fmaf(dv[p], xv[q], gw1[p][q]);
+        }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    __shared__ float ws[8];
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = l;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        float s = 0.f;
-        for (int k = 0; k < (int)(blockDim.x >> 5); ++k) s += ws[k];
-        atomicAdd(sum, s);
+    for (int p = 0; p < 8; ++p)
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            atomicAdd(G + kOffW2 + (u0 + p) * kHid + (q < 4 ? k0 + q : 60 + k0 + q), gw2[p][q]);
+#pragma unroll
+    for (int p = 0; p < 4; ++p)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) atomicAdd(G + kOffW1 + (j0 + p) * kIn + x0 + q, gw1[p][q]);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        atomicAdd(G + kOffW3 + tx + 32 * c, gw3[c]);
+        atomicAdd(G + kOffB2 + tx + 32 * c, gb2[c]);
+        atomicAdd(G + kOffB1 + 4 * tx + c, gb1[c]);
+    }
+    if (tx == 0) {
+        atomicAdd(G + kOffB3, gb3);
+        atomicAdd(G + kParams, ls);
     }
 }
 
-// dZ2[i][j] = dy[i] w3[j] where Z2[i][j] > 0, else 0
-__global__ void __launch_bounds__(256) k_dz2(int n, const float *__restrict__ dy, const float *__restrict__ w3,
-                                             const float *__restrict__ Z2, float *__restrict__ dZ2)
+__device__ __forceinline__ float sum_copies(const float *__restrict__ g, int k)
 {
-    const long q = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= (long)n * kHid) return;
-    const int i = (int)(q / kHid), j = (int)(q % kHid);
-    dZ2[q] = Z2[q] > 0.f ? dy[i] * w3[j] : 0.f;
+    double s = 0.0;
+#pragma unroll
+    for (int c = 0; c < kCopies; ++c) s += g[c * kCopy + k];
+    return (float)s;
 }
 
-// out[j] += sum_i D[i][j] (wt ? wt[i] : 1) over a block's rows
-__global__ void __launch_bounds__(256) k_colsum(int n, int N, const float *__restrict__ D,
-                                                const float *__restrict__ wt, float *__restrict__ out)
-{
-    const int j = threadIdx.x % N, rows_per = blockDim.x / N, sub = threadIdx.x / N;
-    if (sub >= rows_per) return;
-    const int chunk = (n + gridDim.x - 1) / gridDim.x, i0 = blockIdx.x * chunk, i1 = min(n, i0 + chunk);
-    float s = 0.f;
-    for (int i = i0 + sub; i < i1; i += rows_per) s += D[(long)i * N + j] * (wt ? wt[i] : 1.f);
-    atomicAdd(out + j, s);
-}
-
-__global__ void __launch_bounds__(256) k_adam(int P, float *__restrict__ p, const float *__restrict__ g,
-                                              float *__restrict__ m, float *__restrict__ v, float lr, float c1,
-                                              float c2)
+__global__ void __launch_bounds__(256) k_sum_copies(const float *__restrict__ g, float *__restrict__ out)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < kCopy) out[k] = sum_copies(g, k);
+}
+
+// loss: the epoch's loss sum, which the minibatch's is added to
+__global__ void __launch_bounds__(256) k_adam(int P, float *__restrict__ p, const float *__restrict__ g,
+                                              float *__restrict__ m, float *__restrict__ v, float lr, float c1,
+                                              float c2, double *loss)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k == P) *loss += (double)sum_copies(g, P);
     if (k >= P) return;
-    const float gk = g[k];
+    const float gk = sum_copies(g, k);
     const float mk = 0.9f * m[k] + 0.1f * gk, vk = 0.999f * v[k] + 0.001f * gk * gk;
     m[k] = mk;
     v[k] = vk;
     p[k] -= lr * (mk * c1) / (sqrtf(vk * c2) + 1e-8f);
-}
-
-// batch row i = data row (mul * (base + i) + add) mod n (a permutation when gcd(mul, n) = 1)
-__global__ void __launch_bounds__(256) k_gather(int nb, uint64_t base, uint64_t mul, uint64_t add, uint64_t n,
-                                                const float *__restrict__ X, const float *__restrict__ T,
-                                                float *__restrict__ Xb, float *__restrict__ Tb)
-{
-    const long q = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= (long)nb * kIn) return;
-    const int i = (int)(q / kIn), k = (int)(q % kIn);
-    const uint64_t src = (uint64_t)(((unsigned __int128)mul * (base + i) + add) % n);
-    Xb[q] = X[src * kIn + k];
-    if (k == 0) Tb[i] = T[src];
 }
 
 }  // namespace gls
@@ -575,63 +666,22 @@ struct gls_trainer {
     cudaStream_t st = nullptr;
     std::string err;
     uint64_t n = 0, seed = 0, adam_t = 0;
-    uint32_t cap_batch = 0;
-    DevBuf X, T, Xb, Tb, Z1, H1, Z2, H2, Y, DY, DZ2, DZ1, P, G, Mo, Vo, loss;
+    int sm_count = 1;
+    DevBuf X, T, P, G, Mo, Vo;
+    PinBuf host;
+    DevBuf sum;   // an epoch's loss sum; a gradient's entries and loss
 };
 
 namespace {
 
-int tr_alloc_batch(gls_trainer *tr, uint32_t nb)
+// Loss sum and gradient over nb rows (see k_mlp_grad) into the copies of G
+void tr_step_grad(gls_trainer *tr, int nb, uint64_t first, uint64_t mul, uint64_t add, float huber)
 {
-    if (nb <= tr->cap_batch) return GLS_OK;
-    const size_t h = (size_t)nb * kHid * 4;
-    cudaError_t e = cudaSuccess;
-    DevBuf *hb[] = {&tr->Z1, &tr->H1, &tr->Z2, &tr->H2, &tr->DZ2, &tr->DZ1};
-    for (DevBuf *b : hb)
-        if (e == cudaSuccess) e = b->ensure(h);
-    if (e == cudaSuccess) e = tr->Xb.ensure((size_t)nb * kIn * 4);
-    if (e == cudaSuccess) e = tr->Tb.ensure((size_t)nb * 4);
-    if (e == cudaSuccess) e = tr->Y.ensure((size_t)nb * 4);
-    if (e == cudaSuccess) e = tr->DY.ensure((size_t)nb * 4);
-    if (e != cudaSuccess) return setf(&tr->err, GLS_ENOMEM, "trainer batch buffers", e);
-    tr->cap_batch = nb;
-    return GLS_OK;
-}
-
-template <int EPI>
-void gemm(cudaStream_t st, int M, int N, int K, const float *A, long as0, long as1, const float *B, long bs0, long bs1,
-          float *C, long cs, const float *bias = nullptr, const float *mask = nullptr, float *C2 = nullptr)
-{
-    int splits = 1;
-    if (EPI == kEpiStore) splits = std::max(1, std::min(64, K / 512));   // split-K sums land by atomics in cleared C
-    const int kchunk = ((K + splits - 1) / splits + 15) / 16 * 16;
-    splits = (K + kchunk - 1) / kchunk;
-    dim3 grid((N + 63) / 64, (M + 63) / 64, splits);
-    k_gemm<EPI><<<grid, 256, 0, st>>>(M, N, K, kchunk, A, as0, as1, B, bs0, bs1, C, cs, bias, mask, C2);
-}
-
-// forward and backward over rows Xb/Tb (nb); gradients into G (cleared here), loss sum into loss[0]
-void tr_step_grad(gls_trainer *tr, int nb, float huber)
-{
-    cudaStream_t st = tr->st;
-    float *P = tr->P.as<float>(), *G = tr->G.as<float>();
-    const float *Xb = tr->Xb.as<float>(), *Tb = tr->Tb.as<float>();
-    float *Z1 = tr->Z1.as<float>(), *H1 = tr->H1.as<float>(), *Z2 = tr->Z2.as<float>(), *H2 = tr->H2.as<float>();
-    float *Y = tr->Y.as<float>(), *DY = tr->DY.as<float>(), *DZ2 = tr->DZ2.as<float>(), *DZ1 = tr->DZ1.as<float>();
-    cudaMemsetAsync(G, 0, (size_t)kParams * 4, st);
-    gemm<kEpiBiasRelu>(st, nb, kHid, kIn, Xb, kIn, 1, P + kOffW1, 1, kIn, Z1, kHid, P + kOffB1, nullptr, H1);
-    gemm<kEpiBiasRelu>(st, nb, kHid, kHid, H1, kHid, 1, P + kOffW2, 1, kHid, Z2, kHid, P + kOffB2, nullptr, H2);
-    k_rowdot<<<(nb * 32 + 255) / 256, 256, 0, st>>>(nb, H2, P + kOffW3, P + kOffB3, Y);
-    k_loss<<<(nb + 255) / 256, 256, 0, st>>>(nb, Y, Tb, huber, 1.f / nb, DY, tr->loss.as<float>());
-    const int cb = std::max(1, std::min(256, nb / 64));
-    k_colsum<<<cb, 256, 0, st>>>(nb, kHid, H2, DY, G + kOffW3);
-    k_colsum<<<cb, 256, 0, st>>>(nb, 1, DY, nullptr, G + kOffB3);
-    k_dz2<<<(unsigned)(((long)nb * kHid + 255) / 256), 256, 0, st>>>(nb, DY, P + kOffW3, Z2, DZ2);
-    gemm<kEpiStore>(st, kHid, kHid, nb, DZ2, 1, kHid, H1, kHid, 1, G + kOffW2, kHid);
-    k_colsum<<<cb, 256, 0, st>>>(nb, kHid, DZ2, nullptr, G + kOffB2);
-    gemm<kEpiMask>(st, nb, kHid, kHid, DZ2, kHid, 1, P + kOffW2, kHid, 1, DZ1, kHid, nullptr, Z1);
-    gemm<kEpiStore>(st, kHid, kIn, nb, DZ1, 1, kHid, Xb, kIn, 1, G + kOffW1, kIn);
-    k_colsum<<<cb, 256, 0, st>>>(nb, kHid, DZ1, nullptr, G + kOffB1);
+    cudaMemsetAsync(tr->G.p, 0, (size_t)kCopies * kCopy * 4, tr->st);
+    const int tiles = (nb + kRows - 1) / kRows;
+    k_mlp_grad<<<std::min(tiles, tr->sm_count), 256, sizeof(GradSmem), tr->st>>>(
+        nb, first, mul, add, tr->n, tr->X.as<float>(), tr->T.as<float>(), tr->P.as<float>(), huber, 1.f / nb,
+        tr->G.as<float>());
 }
 
 uint64_t splitmix(uint64_t &s)
@@ -664,10 +714,12 @@ extern "C" int gls_trainer_create(int device, uint64_t seed, gls_trainer **out)
     tr->seed = seed;
     cudaError_t e = cudaStreamCreateWithFlags(&tr->st, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = tr->P.ensure(kParams * 4);
-    if (e == cudaSuccess) e = tr->G.ensure(kParams * 4);
+    if (e == cudaSuccess) e = tr->G.ensure(kCopies * kCopy * 4);
+    if (e == cudaSuccess) e = tr->sum.ensure(kCopy * 4 + 16);
     if (e == cudaSuccess) e = tr->Mo.ensure(kParams * 4);
     if (e == cudaSuccess) e = tr->Vo.ensure(kParams * 4);
-    if (e == cudaSuccess) e = tr->loss.ensure(16);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&tr->sm_count, cudaDevAttrMultiProcessorCount, device);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(GradSmem));
     if (e != cudaSuccess) {
         delete tr;
         return GLS_ECUDA;
@@ -690,9 +742,9 @@ extern "C" int gls_trainer_destroy(gls_trainer *tr)
 {
     if (!tr) return GLS_OK;
     cudaSetDevice(tr->device);
-    DevBuf *all[] = {&tr->X, &tr->T, &tr->Xb, &tr->Tb, &tr->Z1, &tr->H1, &tr->Z2, &tr->H2, &tr->Y,
-                     &tr->DY, &tr->DZ2, &tr->DZ1, &tr->P, &tr->G, &tr->Mo, &tr->Vo, &tr->loss};
+    DevBuf *all[] = {&tr->X, &tr->T, &tr->P, &tr->G, &tr->Mo, &tr->Vo, &tr->sum};
     for (DevBuf *b : all) b->release();
+    tr->host.release();
     if (tr->st) cudaStreamDestroy(tr->st);
     delete tr;
     return GLS_OK;
@@ -724,8 +776,6 @@ extern "C" int gls_trainer_fit(gls_trainer *tr, const gls_train_opts *o, float *
     if (!tr || !o || !o->batch || !tr->n) return GLS_EINVAL;
     cudaSetDevice(tr->device);
     const uint32_t nb_max = (uint32_t)std::min<uint64_t>(o->batch, tr->n);
-    int rc = tr_alloc_batch(tr, nb_max);
-    if (rc) return rc;
     uint64_t s = o->seed ^ 0x5DEECE66Dull;
     for (uint32_t ep = 0; ep < o->epochs; ++ep) {
         // a fresh pseudo-random permutation of the rows every epoch
@@ -733,20 +783,19 @@ extern "C" int gls_trainer_fit(gls_trainer *tr, const gls_train_opts *o, float *
         if (mul == 0) mul = 1;
         while (gcd64(mul, tr->n) != 1) mul = mul + 1 < tr->n ? mul + 1 : 1;
         const uint64_t add = splitmix(s) % tr->n;
-        cudaMemsetAsync(tr->loss.p, 0, 4, tr->st);
+        cudaMemsetAsync(tr->sum.p, 0, 8, tr->st);
         for (uint64_t b0 = 0; b0 < tr->n; b0 += nb_max) {
             const int nb = (int)std::min<uint64_t>(nb_max, tr->n - b0);
-            k_gather<<<(unsigned)(((long)nb * kIn + 255) / 256), 256, 0, tr->st>>>(
-                nb, b0, mul, add, tr->n, tr->X.as<float>(), tr->T.as<float>(), tr->Xb.as<float>(), tr->Tb.as<float>());
-            tr_step_grad(tr, nb, o->huber);
+            tr_step_grad(tr, nb, b0, mul, add, o->huber);
             ++tr->adam_t;
             const float c1 = 1.f / (1.f - std::pow(0.9f, (float)tr->adam_t));
             const float c2 = 1.f / (1.f - std::pow(0.999f, (float)tr->adam_t));
-            k_adam<<<(kParams + 255) / 256, 256, 0, tr->st>>>(kParams, tr->P.as<float>(), tr->G.as<float>(),
-                                                               tr->Mo.as<float>(), tr->Vo.as<float>(), o->lr, c1, c2);
+            k_adam<<<kParams / 256 + 1, 256, 0, tr->st>>>(kParams, tr->P.as<float>(), tr->G.as<float>(),
+                                                          tr->Mo.as<float>(), tr->Vo.as<float>(), o->lr, c1, c2,
+                                                          tr->sum.as<double>());
         }
-        float ls = 0.f;
-        cudaMemcpyAsync(&ls, tr->loss.p, 4, cudaMemcpyDeviceToHost, tr->st);
+        double ls = 0.0;
+        cudaMemcpyAsync(&ls, tr->sum.p, 8, cudaMemcpyDeviceToHost, tr->st);
         const cudaError_t e = cudaStreamSynchronize(tr->st);
         if (e != cudaSuccess) return setf(&tr->err, GLS_ECUDA, "training step", e);
         if (loss) loss[ep] = (float)(ls / (double)tr->n);
@@ -758,17 +807,18 @@ extern "C" int gls_trainer_grad(gls_trainer *tr, uint64_t first, uint64_t n, flo
 {
     if (!tr || !grad || !n || first + n > tr->n || n > 0x7FFFFFFFull) return GLS_EINVAL;
     cudaSetDevice(tr->device);
-    int rc = tr_alloc_batch(tr, (uint32_t)n);
-    if (rc) return rc;
-    cudaMemcpyAsync(tr->Xb.p, tr->X.as<float>() + first * kIn, n * kIn * 4, cudaMemcpyDeviceToDevice, tr->st);
-    cudaMemcpyAsync(tr->Tb.p, tr->T.as<float>() + first, n * 4, cudaMemcpyDeviceToDevice, tr->st);
-    cudaMemsetAsync(tr->loss.p, 0, 4, tr->st);
-    tr_step_grad(tr, (int)n, huber);
-    cudaMemcpyAsync(grad, tr->G.p, kParams * 4, cudaMemcpyDeviceToHost, tr->st);
-    float ls = 0.f;
-    cudaMemcpyAsync(&ls, tr->loss.p, 4, cudaMemcpyDeviceToHost, tr->st);
-    const cudaError_t e = cudaStreamSynchronize(tr->st);
+    tr_step_grad(tr, (int)n, first, 0, 0, huber);
+    k_sum_copies<<<kCopy / 256 + 1, 256, 0, tr->st>>>(tr->G.as<float>(), tr->sum.as<float>());
+    // the gradient and the loss sum behind it in one copy, through page-locked
+    // memory kept with the trainer
+    cudaError_t e = cudaSuccess;
+    if (!tr->host.ensure(kCopy * 4)) e = cudaErrorMemoryAllocation;
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(tr->host.p, tr->sum.p, kCopy * 4, cudaMemcpyDeviceToHost, tr->st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(tr->st);
     if (e != cudaSuccess) return setf(&tr->err, GLS_ECUDA, "gradient", e);
+    std::memcpy(grad, tr->host.p, kParams * 4);
+    const float ls = tr->host.as<float>()[kParams];
     if (loss) *loss = ls / (float)n;
     return GLS_OK;
 }
