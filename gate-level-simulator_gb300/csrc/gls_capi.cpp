@@ -178,11 +178,11 @@ extern "C" int gls_create(const gls_opts *opts, gls_ctx **out)
 static void free_window(Window *w)
 {
     w->pool.release(); w->net_off.release(); w->net_len.release();
-    w->init_off.release(); w->init_len.release(); w->saif.release(); w->small.release();
+    w->saif.release(); w->small.release();
     w->stim_dev.release();
     w->dwin.release();
     w->lvl.release();
-    w->h_words.release(); w->h_off.release(); w->h_len.release();
+    w->h_words.release(); w->h_stim.release();
     delete w;
 }
 
@@ -210,7 +210,7 @@ void ctx_drop_graphs(gls_ctx *ctx)
 // its SAIF counts, lengths and flags stay
 static void release_window_pool(gls_ctx *ctx, Window *w)
 {
-    DevBuf *bufs[] = {&w->pool, &w->net_off, &w->init_off, &w->init_len, &w->stim_dev};
+    DevBuf *bufs[] = {&w->pool, &w->net_off, &w->stim_dev};
     for (DevBuf *b : bufs) {
         if (b->p) ctx->spare_bufs.push_back(*b);
         b->p = nullptr;
@@ -266,6 +266,7 @@ extern "C" int gls_destroy(gls_ctx *ctx)
     ctx->fast.release();
     ctx_drop_graphs(ctx);
     ctx->hwave.release();
+    ctx->hsmall.release();
     ctx->pin_out.release();
     ctx->dwave.release();
     ctx->wave_e.release();
@@ -615,9 +616,8 @@ static uint64_t projected_cap(const gls_ctx *ctx, const Window *w)
     return cap;
 }
 
-// Device buffers of a window filled from its host staging.  Without `sync`
-// the copies only precede later work on the context's stream.
-static int upload_window(gls_ctx *ctx, Window *w, bool sync = true)
+// Device buffers of a window filled from its host staging, in stream order.
+static int upload_window(gls_ctx *ctx, Window *w)
 {
     const uint64_t n = ctx->n_nets;
     w->cap = std::max(w->cap, projected_cap(ctx, w));
@@ -626,32 +626,17 @@ static int upload_window(gls_ctx *ctx, Window *w, bool sync = true)
     CK(take_buf(ctx, w->pool, w->cap * wb), "alloc event pool");
     CK(take_buf(ctx, w->net_off, n * 8), "alloc net_off");
     CK(w->net_len.ensure(n * 8), "alloc net_len");   // lengths, then the X times
-    CK(take_buf(ctx, w->init_off, n * 8), "alloc init_off");
-    CK(take_buf(ctx, w->init_len, n * 8), "alloc init_len");
     CK(w->saif.ensure(n * 24), "alloc saif");
     CK(w->small.ensure(256), "alloc counters");
     CK(w->lvl.ensure((ctx->drv_level_start.size()) * sizeof(LevelCtr)), "alloc level counters");
-    CK(take_buf(ctx, w->stim_dev, w->stim_nets.size() * 4 + 16), "alloc stim nets");
+    const size_t stim_bytes = w->stim_nets.size() * 16;
+    CK(take_buf(ctx, w->stim_dev, stim_bytes + 16), "alloc stim nets");
     if (w->stim_events)
         CK(cudaMemcpyAsync(w->pool.p, w->h_words.p, w->stim_events * wb, cudaMemcpyHostToDevice, ctx->stream),
            "upload stimulus");
-    if (!w->h_off.ensure(n * 8) || !w->h_len.ensure(n * 8)) return fail(ctx, GLS_ENOMEM, "pinned staging");
-    uint64_t *off = w->h_off.as<uint64_t>();
-    uint32_t *len = w->h_len.as<uint32_t>();
-    std::memset(off, 0, n * 8);
-    std::memset(len, 0xFF, n * 4);
-    std::memset(len + n, 0, n * 4);   // k_stim_saif and the gate kernels fill it
-    for (size_t k = 0; k < w->stim_nets.size(); ++k) {
-        off[w->stim_nets[k]] = w->stim_off[k];
-        len[w->stim_nets[k]] = w->stim_len[k];
-    }
-    CK(cudaMemcpyAsync(w->init_off.p, off, n * 8, cudaMemcpyHostToDevice, ctx->stream), "upload offsets");
-    CK(cudaMemcpyAsync(w->init_len.p, len, n * 8, cudaMemcpyHostToDevice, ctx->stream), "upload lengths");
-    if (!w->stim_nets.empty())
-        CK(cudaMemcpyAsync(w->stim_dev.p, w->stim_nets.data(), w->stim_nets.size() * 4, cudaMemcpyHostToDevice,
-                           ctx->stream),
+    if (stim_bytes)
+        CK(cudaMemcpyAsync(w->stim_dev.p, w->h_stim.p, stim_bytes, cudaMemcpyHostToDevice, ctx->stream),
            "upload stim nets");
-    if (sync) CK(cudaStreamSynchronize(ctx->stream), "upload sync");
     w->uploaded = true;
     return GLS_OK;
 }
@@ -691,10 +676,6 @@ extern "C" int gls_add_window(gls_ctx *ctx, const gls_stimulus *st, uint64_t t_b
     for (uint32_t net : ctx->ext_inputs)
         if (!seen[net]) { ctx->spare.push_back(w); return fail(ctx, GLS_EINVAL, "net %u is read by a gate but has no stimulus", net); }
     const uint64_t total = at[st->n_nets];
-    if (!w->h_words.ensure(total * 4)) {
-        ctx->spare.push_back(w);
-        return fail(ctx, GLS_ENOMEM, "pinned staging of %llu events", (unsigned long long)total);
-    }
     // validate and pack (time << 2 | value), each net on a 4-event boundary;
     // large stimuli are packed by several host threads.  32-bit words hold
     // times up to 2^30 - 2; a later time repacks the stimulus in 64-bit words.
@@ -734,34 +715,43 @@ extern "C" int gls_add_window(gls_ctx *ctx, const gls_stimulus *st, uint64_t t_b
             }
         }
     };
+    // times increase within a net, so its last one tells which words it needs
+    // (a net out of order is found by the pack)
+    for (uint32_t k = 0; k < st->n_nets; ++k)
+        if (st->ev_start[k + 1] > st->ev_start[k] && st->time[st->ev_start[k + 1] - 1] > kMaxTime) w->w64 = true;
+    // several threads from about 2^17 events on: 110 us for any count up to
+    // 2^18, one thread 129 us at 2^17 and 233 us at 2^18
+    constexpr uint64_t kPackAlone = 1u << 17;
     const unsigned hc = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
-    if (total > (1u << 20) && hc > 1 && st->n_nets > 4 * hc && !ctx->pool) {
+    if (total > kPackAlone && hc > 1 && st->n_nets > 4 * hc && !ctx->pool) {
         try {
             ctx->pool = new WorkPool(hc - 1);
         } catch (...) {   // no threads to be had: pack on this one
             ctx->pool = nullptr;
         }
     }
-    if (total > (1u << 20) && ctx->pool && st->n_nets > 4 * ctx->pool->threads()) {
-        // parts of about equal event counts: part q starts at the first net
-        // whose packed offset reaches q * total / parts
-        const unsigned parts = 4 * ctx->pool->threads();
-        std::vector<uint32_t> first(parts + 1, st->n_nets);
-        for (unsigned q = 0; q < parts; ++q)
-            first[q] = (uint32_t)(std::lower_bound(at.begin(), at.end() - 1, total * q / parts) - at.begin());
-        ctx->pool->parallel_for(parts, [&](unsigned q) {
-            pack(w->h_words.as<uint32_t>(), first[q], std::max(first[q], first[q + 1]));
-        });
-    } else {
-        pack(w->h_words.as<uint32_t>(), 0, st->n_nets);
-    }
-    if (!bad && long_times) {
-        if (!w->h_words.ensure(total * 8)) {
+    auto pack_all = [&](auto *hw) {
+        if (total > kPackAlone && ctx->pool && st->n_nets > 4 * ctx->pool->threads()) {
+            // parts of about equal event counts: part q starts at the first net
+            // whose packed offset reaches q * total / parts
+            const unsigned parts = 4 * ctx->pool->threads();
+            std::vector<uint32_t> first(parts + 1, st->n_nets);
+            for (unsigned q = 0; q < parts; ++q)
+                first[q] = (uint32_t)(std::lower_bound(at.begin(), at.end() - 1, total * q / parts) - at.begin());
+            ctx->pool->parallel_for(parts, [&](unsigned q) { pack(hw, first[q], std::max(first[q], first[q + 1])); });
+        } else {
+            pack(hw, 0, st->n_nets);
+        }
+    };
+    for (;;) {
+        if (!w->h_words.ensure(total * w->word_bytes())) {
             ctx->spare.push_back(w);
             return fail(ctx, GLS_ENOMEM, "pinned staging of %llu events", (unsigned long long)total);
         }
-        w->w64 = true;
-        pack(w->h_words.as<WideWord>(), 0, st->n_nets);
+        if (w->w64) pack_all(w->h_words.as<WideWord>());
+        else pack_all(w->h_words.as<uint32_t>());
+        if (bad || w->w64 || !long_times) break;
+        w->w64 = true;   // a late time before a net's last one: the faults as 64-bit words have them
     }
     if (bad) {
         ctx->spare.push_back(w);
@@ -771,9 +761,17 @@ extern "C" int gls_add_window(gls_ctx *ctx, const gls_stimulus *st, uint64_t t_b
                                              : "times not strictly increasing");
     }
     w->stim_nets.assign(st->net, st->net + st->n_nets);
-    w->stim_off.assign(at.begin(), at.end() - 1);
-    w->stim_len.resize(st->n_nets);
-    for (uint32_t k = 0; k < st->n_nets; ++k) w->stim_len[k] = (uint32_t)(st->ev_start[k + 1] - st->ev_start[k]);
+    if (!w->h_stim.ensure((size_t)st->n_nets * 16)) {
+        ctx->spare.push_back(w);
+        return fail(ctx, GLS_ENOMEM, "pinned staging of %u stimulus nets", st->n_nets);
+    }
+    uint32_t *const h_net = w->h_stim.as<uint32_t>(), *const h_len = h_net + st->n_nets;
+    uint64_t *const h_off = reinterpret_cast<uint64_t *>(h_net + 2ull * st->n_nets);
+    for (uint32_t k = 0; k < st->n_nets; ++k) {
+        h_net[k] = st->net[k];
+        h_len[k] = (uint32_t)(st->ev_start[k + 1] - st->ev_start[k]);
+        h_off[k] = at[k];
+    }
     w->stim_events = total;
     // initial pool capacity: stimulus plus an estimate of every gate's slot
     uint64_t cap = ctx->opts.pool_events;
@@ -822,7 +820,6 @@ static WinDev make_windev(gls_ctx *ctx, Window *w, const LevelScratch &ls, int p
     d.top = sm;
     d.counters = sm + 1;     // 4 counters
     d.err = reinterpret_cast<uint32_t *>(sm + 5);
-    d.n_segs = reinterpret_cast<uint32_t *>(sm + 6);
     d.n_over = sm + 7;
     d.res = (parity ? ls.res1 : ls.res).as<uint32_t>();
     d.pred = ls.pred.as<uint32_t>();
@@ -840,6 +837,7 @@ static WinDev make_windev(gls_ctx *ctx, Window *w, const LevelScratch &ls, int p
     d.seg_cap = ls.seg_cap;
     d.t_begin = w->t_begin;
     d.t_end = w->t_end;
+    d.top0 = w->stim_events + ctx->pool_gap;
     return d;
 }
 
@@ -859,19 +857,6 @@ static void prof_mark(gls_ctx *ctx)
     if (!ctx->opts.profile) return;
     cudaEvent_t e = prof_event(ctx);
     if (e) cudaEventRecord(e, ctx->stream);
-}
-
-// Clear a window's outputs and counters before it runs.
-static int reset_window(gls_ctx *ctx, Window *w)
-{
-    const uint64_t n = ctx->n_nets;
-    CK(cudaMemcpyAsync(w->net_off.p, w->init_off.p, n * 8, cudaMemcpyDeviceToDevice, ctx->stream), "reset offsets");
-    CK(cudaMemcpyAsync(w->net_len.p, w->init_len.p, n * 8, cudaMemcpyDeviceToDevice, ctx->stream), "reset lengths");
-    CK(cudaMemsetAsync(w->saif.p, 0xFF, n * 24, ctx->stream), "reset saif");
-    CK(cudaMemsetAsync(w->lvl.p, 0, ctx->drv_level_start.size() * sizeof(LevelCtr), ctx->stream), "reset level counters");
-    unsigned long long small[8] = {w->stim_events + ctx->pool_gap, 0, 0, 0, 0, 0, 0, 0};
-    CK(cudaMemcpyAsync(w->small.p, small, sizeof small, cudaMemcpyHostToDevice, ctx->stream), "reset counters");
-    return GLS_OK;
 }
 
 // Whether a run's levels go through k_gate: 64-bit windows, and the default
@@ -1115,14 +1100,25 @@ static int enqueue_window(gls_ctx *ctx, Window *w, uint32_t *launches)
     int rc = w->uploaded ? GLS_OK : upload_window(ctx, w);
     if (rc) return rc;
     w->saif_only = false;
-    rc = reset_window(ctx, w);
-    if (rc) return rc;
     const WinDev d[2] = {make_windev(ctx, w, *ctx->lsc[0], 0), make_windev(ctx, w, *ctx->lsc[0], 1)};
     CK(w->dwin.ensure(sizeof d), "alloc window descriptor");
     CK(cudaMemcpyAsync(w->dwin.p, d, sizeof d, cudaMemcpyHostToDevice, ctx->stream), "upload window descriptor");
     const WinDev *dw[2] = {w->dwin.as<WinDev>(), w->dwin.as<WinDev>() + 1};
     const WinDev *hp[2] = {&d[0], &d[1]};
+    launch_reset(dw[0], d[0], 1, d[0].n_stim, ctx->n_nets, (uint32_t)ctx->drv_level_start.size(), ctx->stream);
     return enqueue_levels(ctx, dw, hp, 1, d[0].n_stim, true, launches, w->w64, gate_events_est(ctx, w));
+}
+
+// Copies the flags and counters of windows [w0, w0 + n) to ctx->hsmall, behind
+// what the stream holds.
+static int read_status(gls_ctx *ctx, size_t w0, size_t n)
+{
+    if (!ctx->hsmall.ensure(std::max<size_t>(n, 1) * 64)) return fail(ctx, GLS_ENOMEM, "pinned staging of run flags");
+    for (size_t k = 0; k < n; ++k)
+        CK(cudaMemcpyAsync(ctx->hsmall.as<char>() + k * 64, ctx->windows[w0 + k]->small.p, 64, cudaMemcpyDeviceToHost,
+                           ctx->stream),
+           "read status");
+    return GLS_OK;
 }
 
 // Totals of a run over its windows.
@@ -1146,13 +1142,15 @@ static int widen_window(gls_ctx *ctx, Window *w)
     return upload_window(ctx, w);
 }
 
-// Read a window's flags after its run; on a full pool or work space, grow it
+// A window's flags after its run (status: its eight counters as the run left
+// them); on a full pool or work space, grow it
 // and run the window again on its own (level work space 0), until it fits.
-static int settle_window(gls_ctx *ctx, Window *w, RunAcc &acc)
+static int settle_window(gls_ctx *ctx, Window *w, RunAcc &acc, const unsigned long long *status)
 {
     for (int attempt = 0;; ++attempt) {
         unsigned long long small[8];
-        CK(cudaMemcpy(small, w->small.p, sizeof small, cudaMemcpyDeviceToHost), "read status");
+        if (attempt) CK(cudaMemcpy(small, w->small.p, sizeof small, cudaMemcpyDeviceToHost), "read status");
+        else std::memcpy(small, status, sizeof small);
         const uint32_t err = (uint32_t)small[5];
         if (!err) {
             const double sc = pool_scale(ctx, w);
@@ -1249,6 +1247,7 @@ extern "C" int gls_run(gls_ctx *ctx)
         if (rc) return rc;
     }
     CK(cudaEventRecord(ctx->ev1, ctx->stream), "event");
+    if (int rc = read_status(ctx, 0, ctx->windows.size())) return rc;
     CK(cudaStreamSynchronize(ctx->stream), "run");
     float ms = 0.f;
     cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
@@ -1278,8 +1277,8 @@ extern "C" int gls_run(gls_ctx *ctx)
     RunAcc acc;
     acc.total_ms = total_ms;
     acc.launches = launches;
-    for (Window *w : ctx->windows) {
-        int rc = settle_window(ctx, w, acc);
+    for (size_t k = 0; k < ctx->windows.size(); ++k) {
+        int rc = settle_window(ctx, ctx->windows[k], acc, ctx->hsmall.as<unsigned long long>() + 8 * k);
         if (rc) return rc;
     }
     publish_stats(ctx, acc, kms);
@@ -1321,7 +1320,7 @@ static int batch_setup(gls_ctx *ctx, const gls_batch_opts &o, uint64_t *B)
         fr += spare_bytes(ctx);
         uint64_t per = 0;
         for (Window *w : ctx->windows) per = std::max<uint64_t>(per, projected_cap(ctx, w) * w->word_bytes());
-        per += (uint64_t)ctx->n_nets * 48 + (uint64_t)(ctx->max_width + 1) * 32 +
+        per += (uint64_t)ctx->n_nets * 56 + (uint64_t)(ctx->max_width + 1) * 32 +
                (uint64_t)ctx->seg_cap * (sizeof(SegRec) + sizeof(CopyRec)) + ctx->scr_cap * 4;
         const uint64_t fit = std::max<uint64_t>(1, (uint64_t)(0.85 * (double)fr) / std::max<uint64_t>(per, 1));
         b = std::max<uint64_t>(1, std::min(b, fit));
@@ -1351,8 +1350,7 @@ static int run_wave(gls_ctx *ctx, size_t w0, uint32_t nwin, const gls_batch_opts
         CK(ctx->lsc[k]->ensure(ctx->max_width, ctx->seg_cap, ctx->scr_cap), "alloc level work spaces");
     for (uint32_t k = 0; k < nwin; ++k) {
         Window *w = ctx->windows[w0 + k];
-        int rc = w->uploaded ? GLS_OK : upload_window(ctx, w, false);
-        if (rc == GLS_OK) rc = reset_window(ctx, w);
+        int rc = w->uploaded ? GLS_OK : upload_window(ctx, w);
         if (rc) return rc;
         w->saif_only = false;
         hw[k] = make_windev(ctx, w, *ctx->lsc[k], 0);
@@ -1360,13 +1358,14 @@ static int run_wave(gls_ctx *ctx, size_t w0, uint32_t nwin, const gls_batch_opts
         max_stim = std::max(max_stim, hw[k].n_stim);
         est += gate_events_est(ctx, w) / nwin;
     }
-    CK(cudaEventRecord(e0, ctx->stream), "event");
     for (int p = 0; p < 2; ++p)
         CK(cudaMemcpyAsync(ctx->dwave.as<WinDev>() + p * kMaxWave, hw + p * kMaxWave, nwin * sizeof(WinDev),
                            cudaMemcpyHostToDevice, ctx->stream),
            "upload wave descriptors");
     const WinDev *dw[2] = {ctx->dwave.as<WinDev>(), ctx->dwave.as<WinDev>() + kMaxWave};
     const WinDev *hp[2] = {&hw[0], &hw[kMaxWave]};
+    launch_reset(dw[0], hw[0], nwin, max_stim, ctx->n_nets, (uint32_t)ctx->drv_level_start.size(), ctx->stream);
+    CK(cudaEventRecord(e0, ctx->stream), "event");
     if (o.use_graph && nwin > 1) {
         // one graph per wave shape; the descriptors it reads are rewritten per wave
         gls_ctx::WaveGraph key{nwin, max_stim, ctx->warp_mask, (uint32_t)ctx->opts.alloc_mode, ctx->seg_per_sm,
@@ -1403,6 +1402,7 @@ static int run_wave(gls_ctx *ctx, size_t w0, uint32_t nwin, const gls_batch_opts
         if (rc) return rc;
     }
     CK(cudaEventRecord(e1, ctx->stream), "event");
+    if (int rc = read_status(ctx, w0, nwin)) return rc;
     CK(cudaStreamSynchronize(ctx->stream), "wave");
     float t = 0.f;
     cudaEventElapsedTime(&t, e0, e1);
@@ -1410,15 +1410,14 @@ static int run_wave(gls_ctx *ctx, size_t w0, uint32_t nwin, const gls_batch_opts
     // windows that finished first (and, with saif_only, give their pools
     // back), then the ones that outgrew a buffer, rerun alone with more room
     std::vector<uint32_t> again;
+    const unsigned long long *status = ctx->hsmall.as<unsigned long long>();
     for (uint32_t k = 0; k < nwin; ++k) {
         Window *w = ctx->windows[w0 + k];
-        unsigned long long small[8];
-        CK(cudaMemcpy(small, w->small.p, sizeof small, cudaMemcpyDeviceToHost), "read status");
-        if (small[5]) {
+        if (status[8 * k + 5]) {
             again.push_back(k);
             continue;
         }
-        int rc = settle_window(ctx, w, acc);
+        int rc = settle_window(ctx, w, acc, status + 8 * k);
         if (rc) return rc;
         if (o.saif_only) {
             release_window_pool(ctx, w);
@@ -1429,7 +1428,7 @@ static int run_wave(gls_ctx *ctx, size_t w0, uint32_t nwin, const gls_batch_opts
         for (size_t k = 1; k < ctx->lsc.size(); ++k) ctx->lsc[k]->release();
     for (uint32_t k : again) {
         Window *w = ctx->windows[w0 + k];
-        int rc = settle_window(ctx, w, acc);
+        int rc = settle_window(ctx, w, acc, status + 8 * k);
         if (rc) return rc;
         if (o.saif_only) {
             release_window_pool(ctx, w);
@@ -1462,7 +1461,7 @@ extern "C" int gls_run_batched(gls_ctx *ctx, const gls_batch_opts *opts)
             uint64_t per = 1;
             for (uint64_t k = 0; k < nwin; ++k) {
                 const Window *w = ctx->windows[w0 + k];
-                per = std::max<uint64_t>(per, projected_cap(ctx, w) * w->word_bytes() + (uint64_t)ctx->n_nets * 48);
+                per = std::max<uint64_t>(per, projected_cap(ctx, w) * w->word_bytes() + (uint64_t)ctx->n_nets * 56);
             }
             nwin = std::max<uint64_t>(1, std::min<uint64_t>(nwin, (uint64_t)(0.85 * (double)fr) / per));
         }
@@ -1661,33 +1660,41 @@ extern "C" int gls_waveform(gls_ctx *ctx, uint32_t window, uint32_t net, uint32_
     if (net >= ctx->n_nets) return fail(ctx, GLS_EINVAL, "net %u out of range", net);
     if (w->saif_only) return fail(ctx, GLS_ESTATE, "window %u ran with saif_only: its waveforms were not kept", window);
     cudaSetDevice(ctx->opts.device);
-    uint64_t off = 0;
-    uint32_t len = 0;
-    CK(cudaMemcpy(&off, w->net_off.as<uint64_t>() + net, 8, cudaMemcpyDeviceToHost), "read offset");
-    CK(cudaMemcpy(&len, w->net_len.as<uint32_t>() + net, 4, cudaMemcpyDeviceToHost), "read length");
+    const uint32_t wb = (uint32_t)w->word_bytes();
+    const uint64_t want = (time || value) ? cap : 0;
+    // The length and a short list in one launch that writes page-locked memory
+    // (14 us at 1000 events, 37 us at 2^16; two copies for offset and length
+    // and one for the events 30 and 51 us); one block's stores fall behind a
+    // copy at about 2^18 events (107 us either way).
+    constexpr uint64_t kInline = 1u << 18;
+    const uint64_t first = want > kInline ? 0 : want;
+    if (!ctx->pin_out.ensure(16 + first * wb)) return fail(ctx, GLS_ENOMEM, "pinned staging for a waveform");
+    launch_read_list(w->net_off.as<uint64_t>() + net, w->net_len.as<uint32_t>() + net, w->pool.p, wb, first,
+                     ctx->pin_out.p, ctx->stream);
+    CK(cudaGetLastError(), "read waveform");
+    CK(cudaStreamSynchronize(ctx->stream), "read waveform");
+    const uint64_t len = ctx->pin_out.as<uint64_t>()[0], off = ctx->pin_out.as<uint64_t>()[1];
     if (len == 0xFFFFFFFFu) {
         *n = UINT64_MAX;
         return GLS_OK;
     }
     *n = len;
-    const uint64_t k = std::min<uint64_t>(cap, len);
-    if (k && (time || value)) {
-        if (w->w64) {
-            std::vector<WideWord> words(k);
-            CK(cudaMemcpy(words.data(), w->pool.as<WideWord>() + off, k * 8, cudaMemcpyDeviceToHost), "read events");
-            for (uint64_t e = 0; e < k; ++e) {
-                if (time) time[e] = ev_time(words[e]);
-                if (value) value[e] = (uint8_t)ev_val(words[e]);
-            }
-        } else {
-            std::vector<uint32_t> words(k);
-            CK(cudaMemcpy(words.data(), w->pool.as<uint32_t>() + off, k * 4, cudaMemcpyDeviceToHost), "read events");
-            for (uint64_t e = 0; e < k; ++e) {
-                if (time) time[e] = ev_time(words[e]);
-                if (value) value[e] = (uint8_t)ev_val(words[e]);
-            }
-        }
+    const uint64_t k = std::min<uint64_t>(want, len);
+    std::vector<WideWord> rest;   // 64-bit aligned, for words of either size
+    const char *words = ctx->pin_out.as<char>() + 16;
+    if (k > first) {
+        rest.resize((k * wb + 7) / 8);
+        CK(cudaMemcpy(rest.data(), w->pool.as<char>() + off * wb, k * wb, cudaMemcpyDeviceToHost), "read events");
+        words = reinterpret_cast<const char *>(rest.data());
     }
+    auto unpack = [&](const auto *x) {
+        for (uint64_t e = 0; e < k; ++e) {
+            if (time) time[e] = ev_time(x[e]);
+            if (value) value[e] = (uint8_t)ev_val(x[e]);
+        }
+    };
+    if (w->w64) unpack(reinterpret_cast<const WideWord *>(words));
+    else unpack(reinterpret_cast<const uint32_t *>(words));
     return GLS_OK;
 }
 

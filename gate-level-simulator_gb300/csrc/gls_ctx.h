@@ -191,14 +191,12 @@ struct LevelScratch {
 
 struct Window {
     std::vector<uint32_t> stim_nets;
-    std::vector<uint64_t> stim_off;     // aligned pool offset per stimulus net
-    std::vector<uint32_t> stim_len;
     uint64_t stim_events = 0;           // aligned extent of the stimulus in the pool
     PinBuf h_words;                     // packed stimulus events (kept to re-upload on pool growth)
-    PinBuf h_off, h_len;                // initial net table
+    PinBuf h_stim;                      // per stimulus net: nets, lengths, then (64 bits) aligned pool offsets
     uint64_t t_begin = 0, t_end = 0;
     uint64_t cap = 0;
-    DevBuf pool, net_off, net_len, init_off, init_len, saif, small, stim_dev;
+    DevBuf pool, net_off, net_len, saif, small, stim_dev;
     DevBuf dwin;                        // the window's WinDev on the device (sequential runs)
     DevBuf lvl;                         // LevelCtr per level
     bool done = false;
@@ -275,6 +273,7 @@ struct gls_ctx {
     // batched runs: the wave's window descriptors (host pinned, device) and
     // the captured launch graphs, one per wave shape
     PinBuf hwave;
+    PinBuf hsmall;                   // the windows' flags and counters after a run (64 bytes each)
     PinBuf pin_out;                  // staging of SAIF counts and lengths read back to the host
     WorkPool *pool = nullptr;        // host threads that pack stimuli (made on first use)
     DevBuf dwave;

@@ -177,16 +177,16 @@ struct WinDev {
     uint64_t *scr;              // per driver of the level: segment stacks in the scratch
     SegRec *segs;
     CopyRec *copies;            // per segment, written by k_link
-    uint32_t *n_segs;
     uint32_t *res;              // per driver of the level: events reserved in its slot (exact / learned modes)
     unsigned long long *n_over; // gate outputs placed exactly because the presize was short (learned mode)
     uint32_t *pred;             // per driver of the level: predicted slot length (learned mode)
-    const uint32_t *stim_nets;  // nets the stimulus drives
+    const uint32_t *stim_nets;  // nets the stimulus drives, then their lengths, then (64 bits) their pool offsets
     uint32_t *scratch;          // level scratch: segment stacks (event words)
     LevelCtr *lvl;              // k_gate: counters of every level
     uint64_t cap;               // pool capacity (events)
     uint64_t scr_cap;           // scratch capacity (events)
     uint64_t t_begin, t_end;
+    uint64_t top0;              // the pool pointer before the run
     uint32_t seg_cap;           // SegRec capacity
     uint32_t n_stim;
 };
@@ -227,6 +227,13 @@ __host__ __device__ inline int fanin_class(int m) { return m <= 1 ? 0 : (m == 2 
 
 // A launch covers nwin windows: `h` is window 0's descriptor on the host
 // (used when nwin == 1), `dw` the device array of all nwin descriptors.
+// The windows' net tables, counts, counters and pool pointers as before a run.
+void launch_reset(const WinDev *dw, const WinDev &h, uint32_t nwin, uint32_t max_stim, uint32_t n_nets, uint32_t n_levels,
+                  cudaStream_t st);
+// One list (word: bytes of an event word) from its net's tables to out: its
+// length, its pool offset (64 bits each), then up to cap events.
+void launch_read_list(const uint64_t *off, const uint32_t *len, const void *pool, uint32_t word, uint64_t cap, void *out,
+                      cudaStream_t st);
 void launch_stim_saif(const WinDev *dw, const WinDev &h, uint32_t nwin, uint32_t max_stim, bool wide, uint32_t n_nets,
                       cudaStream_t st);
 void launch_plan(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelArgs &a, cudaStream_t st);

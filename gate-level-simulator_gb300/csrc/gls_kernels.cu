@@ -28,6 +28,7 @@
 // those with o < min(o over all later segments), and a segment's first
 // entry is dropped iff it repeats the value of the last kept entry before it.
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstdint>
 #include <type_traits>
 #include "gls_device.cuh"
@@ -186,7 +187,6 @@ __global__ void __launch_bounds__(1024) k_plan(const WinSet<kBatch> ws, LevelArg
     }
     if (*w.err) {   // a failed window: an empty segment table keeps the later kernels off it
         for (uint32_t i = threadIdx.x; i <= n; i += blockDim.x) w.seg_base[i] = 0;
-        if (threadIdx.x == 0) *w.n_segs = 0;
         return;
     }
     if (threadIdx.x <= kClasses) s_sum[threadIdx.x] = 0;
@@ -273,7 +273,6 @@ __global__ void __launch_bounds__(1024) k_plan(const WinSet<kBatch> ws, LevelArg
     __syncthreads();
     if (*w.err) {
         for (uint32_t i = threadIdx.x; i <= n; i += blockDim.x) w.seg_base[i] = 0;
-        if (threadIdx.x == 0) *w.n_segs = 0;
         return;
     }
     // Pass 2: segments, slot and scratch sizes, placed by a block scan in
@@ -319,7 +318,6 @@ __global__ void __launch_bounds__(1024) k_plan(const WinSet<kBatch> ws, LevelArg
     __shared__ bool s_fail;
     if (threadIdx.x == 0) {
         w.seg_base[n] = run_seg;
-        *w.n_segs = run_seg;
         uint32_t e = 0;
         if (run_seg > w.seg_cap) e |= kErrSegCap;
         if (run_scr > w.scr_cap) e |= kErrScratch;
@@ -334,7 +332,6 @@ __global__ void __launch_bounds__(1024) k_plan(const WinSet<kBatch> ws, LevelArg
     __syncthreads();
     if (s_fail) {
         for (uint32_t i = threadIdx.x; i <= n; i += blockDim.x) w.seg_base[i] = 0;
-        if (threadIdx.x == 0) *w.n_segs = 0;
     }
 }
 
@@ -1547,6 +1544,54 @@ __global__ void __launch_bounds__(256, GLS_COPY_BLOCKS) k_copy(const WinSet<kBat
     }
 }
 
+// ------------------------------------------------------- before a run
+// A window's tables are rebuilt on the device from its stimulus' short ones
+// (net, length, offset per stimulus net): two launches for all windows of a
+// wave, instead of whole tables uploaded per window and five copies and
+// fills per window and run.
+template <bool kBatch>
+__global__ void __launch_bounds__(256) k_reset_nets(const WinSet<kBatch> ws, uint32_t n_nets)
+{
+    const WinDev &w = ws.get(blockIdx.y);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_nets; i += gridDim.x * blockDim.x) {
+        w.net_len[i] = kInf;
+        w.net_len[n_nets + i] = 0;
+        w.saif[i] = ~0ull;
+        w.saif[(uint64_t)n_nets + i] = ~0ull;
+        w.saif[2ull * n_nets + i] = ~0ull;
+    }
+}
+template <bool kBatch>
+__global__ void __launch_bounds__(256) k_reset_stim(const WinSet<kBatch> ws, uint32_t n_levels)
+{
+    const WinDev &w = ws.get(blockIdx.y);
+    const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    const uint32_t *len = w.stim_nets + w.n_stim;
+    const uint64_t *off = reinterpret_cast<const uint64_t *>(w.stim_nets + 2ull * w.n_stim);
+    for (uint32_t i = q; i < w.n_stim; i += step) {
+        const uint32_t net = w.stim_nets[i];
+        w.net_len[net] = len[i];
+        w.net_off[net] = off[i];
+    }
+    for (uint32_t i = q; i < n_levels; i += step) w.lvl[i] = LevelCtr{};
+    if (q < 8) w.top[q] = q == 0 ? w.top0 : 0ull;   // the pool pointer, then the counters and flags
+}
+
+// One block: a list's length, its offset and up to cap of its events into
+// host memory.
+template <class Wd>
+__global__ void __launch_bounds__(1024) k_read_list(const uint64_t *__restrict__ off, const uint32_t *__restrict__ len,
+                                                    const Wd *__restrict__ pool, uint64_t cap, unsigned long long *out)
+{
+    const uint32_t n = *len;
+    if (threadIdx.x == 0) out[0] = n;
+    if (n == kInf) return;
+    const Wd *x = pool + *off;
+    if (threadIdx.x == 0) out[1] = *off;
+    Wd *d = reinterpret_cast<Wd *>(out + 2);
+    for (uint64_t e = threadIdx.x; e < n && e < cap; e += blockDim.x) d[e] = x[e];
+}
+
 // ------------------------------------------------------- stimulus SAIF
 // one warp per stimulus net; blockIdx.y is the window.  Beside the SAIF
 // counts, the time of the net's last X, Z or repeated value, after which it
@@ -1617,6 +1662,22 @@ void launch_stim_saif(const WinDev *dw, const WinDev &h, uint32_t nwin, uint32_t
         return;
     }
     GLS_DISPATCH(h, dw, nwin, (k_stim_saif<decltype(ws)::kIsBatch, uint32_t><<<grid, 256, 0, st>>>(ws, n_nets)));
+}
+
+void launch_reset(const WinDev *dw, const WinDev &h, uint32_t nwin, uint32_t max_stim, uint32_t n_nets, uint32_t n_levels,
+                  cudaStream_t st)
+{
+    const dim3 ga(std::min(1024u, (n_nets + 255) / 256 + 1), nwin), gb(std::min(256u, std::max(max_stim, n_levels) / 256 + 1), nwin);
+    GLS_DISPATCH(h, dw, nwin, (k_reset_nets<decltype(ws)::kIsBatch><<<ga, 256, 0, st>>>(ws, n_nets)));
+    GLS_DISPATCH(h, dw, nwin, (k_reset_stim<decltype(ws)::kIsBatch><<<gb, 256, 0, st>>>(ws, n_levels)));
+}
+
+void launch_read_list(const uint64_t *off, const uint32_t *len, const void *pool, uint32_t word, uint64_t cap, void *out,
+                      cudaStream_t st)
+{
+    unsigned long long *o = static_cast<unsigned long long *>(out);
+    if (word == 8) k_read_list<WideWord><<<1, 1024, 0, st>>>(off, len, static_cast<const WideWord *>(pool), cap, o);
+    else k_read_list<uint32_t><<<1, 1024, 0, st>>>(off, len, static_cast<const uint32_t *>(pool), cap, o);
 }
 
 void launch_wave_events(const WinDev *dw, uint32_t nwin, const LevelArgs &a, cudaStream_t st)

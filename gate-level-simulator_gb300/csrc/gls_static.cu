@@ -132,7 +132,6 @@ extern "C" int gls_run_level_static(gls_ctx *ctx, uint32_t level, uint32_t first
     d.top = d_top;
     d.counters = small + 1;
     d.err = reinterpret_cast<uint32_t *>(small + 5);
-    d.n_segs = reinterpret_cast<uint32_t *>(small + 6);
     d.n_over = small + 7;
     d.seg_base = reinterpret_cast<uint32_t *>(base + kOffSegBase);
     d.slot = reinterpret_cast<uint64_t *>(base + kOffSlot);

@@ -24,6 +24,11 @@
 #include <cstdint>
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
+#include <thread>
+#include <utility>
+#include <vector>
+#include <unistd.h>
 #include "gls.h"
 
 namespace {
@@ -397,12 +402,46 @@ __global__ void __launch_bounds__(256) k_emit(const uint8_t *__restrict__ B, con
     }
 }
 
-struct Dev {
-    void *p = nullptr;
-    ~Dev() { if (p) cudaFree(p); }
-    bool alloc(size_t n) { return cudaMalloc(&p, n ? n : 16) == cudaSuccess; }
-    template <typename T> T *as() const { return static_cast<T *>(p); }
+// Device arrays of one phase, carved from one allocation: 24 allocations and
+// frees one by one took longer than the kernels.
+struct Arena {
+    char *p = nullptr;
+    ~Arena() { if (p) cudaFree(p); }
+    template <typename... T> bool alloc(T... parts)   // parts: {T **, count}
+    {
+        size_t total = 0;
+        ((total += part_bytes(parts)), ...);
+        if (cudaMalloc(reinterpret_cast<void **>(&p), total) != cudaSuccess) return false;
+        char *at = p;
+        ((*parts.ptr = reinterpret_cast<decltype(*parts.ptr)>(at), at += part_bytes(parts)), ...);
+        return true;
+    }
+    template <typename P> static size_t part_bytes(const P &x) { return (x.count * sizeof(**x.ptr) + 255) / 256 * 256; }
 };
+template <typename T> struct Part { T **ptr; size_t count; };
+// Fresh host memory faulted in by several threads before a copy into it: one
+// thread takes 3.2 ms for 48 MB, the copy itself .3 ms.
+void touch_pages(std::initializer_list<std::pair<void *, size_t>> blocks)
+{
+    size_t total = 0;
+    for (const auto &b : blocks) total += b.second;
+    const size_t page = (size_t)std::max(4096l, sysconf(_SC_PAGESIZE));
+    const unsigned n = (unsigned)std::min<size_t>(std::min(8u, std::max(1u, std::thread::hardware_concurrency())), total >> 20);
+    if (n < 2) return;
+    auto part = [&](unsigned q) {
+        for (const auto &b : blocks)
+            for (size_t i = b.second / n * q / page * page, e = q + 1 == n ? b.second : b.second / n * (q + 1); i < e; i += page)
+                static_cast<volatile char *>(b.first)[i] = 0;
+    };
+    std::vector<std::thread> threads;
+    try {
+        for (unsigned q = 1; q < n; ++q) threads.emplace_back(part, q);
+    } catch (...) {   // fewer threads than asked for: the copy faults in what is left
+    }
+    part(0);
+    for (std::thread &t : threads) t.join();
+}
+template <typename T> Part<T> part(T *&ptr, size_t count) { return {&ptr, count}; }
 
 }  // namespace
 
@@ -426,82 +465,85 @@ extern "C" int gls_vcd_scan(int device, const char *body, uint64_t n_bytes, cons
     cudaStream_t st = nullptr;
     if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return GLS_ECUDA;
     int rc = GLS_OK;
-    Dev dB, dTileCnt, dTileAgg, dTok, dLen, dCls, dM1, dM2, dM3, dAgg4, dCnt, dAt, dAgg1, dKey, dVs, dBs, dBits, dBus,
-        dFlag, dSig, dTime, dVal, dBusOut;
+    Arena inputs, tokens, results;
+    uint8_t *dB = nullptr, *dBus = nullptr, *dCls = nullptr, *dVal = nullptr, *dBusOut = nullptr;
+    uint32_t *dTileCnt = nullptr, *dTileAgg = nullptr, *dFlag = nullptr, *dVs = nullptr, *dBs = nullptr, *dBits = nullptr,
+             *dTok = nullptr, *dLen = nullptr, *dSig = nullptr;
+    uint64_t *dKey = nullptr;
+    uint4 *dM1 = nullptr, *dM2 = nullptr, *dM3 = nullptr, *dAgg4 = nullptr;
+    unsigned long long *dCnt = nullptr, *dAt = nullptr, *dAgg1 = nullptr, *dTime = nullptr;
     do {
         const uint32_t tiles = (n + kTileBytes - 1) / kTileBytes;
-        if (!dB.alloc(n) || !dTileCnt.alloc((size_t)tiles * 4) || !dTileAgg.alloc((size_t)tiles * 4) ||
-            !dFlag.alloc(16) || !dKey.alloc((size_t)ids->n_ids * 8) || !dVs.alloc((size_t)(ids->n_ids + 1) * 4) ||
-            !dBs.alloc((size_t)(n_vars + 1) * 4) || !dBits.alloc((size_t)n_bits * 4) || !dBus.alloc(n_vars)) {
+        if (!inputs.alloc(part(dB, n), part(dTileCnt, tiles), part(dTileAgg, tiles), part(dFlag, 4),
+                          part(dKey, ids->n_ids), part(dVs, ids->n_ids + 1), part(dBs, n_vars + 1), part(dBits, n_bits),
+                          part(dBus, n_vars))) {
             rc = GLS_ENOMEM;
             break;
         }
-        if (cudaMemcpyAsync(dB.p, body, n, cudaMemcpyHostToDevice, st) ||
-            cudaMemcpyAsync(dKey.p, ids->key, (size_t)ids->n_ids * 8, cudaMemcpyHostToDevice, st) ||
-            cudaMemcpyAsync(dVs.p, ids->var_start, (size_t)(ids->n_ids + 1) * 4, cudaMemcpyHostToDevice, st) ||
-            cudaMemcpyAsync(dBs.p, ids->bit_start, (size_t)(n_vars + 1) * 4, cudaMemcpyHostToDevice, st) ||
-            (n_bits && cudaMemcpyAsync(dBits.p, ids->bits, (size_t)n_bits * 4, cudaMemcpyHostToDevice, st)) ||
-            (n_vars && cudaMemcpyAsync(dBus.p, ids->bus, n_vars, cudaMemcpyHostToDevice, st)) ||
-            cudaMemsetAsync(dFlag.p, 0, 16, st)) {
+        if (cudaMemcpyAsync(dB, body, n, cudaMemcpyHostToDevice, st) ||
+            cudaMemcpyAsync(dKey, ids->key, (size_t)ids->n_ids * 8, cudaMemcpyHostToDevice, st) ||
+            cudaMemcpyAsync(dVs, ids->var_start, (size_t)(ids->n_ids + 1) * 4, cudaMemcpyHostToDevice, st) ||
+            cudaMemcpyAsync(dBs, ids->bit_start, (size_t)(n_vars + 1) * 4, cudaMemcpyHostToDevice, st) ||
+            (n_bits && cudaMemcpyAsync(dBits, ids->bits, (size_t)n_bits * 4, cudaMemcpyHostToDevice, st)) ||
+            (n_vars && cudaMemcpyAsync(dBus, ids->bus, n_vars, cudaMemcpyHostToDevice, st)) ||
+            cudaMemsetAsync(dFlag, 0, 16, st)) {
             rc = GLS_ECUDA;
             break;
         }
-        const uint8_t *B = dB.as<uint8_t>();
-        k_count_starts<<<tiles, 256, 0, st>>>(B, n, dTileCnt.as<uint32_t>());
-        if (device_incl_scan<uint32_t>(dTileCnt.as<uint32_t>(), dTileCnt.as<uint32_t>(), tiles,
-                                       dTileAgg.as<uint32_t>(), Sum(), st)) {
+        const uint8_t *B = dB;
+        k_count_starts<<<tiles, 256, 0, st>>>(B, n, dTileCnt);
+        if (device_incl_scan<uint32_t>(dTileCnt, dTileCnt, tiles,
+                                       dTileAgg, Sum(), st)) {
             rc = GLS_ECUDA;
             break;
         }
         uint32_t T = 0;
-        if (cudaMemcpyAsync(&T, dTileCnt.as<uint32_t>() + tiles - 1, 4, cudaMemcpyDeviceToHost, st) ||
+        if (cudaMemcpyAsync(&T, dTileCnt + tiles - 1, 4, cudaMemcpyDeviceToHost, st) ||
             cudaStreamSynchronize(st)) {
             rc = GLS_ECUDA;
             break;
         }
         if (T == 0) break;
         const uint32_t T_tiles = (T + kScanTile - 1) / kScanTile;
-        if (!dTok.alloc((size_t)T * 4) || !dLen.alloc((size_t)T * 4) || !dCls.alloc(T) ||
-            !dM1.alloc((size_t)T * 16) || !dM2.alloc((size_t)T * 16) || !dM3.alloc((size_t)T * 16) ||
-            !dAgg4.alloc((size_t)T_tiles * 16) || !dCnt.alloc((size_t)T * 8) || !dAt.alloc((size_t)T * 8) ||
-            !dAgg1.alloc((size_t)T_tiles * 8)) {
+        if (!tokens.alloc(part(dTok, T), part(dLen, T), part(dCls, T), part(dM1, T), part(dM2, T), part(dM3, T),
+                          part(dAgg4, T_tiles), part(dCnt, T), part(dAt, T), part(dAgg1, T_tiles))) {
             rc = GLS_ENOMEM;
             break;
         }
-        k_write_starts<<<tiles, 256, 0, st>>>(B, n, dTileCnt.as<uint32_t>(), dTok.as<uint32_t>());
+        k_write_starts<<<tiles, 256, 0, st>>>(B, n, dTileCnt, dTok);
         int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
         const uint32_t grid = (uint32_t)std::max(1, sms) * 8;
-        k_classify<<<grid, 256, 0, st>>>(B, n, dTok.as<uint32_t>(), T, dCls.as<uint8_t>(), dLen.as<uint32_t>());
-        k_marks1<<<grid, 256, 0, st>>>(dCls.as<uint8_t>(), T, dM1.as<uint4>());
-        if (device_incl_scan<uint4>(dM1.as<uint4>(), dM1.as<uint4>(), T, dAgg4.as<uint4>(), Max4(), st)) {
+        k_classify<<<grid, 256, 0, st>>>(B, n, dTok, T, dCls, dLen);
+        k_marks1<<<grid, 256, 0, st>>>(dCls, T, dM1);
+        if (device_incl_scan<uint4>(dM1, dM1, T, dAgg4, Max4(), st)) {
             rc = GLS_ECUDA;
             break;
         }
-        k_marks2<<<grid, 256, 0, st>>>(dCls.as<uint8_t>(), T, dM1.as<uint4>(), dM2.as<uint4>());
-        if (device_incl_scan<uint4>(dM2.as<uint4>(), dM2.as<uint4>(), T, dAgg4.as<uint4>(), Max4(), st)) {
+        k_marks2<<<grid, 256, 0, st>>>(dCls, T, dM1, dM2);
+        if (device_incl_scan<uint4>(dM2, dM2, T, dAgg4, Max4(), st)) {
             rc = GLS_ECUDA;
             break;
         }
-        k_marks3<<<grid, 256, 0, st>>>(dCls.as<uint8_t>(), T, dM1.as<uint4>(), dM2.as<uint4>(), dM3.as<uint4>(),
-                                       dFlag.as<uint32_t>());
-        if (device_incl_scan<uint4>(dM3.as<uint4>(), dM3.as<uint4>(), T, dAgg4.as<uint4>(), Max4(), st)) {
+        k_marks3<<<grid, 256, 0, st>>>(dCls, T, dM1, dM2, dM3,
+                                       dFlag);
+        if (device_incl_scan<uint4>(dM3, dM3, T, dAgg4, Max4(), st)) {
             rc = GLS_ECUDA;
             break;
         }
-        Ids di{dKey.as<uint64_t>(), dVs.as<uint32_t>(), dBs.as<uint32_t>(), dBits.as<uint32_t>(), dBus.as<uint8_t>(),
+        Ids di{dKey, dVs, dBs, dBits, dBus,
                ids->n_ids};
-        k_count_bits<<<grid, 256, 0, st>>>(B, dTok.as<uint32_t>(), dLen.as<uint32_t>(), dCls.as<uint8_t>(), T,
-                                           dM1.as<uint4>(), dM2.as<uint4>(), di, dCnt.as<unsigned long long>());
-        if (device_incl_scan<unsigned long long>(dCnt.as<unsigned long long>(), dAt.as<unsigned long long>(), T,
-                                                 dAgg1.as<unsigned long long>(), Sum64(), st)) {
+        k_count_bits<<<grid, 256, 0, st>>>(B, dTok, dLen, dCls, T,
+                                           dM1, dM2, di, dCnt);
+        if (device_incl_scan<unsigned long long>(dCnt, dAt, T,
+                                                 dAgg1, Sum64(), st)) {
             rc = GLS_ECUDA;
             break;
         }
         uint32_t flag = 0;
         unsigned long long total = 0;
-        if (cudaMemcpyAsync(&flag, dFlag.p, 4, cudaMemcpyDeviceToHost, st) ||
-            cudaMemcpyAsync(&total, dAt.as<unsigned long long>() + T - 1, 8, cudaMemcpyDeviceToHost, st) ||
+        if (cudaMemcpyAsync(&flag, dFlag, 4, cudaMemcpyDeviceToHost, st) ||
+            cudaMemcpyAsync(&total, dAt + T - 1, 8, cudaMemcpyDeviceToHost, st) ||
             cudaStreamSynchronize(st)) {
             rc = GLS_ECUDA;
             break;
@@ -511,15 +553,14 @@ extern "C" int gls_vcd_scan(int device, const char *body, uint64_t n_bytes, cons
             break;
         }
         if (total == 0) break;
-        if (!dSig.alloc((size_t)total * 4) || !dTime.alloc((size_t)total * 8) || !dVal.alloc(total) ||
-            !dBusOut.alloc(total)) {
+        if (!results.alloc(part(dTime, total), part(dSig, total), part(dVal, total), part(dBusOut, total))) {
             rc = GLS_ENOMEM;
             break;
         }
-        k_emit<<<grid, 256, 0, st>>>(B, dTok.as<uint32_t>(), dLen.as<uint32_t>(), dCls.as<uint8_t>(), T,
-                                     dM3.as<uint4>(), di, dCnt.as<unsigned long long>(), dAt.as<unsigned long long>(),
-                                     dSig.as<uint32_t>(),
-                                     dTime.as<unsigned long long>(), dVal.as<uint8_t>(), dBusOut.as<uint8_t>());
+        k_emit<<<grid, 256, 0, st>>>(B, dTok, dLen, dCls, T,
+                                     dM3, di, dCnt, dAt,
+                                     dSig,
+                                     dTime, dVal, dBusOut);
         out->signal = static_cast<uint32_t *>(std::malloc((size_t)total * 4));
         out->time = static_cast<uint64_t *>(std::malloc((size_t)total * 8));
         out->value = static_cast<uint8_t *>(std::malloc(total));
@@ -528,10 +569,11 @@ extern "C" int gls_vcd_scan(int device, const char *body, uint64_t n_bytes, cons
             rc = GLS_ENOMEM;
             break;
         }
-        if (cudaMemcpyAsync(out->signal, dSig.p, (size_t)total * 4, cudaMemcpyDeviceToHost, st) ||
-            cudaMemcpyAsync(out->time, dTime.p, (size_t)total * 8, cudaMemcpyDeviceToHost, st) ||
-            cudaMemcpyAsync(out->value, dVal.p, total, cudaMemcpyDeviceToHost, st) ||
-            cudaMemcpyAsync(out->bus, dBusOut.p, total, cudaMemcpyDeviceToHost, st) || cudaStreamSynchronize(st)) {
+        touch_pages({{out->signal, (size_t)total * 4}, {out->time, (size_t)total * 8}, {out->value, total}, {out->bus, total}});
+        if (cudaMemcpyAsync(out->signal, dSig, (size_t)total * 4, cudaMemcpyDeviceToHost, st) ||
+            cudaMemcpyAsync(out->time, dTime, (size_t)total * 8, cudaMemcpyDeviceToHost, st) ||
+            cudaMemcpyAsync(out->value, dVal, total, cudaMemcpyDeviceToHost, st) ||
+            cudaMemcpyAsync(out->bus, dBusOut, total, cudaMemcpyDeviceToHost, st) || cudaStreamSynchronize(st)) {
             rc = GLS_ECUDA;
             break;
         }

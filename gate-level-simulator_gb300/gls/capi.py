@@ -8,6 +8,7 @@ libgls.so is missing or no CUDA device is present, calls raise.
 from __future__ import annotations
 
 import ctypes as C
+from itertools import chain
 from pathlib import Path
 
 import numpy as np
@@ -271,41 +272,52 @@ class VcdChanges(C.Structure):
                 ("value", C.POINTER(C.c_uint8)), ("bus", C.POINTER(C.c_uint8)), ("fallback", C.c_int)]
 
 
+class _VcdResult:
+    """gls_vcd_scan's arrays.  The numpy arrays are views of the library's
+    memory (a copy of them would fault in as much fresh memory again); it is
+    freed with the last of them."""
+    def __init__(self, lib):
+        self.lib, self.changes = lib, VcdChanges()
+
+    def __del__(self):
+        self.lib.gls_vcd_free(C.byref(self.changes))
+
+    def array(self, field, dtype):
+        n = int(self.changes.n)
+        if n == 0:
+            return np.zeros(0, dtype)
+        mem = (C.c_char * (n * np.dtype(dtype).itemsize)).from_address(
+            C.cast(getattr(self.changes, field), C.c_void_p).value)
+        mem.owner = self
+        return np.frombuffer(mem, dtype)
+
+
 def vcd_scan(body: bytes, codes: dict[str, list[tuple[list[int], bool]]], device: int = 0):
     """Bit changes of a VCD body on the GPU (gls_vcd_scan).  codes: identifier
     code -> declarations (bit signals msb first, bus flag).  Returns
     (signal, time, value, bus, fallback) in file order."""
     lib = load_library()
-    keyed = []
-    for code, decls in codes.items():
-        b = code.encode()
-        if not 0 < len(b) <= 8:
-            raise ValueError("identifier codes of 1 to 8 bytes")
-        keyed.append((int.from_bytes(b, "little"), decls))
-    keyed.sort(key=lambda x: x[0])
-    key = np.array([k for k, _ in keyed], np.uint64)
-    var_start, bit_start, bits, bus = [0], [0], [], []
-    for _, decls in keyed:
-        for sig, is_bus in decls:
-            bits.extend(sig)
-            bit_start.append(len(bits))
-            bus.append(1 if is_bus else 0)
-        var_start.append(len(bus))
-    arrs = [key, np.array(var_start, np.uint32), np.array(bit_start, np.uint32), np.array(bits, np.uint32),
-            np.array(bus, np.uint8)]
+    names = [code.encode() for code in codes]
+    if names and not (min(map(len, names)) > 0 and max(map(len, names)) <= 8):
+        raise ValueError("identifier codes of 1 to 8 bytes")
+    key = np.frombuffer(b"".join([b.ljust(8, b"\0") for b in names]), "<u8")
+    order = np.argsort(key, kind="stable")
+    vals = list(codes.values())
+    vals = [vals[i] for i in order.tolist()]
+    decls = list(chain.from_iterable(vals))
+    sigs = [sig for sig, _ in decls]
+    starts = lambda counts: np.concatenate([np.zeros(1, np.uint32), np.cumsum(list(map(len, counts)), dtype=np.uint32)])
+    arrs = [key[order], starts(vals), starts(sigs), np.array(list(chain.from_iterable(sigs)), np.uint32),
+            np.array([1 if is_bus else 0 for _, is_bus in decls], np.uint8)]
     ids = VcdIds(len(key), *[_ptr(a) if len(a) else None for a in arrs])
-    out = VcdChanges()
-    buf = C.create_string_buffer(body, len(body))
-    rc = lib.gls_vcd_scan(device, buf, len(body), C.byref(ids), C.byref(out))
+    if not isinstance(body, bytes):
+        raise TypeError("body must be bytes")
+    out = _VcdResult(lib)
+    rc = lib.gls_vcd_scan(device, body, len(body), C.byref(ids), C.byref(out.changes))
     if rc:
         raise GlsError(rc, "gls_vcd_scan")
-    try:
-        n = int(out.n)
-        take = lambda p, dt: np.ctypeslib.as_array(p, (n,)).astype(dt) if n else np.zeros(0, dt)
-        return (take(out.signal, np.uint32), take(out.time, np.uint64), take(out.value, np.uint8),
-                take(out.bus, np.uint8), bool(out.fallback))
-    finally:
-        lib.gls_vcd_free(C.byref(out))
+    return (out.array("signal", np.uint32), out.array("time", np.uint64), out.array("value", np.uint8),
+            out.array("bus", np.uint8), bool(out.changes.fallback))
 
 
 def netlist_preds(in_nets: list[list[int]], out_nets: list[list[int]]):
@@ -433,9 +445,13 @@ class Simulator:
 
     def waveform(self, net: int, window: int = 0):
         n = C.c_uint64()
-        self._check(self.lib.gls_waveform(self.h, window, net, None, None, 0, C.byref(n)), "waveform")
+        t = np.empty(1024, np.uint32)   # most lists are short: read with their length in one call
+        v = np.empty(1024, np.uint8)
+        self._check(self.lib.gls_waveform(self.h, window, net, _ptr(t), _ptr(v), len(t), C.byref(n)), "waveform")
         if n.value == 2**64 - 1:
             return None
+        if n.value <= len(t):
+            return t[:n.value].copy(), v[:n.value].copy()
         t = np.zeros(n.value, np.uint32)
         v = np.zeros(n.value, np.uint8)
         self._check(self.lib.gls_waveform(self.h, window, net, _ptr(t), _ptr(v), n.value, C.byref(n)), "waveform")
