@@ -342,7 +342,7 @@ struct ListReader<uint32_t> {
     static __device__ __forceinline__ uint32_t ld_if(const uint32_t *q, bool go)
     {
         uint32_t v;
-        asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\tmov.u32 %0, 0xFFFFFFFF;\n\t@p ld.global.nc.u32 %0, [%1];\n\t}"
+        asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\tmov.u32 %0, 0xFFFFFFFF;\n\t@p ld.global.u32 %0, [%1];\n\t}"
             : "=r"(v) : "l"(q), "r"((uint32_t)go));
         return v;
     }
@@ -358,7 +358,7 @@ struct ListReader<uint32_t> {
         const bool more = go && (uint32_t)(uintptr_t)q != qe;
         h = go ? n : h;
         asm("{\n\t.reg .pred p, r;\n\tsetp.ne.u32 p, %2, 0;\n\tsetp.ne.u32 r, %3, 0;\n\t@p mov.u32 %0, 0xFFFFFFFF;\n\t"
-            "@r ld.global.nc.u32 %0, [%1];\n\t}"
+            "@r ld.global.u32 %0, [%1];\n\t}"
             : "+r"(n) : "l"(q), "r"((uint32_t)go), "r"((uint32_t)more));
         q += more ? 1 : 0;
     }
@@ -371,7 +371,7 @@ struct ListReader<WideWord> {   // a list of up to 2^32 events: its end is a who
     static __device__ __forceinline__ WideWord ld_if(const WideWord *q, bool go)
     {
         WideWord v;
-        asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\tmov.u64 %0, -1;\n\t@p ld.global.nc.u64 %0, [%1];\n\t}"
+        asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\tmov.u64 %0, -1;\n\t@p ld.global.u64 %0, [%1];\n\t}"
             : "=l"(v) : "l"(q), "r"((uint32_t)go));
         return v;
     }
@@ -387,7 +387,7 @@ struct ListReader<WideWord> {   // a list of up to 2^32 events: its end is a who
         const bool more = go && q != qe;
         h = go ? n : h;
         asm("{\n\t.reg .pred p, r;\n\tsetp.ne.u32 p, %2, 0;\n\tsetp.ne.u32 r, %3, 0;\n\t@p mov.u64 %0, -1;\n\t"
-            "@r ld.global.nc.u64 %0, [%1];\n\t}"
+            "@r ld.global.u64 %0, [%1];\n\t}"
             : "+l"(n) : "l"(q), "r"((uint32_t)go), "r"((uint32_t)more));
         q += more ? 1 : 0;
     }

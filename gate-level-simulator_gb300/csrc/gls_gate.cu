@@ -46,14 +46,12 @@ struct GateSmem {
     uint32_t xt;                 // latest X or Z of the list but its first entry
 };
 
-// Per thread of the block, one time segment: shared arrays behind GateSmem.
-struct SegSmem {
-    uint32_t *tcut;   // time it starts at
-    uint32_t *src;    // its first kept entry, from the gate output's stacks on
-    uint32_t *n;      // entries kept
-    uint32_t *pos;    // their place in the list
-    uint32_t *pv;     // value before them
-};
+// kWarp: blocks of one warp
+template <bool kWarp> __device__ __forceinline__ void sync_block()
+{
+    if (kWarp) __syncwarp();
+    else __syncthreads();
+}
 
 // The thread's part of a gate output after the walk.
 template <class Wd>
@@ -67,9 +65,10 @@ struct Walked {
 // Cut and walk gate output i of the level.
 template <int M, bool kTab, class Wd>
 __device__ __forceinline__ Walked<Wd> walk_gate(const WinDev &w, const LevelArgs &a, uint32_t i, GateSmem &sm,
-                                            const SegSmem &sg)
+                                            uint32_t *s_seg)
 {
-    const uint32_t tid = threadIdx.x, nthr = blockDim.x;
+    constexpr bool kWarp = !kTab && M <= 3;
+    const uint32_t tid = threadIdx.x, nthr = kWarp ? 32u : blockDim.x;
     const uint32_t drv = a.lo + i;
     const Wd *const pool = reinterpret_cast<const Wd *>(w.pool);
     const DrvMeta *__restrict__ mdp = a.meta + drv;
@@ -95,7 +94,7 @@ __device__ __forceinline__ Walked<Wd> walk_gate(const WinDev &w, const LevelArgs
             len[j] = w.net_len[net];
             E += len[j];
             lmin = min(lmin, len[j]);
-            if (kTab) xmax = max(xmax, w.net_len[a.n_nets + net]);
+            if (kTab && a.x_times) xmax = max(xmax, w.net_len[a.n_nets + net]);
             if (len[j] > plen) { sec = piv; slen = plen; plen = len[j]; piv = j; }
             else if (sec < 0 || len[j] > slen) { sec = j; slen = len[j]; }
         }
@@ -113,7 +112,7 @@ __device__ __forceinline__ Walked<Wd> walk_gate(const WinDev &w, const LevelArgs
     const unsigned long long scr_need = (E + S + 3) & ~3ull;
     unsigned long long scr_at = 0;   // thread 0; used once the cuts are found
     if (tid == 0) scr_at = atomicAdd(&w.lvl[a.level].scr, scr_need);
-    const bool usable = kTab && f1.w != 0u;   // the step table is
+    const bool usable = kTab && a.x_times && f1.w != 0u;   // the step table is
     uint32_t tabw = 0;   // a word of the tables, stored once the cuts are found
     const uint32_t tk = nthr - 1 - tid;
     if constexpr (kSm) {
@@ -131,7 +130,7 @@ __device__ __forceinline__ Walked<Wd> walk_gate(const WinDev &w, const LevelArgs
     for (int j = 0; j < M; ++j) cb[j] = 0;
     if (mine && tid > 0)
         tcut = cut_at<M, !kTab>(pool, off, len, m, piv, sec, poff, soff, plen, slen, sk, sn, cb);
-    if (mine) sg.tcut[tid] = tcut;
+    if (mine) s_seg[tid] = tcut;
     if constexpr (kTab) {
         if (usable)
             for (uint32_t e = tid; e < 1u << (2 * M); e += nthr) sm.tab.step[e] = step_entry<M>(f0, f1, e);
@@ -143,7 +142,7 @@ __device__ __forceinline__ Walked<Wd> walk_gate(const WinDev &w, const LevelArgs
         sm.ok = scr_at + scr_need <= w.scr_cap;
         if (!sm.ok) atomicOr(w.err, kErrScratch);
     }
-    __syncthreads();
+    sync_block<kWarp>();
     Wd *const scr = reinterpret_cast<Wd *>(w.scratch) + sm.scr;
     uint32_t region = tid;
     WalkOut<Wd> o = {0, EvW<Wd>::kInfW, 0, 0};
@@ -161,7 +160,7 @@ __device__ __forceinline__ Walked<Wd> walk_gate(const WinDev &w, const LevelArgs
             }
             rd[j].start(x, cb[j], len[j]);
         }
-        const uint32_t tnext = tid + 1 < S ? sg.tcut[tid + 1] : kInf;
+        const uint32_t tnext = tid + 1 < S ? s_seg[tid + 1] : kInf;
         if (tnext != kInf) {
             tmax = tnext;
         } else {
@@ -188,19 +187,20 @@ __device__ __forceinline__ Walked<Wd> walk_gate(const WinDev &w, const LevelArgs
 // fetch: thread 0 sets sm.q and sm.skip to the block's next gate output; called
 // where the wait for it overlaps others and every thread has read the present
 // one.
-template <class Wd, class Fetch>
+template <bool kWarp, class Wd, class Fetch>
 __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a, uint32_t i, GateSmem &sm,
-                                            const SegSmem &sg, const Walked<Wd> &wk, Fetch fetch)
+                                            uint32_t *s_seg, const Walked<Wd> &wk, Fetch fetch)
 {
     const unsigned FULL = 0xffffffffu;
-    const uint32_t tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31u, wid = tid >> 5, nw = nthr >> 5;
+    const uint32_t tid = threadIdx.x, nthr = kWarp ? 32u : blockDim.x;
+    const uint32_t lane = tid & 31u, wid = kWarp ? 0u : tid >> 5, nw = nthr >> 5;
     const DrvMeta *__restrict__ mdp = a.meta + a.lo + i;
     const WalkOut<Wd> &o = wk.o;
     const uint32_t region = wk.region, S = wk.S;
     const unsigned long long E = wk.E;
     const bool mine = tid < S;
     if (!sm.ok) {   // no room for its stacks; the same for the whole block
-        __syncthreads();
+        sync_block<kWarp>();
         if (tid == 0) fetch();
         return;
     }
@@ -214,10 +214,10 @@ __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a,
         const Wd y = __shfl_down_sync(FULL, x, k);
         if (lane + k < 32) x = min(x, y);
     }
-    if (lane == 0) sm.wmin[wid] = x;
+    if (!kWarp && lane == 0) sm.wmin[wid] = x;
     Wd later = __shfl_down_sync(FULL, x, 1);
     if (lane == 31) later = EvW<Wd>::kInfW;
-    __syncthreads();
+    if (!kWarp) __syncthreads();
     for (uint32_t k = wid + 1; k < nw; ++k) later = min(later, (Wd)sm.wmin[k]);
     uint32_t keep = o.cnt, firstv = 0, lastv = 0;
     if (keep && later != EvW<Wd>::kInfW)
@@ -232,7 +232,7 @@ __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a,
     uint32_t vprev = __shfl_sync(FULL, lastv, prior ? 31 - __clz(prior) : 0);
     const uint32_t vtop = __shfl_sync(FULL, lastv, bal ? 31 - __clz(bal) : 0);
     if (lane == 0) sm.wlast[wid] = bal ? vtop : 4u;
-    __syncthreads();
+    if (!kWarp) __syncthreads();
     if (!prior) {
         vprev = kVX;
         for (int k = (int)wid - 1; k >= 0; --k)
@@ -246,19 +246,23 @@ __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a,
         const uint32_t y = __shfl_up_sync(FULL, inc, k);
         if (lane >= k) inc += y;
     }
-    if (lane == 31) sm.wsum[wid] = inc;
-    __syncthreads();
     uint32_t pos = inc - fin, total = 0;
-    for (uint32_t k = 0; k < nw; ++k) {
-        if (k < wid) pos += sm.wsum[k];
-        total += sm.wsum[k];
+    if (kWarp) {
+        total = __shfl_sync(FULL, inc, 31);
+    } else {
+        if (lane == 31) sm.wsum[wid] = inc;
+        __syncthreads();
+        for (uint32_t k = 0; k < nw; ++k) {
+            if (k < wid) pos += sm.wsum[k];
+            total += sm.wsum[k];
+        }
     }
-    if (mine) {
-        sg.src[tid] = region + drop;
-        sg.n[tid] = fin;
-        sg.pos[tid] = pos;
-        sg.pv[tid] = vprev;
-    }
+    // per warp, the segments that keep entries: where in the stacks the list's
+    // entry 0 would be
+    const unsigned some = __ballot_sync(FULL, fin > 0);
+    uint32_t *const delta = s_seg + (tid & ~31u);
+    __syncwarp();   // the cut times that were here have been read
+    if (fin) delta[__popc(some & ((1u << lane) - 1u))] = region + drop - pos;
     if (tid == 0) {
         // the list's place: reserved up front for its bound or its predicted
         // length, or (exact placement, or a list longer than predicted) as long as it is
@@ -292,52 +296,51 @@ __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a,
                 for (int p = 0; p < mdp->n_pins; ++p) sm.ctr[0] += w.net_len[mdp->net[(mdp->pin_slot >> (3 * p)) & 7u]];
         }
     }
-    __syncthreads();
+    sync_block<kWarp>();
     if (!sm.ok) return;
-    // Copy, eight lanes a segment, with the SAIF integral: an entry at time t
-    // ends the hold of the value before it and starts its own, so class c's
-    // time is the sum of t over the entries after a value of class c minus
-    // the sum over those of class c, plus t_end for the last value's class.
-    // Times are window-relative and below 2^30: the sums wrap in 32 bits and
-    // are read back as signed.  (Four consecutive entries of the list a
-    // thread, found by bisection, and one 16-byte store: 75.1 ms instead of
-    // 74.4 on the 2 M cell design, 32.8 instead of 29.1 in waves.)
-    constexpr uint32_t W = 8, U = 4;
-    const uint32_t sub = tid & (W - 1);
+    // Copy, with the SAIF integral: an entry at time t ends the hold of the
+    // value before it and starts its own, so class c's time is the sum of t
+    // over the entries after a value of class c minus the sum over those of
+    // class c, plus t_end for the last value's class.  Times are
+    // window-relative and below 2^30: the sums wrap in 32 bits and are read
+    // back as signed.  A warp's segments make a contiguous part of the list:
+    // it copies 32 entries at a time, and finds each one's segment by counting
+    // the segments that start up to there.  The stacks come from L2, so U
+    // times 32 entries are loaded before the first is stored.  Against eight
+    // lanes a segment, four entries each at a time, device ms: 2 M cells 73.8
+    // -> 69.6 (U = 1 / 2 / 4 / 6 / 8: 78.7 / 73.4 / 71.1 / 69.5 / 69.7),
+    // 200,000 cells 13.7 -> 12.7 (15.1 / 13.8 / 13.1 / 12.8 / 12.7), waves of
+    // 200,000 cells, whose warps hold some 300 entries, 23.3 -> 20.8 (- / 20.9
+    // / 21.7 / - / -).
+    constexpr uint32_t U = kWarp ? 2 : 8;
     using P = SaifP<Wd>;
     const RelClampT<P> rc(w.t_begin, w.t_end);
     P s0 = 0, s1 = 0;
     Wd *const dst = reinterpret_cast<Wd *>(w.pool) + sm.dst;
-    for (uint32_t b = wid * (32 / W); b < S; b += nthr / W) {   // a warp's four segments
-        const uint32_t k = b + (lane / W);
-        const uint32_t n = k < S ? sg.n[k] : 0u;
-        uint32_t nmax = n;
-        nmax = max(nmax, __shfl_xor_sync(FULL, nmax, 8));
-        nmax = max(nmax, __shfl_xor_sync(FULL, nmax, 16));
-        if (nmax == 0) continue;
-        const Wd *sp = scr + (k < S ? sg.src[k] : 0u);
-        Wd *dp = dst + (k < S ? sg.pos[k] : 0u);
-        uint32_t pv = k < S ? sg.pv[k] : 0u;
-        for (uint32_t e0 = 0; e0 < nmax; e0 += W * U) {
-            Wd wd[U];
+    const uint32_t end = __shfl_sync(FULL, pos + fin, 31);
+    const uint32_t upto = 0xFFFFFFFFu >> (31 - lane);   // this lane and the ones below
+    uint32_t first = 0u - 1u;                           // segments that start before the 32 entries, less one
+    uint32_t before1 = __shfl_sync(FULL, vprev, 0);     // the value before them
+    for (uint32_t c = __shfl_sync(FULL, pos, 0); c < end; c += 32 * U) {
+        Wd wd[U];
 #pragma unroll
-            for (uint32_t u = 0; u < U; ++u) {
-                const uint32_t e = e0 + u * W + sub;
-                wd[u] = e < n ? sp[e] : Wd(0);
-            }
+        for (uint32_t u = 0; u < U; ++u) {
+            const uint32_t rel = pos - (c + 32 * u), e = c + 32 * u + lane;
+            const unsigned starts = __reduce_or_sync(FULL, fin > 0 && rel < 32 ? 1u << rel : 0u);
+            wd[u] = e < end ? scr[delta[first + __popc(starts & upto)] + e] : Wd(0);
+            first += __popc(starts);
+        }
 #pragma unroll
-            for (uint32_t u = 0; u < U; ++u) {
-                const uint32_t e = e0 + u * W + sub;
-                uint32_t before = __shfl_up_sync(FULL, ev_val(wd[u]), 1, W);
-                if (sub == 0) before = pv;
-                pv = __shfl_sync(FULL, ev_val(wd[u]), W - 1, W);
-                if (e < n) {
-                    dp[e] = wd[u];
-                    const P t = rc(ev_time(wd[u]));
-                    const uint32_t c = ev_val(wd[u]);
-                    s0 += (before == kV0 ? t : P(0)) - (c == kV0 ? t : P(0));
-                    s1 += (before == kV1 ? t : P(0)) - (c == kV1 ? t : P(0));
-                }
+        for (uint32_t u = 0; u < U; ++u) {
+            const uint32_t e = c + 32 * u + lane, v = ev_val(wd[u]);
+            uint32_t before = __shfl_up_sync(FULL, v, 1);
+            if (lane == 0) before = before1;
+            before1 = __shfl_sync(FULL, v, 31);
+            if (e < end) {
+                dst[e] = wd[u];
+                const P t = rc(ev_time(wd[u]));
+                s0 += (before == kV0 ? t : P(0)) - (v == kV0 ? t : P(0));
+                s1 += (before == kV1 ? t : P(0)) - (v == kV1 ? t : P(0));
             }
         }
     }
@@ -346,15 +349,22 @@ __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a,
         s0 += __shfl_xor_sync(FULL, s0, k);
         s1 += __shfl_xor_sync(FULL, s1, k);
     }
-    if (lane == 0) { sm.s0[wid] = s0; sm.s1[wid] = s1; }
-    __syncthreads();
+    uint32_t last = vtop;   // one warp: that of its last kept entry
+    if (kWarp) {
+        if (!bal) last = kVX;
+    } else {
+        if (lane == 0) { sm.s0[wid] = s0; sm.s1[wid] = s1; }
+        __syncthreads();
+    }
     if (tid == 0) {
-        uint32_t last = kVX;
-        s0 = s1 = 0;
-        for (uint32_t k = 0; k < nw; ++k) {
-            s0 += (P)sm.s0[k];
-            s1 += (P)sm.s1[k];
-            if (sm.wlast[k] < 4u) last = sm.wlast[k];
+        if (!kWarp) {
+            last = kVX;
+            s0 = s1 = 0;
+            for (uint32_t k = 0; k < nw; ++k) {
+                s0 += (P)sm.s0[k];
+                s1 += (P)sm.s1[k];
+                if (sm.wlast[k] < 4u) last = sm.wlast[k];
+            }
         }
         using Sg = typename std::make_signed<P>::type;
         const unsigned long long D = w.t_end - w.t_begin;
@@ -369,25 +379,28 @@ __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a,
 
 }  // namespace
 
-// kTab = false is the kernel of one-warp blocks.  Their 32 warps on an SM run
-// all over it, and it is bound by instruction fetch (2.7 warps waiting for
-// instructions per issue): finish_gate is no template (three copies of it cost
-// 28.6 instead of 26.7 ms on 8 windows of 200,000 cells), and the cut searches
-// and irregular delays are calls (22.2 ms; on the 2 M cell design, whose
-// blocks of four warps run the other kernel, calls cost 75.8 instead of 73.9).
+// kTab = false is the kernel of one-warp blocks (and of the class of four to
+// six input nets).  Their 32 warps on an SM run all over it, and it is bound
+// by instruction fetch (2.3 warps waiting for instructions per issue): it has
+// one copy of finish_gate (three copies cost 28.6 instead of 26.7 ms on 8
+// windows of 200,000 cells), the cut searches and irregular delays are calls
+// (22.2 ms; on the 2 M cell design, whose blocks of four warps run the other
+// kernel, calls cost 75.8 instead of 73.9), and what only meets between warps
+// is left out (23.3 -> 20.8 ms).
 //
 // Gate outputs [d0, d1) of the level of every window of the launch (kSix: the
 // class of four to six input nets, else the narrower ones; c1, c2: where the
 // 2- and 3-input ones start).  Blocks take gate outputs from the back, the
 // widest first, as they become free.
 template <bool kBatch, bool kSix, bool kTab, class Wd>
-__global__ void __launch_bounds__(kGateMaxThreads, kSix ? 1 : gate_resident<Wd>() / kGateMaxThreads)
+__global__ void __launch_bounds__(kSix || kTab ? kGateMaxThreads : 32,
+                                  kSix ? 1 : gate_resident<Wd>() / (kTab ? kGateMaxThreads : 32))
     k_gate(const WinSet<kBatch> ws, LevelArgs a, uint32_t d0, uint32_t d1, uint32_t c1, uint32_t c2)
 {
     __shared__ GateSmem sm;
-    extern __shared__ uint32_t s_seg[];
-    const uint32_t nthr = blockDim.x;
-    const SegSmem sg = {s_seg, s_seg + nthr, s_seg + 2 * nthr, s_seg + 3 * nthr, s_seg + 4 * nthr};
+    extern __shared__ uint32_t s_seg[];   // per thread the time its segment starts at; then see finish_gate
+    constexpr bool kWarp = !kSix && !kTab;
+    const uint32_t nthr = kWarp ? 32u : blockDim.x;
     const uint32_t n = d1 - d0, total = n * ws.size();
     auto fetch = [&](uint32_t q) {   // thread 0
         sm.q = q < total ? q : kInf;
@@ -410,7 +423,7 @@ __global__ void __launch_bounds__(kGateMaxThreads, kSix ? 1 : gate_resident<Wd>(
         fetch(blockIdx.x);   // the grid has at most one block per gate output
     }
     for (;;) {
-        __syncthreads();
+        sync_block<kWarp>();
         const uint32_t q = sm.q;
         if (q == kInf) break;
         const bool skip = sm.skip != 0;
@@ -418,7 +431,7 @@ __global__ void __launch_bounds__(kGateMaxThreads, kSix ? 1 : gate_resident<Wd>(
         if constexpr (kBatch) {
             // the window's descriptor in shared memory, out of the way of the walks
             const uint32_t cw = sm.cw;
-            __syncthreads();
+            sync_block<kWarp>();
             if (win != cw) {
                 if (threadIdx.x == 0) {
                     if (cw != kInf) flush();
@@ -426,13 +439,13 @@ __global__ void __launch_bounds__(kGateMaxThreads, kSix ? 1 : gate_resident<Wd>(
                 }
                 const uint32_t *src = reinterpret_cast<const uint32_t *>(&ws.get(win));
                 uint32_t *d = reinterpret_cast<uint32_t *>(&sm.win);
-                for (uint32_t k = threadIdx.x; k < sizeof(WinDev) / 4; k += blockDim.x) d[k] = src[k];
-                __syncthreads();
+                for (uint32_t k = threadIdx.x; k < sizeof(WinDev) / 4; k += nthr) d[k] = src[k];
+                sync_block<kWarp>();
             }
         }
         auto next = [&]() { fetch(gridDim.x == total ? total : gridDim.x + atomicAdd(&ws.get(0).lvl[a.level].next[kSix ? 0 : 1], 1u)); };
         if (skip) {
-            __syncthreads();   // sm.q is read
+            sync_block<kWarp>();   // sm.q is read
             if (threadIdx.x == 0) next();
             continue;
         }
@@ -440,13 +453,13 @@ __global__ void __launch_bounds__(kGateMaxThreads, kSix ? 1 : gate_resident<Wd>(
         auto go = [&](const WinDev &w) {
             Walked<Wd> wk;
             if constexpr (kSix) {
-                wk = walk_gate<kMaxSlots, false, Wd>(w, a, i, sm, sg);
+                wk = walk_gate<kMaxSlots, false, Wd>(w, a, i, sm, s_seg);
             } else {
-                if (i >= c2) wk = walk_gate<3, kTab, Wd>(w, a, i, sm, sg);
-                else if (i >= c1) wk = walk_gate<2, kTab, Wd>(w, a, i, sm, sg);
-                else wk = walk_gate<1, kTab, Wd>(w, a, i, sm, sg);
+                if (i >= c2) wk = walk_gate<3, kTab, Wd>(w, a, i, sm, s_seg);
+                else if (i >= c1) wk = walk_gate<2, kTab, Wd>(w, a, i, sm, s_seg);
+                else wk = walk_gate<1, kTab, Wd>(w, a, i, sm, s_seg);
             }
-            finish_gate(w, a, i, sm, sg, wk, next);
+            finish_gate<kWarp>(w, a, i, sm, s_seg, wk, next);
         };
         if constexpr (kBatch) go(sm.win);
         else go(ws.get(0));
@@ -454,10 +467,12 @@ __global__ void __launch_bounds__(kGateMaxThreads, kSix ? 1 : gate_resident<Wd>(
     if (threadIdx.x == 0 && (!kBatch || sm.cw != kInf)) flush();
 }
 
-void launch_gate(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelArgs &a, const uint32_t *cls,
+void launch_gate(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelArgs &level, const uint32_t *cls,
                  uint32_t threads, bool table, int sm_count, cudaStream_t st, uint32_t *launches)
 {
-    const uint32_t smem = threads * 5 * 4;
+    LevelArgs a = level;
+    a.x_times = table ? 1u : 0u;
+    const uint32_t smem = threads * 4;
     auto go = [&](auto six, auto tab, uint32_t d0, uint32_t d1) {
         constexpr bool kSix = decltype(six)::value, kTab = decltype(tab)::value;
         if (d1 <= d0) return;
@@ -488,7 +503,7 @@ void launch_gate(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelAr
     go(T(), F(), cls[3], cls[4]);
     // the step table is for warps none of whose segments starts at X: in a
     // block of one warp the first one does
-    if (table && threads > 32) go(F(), T(), 0u, cls[3]);
+    if (threads > 32) go(F(), T(), 0u, cls[3]);
     else go(F(), F(), 0u, cls[3]);
 }
 

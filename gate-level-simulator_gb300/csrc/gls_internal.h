@@ -214,6 +214,7 @@ struct LevelArgs {
     float bal_weight;           // learned mode: segment work = fan-in events + bal_weight * predicted output events
     uint32_t level;             // the level's number
     uint32_t n_nets;
+    uint32_t x_times;           // k_gate: the X times of the level's fan-in nets are known
     uint32_t plan_part;         // k_plan: 0 all of it; learned mode split in two: 1 segments and stacks
                                 // (slots left open), 2 slot placement from the predictions
 };

@@ -85,3 +85,26 @@ def test_wave_with_uneven_windows(threads, gpu, oracle_bin):
             lens = s.lengths(wid)
             gw = {n: s.waveform(n, wid) for n in range(nl.n_nets) if lens[n] != 2**32 - 1}
             assert_same(gw, s.saif(wid), ow, osaif, f"wave window {wid}")
+
+
+@pytest.mark.parametrize("every", [1, 3, 40, 400])
+@pytest.mark.parametrize("kept", [31, 32, 33, 64, 65, 255, 257, 513])
+def test_copy_of_sparse_segments(kept, every, gpu, oracle_bin):
+    """Glitch trains that a slow buffer swallows, with `every` events around
+    each edge that it keeps: lists of `kept` entries from segments of which
+    most keep nothing, or one entry each."""
+    c = LIBRARY["GEN_BUF_D1"]
+    nl = assemble([(c.name, [0], [1], default_arcs(c, 100.0, 100.0))], n_nets=2)
+    ev, t, v = [(0, 0)], 0, 0
+    for _ in range(kept):
+        for _ in range(2 * (every // 2)):   # glitches shorter than the delay
+            t, v = t + 3, 3 - v
+            ev.append((t, v))
+        t, v = t + 3, 3 - v
+        ev.append((t, v))
+        t += 500
+    st = stimulus({0: ev})
+    ow, osaif, _ = run_oracle(nl, st, 0, t + 50)
+    for threads in ("32", "128", "256"):
+        gw, gs, _, _ = gpu_run(nl, st, 0, t + 50, env={"GLS_GATE_THREADS": threads})
+        assert_same(gw, gs, ow, osaif, f"{threads} threads")
