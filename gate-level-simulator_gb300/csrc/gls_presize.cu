@@ -9,6 +9,36 @@
 namespace gls {
 
 // ------------------------------------------------------------- features
+// Expected output changes (est) and probability of a 1 (pone) of a gate output
+// of M input nets, from their lengths and 1-probabilities and its truth table
+// over their values; unrolled, so that nothing is looked up in memory.
+template <int M>
+__device__ __forceinline__ void sensitized(const uint4 &t, const float *len, const float *p1, float &est, float &pone)
+{
+    uint32_t F[1 << M];
+#pragma unroll
+    for (uint32_t b = 0; b < (1u << M); ++b)
+        F[b] = (((b & 4u) ? t.w : t.x) >> (((b & 1u) ? 6u : 0u) + ((b & 2u) ? 24u : 0u))) & 3u;
+#pragma unroll
+    for (uint32_t b = 0; b < (1u << M); ++b) {
+        float w = 1.f;
+#pragma unroll
+        for (int j = 0; j < M; ++j) w *= ((b >> j) & 1u) ? p1[j] : 1.f - p1[j];
+        if (F[b] == kV1) pone += w;
+#pragma unroll
+        for (int j = 0; j < M; ++j) {
+            if ((b >> j) & 1u) continue;
+            if (F[b | (1u << j)] != F[b]) {
+                float wo = 1.f;   // probability of the other inputs' values
+#pragma unroll
+                for (int i = 0; i < M; ++i)
+                    if (i != j) wo *= ((b >> i) & 1u) ? p1[i] : 1.f - p1[i];
+                est += wo * len[j];
+            }
+        }
+    }
+}
+
 // Row of a gate output: its static features (cell, pins, delays, fan-out,
 // truth-table sensitivity) with the input-net entries filled from the
 // lengths of its input nets' change lists.
@@ -55,6 +85,11 @@ __device__ __forceinline__ void gate_features(const PresizeArgs &a, uint32_t r, 
     const uint8_t *lut = a.lut + md.lut_off;
     const int m = md.m;
     float est = 0.f, pone = 0.f, pmean = 0.f;
+    const uint4 t = __ldg(a.slut + d);   // of up to three input nets
+    if (m == 1) sensitized<1>(t, len, p1, est, pone);
+    else if (m == 2) sensitized<2>(t, len, p1, est, pone);
+    else if (m == 3) sensitized<3>(t, len, p1, est, pone);
+    else
     for (uint32_t b = 0; b < (1u << m); ++b) {
         uint32_t idx = 0;
         for (int p = 0; p < md.n_pins; ++p)
@@ -77,7 +112,9 @@ __device__ __forceinline__ void gate_features(const PresizeArgs &a, uint32_t r, 
             }
         }
     }
-    for (int j = 0; j < m; ++j) pmean += p1[j];
+#pragma unroll
+    for (int j = 0; j < kMaxSlots; ++j)
+        if (j < m) pmean += p1[j];
     x[21] = log1pf(est) * (1.f / 12.f);
     x[22] = pone;
     x[23] = m ? pmean / m : 0.f;
@@ -246,6 +283,12 @@ __global__ void __launch_bounds__(128, 1) k_presize_tc(PresizeArgs a0)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    // launched while the level before still runs, whose lists the features are
+    // made of.  The level's gate outputs wait for the end of this kernel: their
+    // blocks stay on an SM for the whole level, and next to this kernel's
+    // shared memory they have little L1 (75.8 instead of 67.7 ms on the 2 M
+    // cell design; launched one after the other 69.7).
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     // A1: this thread's feature row in BF16, 16 bytes per 8 features
     const uint32_t r = blockIdx.x * 128 + tid;
     {
@@ -361,8 +404,19 @@ void launch_presize(const PresizeArgs &a, bool tensor_cores, cudaStream_t st)
 {
     if (!a.n) return;
     const dim3 grid((a.n + 127) / 128, a.wv ? a.nwin : 1);
-    if (tensor_cores) k_presize_tc<<<grid, 128, kSmTotal, st>>>(a);
-    else k_presize_f32<<<grid, 128, kParams * 4, st>>>(a);
+    if (tensor_cores) {
+        cudaLaunchAttribute at;
+        at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at.val.programmaticStreamSerializationAllowed = 1;
+        cudaLaunchConfig_t lc = {};
+        lc.gridDim = grid;
+        lc.blockDim = dim3(128);
+        lc.dynamicSmemBytes = kSmTotal;
+        lc.stream = st;
+        lc.attrs = &at;
+        lc.numAttrs = 1;
+        cudaLaunchKernelEx(&lc, k_presize_tc, a);
+    } else k_presize_f32<<<grid, 128, kParams * 4, st>>>(a);
 }
 
 // ------------------------------------------------------------- training
@@ -870,6 +924,7 @@ void ctx_presize_args(const gls_ctx *ctx, PresizeArgs *a)
     a->feat_static = ctx->feat_static.as<float>();
     a->meta = ctx->meta.as<DrvMeta>();
     a->lut = ctx->lut.as<uint8_t>();
+    a->slut = ctx->slut.as<uint4>();
     a->params = ctx->mlp_params.as<float>();
     a->img = ctx->mlp_img.as<uint4>();
     a->margin = ctx->margin;

@@ -32,6 +32,7 @@ struct PresizeArgs {
     const float *feat_static;     // per driver x 32
     const DrvMeta *meta;
     const uint8_t *lut;           // cell truth tables
+    const uint4 *slut;            // per driver with at most 3 input nets: truth table over its input nets' values
     const uint32_t *net_len;
     const unsigned long long *saif;   // T0 / T1 / TX per net (input nets are complete)
     uint32_t lo, n;
