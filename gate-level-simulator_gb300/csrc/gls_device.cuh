@@ -453,8 +453,9 @@ __device__ __forceinline__ uint32_t step_entry(const uint4 &f0, const uint4 &f1,
     return d << 2 | (F ? kV1 : kV0);
 }
 
-// What a gate output's walks read from shared memory (tab: its address).
-struct __align__(256) GateTab {
+// What a gate output's walks read from shared memory (tab: its address, a
+// multiple of 256: rows of the step table are found by ORing).
+struct GateTab {
     uint32_t step[64];   // the step table
     uint32_t slut[4];    // the truth table (LevelArgs::slut)
     uint32_t nd[24];     // its input nets' NetDelay entries (regular gate outputs)

@@ -30,18 +30,32 @@ constexpr int kMaxWarps = kGateMaxThreads / 32;
 // threads per SM the narrow classes' kernel is compiled for
 template <class Wd> __host__ __device__ constexpr uint32_t gate_resident() { return sizeof(Wd) == 4 ? 1024u : 768u; }
 
-struct GateSmem {
-    GateTab tab;                 // the gate output's tables
+// Shared memory is L1 lost: each kernel has only what it uses, the step table
+// (kTab), what meets between warps (not kWarp) and the window's descriptor
+// (kBatch).  With 512 bytes before the segments' a 1,024-thread SM gets by
+// with 16 KB (one step of the split more: 2 M cells 68.7 instead of 68.3 ms,
+// 200,000 cells 13.1 instead of 12.9); one-warp blocks with 272 bytes instead
+// of 1,280: 8 windows of 200,000 cells 19.8 -> 19.5, 48 of 2,000 cells .89 ->
+// .87.
+template <bool kTab> struct TabSmem { GateTab tab; };   // the gate output's tables
+template <> struct TabSmem<false> {};
+template <bool kWarp, class Wd> struct WarpsSmem {
+    Wd a[kMaxWarps];             // per warp: smallest candidate of its segments; at the end its part of T0
+    Wd b[kMaxWarps];             // kept entries; at the end its part of T1
+    uint8_t wlast[kMaxWarps];    // value of its last kept entry (4: none)
+};
+template <class Wd> struct WarpsSmem<true, Wd> {};
+template <bool kBatch> struct WindowSmem {
     WinDev win;                  // wave of windows: the descriptor of the block's current window
     uint32_t cw;                 // its number
+};
+template <> struct WindowSmem<false> {};
+template <bool kBatch, bool kTab, bool kWarp, class Wd>
+struct GateSmem : TabSmem<kTab>, WarpsSmem<kWarp, Wd>, WindowSmem<kBatch> {
+    unsigned long long ctr[4];   // gate events, output events, segments, fan-in events of the window at hand
+    unsigned long long scr, dst; // the gate output's stacks in the scratch, its list in the pool
     uint32_t q;                  // the block's gate output, kInf: none left
     uint32_t skip;               // its window has failed
-    unsigned long long ctr[4];   // gate events, output events, segments, fan-in events of the window at hand
-    WideWord wmin[kMaxWarps];    // smallest candidate of every warp's segments
-    uint32_t wlast[kMaxWarps];   // value of the last kept entry of every warp's segments (4: none)
-    uint32_t wsum[kMaxWarps];    // kept entries
-    WideWord s0[kMaxWarps], s1[kMaxWarps];
-    unsigned long long scr, dst; // the gate output's stacks in the scratch, its list in the pool
     uint32_t ok;                 // the list has its place
     uint32_t xt;                 // latest X or Z of the list but its first entry
 };
@@ -63,8 +77,8 @@ struct Walked {
 };
 
 // Cut and walk gate output i of the level.
-template <int M, bool kTab, class Wd>
-__device__ __forceinline__ Walked<Wd> walk_gate(const WinDev &w, const LevelArgs &a, uint32_t i, GateSmem &sm,
+template <int M, bool kTab, class Wd, class Smem>
+__device__ __forceinline__ Walked<Wd> walk_gate(const WinDev &w, const LevelArgs &a, uint32_t i, Smem &sm,
                                             uint32_t *s_seg)
 {
     constexpr bool kWarp = !kTab && M <= 3;
@@ -135,7 +149,9 @@ __device__ __forceinline__ Walked<Wd> walk_gate(const WinDev &w, const LevelArgs
         if (usable)
             for (uint32_t e = tid; e < 1u << (2 * M); e += nthr) sm.tab.step[e] = step_entry<M>(f0, f1, e);
     }
-    if (kSm && tk < 28) (&sm.tab.slut[0])[tk] = tabw;   // slut, then nd
+    if constexpr (kSm) {
+        if (tk < 28) (&sm.tab.slut[0])[tk] = tabw;   // slut, then nd
+    }
     if (tid == 0) {
         sm.xt = 0;
         sm.scr = scr_at;
@@ -176,8 +192,9 @@ __device__ __forceinline__ Walked<Wd> walk_gate(const WinDev &w, const LevelArgs
             clean = usable && tmax <= EvW<Wd>::kMax - 0x10000u && tcut > xmax && ((curp ^ (curp >> 1)) & 0x15u) == 0u;
             clean = __all_sync(__activemask(), clean);
         }
-        o = walk_segment<M, kTab, kSm, !kTab>(w, a, drv, tid, rd, curp, before, tnext, tmax, scr + region,
-                                       (uint32_t)__cvta_generic_to_shared(&sm.tab), clean);
+        uint32_t tab = 0;
+        if constexpr (kSm) tab = (uint32_t)__cvta_generic_to_shared(&sm.tab);
+        o = walk_segment<M, kTab, kSm, !kTab>(w, a, drv, tid, rd, curp, before, tnext, tmax, scr + region, tab, clean);
         if (o.xt) atomicMax(&sm.xt, o.xt);
     }
     return {o, region, S, E};
@@ -187,8 +204,8 @@ __device__ __forceinline__ Walked<Wd> walk_gate(const WinDev &w, const LevelArgs
 // fetch: thread 0 sets sm.q and sm.skip to the block's next gate output; called
 // where the wait for it overlaps others and every thread has read the present
 // one.
-template <bool kWarp, class Wd, class Fetch>
-__device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a, uint32_t i, GateSmem &sm,
+template <bool kWarp, class Wd, class Smem, class Fetch>
+__device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a, uint32_t i, Smem &sm,
                                             uint32_t *s_seg, const Walked<Wd> &wk, Fetch fetch)
 {
     const unsigned FULL = 0xffffffffu;
@@ -214,11 +231,13 @@ __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a,
         const Wd y = __shfl_down_sync(FULL, x, k);
         if (lane + k < 32) x = min(x, y);
     }
-    if (!kWarp && lane == 0) sm.wmin[wid] = x;
     Wd later = __shfl_down_sync(FULL, x, 1);
     if (lane == 31) later = EvW<Wd>::kInfW;
-    if (!kWarp) __syncthreads();
-    for (uint32_t k = wid + 1; k < nw; ++k) later = min(later, (Wd)sm.wmin[k]);
+    if constexpr (!kWarp) {
+        if (lane == 0) sm.a[wid] = x;
+        __syncthreads();
+        for (uint32_t k = wid + 1; k < nw; ++k) later = min(later, sm.a[k]);
+    }
     uint32_t keep = o.cnt, firstv = 0, lastv = 0;
     if (keep && later != EvW<Wd>::kInfW)
         while (keep && ((keep == o.cnt ? o.top : ot[keep - 1]) | 3u) >= later) --keep;
@@ -231,12 +250,13 @@ __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a,
     const unsigned prior = bal & ((1u << lane) - 1u);
     uint32_t vprev = __shfl_sync(FULL, lastv, prior ? 31 - __clz(prior) : 0);
     const uint32_t vtop = __shfl_sync(FULL, lastv, bal ? 31 - __clz(bal) : 0);
-    if (lane == 0) sm.wlast[wid] = bal ? vtop : 4u;
-    if (!kWarp) __syncthreads();
-    if (!prior) {
-        vprev = kVX;
-        for (int k = (int)wid - 1; k >= 0; --k)
-            if (sm.wlast[k] < 4u) { vprev = sm.wlast[k]; break; }
+    if (!prior) vprev = kVX;
+    if constexpr (!kWarp) {
+        if (lane == 0) sm.wlast[wid] = bal ? vtop : 4u;
+        __syncthreads();
+        if (!prior)
+            for (int k = (int)wid - 1; k >= 0; --k)
+                if (sm.wlast[k] < 4u) { vprev = sm.wlast[k]; break; }
     }
     const uint32_t drop = (tid > 0 && keep > 0 && firstv == vprev) ? 1u : 0u;
     const uint32_t fin = keep - drop;
@@ -247,14 +267,15 @@ __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a,
         if (lane >= k) inc += y;
     }
     uint32_t pos = inc - fin, total = 0;
-    if (kWarp) {
+    if constexpr (kWarp) {
         total = __shfl_sync(FULL, inc, 31);
     } else {
-        if (lane == 31) sm.wsum[wid] = inc;
+        if (lane == 31) sm.b[wid] = inc;
         __syncthreads();
         for (uint32_t k = 0; k < nw; ++k) {
-            if (k < wid) pos += sm.wsum[k];
-            total += sm.wsum[k];
+            const uint32_t n = (uint32_t)sm.b[k];
+            if (k < wid) pos += n;
+            total += n;
         }
     }
     // per warp, the segments that keep entries: where in the stacks the list's
@@ -350,19 +371,19 @@ __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a,
         s1 += __shfl_xor_sync(FULL, s1, k);
     }
     uint32_t last = vtop;   // one warp: that of its last kept entry
-    if (kWarp) {
+    if constexpr (kWarp) {
         if (!bal) last = kVX;
     } else {
-        if (lane == 0) { sm.s0[wid] = s0; sm.s1[wid] = s1; }
+        if (lane == 0) { sm.a[wid] = s0; sm.b[wid] = s1; }
         __syncthreads();
     }
     if (tid == 0) {
-        if (!kWarp) {
+        if constexpr (!kWarp) {
             last = kVX;
             s0 = s1 = 0;
             for (uint32_t k = 0; k < nw; ++k) {
-                s0 += (P)sm.s0[k];
-                s1 += (P)sm.s1[k];
+                s0 += sm.a[k];
+                s1 += sm.b[k];
                 if (sm.wlast[k] < 4u) last = sm.wlast[k];
             }
         }
@@ -397,9 +418,9 @@ __global__ void __launch_bounds__(kSix || kTab ? kGateMaxThreads : 32,
                                   kSix ? 1 : gate_resident<Wd>() / (kTab ? kGateMaxThreads : 32))
     k_gate(const WinSet<kBatch> ws, LevelArgs a, uint32_t d0, uint32_t d1, uint32_t c1, uint32_t c2)
 {
-    __shared__ GateSmem sm;
-    extern __shared__ uint32_t s_seg[];   // per thread the time its segment starts at; then see finish_gate
     constexpr bool kWarp = !kSix && !kTab;
+    __shared__ __align__(256) GateSmem<kBatch, kTab, kWarp, Wd> sm;
+    extern __shared__ uint32_t s_seg[];   // per thread the time its segment starts at; then see finish_gate
     const uint32_t nthr = kWarp ? 32u : blockDim.x;
     const uint32_t n = d1 - d0, total = n * ws.size();
     auto fetch = [&](uint32_t q) {   // thread 0
@@ -407,7 +428,9 @@ __global__ void __launch_bounds__(kSix || kTab ? kGateMaxThreads : 32,
         if (q < total) sm.skip = *(volatile uint32_t *)ws.get(kBatch ? q / n : 0u).err != 0;
     };
     auto flush = [&]() {
-        const WinDev &w = ws.get(kBatch ? sm.cw : 0u);
+        uint32_t win = 0;
+        if constexpr (kBatch) win = sm.cw;
+        const WinDev &w = ws.get(win);
         for (int k = 0; k < 4; ++k) {
             if (sm.ctr[k]) atomicAdd(&w.counters[k], sm.ctr[k]);
             sm.ctr[k] = 0;
@@ -418,7 +441,7 @@ __global__ void __launch_bounds__(kSix || kTab ? kGateMaxThreads : 32,
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (threadIdx.x == 0) {
-        sm.cw = kInf;
+        if constexpr (kBatch) sm.cw = kInf;
         for (int k = 0; k < 4; ++k) sm.ctr[k] = 0;
         fetch(blockIdx.x);   // the grid has at most one block per gate output
     }
@@ -459,12 +482,14 @@ __global__ void __launch_bounds__(kSix || kTab ? kGateMaxThreads : 32,
                 else if (i >= c1) wk = walk_gate<2, kTab, Wd>(w, a, i, sm, s_seg);
                 else wk = walk_gate<1, kTab, Wd>(w, a, i, sm, s_seg);
             }
-            finish_gate<kWarp>(w, a, i, sm, s_seg, wk, next);
+            finish_gate<kWarp, Wd>(w, a, i, sm, s_seg, wk, next);
         };
         if constexpr (kBatch) go(sm.win);
         else go(ws.get(0));
     }
-    if (threadIdx.x == 0 && (!kBatch || sm.cw != kInf)) flush();
+    bool any = true;
+    if constexpr (kBatch) any = sm.cw != kInf;
+    if (threadIdx.x == 0 && any) flush();
 }
 
 void launch_gate(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelArgs &level, const uint32_t *cls,
