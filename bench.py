@@ -390,7 +390,7 @@ def gls_arm(args):
     sim_ms_step = sim_ms / prof_steps
     achieved = sim_bytes / (sim_ms_step / 1000.0) / 1e9
     peak, src = peak_hbm()
-    traffic, traffic_basis = scaled_traffic(args, stats)
+    traffic, traffic_basis = scaled_traffic(args, stats, gate_kernel(sched))
     # whole-step algorithmic bytes (fan-in read + outputs written + SAIF)
     step_bytes = sim_bytes + 5 * stats["output_events"] * 2 + 24 * nl.n_nets
     line = {
@@ -402,14 +402,15 @@ def gls_arm(args):
         "sim_cycles_per_s": sim_cycles,
         "gate_events_per_step": gate_ev, "output_events_per_step": stats["output_events"],
         "fanin_events_per_step": stats["fanin_bytes"] // 5,
-        "roofline": {"bound": "hbm", "kernel": "k_sim", "achieved": achieved, "peak": peak, "unit": "GB/s",
+        "roofline": {"bound": "hbm", "kernel": gate_kernel(sched), "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "traffic": traffic, "traffic_basis": traffic_basis,
                      "peak_source": src,
                      "algorithmic_bytes_per_step": sim_bytes,
-                     "kernel_ms_per_step": {"k_sim": sim_ms_step, "k_combine": comb_ms / prof_steps,
+                     "kernel_ms_per_step": {gate_kernel(sched): sim_ms_step, "k_combine": comb_ms / prof_steps,
                                             "k_plan": plan_ms / prof_steps,
-                                            "timed": f"profiled run with the fan-in classes in turn, "
-                                                     f"mean of {prof_steps}"},
+                                            "timed": f"profiled run, the kernels of a level in turn, "
+                                                     f"mean of {prof_steps} (with k_gate, k_plan is the presize, "
+                                                     f"k_combine nothing)"},
                      "step_achieved_gbs": step_bytes / (step_ms / 1000.0) / 1e9},
         "e2e": {"value": e2e, "unit": "gate-events/s", "h2d_bytes_per_step": int(h2d),
                 "d2h_bytes_per_step": int(d2h), "ms_per_step": 1000.0 * e2e_s},
@@ -434,11 +435,17 @@ def gls_arm(args):
         torch.distributed.destroy_process_group()
 
 
-def scaled_traffic(args, stats):
+def gate_kernel(sched):
+    """The kernel that walks the gates under a schedule: k_gate, or k_sim with
+    warp-per-segment classes, 256-thread blocks, wider loads or learned balance."""
+    return "k_sim" if sched["warp_mask"] or sched["flags"] & 14 else "k_gate"
+
+
+def scaled_traffic(args, stats, kernel):
     """DRAM bytes of the gate kernels per step, scaled from an ncu capture
     of a smaller case of the same generator by the fan-in events processed
     (the kernels' traffic grows with the events they read and write)."""
-    tp = REPO / "profiles" / "k_sim_traffic_c3-100k-depth6-profiling-case.json"
+    tp = REPO / "profiles" / f"{kernel}_traffic_c3-100k-depth6-profiling-case.json"
     if not tp.exists() or args.cells or args.depth or args.cycles:
         return None, None
     tr = json.loads(tp.read_text())
@@ -446,7 +453,7 @@ def scaled_traffic(args, stats):
     if not per_ev:
         return None, None
     fanin_events = stats["fanin_bytes"] / 5
-    return per_ev * fanin_events, (f"{per_ev:.3f} DRAM bytes per fan-in event over the k_sim launches of "
+    return per_ev * fanin_events, (f"{per_ev:.3f} DRAM bytes per fan-in event over the {kernel} launches of "
                                    f"{tr.get('case', 'a smaller case')} (ncu), times this step's fan-in events")
 
 

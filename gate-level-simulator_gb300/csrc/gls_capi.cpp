@@ -870,12 +870,11 @@ static bool gate_path(const gls_ctx *ctx, const LevelArgs &a)
 // `outs` gate outputs of about `est` fan-in events each.  Fewer, longer
 // segments spend less on cut searches and linking; more of them even out the
 // level's end and fill the GPU where the level is narrow.  Measured (device
-// ms, threads 32 / 64 / 128 / 256 / 512): 16,667 outputs of 5,300 events a
-// level 102 / 88 / 82 / 96 / 138; 3,333 of 9,600 38 / 24 / 16.7 / 14.9 /
-// 17.8; 800 of 2,900 5.1 / 3.0 / 2.0 / 1.8 / 2.3; 100 of 670 .53 / .40 / .34
-// / .34 / .34; 26,700 of 1,200 25.1 / 29.1 / 27.6 / 40 / 73.  So: at least 24
-// estimated events a thread; while one and a half rounds of blocks take the
-// whole level, six.
+// ms, threads 64 / 128 / 256): 16,667 outputs of 5,300 events a level 82.7 /
+// 69.6 / 74.7; 3,333 of 9,600 22.7 / 15.7 / 12.7; 800 of 2,900 2.84 / 2.07 /
+// 1.46; 100 of 670 .32 / .28 / .28; 26,700 of 1,200 29.5 / 27.1 / 36.2, in
+// blocks of 32 threads 20.8.  So: at least 24 estimated events a thread; while
+// one and a half rounds of blocks take the whole level, six.
 static uint32_t gate_block(const gls_ctx *ctx, uint64_t outs, double est)
 {
     uint32_t t = 32;
@@ -889,7 +888,8 @@ static uint32_t gate_block(const gls_ctx *ctx, uint64_t outs, double est)
 }
 
 // The launches of a run of nwin windows: stimulus SAIF, then per level the
-// presize (learned mode), plan, simulate per fan-in class, link and copy.
+// presize (learned mode) and k_gate, or (see gate_path) plan, simulate per
+// fan-in class, link and copy.
 // dw[p] / h[p] are the descriptors (device array / window 0 on the host)
 // whose per-gate-output tables serve levels of parity p.  With `prof` the
 // kernel classes are bracketed with events (not during stream capture).

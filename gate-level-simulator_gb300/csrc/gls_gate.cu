@@ -6,15 +6,17 @@
 // Nothing but the finished list leaves the block, so a level needs no plan,
 // no segment tables and no launches in between.
 //
-// What bounds it: issue (60 %) and the integer pipe (67 %) on wide levels, the
-// chain of dependent loads of one gate output (its record, its lists' places,
-// the cut search, the walk) on narrow ones.  Against plan, three classes of
-// simulate, link and copy kernels with one thread per segment of a level-wide
-// segment list (device ms): 2,000 cells over 1,000 cycles .95 -> .34; 37,501
-// cells, 3,333 cycles 3.97 -> 1.80; 200,000 cells, 10,000 cycles 20.1 -> 14.9;
-// 2 M cells, 5,000 cycles 95.8 -> 84.  The segment search is made once per
-// segment instead of at both ends, the lanes of a warp walk the same gate
-// output, and link and copy find the stacks in L1 and L2.
+// What bounds it: on wide levels issue (59 % of the cycles, the integer pipe
+// 58 %) by 32 warps an SM of 64 registers a thread, a quarter of whose time
+// goes into waiting for the slowest warp of the block; on narrow levels the
+// chain of dependent steps of one gate output (its record, its lists' places,
+// the cut search, the walk).  Against plan, three classes of simulate, link
+// and copy kernels with one thread per segment of a level-wide segment list
+// (device ms): 2,000 cells over 1,000 cycles .95 -> .28; 37,501 cells, 3,333
+// cycles 3.97 -> 1.47; 200,000 cells, 10,000 cycles 20.1 -> 12.7; 2 M cells,
+// 5,000 cycles 95.8 -> 67.7.  The segment search is made once per segment
+// instead of at both ends, the lanes of a warp walk the same gate output, and
+// link and copy find the stacks in L1 and L2.
 //
 // The stack contract of a segment and why the split is exact: see the head of
 // gls_kernels.cu.

@@ -1,6 +1,11 @@
 // Level kernels of the GB300 gate-level simulator (sm_103a).
 //
-// One level of gates is simulated by four kinds of launches:
+// The default schedule simulates a level in one launch of k_gate
+// (gls_gate.cu).  Here are the kernels beside it (stimulus SAIF, tables
+// before a run, waveforms read back) and the older form of a level, which the
+// schedules with warp-per-segment classes, 256-thread blocks, wider loads or
+// learned balance, and the allocation-free entry point, take: four kinds of
+// launches,
 //   k_plan     (1 CTA)   sizes every gate output's slot in the event pool and
 //                        its segment stacks in the level scratch, and splits
 //                        its fan-in timeline into time segments.

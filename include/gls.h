@@ -141,9 +141,11 @@ typedef struct {
     uint64_t pool_bytes;      /* device bytes held by the pool */
     uint64_t overflow_retries;/* pool regrowths */
     double kernel_ms;         /* device time of the last gls_run */
-    uint32_t launches;        /* kernels launched by the last gls_run */
+    uint32_t launches;        /* kernels launched by the last gls_run (its levels, the stimulus SAIF) */
     uint32_t n_windows;
-    /* with opts.profile: device time per kernel class in the last gls_run */
+    /* with opts.profile: device time per kernel class in the last gls_run.  In
+     * the default schedule one kernel does a level: its time is sim_ms, plan_ms
+     * the presize (GLS_ALLOC_LEARNED), combine_ms nothing */
     double plan_ms, sim_ms, combine_ms, stim_ms;
     uint64_t fanin_bytes;     /* fan-in event bytes the gate kernels read (5 B per event per net) */
     uint64_t presize_overflows; /* GLS_ALLOC_LEARNED: gate outputs longer than their predicted slot */
@@ -199,7 +201,9 @@ int gls_run_batched(gls_ctx *ctx, const gls_batch_opts *opts);
  * then, on the best of those, each of priority class streams, 256-thread
  * gate-kernel blocks, wider event loads, and both of the last two (13
  * candidates), and with GLS_ALLOC_LEARNED the learned balance of segments
- * (14).  Results never depend on the schedule. */
+ * (14).  Without warp-per-segment classes and flags other than class priority
+ * a level is one launch with a block per gate output, which sizes its segments
+ * itself: those candidates run alike.  Results never depend on the schedule. */
 #define GLS_SCHED_CLASS_PRIORITY 1u   /* wider fan-in classes on higher-priority streams */
 #define GLS_SCHED_BLOCK256 2u         /* thread-per-segment gate kernels in blocks of 256 threads (else 128) */
 #define GLS_SCHED_WIDE_LOADS 4u       /* thread-per-segment gate kernels load 4 events at a time for 1- and
