@@ -872,9 +872,10 @@ static bool gate_path(const gls_ctx *ctx, const LevelArgs &a)
 // level's end and fill the GPU where the level is narrow.  Measured (device
 // ms, threads 64 / 128 / 256): 16,667 outputs of 5,300 events a level 82.7 /
 // 69.6 / 74.7; 3,333 of 9,600 22.7 / 15.7 / 12.7; 800 of 2,900 2.84 / 2.07 /
-// 1.46; 100 of 670 .32 / .28 / .28; 26,700 of 1,200 29.5 / 27.1 / 36.2, in
-// blocks of 32 threads 20.8.  So: at least 24 estimated events a thread; while
-// one and a half rounds of blocks take the whole level, six.
+// 1.42; 100 of 670 .32 / .24 / .22; 26,700 of 1,200 29.5 / 27.1 / 36.2, in
+// blocks of 32 threads 20.8; 4,800 of 200 1.28 / 1.42 / 2.02, 32 threads .84.
+// So: at least 24 estimated events a thread; while one and a half rounds of
+// blocks take the whole level, two.
 static uint32_t gate_block(const gls_ctx *ctx, uint64_t outs, double est)
 {
     uint32_t t = 32;
@@ -883,7 +884,7 @@ static uint32_t gate_block(const gls_ctx *ctx, uint64_t outs, double est)
         return t;
     }
     while (t < 256 && est >= 2.0 * 24 * t) t *= 2;
-    while (t < 256 && outs * t * 2 <= (uint64_t)ctx->sm_count * 1536 && est >= 2.0 * 6 * t) t *= 2;
+    while (t < 256 && outs * t * 2 <= (uint64_t)ctx->sm_count * 1536 && est >= 2.0 * 2 * t) t *= 2;
     return t;
 }
 

@@ -253,7 +253,12 @@ void launch_copy(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelAr
 // four to six input nets exist).  cls: the level's fan-in class starts
 // (kClasses + 1); threads per block: 32 .. kGateMaxThreads, a power of two.
 constexpr uint32_t kGateMaxThreads = 256;
-constexpr uint32_t kGateMinSeg = 16;   // fan-in events a time segment is worth a search
+// Fan-in events a time segment of k_gate is worth a search.  A block's threads
+// are there anyway, and its time is that of its longest segment: 32 / 16 / 8 /
+// 4 / 2 measured .36 / .28 / .24 / .23 / .23 ms on 2,000 cells over 1,000
+// cycles, .82 / .61 / .49 / .46 / .46 on 20,000 cells with calc literal, 68.9 /
+// 67.3 / 66.5 / 66.8 / 66.8 on 2 M cells.
+constexpr uint32_t kGateMinSeg = 4;
 void launch_gate(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelArgs &a, const uint32_t *cls,
                  uint32_t threads, bool table, int sm_count, cudaStream_t st, uint32_t *launches);
 

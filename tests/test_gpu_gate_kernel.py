@@ -108,3 +108,15 @@ def test_copy_of_sparse_segments(kept, every, gpu, oracle_bin):
     for threads in ("32", "128", "256"):
         gw, gs, _, _ = gpu_run(nl, st, 0, t + 50, env={"GLS_GATE_THREADS": threads})
         assert_same(gw, gs, ow, osaif, f"{threads} threads")
+
+
+@pytest.mark.parametrize("events", [2, 3, 4, 5, 6, 8, 43, 85, 86, 170, 342])
+def test_smallest_segments(events, gpu, oracle_bin):
+    """Lists around the smallest segment, and around one smallest segment for
+    every thread of a block, in every block size and the one the rule takes."""
+    nl, st = fan_design(), even_lists(events)
+    t_end = 20 * events + 500
+    ow, osaif, _ = run_oracle(nl, st, 0, t_end)
+    for env in [{"GLS_GATE_THREADS": str(t)} for t in (32, 64, 128, 256)] + [{}]:
+        gw, gs, _, _ = gpu_run(nl, st, 0, t_end, env=env)
+        assert_same(gw, gs, ow, osaif, f"{env}, {events} events")
