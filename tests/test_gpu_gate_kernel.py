@@ -7,7 +7,7 @@ import pytest
 
 from cases import random_case, stimulus
 from gls import synth
-from gls.cells import LIBRARY
+from gls.cells import LIBRARY, CellDef
 from gls.levelize import assemble, default_arcs
 from gls.capi import ALLOC_EXACT
 from gpu_util import assert_same, gpu_run, simulator
@@ -120,3 +120,37 @@ def test_smallest_segments(events, gpu, oracle_bin):
     for env in [{"GLS_GATE_THREADS": str(t)} for t in (32, 64, 128, 256)] + [{}]:
         gw, gs, _, _ = gpu_run(nl, st, 0, t_end, env=env)
         assert_same(gw, gs, ow, osaif, f"{env}, {events} events")
+
+
+def wide_cells():
+    return [CellDef(f"T_{fn.upper()}{k}", [f"a{i}" for i in range(k)], ["z"], [(fn, "z", [f"a{i}" for i in range(k)])],
+                    [(2, f"a{i}", "z") for i in range(k)])
+            for fn, k in (("and", 4), ("xor", 4), ("nor", 5), ("or", 6), ("xor", 6))]
+
+
+@pytest.mark.parametrize("base", [0, 3_000_000_000])
+@pytest.mark.parametrize("events", [3, 17, 300, 4000])
+@pytest.mark.parametrize("threads", [32, 64, 256])
+def test_four_to_six_input_nets(threads, events, base, gpu, oracle_bin):
+    """The class of four to six input nets, in both word sizes, beside a
+    level's narrower gate outputs."""
+    library = {**LIBRARY, **{c.name: c for c in wide_cells()}}
+    names = [c.name for c in wide_cells()] + CELLS
+    rng = np.random.default_rng(events)
+    insts, src, nn = [], list(range(6)), 6
+    for _ in range(3):
+        for k, name in enumerate(names):
+            c = library[name]
+            ins = [int(x) for x in rng.choice(src, c.n_in, replace=False)]
+            insts.append((name, ins, [nn + k], default_arcs(c, 4.0 + k, 9.0 - k % 5)))
+        src, nn = list(range(nn, nn + len(names))), nn + len(names)
+    nl = assemble(insts, n_nets=nn, cells=library)
+    d = {}
+    for net in range(6):
+        t = base + np.cumsum(rng.integers(1, 30, events))
+        d[net] = list(zip(t.tolist(), rng.choice([0, 3, 1, 2], events, p=[.48, .48, .02, .02]).tolist()))
+    st = stimulus(d)
+    t_end = base + 30 * events + 200
+    ow, osaif, _ = run_oracle(nl, st, base + 5, t_end)
+    gw, gs, _, _ = gpu_run(nl, st, base + 5, t_end, env={"GLS_GATE_THREADS": str(threads)})
+    assert_same(gw, gs, ow, osaif, f"{threads} threads, {events} events")
