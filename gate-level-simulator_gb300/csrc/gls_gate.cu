@@ -29,8 +29,15 @@ namespace gls {
 namespace {
 
 constexpr int kMaxWarps = kGateMaxThreads / 32;
-// threads per SM the narrow classes' kernel is compiled for
-template <class Wd> __host__ __device__ constexpr uint32_t gate_resident() { return sizeof(Wd) == 4 ? 1024u : 768u; }
+// threads per SM the kernels are compiled for.  kSix: the class of four to six
+// input nets, which walks by general steps in more registers (12 levels of
+// 3,000 such gate outputs of 140,000 events: 256 / 512 / 768 / 1,024 threads
+// 113 / 71 / 59 / 63 ms, the last with spills; of 100 such gate outputs of
+// 36,000 events 3.6 / 3.4 / 3.4 / 4.0).
+template <bool kSix, class Wd> __host__ __device__ constexpr uint32_t gate_resident()
+{
+    return kSix ? (sizeof(Wd) == 4 ? 768u : 512u) : (sizeof(Wd) == 4 ? 1024u : 768u);
+}
 
 // Shared memory is L1 lost: each kernel has only what it uses, the step table
 // (kTab), what meets between warps (not kWarp) and the window's descriptor
@@ -417,7 +424,7 @@ __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a,
 // widest first, as they become free.
 template <bool kBatch, bool kSix, bool kTab, class Wd>
 __global__ void __launch_bounds__(kSix || kTab ? kGateMaxThreads : 32,
-                                  kSix ? 1 : gate_resident<Wd>() / (kTab ? kGateMaxThreads : 32))
+                                  gate_resident<kSix, Wd>() / (kSix || kTab ? kGateMaxThreads : 32))
     k_gate(const WinSet<kBatch> ws, LevelArgs a, uint32_t d0, uint32_t d1, uint32_t c1, uint32_t c2)
 {
     constexpr bool kWarp = !kSix && !kTab;
@@ -505,7 +512,7 @@ void launch_gate(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelAr
         if (d1 <= d0) return;
         const uint64_t total = (uint64_t)(d1 - d0) * nwin;
         const uint64_t room =
-            (uint64_t)sm_count * ((kSix ? kGateMaxThreads : (a.wide ? gate_resident<WideWord>() : gate_resident<uint32_t>())) / threads);
+            (uint64_t)sm_count * ((a.wide ? gate_resident<kSix, WideWord>() : gate_resident<kSix, uint32_t>()) / threads);
         const uint32_t grid = (uint32_t)(total < room ? total : room);
         cudaLaunchAttribute at;
         at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
