@@ -12,9 +12,9 @@
 // chain of dependent steps of one gate output (its record, its lists' places,
 // the cut search, the walk).  Against plan, three classes of simulate, link
 // and copy kernels with one thread per segment of a level-wide segment list
-// (device ms): 2,000 cells over 1,000 cycles .95 -> .28; 37,501 cells, 3,333
-// cycles 3.97 -> 1.47; 200,000 cells, 10,000 cycles 20.1 -> 12.7; 2 M cells,
-// 5,000 cycles 95.8 -> 67.7.  The segment search is made once per segment
+// (device ms): 2,000 cells over 1,000 cycles .95 -> .23; 37,501 cells, 3,333
+// cycles 3.97 -> 1.43; 200,000 cells, 10,000 cycles 20.1 -> 12.7; 2 M cells,
+// 5,000 cycles 95.8 -> 66.8.  The segment search is made once per segment
 // instead of at both ends, the lanes of a warp walk the same gate output, and
 // link and copy find the stacks in L1 and L2.
 //

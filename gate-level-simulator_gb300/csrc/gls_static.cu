@@ -33,7 +33,7 @@ constexpr uint64_t kStaticMaxWords = 4194304;        // segment-stack words per 
 
 // Layout of the static scratch (byte offsets, each 256-byte aligned).
 constexpr uint64_t al256(uint64_t x) { return (x + 255) & ~255ull; }
-constexpr uint64_t kOffSmall = 0;   // 8 x u64: saved pool pointer, 4 counters, err, n_segs, presize overflows
+constexpr uint64_t kOffSmall = 0;   // 8 x u64: saved pool pointer, 4 counters, err, unused, presize overflows
 constexpr uint64_t kOffWin = 64;                                             // the level kernels' WinDev
 constexpr uint64_t kOffSegBase = al256(kOffWin + sizeof(WinDev));
 constexpr uint64_t kOffSlot = al256(kOffSegBase + 4ull * (kStaticMaxOutputs + 1));
