@@ -1659,7 +1659,10 @@ extern "C" int gls_waveform(gls_ctx *ctx, uint32_t window, uint32_t net, uint32_
     Window *w = get_done(ctx, window);
     if (!w) return fail(ctx, GLS_ESTATE, "window %u not simulated", window);
     if (net >= ctx->n_nets) return fail(ctx, GLS_EINVAL, "net %u out of range", net);
-    if (w->saif_only) return fail(ctx, GLS_ESTATE, "window %u ran with saif_only: its waveforms were not kept", window);
+    // saif_only calls give every window's pool back before their first wave,
+    // also those of windows that they then do not run (autotune, a failed wave)
+    if (w->saif_only || !w->pool.p || !w->net_off.p)
+        return fail(ctx, GLS_ESTATE, "window %u's pool went in a saif_only run: its waveforms were not kept", window);
     cudaSetDevice(ctx->opts.device);
     const uint32_t wb = (uint32_t)w->word_bytes();
     const uint64_t want = (time || value) ? cap : 0;
@@ -1670,11 +1673,12 @@ extern "C" int gls_waveform(gls_ctx *ctx, uint32_t window, uint32_t net, uint32_
     constexpr uint64_t kInline = 1u << 18;
     const uint64_t first = want > kInline ? 0 : want;
     if (!ctx->pin_out.ensure(16 + first * wb)) return fail(ctx, GLS_ENOMEM, "pinned staging for a waveform");
-    launch_read_list(w->net_off.as<uint64_t>() + net, w->net_len.as<uint32_t>() + net, w->pool.p, wb, first,
+    launch_read_list(w->net_off.as<uint64_t>() + net, w->net_len.as<uint32_t>() + net, w->pool.p, w->pool.bytes, wb, first,
                      ctx->pin_out.p, ctx->stream);
     CK(cudaGetLastError(), "read waveform");
     CK(cudaStreamSynchronize(ctx->stream), "read waveform");
     const uint64_t len = ctx->pin_out.as<uint64_t>()[0], off = ctx->pin_out.as<uint64_t>()[1];
+    if (len == kListOutside) return fail(ctx, GLS_ECUDA, "net %u: its list does not lie in window %u's pool", net, window);
     if (len == 0xFFFFFFFFu) {
         *n = UINT64_MAX;
         return GLS_OK;

@@ -232,9 +232,11 @@ __host__ __device__ inline int fanin_class(int m) { return m <= 1 ? 0 : (m == 2 
 void launch_reset(const WinDev *dw, const WinDev &h, uint32_t nwin, uint32_t max_stim, uint32_t n_nets, uint32_t n_levels,
                   cudaStream_t st);
 // One list (word: bytes of an event word) from its net's tables to out: its
-// length, its pool offset (64 bits each), then up to cap events.
-void launch_read_list(const uint64_t *off, const uint32_t *len, const void *pool, uint32_t word, uint64_t cap, void *out,
-                      cudaStream_t st);
+// length (kListOutside: it does not lie in the pool), its pool offset (64 bits
+// each), then up to cap events.
+constexpr unsigned long long kListOutside = ~0ull;
+void launch_read_list(const uint64_t *off, const uint32_t *len, const void *pool, uint64_t pool_bytes, uint32_t word,
+                      uint64_t cap, void *out, cudaStream_t st);
 void launch_stim_saif(const WinDev *dw, const WinDev &h, uint32_t nwin, uint32_t max_stim, bool wide, uint32_t n_nets,
                       cudaStream_t st);
 void launch_plan(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelArgs &a, cudaStream_t st);

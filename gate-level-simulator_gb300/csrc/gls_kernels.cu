@@ -1583,16 +1583,22 @@ __global__ void __launch_bounds__(256) k_reset_stim(const WinSet<kBatch> ws, uin
 }
 
 // One block: a list's length, its offset and up to cap of its events into
-// host memory.
+// host memory; kListOutside as the length where the list does not lie in the
+// pool's `room` events (tables that a run which failed left behind).
 template <class Wd>
 __global__ void __launch_bounds__(1024) k_read_list(const uint64_t *__restrict__ off, const uint32_t *__restrict__ len,
-                                                    const Wd *__restrict__ pool, uint64_t cap, unsigned long long *out)
+                                                    const Wd *__restrict__ pool, uint64_t room, uint64_t cap,
+                                                    unsigned long long *out)
 {
     const uint32_t n = *len;
-    if (threadIdx.x == 0) out[0] = n;
-    if (n == kInf) return;
-    const Wd *x = pool + *off;
-    if (threadIdx.x == 0) out[1] = *off;
+    const uint64_t at = *off;
+    const bool outside = n != kInf && (at > room || n > room - at);
+    if (threadIdx.x == 0) {
+        out[0] = outside ? kListOutside : n;
+        out[1] = at;
+    }
+    if (n == kInf || outside) return;
+    const Wd *x = pool + at;
     Wd *d = reinterpret_cast<Wd *>(out + 2);
     for (uint64_t e = threadIdx.x; e < n && e < cap; e += blockDim.x) d[e] = x[e];
 }
@@ -1677,12 +1683,13 @@ void launch_reset(const WinDev *dw, const WinDev &h, uint32_t nwin, uint32_t max
     GLS_DISPATCH(h, dw, nwin, (k_reset_stim<decltype(ws)::kIsBatch><<<gb, 256, 0, st>>>(ws, n_levels)));
 }
 
-void launch_read_list(const uint64_t *off, const uint32_t *len, const void *pool, uint32_t word, uint64_t cap, void *out,
-                      cudaStream_t st)
+void launch_read_list(const uint64_t *off, const uint32_t *len, const void *pool, uint64_t pool_bytes, uint32_t word,
+                      uint64_t cap, void *out, cudaStream_t st)
 {
     unsigned long long *o = static_cast<unsigned long long *>(out);
-    if (word == 8) k_read_list<WideWord><<<1, 1024, 0, st>>>(off, len, static_cast<const WideWord *>(pool), cap, o);
-    else k_read_list<uint32_t><<<1, 1024, 0, st>>>(off, len, static_cast<const uint32_t *>(pool), cap, o);
+    const uint64_t room = pool_bytes / word;
+    if (word == 8) k_read_list<WideWord><<<1, 1024, 0, st>>>(off, len, static_cast<const WideWord *>(pool), room, cap, o);
+    else k_read_list<uint32_t><<<1, 1024, 0, st>>>(off, len, static_cast<const uint32_t *>(pool), room, cap, o);
 }
 
 void launch_wave_events(const WinDev *dw, uint32_t nwin, const LevelArgs &a, cudaStream_t st)
