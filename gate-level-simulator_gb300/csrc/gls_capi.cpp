@@ -1338,6 +1338,16 @@ static int batch_setup(gls_ctx *ctx, const gls_batch_opts &o, uint64_t *B)
     return GLS_OK;
 }
 
+// How many of windows [w0, w0 + nwin) run together: a window of 64-bit event
+// words runs alone, and a wave stops before one.
+static uint64_t wave_length(const gls_ctx *ctx, size_t w0, uint64_t nwin)
+{
+    if (ctx->windows[w0]->w64) return 1;
+    for (uint64_t k = 1; k < nwin; ++k)
+        if (ctx->windows[w0 + k]->w64) return k;
+    return nwin;
+}
+
 // One wave: windows [w0, w0 + nwin) together; *ms receives its device time
 // (upload of new stimuli excluded, reruns of windows that outgrew a buffer
 // included in acc).
@@ -1466,16 +1476,7 @@ extern "C" int gls_run_batched(gls_ctx *ctx, const gls_batch_opts *opts)
             }
             nwin = std::max<uint64_t>(1, std::min<uint64_t>(nwin, (uint64_t)(0.85 * (double)fr) / per));
         }
-        // a window of 64-bit event words runs alone; a wave stops before one
-        if (ctx->windows[w0]->w64) {
-            nwin = 1;
-        } else {
-            for (uint64_t k = 1; k < nwin; ++k)
-                if (ctx->windows[w0 + k]->w64) {
-                    nwin = k;
-                    break;
-                }
-        }
+        nwin = wave_length(ctx, w0, nwin);
         float ms = 0.f;
         rc = run_wave(ctx, w0, (uint32_t)nwin, o, acc, &ms, e0, e1);
         acc.total_ms += ms;
@@ -1509,7 +1510,7 @@ extern "C" int gls_autotune(gls_ctx *ctx, const gls_batch_opts *opts, gls_tune_r
     uint64_t B = 1;
     int rc = batch_setup(ctx, o, &B);
     if (rc) return rc;
-    const uint32_t nwin = (uint32_t)std::min<uint64_t>(B, ctx->windows.size());
+    uint32_t nwin = (uint32_t)wave_length(ctx, 0, std::min<uint64_t>(B, ctx->windows.size()));
     // Stage 1: time segments per SM for the thread-per-segment kernel times
     // which fan-in classes run warp-per-segment.  Stage 2, on the best of
     // those: class-stream priority, the gate kernel's block size and load
@@ -1535,6 +1536,14 @@ extern "C" int gls_autotune(gls_ctx *ctx, const gls_batch_opts *opts, gls_tune_r
             float tr = 0.f;
             rc = run_wave(ctx, 0, nwin, o, acc, &tr, e0, e1);
             if (rep) t = std::min(t, tr);
+            // a window whose output times turned out to need 64-bit words
+            // (the first run tells) leaves the wave that is timed
+            const uint32_t together = (uint32_t)wave_length(ctx, 0, nwin);
+            if (rc == GLS_OK && together < nwin) {
+                nwin = together;
+                rep = -1;
+                t = 1e30f;
+            }
         }
         r.ms[c] = t;
         r.seg_per_sm[c] = segs;

@@ -38,3 +38,51 @@ def test_waveform_of_a_window_whose_pool_went(design, gpu):
         for w in ids:
             t, v = s.waveform(out, w)
             assert np.array_equal(t, waves[w][0]) and np.array_equal(v, waves[w][1])
+
+
+@pytest.mark.parametrize("late", [0, 1, 2])
+def test_autotune_stops_before_a_window_of_64_bit_words(late, design, gpu):
+    """Windows of 64-bit event words run alone: the wave that autotune times
+    ends before one, is that one when it comes first, and leaves every window
+    that it ran as gls_run leaves it."""
+    cfg, nl = design
+    far = synth.scaled(cfg)
+    far.period = 20_000_000   # times past 2^30 - 2
+    wins = [far if k == late else cfg for k in range(3)]
+    with Simulator() as s:
+        s.load(nl)
+        ids = [s.add_window(synth.make_stimulus(c, nl.ppi_nets, seed=60 + k), 0, c.t_end) for k, c in enumerate(wins)]
+        assert s.autotune()["windows"] == (1 if late == 0 else late)
+        ran = [w for w in ids if w < max(1, late)]
+        tuned = [s.saif(w).copy() for w in ran]
+        s.run()
+        assert s.stats()["wide_windows"] == 1
+        for w, a in zip(ran, tuned):
+            assert np.array_equal(a, s.saif(w))
+
+
+def test_autotune_of_windows_that_grow_past_32_bit_times(design, gpu):
+    """A window whose stimulus fits 32-bit words and whose gate outputs do not
+    is found by the first run of the wave, which then goes on without it."""
+    cfg, nl = design
+    end = 2**30 - 2
+    sts = []
+    for k in range(3):
+        st = synth.make_stimulus(cfg, nl.ppi_nets, seed=70 + k)
+        if k == 1:   # the last event of every net at the largest 32-bit time
+            last = st.ev_start[1:].astype(np.int64) - 1
+            st.time[last[st.ev_start[1:] - st.ev_start[:-1] > 1]] = end
+        sts.append(st)
+    with Simulator() as s:
+        s.load(nl)
+        ids = [s.add_window(st, 0, 2**30 + 10_000) for st in sts]
+        assert s.autotune()["windows"] == 1
+        tuned = [s.saif(w).copy() for w in ids]
+        with Simulator() as r:
+            r.load(nl)
+            for st in sts:
+                r.add_window(st, 0, 2**30 + 10_000)
+            r.run()
+            assert r.stats()["wide_windows"] == 1
+            for w in ids:
+                assert np.array_equal(tuned[w], r.saif(w))
