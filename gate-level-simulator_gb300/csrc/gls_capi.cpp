@@ -861,9 +861,9 @@ static void prof_mark(gls_ctx *ctx)
 
 // Whether a run's levels go through k_gate: 64-bit windows, and the default
 // thread-per-segment schedule.
-static bool gate_path(const gls_ctx *ctx, const LevelArgs &a)
+static bool gate_path(const gls_ctx *ctx, bool w64)
 {
-    return a.wide || (ctx->gate_kernel && a.warp_mask == 0 && a.sim_variant == 0 && a.bal_weight <= 0.f);
+    return w64 || (ctx->gate_kernel && ctx->warp_mask == 0 && ctx->sim_variant == 0 && ctx->bal_weight <= 0.f);
 }
 
 // k_gate's threads (and so time segments) per gate output, for a level of
@@ -888,14 +888,26 @@ static uint32_t gate_block(const gls_ctx *ctx, uint64_t outs, double est)
     return t;
 }
 
+// k_gate's threads at every level of a run of nwin windows together; empty
+// where the run does not go through it.
+static std::vector<uint32_t> gate_blocks(const gls_ctx *ctx, uint32_t nwin, bool w64, double est)
+{
+    if (!gate_path(ctx, w64)) return {};
+    std::vector<uint32_t> t(ctx->drv_level_start.size() - 1);
+    for (size_t L = 0; L < t.size(); ++L)
+        t[L] = gate_block(ctx, (uint64_t)(ctx->drv_level_start[L + 1] - ctx->drv_level_start[L]) * nwin, est);
+    return t;
+}
+
 // The launches of a run of nwin windows: stimulus SAIF, then per level the
-// presize (learned mode) and k_gate, or (see gate_path) plan, simulate per
-// fan-in class, link and copy.
+// presize (learned mode) and k_gate (threads: its block at every level), or
+// (see gate_path) plan, simulate per fan-in class, link and copy.
 // dw[p] / h[p] are the descriptors (device array / window 0 on the host)
 // whose per-gate-output tables serve levels of parity p.  With `prof` the
 // kernel classes are bracketed with events (not during stream capture).
 static int enqueue_levels(gls_ctx *ctx, const WinDev *const dw[2], const WinDev *const h[2], uint32_t nwin,
-                          uint32_t max_stim, bool prof, uint32_t *launches, bool w64, double est)
+                          uint32_t max_stim, bool prof, uint32_t *launches, bool w64,
+                          const std::vector<uint32_t> &threads)
 {
     LevelArgs a;
     ctx_level_args(ctx, &a);
@@ -915,7 +927,7 @@ static int enqueue_levels(gls_ctx *ctx, const WinDev *const dw[2], const WinDev 
     // from the predictions: it keeps the plan whole, after the copies.)
     const bool learned = a.alloc_mode == kAllocLearned;
     const bool split = learned && ctx->bal_weight <= 0.f;
-    const bool gates = gate_path(ctx, a);
+    const bool gates = gate_path(ctx, w64);
     const bool overlap_ok = ctx->concurrent && ctx->pipeline && ctx->plan_overlap && !(prof && ctx->opts.profile) &&
                             (!learned || split);
     if (prof) prof_mark(ctx);
@@ -950,9 +962,8 @@ static int enqueue_levels(gls_ctx *ctx, const WinDev *const dw[2], const WinDev 
                 ++*launches;
             }
             if (prof) prof_mark(ctx);
-            launch_gate(dw[0], *h[0], nwin, a, &ctx->cls_start[(kClasses + 1) * L],
-                        gate_block(ctx, (uint64_t)(a.hi - a.lo) * nwin, est), !stim_beside, ctx->sm_count, ctx->stream,
-                        launches);
+            launch_gate(dw[0], *h[0], nwin, a, &ctx->cls_start[(kClasses + 1) * L], threads[L], !stim_beside,
+                        ctx->sm_count, ctx->stream, launches);
             if (stim_beside) {   // the first level ran without the stimulus nets' X times
                 CK(cudaStreamWaitEvent(ctx->stream, ctx->stim_join, 0), "stim join wait");
                 stim_beside = false;
@@ -1107,7 +1118,8 @@ static int enqueue_window(gls_ctx *ctx, Window *w, uint32_t *launches)
     const WinDev *dw[2] = {w->dwin.as<WinDev>(), w->dwin.as<WinDev>() + 1};
     const WinDev *hp[2] = {&d[0], &d[1]};
     launch_reset(dw[0], d[0], 1, d[0].n_stim, ctx->n_nets, (uint32_t)ctx->drv_level_start.size(), ctx->stream);
-    return enqueue_levels(ctx, dw, hp, 1, d[0].n_stim, true, launches, w->w64, gate_events_est(ctx, w));
+    return enqueue_levels(ctx, dw, hp, 1, d[0].n_stim, true, launches, w->w64,
+                          gate_blocks(ctx, 1, w->w64, gate_events_est(ctx, w)));
 }
 
 // Copies the flags and counters of windows [w0, w0 + n) to ctx->hsmall, behind
@@ -1376,11 +1388,13 @@ static int run_wave(gls_ctx *ctx, size_t w0, uint32_t nwin, const gls_batch_opts
     const WinDev *dw[2] = {ctx->dwave.as<WinDev>(), ctx->dwave.as<WinDev>() + kMaxWave};
     const WinDev *hp[2] = {&hw[0], &hw[kMaxWave]};
     launch_reset(dw[0], hw[0], nwin, max_stim, ctx->n_nets, (uint32_t)ctx->drv_level_start.size(), ctx->stream);
+    const bool w64 = nwin == 1 && ctx->windows[w0]->w64;
+    const std::vector<uint32_t> threads = gate_blocks(ctx, nwin, w64, est);
     CK(cudaEventRecord(e0, ctx->stream), "event");
     if (o.use_graph && nwin > 1) {
         // one graph per wave shape; the descriptors it reads are rewritten per wave
         gls_ctx::WaveGraph key{nwin, max_stim, ctx->warp_mask, (uint32_t)ctx->opts.alloc_mode, ctx->seg_per_sm,
-                               schedule_flags(ctx), nullptr, 0};
+                               schedule_flags(ctx), threads, nullptr, 0};
         cudaGraphExec_t ge = nullptr;
         uint32_t l = 0;
         for (auto &g : ctx->graphs)
@@ -1393,7 +1407,7 @@ static int run_wave(gls_ctx *ctx, size_t w0, uint32_t nwin, const gls_batch_opts
             cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
             int rc = GLS_OK;
             if (e == cudaSuccess) {
-                rc = enqueue_levels(ctx, dw, hp, nwin, max_stim, false, &l, false, est);
+                rc = enqueue_levels(ctx, dw, hp, nwin, max_stim, false, &l, false, threads);
                 const cudaError_t e2 = cudaStreamEndCapture(ctx->stream, &g);
                 if (rc == GLS_OK && e2 != cudaSuccess) e = e2;
             }
@@ -1408,8 +1422,7 @@ static int run_wave(gls_ctx *ctx, size_t w0, uint32_t nwin, const gls_batch_opts
         CK(cudaGraphLaunch(ge, ctx->stream), "graph launch");
         acc.launches += l;
     } else {
-        int rc = enqueue_levels(ctx, dw, hp, nwin, max_stim, false, &acc.launches,
-                                nwin == 1 && ctx->windows[w0]->w64, est);
+        int rc = enqueue_levels(ctx, dw, hp, nwin, max_stim, false, &acc.launches, w64, threads);
         if (rc) return rc;
     }
     CK(cudaEventRecord(e1, ctx->stream), "event");

@@ -281,12 +281,14 @@ struct gls_ctx {
     std::vector<DevBuf> spare_bufs;  // device buffers of windows that ran saif_only, reused by later windows
     struct WaveGraph {
         uint32_t nwin, max_stim, warp_mask, alloc_mode, seg_per_sm, flags;   // flags: GLS_SCHED_*
+        std::vector<uint32_t> threads;   // k_gate's block at every level: the windows' list lengths decide it
         cudaGraphExec_t exec;
         uint32_t launches;
         bool same(const WaveGraph &o) const
         {
             return nwin == o.nwin && max_stim == o.max_stim && warp_mask == o.warp_mask &&
-                   alloc_mode == o.alloc_mode && seg_per_sm == o.seg_per_sm && flags == o.flags;
+                   alloc_mode == o.alloc_mode && seg_per_sm == o.seg_per_sm && flags == o.flags &&
+                   threads == o.threads;
         }
     };
     std::vector<WaveGraph> graphs;

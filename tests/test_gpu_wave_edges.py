@@ -86,3 +86,29 @@ def test_autotune_of_windows_that_grow_past_32_bit_times(design, gpu):
             assert r.stats()["wide_windows"] == 1
             for w in ids:
                 assert np.array_equal(tuned[w], r.saif(w))
+
+
+@pytest.mark.parametrize("order", [(30, 4000), (4000, 30)])
+def test_graph_of_a_wave_fits_its_windows(order, design, gpu):
+    """Waves of as many windows over the same nets, one of short and one of
+    long lists, through one context: each is launched as in a context of its
+    own (the segment count tells the gate kernel's block sizes), and gives the
+    same counts."""
+    cfg, nl = design
+
+    def wave(s, cycles):
+        s.clear_windows()
+        ids = [s.add_window(synth.make_stimulus(cfg, nl.ppi_nets, seed=80 + k, cycles=cycles), 0, cycles * cfg.period)
+               for k in range(40)]
+        s.run_batched()
+        return s.stats()["segments"], [s.saif(w).copy() for w in ids]
+
+    with Simulator() as both:
+        both.load(nl)
+        for cycles in order:
+            segments, saif = wave(both, cycles)
+            with Simulator() as alone:
+                alone.load(nl)
+                s0, f0 = wave(alone, cycles)
+            assert segments == s0
+            assert all(np.array_equal(a, b) for a, b in zip(saif, f0))
