@@ -597,10 +597,19 @@ static double pool_scale(const gls_ctx *ctx, const Window *w)
     return avg * (double)ctx->pins_total;
 }
 
-// about the fan-in events of one gate output
-static double gate_events_est(const gls_ctx *ctx, const Window *w)
+// About the fan-in events of one gate output: on the mean, and of one whose
+// input nets are as busy as the busiest stimulus net that a gate reads.
+struct GateEvents {
+    double mean = 0.0, busiest = 0.0;
+};
+static GateEvents gate_events_est(const gls_ctx *ctx, const Window *w)
 {
-    return ctx->n_drv ? 2.5 * pool_scale(ctx, w) / ctx->n_drv : 0.0;
+    GateEvents e;
+    if (!ctx->n_drv) return e;
+    const double per_event = 2.5 * (double)ctx->pins_total / ctx->n_drv;
+    e.mean = 2.5 * pool_scale(ctx, w) / ctx->n_drv;
+    e.busiest = std::max(e.mean, per_event * (double)w->stim_longest);
+    return e;
 }
 
 // the pool a window is given: its estimate, raised to what earlier windows
@@ -673,8 +682,12 @@ extern "C" int gls_add_window(gls_ctx *ctx, const gls_stimulus *st, uint64_t t_b
         if (st->ev_start[k + 1] < st->ev_start[k]) { ctx->spare.push_back(w); return fail(ctx, GLS_EINVAL, "stimulus ev_start not monotone"); }
         at[k + 1] = at[k] + round4(st->ev_start[k + 1] - st->ev_start[k]);
     }
+    uint64_t longest = 0;
+    for (uint32_t net : ctx->ext_inputs) seen[net] |= 2;
+    for (uint32_t k = 0; k < st->n_nets; ++k)
+        if (seen[st->net[k]] & 2) longest = std::max(longest, at[k + 1] - at[k]);
     for (uint32_t net : ctx->ext_inputs)
-        if (!seen[net]) { ctx->spare.push_back(w); return fail(ctx, GLS_EINVAL, "net %u is read by a gate but has no stimulus", net); }
+        if (!(seen[net] & 1)) { ctx->spare.push_back(w); return fail(ctx, GLS_EINVAL, "net %u is read by a gate but has no stimulus", net); }
     const uint64_t total = at[st->n_nets];
     // validate and pack (time << 2 | value), each net on a 4-event boundary;
     // large stimuli are packed by several host threads.  32-bit words hold
@@ -773,6 +786,7 @@ extern "C" int gls_add_window(gls_ctx *ctx, const gls_stimulus *st, uint64_t t_b
         h_off[k] = at[k];
     }
     w->stim_events = total;
+    w->stim_longest = longest;
     // initial pool capacity: stimulus plus an estimate of every gate's slot
     uint64_t cap = ctx->opts.pool_events;
     if (!cap) {
@@ -859,43 +873,81 @@ static void prof_mark(gls_ctx *ctx)
     if (e) cudaEventRecord(e, ctx->stream);
 }
 
-// Whether a run's levels go through k_gate: 64-bit windows, and the default
-// thread-per-segment schedule.
+// Whether a schedule's levels may go through k_gate: 64-bit windows, and the
+// default thread-per-segment schedule.
 static bool gate_path(const gls_ctx *ctx, bool w64)
 {
     return w64 || (ctx->gate_kernel && ctx->warp_mask == 0 && ctx->sim_variant == 0 && ctx->bal_weight <= 0.f);
 }
 
 // k_gate's threads (and so time segments) per gate output, for a level of
-// `outs` gate outputs of about `est` fan-in events each.  Fewer, longer
-// segments spend less on cut searches and linking; more of them even out the
-// level's end and fill the GPU where the level is narrow.  Measured (device
-// ms, threads 64 / 128 / 256): 16,667 outputs of 5,300 events a level 82.7 /
-// 69.6 / 74.7; 3,333 of 9,600 22.7 / 15.7 / 12.7; 800 of 2,900 2.84 / 2.07 /
-// 1.42; 100 of 670 .32 / .24 / .22; 26,700 of 1,200 29.5 / 27.1 / 36.2, in
-// blocks of 32 threads 20.8; 4,800 of 200 1.28 / 1.42 / 2.02, 32 threads .84.
-// So: at least 24 estimated events a thread; while one and a half rounds of
-// blocks take the whole level, two.
-static uint32_t gate_block(const gls_ctx *ctx, uint64_t outs, double est)
+// `outs` gate outputs, `six` of them with four to six input nets.  Fewer,
+// longer segments spend less on cut searches and linking; more of them even
+// out the level's end and fill the GPU where the level is narrow.  Measured
+// (device ms, threads 64 / 128 / 256): 16,667 outputs of 5,300 events a level
+// 82.7 / 69.6 / 74.7; 3,333 of 9,600 22.7 / 15.7 / 12.7; 800 of 2,900 2.84 /
+// 2.07 / 1.42; 100 of 670 .32 / .24 / .22; 26,700 of 1,200 29.5 / 27.1 / 36.2,
+// in blocks of 32 threads 20.8; 4,800 of 200 1.28 / 1.42 / 2.02, 32 threads
+// .84.  So: at least 24 estimated events a thread; while one and a half rounds
+// of blocks take the whole level, two.
+static GateThreads gate_block(const gls_ctx *ctx, uint64_t outs, uint64_t six, const GateEvents &est)
 {
+    const double sms = ctx->sm_count;
     uint32_t t = 32;
     if (ctx->gate_threads) {
         while (t < kGateMaxThreads && t < ctx->gate_threads) t *= 2;
-        return t;
+        return {t, ctx->gate_threads >= kGateMaxSix ? kGateMaxSix : t};
     }
-    while (t < 256 && est >= 2.0 * 24 * t) t *= 2;
-    while (t < 256 && outs * t * 2 <= (uint64_t)ctx->sm_count * 1536 && est >= 2.0 * 2 * t) t *= 2;
-    return t;
+    while (t < 256 && est.mean >= 2.0 * 24 * t) t *= 2;
+    while (t < 256 && outs * t * 2 <= (uint64_t)ctx->sm_count * 1536 && est.mean >= 2.0 * 2 * t) t *= 2;
+    // A level lasts as long as its busiest gate output, about a microsecond a
+    // step of its threads with its blocks' growth over the levels, and the
+    // others about 8 us per round of blocks: where the busiest has many more
+    // steps than the mean thread, blocks double while that halves more than
+    // the rounds add.  10 levels where 1 % of the gate outputs read nets of 100
+    // times the others' events, threads by the mean / 256 / 512 / 1,024 (as
+    // chosen; the segment kernels): 16,000 outputs, 20,000 cycles 15.7 / 4.2 /
+    // 6.0 / 11.8 (4.2; 4.6); 3,000 outputs 5.7 / 2.0 / 1.9 / 2.8 (1.8; 2.9),
+    // 100,000 cycles 18.3 / 10.0 / 6.8 / 6.7 (6.8; 11.9).  100 gate outputs of
+    // 2.7 M events: 32.3 / - / 18.8 / 15.7 (18.6; 31.6).
+    const double even = 64.0 + 1.5 * (double)outs * est.mean / (1024.0 * sms);   // steps of the busiest that even out
+    while (t < kGateMaxThreads && est.busiest > even * t && (double)t * t * outs < 64.0 * sms * est.busiest) t *= 2;
+    // Four to six input nets: more events and general steps, fewer gate
+    // outputs.  12 levels, share of the class .3 (.05), its threads as the
+    // others' / 128 / 256 / 512 / 768 (the segment kernels): 12,000 outputs of
+    // 300 events a stimulus net 15.5 / 13.2 / 12.4 / 15.2 / 14.7 (15.8), (6.8 /
+    // 5.6 / 5.0 / 5.3 / 5.3 (5.6)); 3,000 outputs 9.1 / 6.4 / 5.4 / 5.6 / 5.6
+    // (5.5), (3.6 / 2.7 / 2.2 / 2.0 / 2.1 (2.2)); 100 outputs of 6,000 events
+    // 23.0 / 36.7 / 23.0 / 17.1 / 15.2 (15.4), (9.2 / 14.2 / 9.3 / 7.1 / 6.5 (6.9)).
+    uint32_t t6 = t;
+    while (t6 < kGateMaxSix && est.mean >= 4.0 * t6 && (double)t6 * t6 * six < 160.0 * sms * est.mean)
+        t6 = std::min(2 * t6, kGateMaxSix);
+    // Too many quiet gate outputs for blocks that would fit the busiest: the
+    // segment kernels, which cut every list to one length.  8 windows of 3,000
+    // outputs as above over 3,000 cycles: 2.76 in 32-thread blocks, 2.35 in
+    // 64-thread ones, 1.50 there.
+    if (t < 256 && est.busiest > even * t) return {0, 0};
+    return {t, t6};
 }
 
 // k_gate's threads at every level of a run of nwin windows together; empty
-// where the run does not go through it.
-static std::vector<uint32_t> gate_blocks(const gls_ctx *ctx, uint32_t nwin, bool w64, double est)
+// where the run goes through the segment kernels: by its schedule, or because
+// gate_block asks for them at most of its gate outputs (they keep no X times,
+// so a run goes one way throughout).
+static std::vector<GateThreads> gate_blocks(const gls_ctx *ctx, uint32_t nwin, bool w64, const GateEvents &est)
 {
     if (!gate_path(ctx, w64)) return {};
-    std::vector<uint32_t> t(ctx->drv_level_start.size() - 1);
-    for (size_t L = 0; L < t.size(); ++L)
-        t[L] = gate_block(ctx, (uint64_t)(ctx->drv_level_start[L + 1] - ctx->drv_level_start[L]) * nwin, est);
+    std::vector<GateThreads> t(ctx->drv_level_start.size() - 1);
+    uint64_t elsewhere = 0;
+    for (size_t L = 0; L < t.size(); ++L) {
+        const uint32_t *cls = &ctx->cls_start[(kClasses + 1) * L];
+        t[L] = gate_block(ctx, (uint64_t)cls[kClasses] * nwin, (uint64_t)(cls[kClasses] - cls[3]) * nwin, est);
+        if (!t[L].narrow) {
+            elsewhere += cls[kClasses];
+            t[L] = {128, 256};
+        }
+    }
+    if (2 * elsewhere > ctx->n_drv && !w64) return {};
     return t;
 }
 
@@ -907,7 +959,7 @@ static std::vector<uint32_t> gate_blocks(const gls_ctx *ctx, uint32_t nwin, bool
 // kernel classes are bracketed with events (not during stream capture).
 static int enqueue_levels(gls_ctx *ctx, const WinDev *const dw[2], const WinDev *const h[2], uint32_t nwin,
                           uint32_t max_stim, bool prof, uint32_t *launches, bool w64,
-                          const std::vector<uint32_t> &threads)
+                          const std::vector<GateThreads> &threads)
 {
     LevelArgs a;
     ctx_level_args(ctx, &a);
@@ -927,7 +979,7 @@ static int enqueue_levels(gls_ctx *ctx, const WinDev *const dw[2], const WinDev 
     // from the predictions: it keeps the plan whole, after the copies.)
     const bool learned = a.alloc_mode == kAllocLearned;
     const bool split = learned && ctx->bal_weight <= 0.f;
-    const bool gates = gate_path(ctx, w64);
+    const bool gates = !threads.empty();
     const bool overlap_ok = ctx->concurrent && ctx->pipeline && ctx->plan_overlap && !(prof && ctx->opts.profile) &&
                             (!learned || split);
     if (prof) prof_mark(ctx);
@@ -1368,7 +1420,7 @@ static int run_wave(gls_ctx *ctx, size_t w0, uint32_t nwin, const gls_batch_opts
 {
     WinDev *hw = ctx->hwave.as<WinDev>();
     uint32_t max_stim = 0;
-    double est = 0.0;
+    GateEvents est;
     for (uint32_t k = 0; k < nwin; ++k)
         CK(ctx->lsc[k]->ensure(ctx->max_width, ctx->seg_cap, ctx->scr_cap), "alloc level work spaces");
     for (uint32_t k = 0; k < nwin; ++k) {
@@ -1379,7 +1431,9 @@ static int run_wave(gls_ctx *ctx, size_t w0, uint32_t nwin, const gls_batch_opts
         hw[k] = make_windev(ctx, w, *ctx->lsc[k], 0);
         hw[kMaxWave + k] = make_windev(ctx, w, *ctx->lsc[k], 1);
         max_stim = std::max(max_stim, hw[k].n_stim);
-        est += gate_events_est(ctx, w) / nwin;
+        const GateEvents e = gate_events_est(ctx, w);
+        est.mean += e.mean / nwin;
+        est.busiest = std::max(est.busiest, e.busiest);
     }
     for (int p = 0; p < 2; ++p)
         CK(cudaMemcpyAsync(ctx->dwave.as<WinDev>() + p * kMaxWave, hw + p * kMaxWave, nwin * sizeof(WinDev),
@@ -1389,7 +1443,7 @@ static int run_wave(gls_ctx *ctx, size_t w0, uint32_t nwin, const gls_batch_opts
     const WinDev *hp[2] = {&hw[0], &hw[kMaxWave]};
     launch_reset(dw[0], hw[0], nwin, max_stim, ctx->n_nets, (uint32_t)ctx->drv_level_start.size(), ctx->stream);
     const bool w64 = nwin == 1 && ctx->windows[w0]->w64;
-    const std::vector<uint32_t> threads = gate_blocks(ctx, nwin, w64, est);
+    const std::vector<GateThreads> threads = gate_blocks(ctx, nwin, w64, est);
     CK(cudaEventRecord(e0, ctx->stream), "event");
     if (o.use_graph && nwin > 1) {
         // one graph per wave shape; the descriptors it reads are rewritten per wave

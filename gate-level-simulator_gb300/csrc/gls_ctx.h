@@ -192,6 +192,7 @@ struct LevelScratch {
 struct Window {
     std::vector<uint32_t> stim_nets;
     uint64_t stim_events = 0;           // aligned extent of the stimulus in the pool
+    uint64_t stim_longest = 0;          // the longest list (aligned) of a net that a gate reads
     PinBuf h_words;                     // packed stimulus events (kept to re-upload on pool growth)
     PinBuf h_stim;                      // per stimulus net: nets, lengths, then (64 bits) aligned pool offsets
     uint64_t t_begin = 0, t_end = 0;
@@ -233,7 +234,7 @@ struct gls_ctx {
     float bal_weight = 0.f;          // learned balance of segments in use (0: off)
     float bal_weight_on = 0.5f;      // its factor when GLS_SCHED_LEARNED_BALANCE is set (GLS_BALANCE_WEIGHT)
     bool pipeline = true;            // with concurrent classes: each class links and copies on its own stream
-    uint32_t gate_threads = 0;       // k_gate's block (GLS_GATE_THREADS; 0: by the level's width)
+    uint32_t gate_threads = 0;       // k_gate's block (GLS_GATE_THREADS; 0: by the level's width and lists)
     bool gate_kernel = true;         // levels run in one launch (GLS_GATE=0: the segment kernels)
     uint32_t copy_lanes = 8;         // lanes per segment of the copy kernel (GLS_COPY_LANES: 4, 8, 16, 32)
     int sm_count = 0;
@@ -281,7 +282,7 @@ struct gls_ctx {
     std::vector<DevBuf> spare_bufs;  // device buffers of windows that ran saif_only, reused by later windows
     struct WaveGraph {
         uint32_t nwin, max_stim, warp_mask, alloc_mode, seg_per_sm, flags;   // flags: GLS_SCHED_*
-        std::vector<uint32_t> threads;   // k_gate's block at every level: the windows' list lengths decide it
+        std::vector<gls::GateThreads> threads;   // k_gate's block at every level: the windows' list lengths decide it
         cudaGraphExec_t exec;
         uint32_t launches;
         bool same(const WaveGraph &o) const

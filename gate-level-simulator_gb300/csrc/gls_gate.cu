@@ -28,7 +28,6 @@ namespace gls {
 
 namespace {
 
-constexpr int kMaxWarps = kGateMaxThreads / 32;
 // threads per SM the kernels are compiled for.  kSix: the class of four to six
 // input nets, which walks by general steps in more registers (12 levels of
 // 3,000 such gate outputs of 140,000 events: 256 / 512 / 768 / 1,024 threads
@@ -40,27 +39,29 @@ template <bool kSix, class Wd> __host__ __device__ constexpr uint32_t gate_resid
 }
 
 // Shared memory is L1 lost: each kernel has only what it uses, the step table
-// (kTab), what meets between warps (not kWarp) and the window's descriptor
-// (kBatch).  With 512 bytes before the segments' a 1,024-thread SM gets by
+// (kTab) and the window's descriptor (kBatch), and behind the segments' words
+// what meets between the warps there are (WarpParts).  With 512 bytes before the segments' a 1,024-thread SM gets by
 // with 16 KB (one step of the split more: 2 M cells 68.7 instead of 68.3 ms,
 // 200,000 cells 13.1 instead of 12.9); one-warp blocks with 272 bytes instead
 // of 1,280: 8 windows of 200,000 cells 19.8 -> 19.5, 48 of 2,000 cells .89 ->
 // .87.
 template <bool kTab> struct TabSmem { GateTab tab; };   // the gate output's tables
 template <> struct TabSmem<false> {};
-template <bool kWarp, class Wd> struct WarpsSmem {
-    Wd a[kMaxWarps];             // per warp: smallest candidate of its segments; at the end its part of T0
-    Wd b[kMaxWarps];             // kept entries; at the end its part of T1
-    uint8_t wlast[kMaxWarps];    // value of its last kept entry (4: none)
+template <class Wd> struct WarpParts {   // an entry per warp, at the end of the dynamic shared memory
+    Wd *a;              // smallest candidate of its segments; at the end its part of T0
+    Wd *b;              // kept entries; at the end its part of T1
+    uint8_t *last;      // value of its last kept entry (4: none)
+    __device__ __forceinline__ WarpParts(void *at, uint32_t nw)
+        : a(static_cast<Wd *>(at)), b(a + nw), last(reinterpret_cast<uint8_t *>(b + nw)) {}
+    static constexpr uint32_t kBytes = 2 * sizeof(Wd) + 1;   // per warp
 };
-template <class Wd> struct WarpsSmem<true, Wd> {};
 template <bool kBatch> struct WindowSmem {
     WinDev win;                  // wave of windows: the descriptor of the block's current window
     uint32_t cw;                 // its number
 };
 template <> struct WindowSmem<false> {};
-template <bool kBatch, bool kTab, bool kWarp, class Wd>
-struct GateSmem : TabSmem<kTab>, WarpsSmem<kWarp, Wd>, WindowSmem<kBatch> {
+template <bool kBatch, bool kTab>
+struct GateSmem : TabSmem<kTab>, WindowSmem<kBatch> {
     unsigned long long ctr[4];   // gate events, output events, segments, fan-in events of the window at hand
     unsigned long long scr, dst; // the gate output's stacks in the scratch, its list in the pool
     uint32_t q;                  // the block's gate output, kInf: none left
@@ -225,6 +226,7 @@ __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a,
     const uint32_t region = wk.region, S = wk.S;
     const unsigned long long E = wk.E;
     const bool mine = tid < S;
+    const WarpParts<Wd> wp(s_seg + nthr, nw);
     if (!sm.ok) {   // no room for its stacks; the same for the whole block
         sync_block<kWarp>();
         if (tid == 0) fetch();
@@ -243,9 +245,9 @@ __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a,
     Wd later = __shfl_down_sync(FULL, x, 1);
     if (lane == 31) later = EvW<Wd>::kInfW;
     if constexpr (!kWarp) {
-        if (lane == 0) sm.a[wid] = x;
+        if (lane == 0) wp.a[wid] = x;
         __syncthreads();
-        for (uint32_t k = wid + 1; k < nw; ++k) later = min(later, sm.a[k]);
+        for (uint32_t k = wid + 1; k < nw; ++k) later = min(later, wp.a[k]);
     }
     uint32_t keep = o.cnt, firstv = 0, lastv = 0;
     if (keep && later != EvW<Wd>::kInfW)
@@ -261,11 +263,11 @@ __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a,
     const uint32_t vtop = __shfl_sync(FULL, lastv, bal ? 31 - __clz(bal) : 0);
     if (!prior) vprev = kVX;
     if constexpr (!kWarp) {
-        if (lane == 0) sm.wlast[wid] = bal ? vtop : 4u;
+        if (lane == 0) wp.last[wid] = bal ? vtop : 4u;
         __syncthreads();
         if (!prior)
             for (int k = (int)wid - 1; k >= 0; --k)
-                if (sm.wlast[k] < 4u) { vprev = sm.wlast[k]; break; }
+                if (wp.last[k] < 4u) { vprev = wp.last[k]; break; }
     }
     const uint32_t drop = (tid > 0 && keep > 0 && firstv == vprev) ? 1u : 0u;
     const uint32_t fin = keep - drop;
@@ -279,10 +281,10 @@ __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a,
     if constexpr (kWarp) {
         total = __shfl_sync(FULL, inc, 31);
     } else {
-        if (lane == 31) sm.b[wid] = inc;
+        if (lane == 31) wp.b[wid] = inc;
         __syncthreads();
         for (uint32_t k = 0; k < nw; ++k) {
-            const uint32_t n = (uint32_t)sm.b[k];
+            const uint32_t n = (uint32_t)wp.b[k];
             if (k < wid) pos += n;
             total += n;
         }
@@ -383,7 +385,7 @@ __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a,
     if constexpr (kWarp) {
         if (!bal) last = kVX;
     } else {
-        if (lane == 0) { sm.a[wid] = s0; sm.b[wid] = s1; }
+        if (lane == 0) { wp.a[wid] = s0; wp.b[wid] = s1; }
         __syncthreads();
     }
     if (tid == 0) {
@@ -391,9 +393,9 @@ __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a,
             last = kVX;
             s0 = s1 = 0;
             for (uint32_t k = 0; k < nw; ++k) {
-                s0 += sm.a[k];
-                s1 += sm.b[k];
-                if (sm.wlast[k] < 4u) last = sm.wlast[k];
+                s0 += wp.a[k];
+                s1 += wp.b[k];
+                if (wp.last[k] < 4u) last = wp.last[k];
             }
         }
         using Sg = typename std::make_signed<P>::type;
@@ -423,13 +425,14 @@ __device__ __forceinline__ void finish_gate(const WinDev &w, const LevelArgs &a,
 // 2- and 3-input ones start).  Blocks take gate outputs from the back, the
 // widest first, as they become free.
 template <bool kBatch, bool kSix, bool kTab, class Wd>
-__global__ void __launch_bounds__(kSix || kTab ? kGateMaxThreads : 32,
-                                  gate_resident<kSix, Wd>() / (kSix || kTab ? kGateMaxThreads : 32))
+__global__ void __launch_bounds__(kSix || kTab ? gate_resident<kSix, Wd>() : 32,
+                                  kSix || kTab ? 1 : gate_resident<kSix, Wd>() / 32)
     k_gate(const WinSet<kBatch> ws, LevelArgs a, uint32_t d0, uint32_t d1, uint32_t c1, uint32_t c2)
 {
     constexpr bool kWarp = !kSix && !kTab;
-    __shared__ __align__(256) GateSmem<kBatch, kTab, kWarp, Wd> sm;
-    extern __shared__ uint32_t s_seg[];   // per thread the time its segment starts at; then see finish_gate
+    __shared__ __align__(256) GateSmem<kBatch, kTab> sm;
+    // per thread the time its segment starts at (then see finish_gate), then WarpParts
+    extern __shared__ __align__(8) uint32_t s_seg[];
     const uint32_t nthr = kWarp ? 32u : blockDim.x;
     const uint32_t n = d1 - d0, total = n * ws.size();
     auto fetch = [&](uint32_t q) {   // thread 0
@@ -502,17 +505,19 @@ __global__ void __launch_bounds__(kSix || kTab ? kGateMaxThreads : 32,
 }
 
 void launch_gate(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelArgs &level, const uint32_t *cls,
-                 uint32_t threads, bool table, int sm_count, cudaStream_t st, uint32_t *launches)
+                 GateThreads block, bool table, int sm_count, cudaStream_t st, uint32_t *launches)
 {
     LevelArgs a = level;
     a.x_times = table ? 1u : 0u;
-    const uint32_t smem = threads * 4;
     auto go = [&](auto six, auto tab, uint32_t d0, uint32_t d1) {
         constexpr bool kSix = decltype(six)::value, kTab = decltype(tab)::value;
         if (d1 <= d0) return;
         const uint64_t total = (uint64_t)(d1 - d0) * nwin;
-        const uint64_t room =
-            (uint64_t)sm_count * ((a.wide ? gate_resident<kSix, WideWord>() : gate_resident<kSix, uint32_t>()) / threads);
+        const uint32_t resident = a.wide ? gate_resident<kSix, WideWord>() : gate_resident<kSix, uint32_t>();
+        const uint32_t threads = kSix ? (block.six < resident ? block.six : resident) : block.narrow;
+        const uint32_t parts = a.wide ? WarpParts<WideWord>::kBytes : WarpParts<uint32_t>::kBytes;
+        const uint32_t smem = threads * 4 + (kSix || kTab ? threads / 32 * parts : 0);
+        const uint64_t room = (uint64_t)sm_count * (resident / threads);
         const uint32_t grid = (uint32_t)(total < room ? total : room);
         cudaLaunchAttribute at;
         at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -537,7 +542,7 @@ void launch_gate(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelAr
     go(T(), F(), cls[3], cls[4]);
     // the step table is for warps none of whose segments starts at X: in a
     // block of one warp the first one does
-    if (threads > 32) go(F(), T(), 0u, cls[3]);
+    if (block.narrow > 32) go(F(), T(), 0u, cls[3]);
     else go(F(), F(), 0u, cls[3]);
 }
 

@@ -253,8 +253,12 @@ void launch_copy(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelAr
 
 // One level in one launch (a second one where gate outputs with
 // four to six input nets exist).  cls: the level's fan-in class starts
-// (kClasses + 1); threads per block: 32 .. kGateMaxThreads, a power of two.
-constexpr uint32_t kGateMaxThreads = 256;
+// (kClasses + 1).
+struct GateThreads {            // threads per block, multiples of 32
+    uint32_t narrow, six;       // of gate outputs with up to three input nets, with four to six
+    bool operator==(const GateThreads &o) const { return narrow == o.narrow && six == o.six; }
+};
+constexpr uint32_t kGateMaxThreads = 512, kGateMaxSix = 768;   // 512 in 64-bit windows
 // Fan-in events a time segment of k_gate is worth a search.  A block's threads
 // are there anyway, and its time is that of its longest segment: 32 / 16 / 8 /
 // 4 / 2 measured .36 / .28 / .24 / .23 / .23 ms on 2,000 cells over 1,000
@@ -262,6 +266,6 @@ constexpr uint32_t kGateMaxThreads = 256;
 // 67.3 / 66.5 / 66.8 / 66.8 on 2 M cells.
 constexpr uint32_t kGateMinSeg = 4;
 void launch_gate(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelArgs &a, const uint32_t *cls,
-                 uint32_t threads, bool table, int sm_count, cudaStream_t st, uint32_t *launches);
+                 GateThreads block, bool table, int sm_count, cudaStream_t st, uint32_t *launches);
 
 }  // namespace gls
