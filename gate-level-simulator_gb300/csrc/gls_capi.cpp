@@ -824,6 +824,8 @@ extern "C" int gls_add_window(gls_ctx *ctx, const gls_stimulus *st, uint64_t t_b
 // parity 1: the per-gate-output tables of odd levels
 static WinDev make_windev(gls_ctx *ctx, Window *w, const LevelScratch &ls, int parity = 0)
 {
+    w->ran_segs = ls.seg_cap;
+    w->ran_scr = ls.scr_cap;
     WinDev d;
     std::memset(&d, 0, sizeof d);
     d.net_off = w->net_off.as<uint64_t>();
@@ -1245,8 +1247,11 @@ static int settle_window(gls_ctx *ctx, Window *w, RunAcc &acc, const unsigned lo
                                                            : "segment region overflow");
         }
         if (attempt > 12) return fail(ctx, GLS_EOVERFLOW, "event pool could not grow enough");
-        if (err & kErrSegCap) ctx->seg_cap = std::max<uint32_t>(ctx->seg_cap, ctx->lsc[0]->seg_cap) * 2;
-        if (err & kErrScratch) ctx->scr_cap = std::max<uint64_t>(ctx->scr_cap, ctx->lsc[0]->scr_cap) * 2;
+        // a window before this one may have grown the work space already
+        ctx->seg_cap = std::max<uint32_t>(ctx->seg_cap, ctx->lsc[0]->seg_cap);
+        ctx->scr_cap = std::max<uint64_t>(ctx->scr_cap, ctx->lsc[0]->scr_cap);
+        if ((err & kErrSegCap) && w->ran_segs >= ctx->seg_cap) ctx->seg_cap *= 2;
+        if ((err & kErrScratch) && w->ran_scr >= ctx->scr_cap) ctx->scr_cap *= 2;
         {
             const cudaError_t e = ctx->lsc[0]->ensure(ctx->max_width, ctx->seg_cap, ctx->scr_cap);
             if (e != cudaSuccess)

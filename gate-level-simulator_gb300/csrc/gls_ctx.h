@@ -197,6 +197,8 @@ struct Window {
     PinBuf h_stim;                      // per stimulus net: nets, lengths, then (64 bits) aligned pool offsets
     uint64_t t_begin = 0, t_end = 0;
     uint64_t cap = 0;
+    uint32_t ran_segs = 0;              // the work space its last run had: segments, stack words
+    uint64_t ran_scr = 0;
     DevBuf pool, net_off, net_len, saif, small, stim_dev;
     DevBuf dwin;                        // the window's WinDev on the device (sequential runs)
     DevBuf lvl;                         // LevelCtr per level

@@ -3,8 +3,11 @@ gave back without running them."""
 import numpy as np
 import pytest
 
+from cases import stimulus
 from gls import synth
 from gls.capi import GlsError, Simulator
+from gls.cells import LIBRARY
+from gls.levelize import assemble, default_arcs
 
 pytestmark = pytest.mark.gpu
 
@@ -112,3 +115,39 @@ def test_graph_of_a_wave_fits_its_windows(order, design, gpu):
                 s0, f0 = wave(alone, cycles)
             assert segments == s0
             assert all(np.array_equal(a, b) for a, b in zip(saif, f0))
+
+
+@pytest.mark.parametrize("batched", [False, True])
+def test_windows_that_all_outgrow_the_work_space(batched, gpu):
+    """Glitching XOR levels need far more stack space than the stimulus lets
+    expect, in every one of 40 windows of a fresh context: the space grows with
+    the need, not once more for every window."""
+    rng = np.random.default_rng(3)
+    c = LIBRARY["GEN_XOR2_D1"]
+    insts, src, nn = [], list(range(24)), 24
+    for _ in range(10):
+        for k in range(40):
+            a, b = (int(x) for x in rng.choice(src, 2, replace=False))
+            insts.append((c.name, [a, b], [nn + k], default_arcs(c, float(rng.integers(2, 9)), float(rng.integers(2, 9)))))
+        src, nn = list(range(nn, nn + 40)), nn + 40
+    nl = assemble(insts, n_nets=nn)
+
+    def window(seed):
+        r = np.random.default_rng(seed)
+        return stimulus({n: [(0, 0)] + [(1000 * e + int(r.integers(1, 900)), 0 if e % 2 else 3) for e in range(120)]
+                         for n in range(24)})
+
+    wins = [window(100 + k) for k in range(40)]
+    with Simulator() as s:
+        s.load(nl)
+        ids = [s.add_window(st, 0, 121_000) for st in wins]
+        if batched:
+            s.run_batched()
+        else:
+            s.run()
+        for w in ids[::13]:
+            with Simulator() as one:
+                one.load(nl)
+                v = one.add_window(wins[w], 0, 121_000)
+                one.run()
+                assert np.array_equal(one.saif(v), s.saif(w)) and np.array_equal(one.lengths(v), s.lengths(w))
