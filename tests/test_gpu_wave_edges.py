@@ -151,3 +151,28 @@ def test_windows_that_all_outgrow_the_work_space(batched, gpu):
                 v = one.add_window(wins[w], 0, 121_000)
                 one.run()
                 assert np.array_equal(one.saif(v), s.saif(w)) and np.array_equal(one.lengths(v), s.lengths(w))
+
+
+@pytest.mark.parametrize("period", [1_000, 20_000_000])
+def test_first_run_of_a_context_is_its_only_one(period, gpu):
+    """Two levels of XORs whose inputs never move together: the second level's
+    lists are twice the stimulus', as long as the stack space is sized for.
+    The first run takes no more launches than the next, whatever the segments
+    add, in 32-bit and in 64-bit event words."""
+    w, events = 200, 100
+    c = LIBRARY["GEN_XOR2_D1"]
+    insts = [(c.name, [2 * k, 2 * k + 1], [4 * w + k], default_arcs(c, 3.0, 5.0)) for k in range(2 * w)]
+    insts += [(c.name, [4 * w + 2 * k, 4 * w + 2 * k + 1], [6 * w + k], default_arcs(c, 4.0, 6.0)) for k in range(w)]
+    insts += [(c.name, [4 * w + 2 * k, 4 * w + (2 * k + 3) % (2 * w)], [7 * w + k], default_arcs(c, 4.0, 6.0)) for k in range(w)]
+    nl = assemble(insts, n_nets=8 * w)
+    st = stimulus({n: [(0, 0)] + [(period * e + period // 4 * (n % 4), 0 if e % 2 else 3) for e in range(1, events)]
+                   for n in range(4 * w)})
+    with Simulator() as s:
+        s.load(nl)
+        v = s.add_window(st, 0, period * events)
+        s.run()
+        first, lens = s.stats()["launches"], s.lengths(v)
+        assert lens[6 * w:].min() > 3.5 * events   # the estimate's limit: two such lists a gate output of the third level
+        s.run()
+        assert s.stats()["launches"] == first == 3
+        assert s.stats()["wide_windows"] == (1 if period > 1_000_000 else 0)
