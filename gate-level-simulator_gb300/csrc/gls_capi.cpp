@@ -733,14 +733,19 @@ extern "C" int gls_add_window(gls_ctx *ctx, const gls_stimulus *st, uint64_t t_b
     for (uint32_t k = 0; k < st->n_nets; ++k)
         if (st->ev_start[k + 1] > st->ev_start[k] && st->time[st->ev_start[k + 1] - 1] > kMaxTime) w->w64 = true;
     // several threads from about 2^17 events on: 110 us for any count up to
-    // 2^18, one thread 129 us at 2^17 and 233 us at 2^18
-    constexpr uint64_t kPackAlone = 1u << 17;
+    // 2^18, one thread 129 us at 2^17 and 233 us at 2^18.  Making them takes as
+    // long as packing 2^19 events alone (.4 ms), so they are made for a
+    // stimulus of 2^20, or once the context has packed as many without them.
+    constexpr uint64_t kPackAlone = 1u << 17, kPackThreads = 1u << 20;
     const unsigned hc = std::max(1u, std::min(16u, std::thread::hardware_concurrency()));
     if (total > kPackAlone && hc > 1 && st->n_nets > 4 * hc && !ctx->pool) {
-        try {
-            ctx->pool = new WorkPool(hc - 1);
-        } catch (...) {   // no threads to be had: pack on this one
-            ctx->pool = nullptr;
+        ctx->packed_alone += total;
+        if (ctx->packed_alone > kPackThreads) {
+            try {
+                ctx->pool = new WorkPool(hc - 1);
+            } catch (...) {   // no threads to be had: pack on this one
+                ctx->pool = nullptr;
+            }
         }
     }
     auto pack_all = [&](auto *hw) {

@@ -278,7 +278,8 @@ struct gls_ctx {
     PinBuf hwave;
     PinBuf hsmall;                   // the windows' flags and counters after a run (64 bytes each)
     PinBuf pin_out;                  // staging of SAIF counts and lengths read back to the host
-    WorkPool *pool = nullptr;        // host threads that pack stimuli (made on first use)
+    WorkPool *pool = nullptr;        // host threads that pack stimuli (made once they are worth it)
+    uint64_t packed_alone = 0;       // events of larger stimuli packed without them
     DevBuf dwave;
     DevBuf wave_e;                   // per level: a wave's fan-in events per class
     std::vector<DevBuf> spare_bufs;  // device buffers of windows that ran saif_only, reused by later windows
