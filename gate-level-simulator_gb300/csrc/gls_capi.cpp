@@ -1438,6 +1438,18 @@ static uint64_t wave_length(const gls_ctx *ctx, size_t w0, uint64_t nwin)
     return nwin;
 }
 
+// The fan-in events of the gate outputs of windows [w0, w0 + nwin).
+static GateEvents wave_events(const gls_ctx *ctx, size_t w0, uint32_t nwin)
+{
+    GateEvents est;
+    for (uint32_t k = 0; k < nwin; ++k) {
+        const GateEvents e = gate_events_est(ctx, ctx->windows[w0 + k]);
+        est.mean += e.mean / nwin;
+        est.busiest = std::max(est.busiest, e.busiest);
+    }
+    return est;
+}
+
 // One wave: windows [w0, w0 + nwin) together; *ms receives its device time
 // (upload of new stimuli excluded, reruns of windows that outgrew a buffer
 // included in acc).
@@ -1446,7 +1458,6 @@ static int run_wave(gls_ctx *ctx, size_t w0, uint32_t nwin, const gls_batch_opts
 {
     WinDev *hw = ctx->hwave.as<WinDev>();
     uint32_t max_stim = 0;
-    GateEvents est;
     for (uint32_t k = 0; k < nwin; ++k)
         CK(ctx->lsc[k]->ensure(ctx->max_width, ctx->seg_cap, ctx->scr_cap), "alloc level work spaces");
     for (uint32_t k = 0; k < nwin; ++k) {
@@ -1457,9 +1468,6 @@ static int run_wave(gls_ctx *ctx, size_t w0, uint32_t nwin, const gls_batch_opts
         hw[k] = make_windev(ctx, w, *ctx->lsc[k], 0);
         hw[kMaxWave + k] = make_windev(ctx, w, *ctx->lsc[k], 1);
         max_stim = std::max(max_stim, hw[k].n_stim);
-        const GateEvents e = gate_events_est(ctx, w);
-        est.mean += e.mean / nwin;
-        est.busiest = std::max(est.busiest, e.busiest);
     }
     for (int p = 0; p < 2; ++p)
         CK(cudaMemcpyAsync(ctx->dwave.as<WinDev>() + p * kMaxWave, hw + p * kMaxWave, nwin * sizeof(WinDev),
@@ -1469,7 +1477,7 @@ static int run_wave(gls_ctx *ctx, size_t w0, uint32_t nwin, const gls_batch_opts
     const WinDev *hp[2] = {&hw[0], &hw[kMaxWave]};
     launch_reset(dw[0], hw[0], nwin, max_stim, ctx->n_nets, (uint32_t)ctx->drv_level_start.size(), ctx->stream);
     const bool w64 = nwin == 1 && ctx->windows[w0]->w64;
-    const std::vector<GateThreads> threads = gate_blocks(ctx, nwin, w64, est);
+    const std::vector<GateThreads> threads = gate_blocks(ctx, nwin, w64, wave_events(ctx, w0, nwin));
     CK(cudaEventRecord(e0, ctx->stream), "event");
     if (o.use_graph && nwin > 1) {
         // one graph per wave shape; the descriptors it reads are rewritten per wave
@@ -1608,7 +1616,7 @@ extern "C" int gls_autotune(gls_ctx *ctx, const gls_batch_opts *opts, gls_tune_r
     // which fan-in classes run warp-per-segment.  Stage 2, on the best of
     // those: class-stream priority, the gate kernel's block size and load
     // width (the variants change nothing but speed).
-    static const uint32_t kSegs[] = {1024, 2048, 4096};
+    static const uint32_t kSegs[] = {2048, 1024, 4096};
     static const uint32_t kMasks[] = {0, 1, 7};
     static const uint32_t kFlags2[] = {GLS_SCHED_CLASS_PRIORITY, GLS_SCHED_BLOCK256, GLS_SCHED_WIDE_LOADS,
                                        GLS_SCHED_BLOCK256 | GLS_SCHED_WIDE_LOADS};
@@ -1620,23 +1628,35 @@ extern "C" int gls_autotune(gls_ctx *ctx, const gls_batch_opts *opts, gls_tune_r
     CK(cudaEventCreate(&e1), "event");
     const uint32_t keep_segs = ctx->seg_per_sm, keep_mask = ctx->warp_mask, keep_flags = schedule_flags(ctx);
     uint32_t c = 0;
+    // Candidates that make the same launches (a level in one launch knows no
+    // segments per SM and no class streams; windows of 64-bit words no schedule
+    // at all) are timed once, and the first of them, the default, stands.
+    float one_launch_ms = -1.f;
     auto trial = [&](uint32_t segs, uint32_t mask, uint32_t flags) {
         apply_schedule(ctx, segs, mask, flags);
-        RunAcc acc;
+        auto one_launch = [&]() {
+            return !gate_blocks(ctx, nwin, nwin == 1 && ctx->windows[0]->w64, wave_events(ctx, 0, nwin)).empty();
+        };
         float t = 1e30f;
-        // the first run of a shape captures its graph; the best of the next two counts
-        for (int rep = 0; rep < 3 && rc == GLS_OK; ++rep) {
-            float tr = 0.f;
-            rc = run_wave(ctx, 0, nwin, o, acc, &tr, e0, e1);
-            if (rep) t = std::min(t, tr);
-            // a window whose output times turned out to need 64-bit words
-            // (the first run tells) leaves the wave that is timed
-            const uint32_t together = (uint32_t)wave_length(ctx, 0, nwin);
-            if (rc == GLS_OK && together < nwin) {
-                nwin = together;
-                rep = -1;
-                t = 1e30f;
+        if (one_launch_ms >= 0.f && one_launch()) {
+            t = one_launch_ms;
+        } else {
+            RunAcc acc;
+            // the first run of a shape captures its graph; the best of the next two counts
+            for (int rep = 0; rep < 3 && rc == GLS_OK; ++rep) {
+                float tr = 0.f;
+                rc = run_wave(ctx, 0, nwin, o, acc, &tr, e0, e1);
+                if (rep) t = std::min(t, tr);
+                // a window whose output times turned out to need 64-bit words
+                // (the first run tells) leaves the wave that is timed
+                const uint32_t together = (uint32_t)wave_length(ctx, 0, nwin);
+                if (rc == GLS_OK && together < nwin) {
+                    nwin = together;
+                    rep = -1;
+                    t = 1e30f;
+                }
             }
+            if (rc == GLS_OK && one_launch()) one_launch_ms = t;
         }
         r.ms[c] = t;
         r.seg_per_sm[c] = segs;

@@ -176,3 +176,27 @@ def test_first_run_of_a_context_is_its_only_one(period, gpu):
         s.run()
         assert s.stats()["launches"] == first == 3
         assert s.stats()["wide_windows"] == (1 if period > 1_000_000 else 0)
+
+
+@pytest.mark.parametrize("late", [False, True])
+def test_autotune_times_equal_schedules_once(late, design, gpu):
+    """Schedules that make the same launches have one time, and do not replace
+    each other by chance: a level in one launch knows no segments per SM and no
+    class streams, a window of 64-bit words no schedule at all."""
+    cfg, nl = design
+    cfg = synth.scaled(cfg)
+    cfg.period = 20_000_000 if late else cfg.period
+    with Simulator() as s:
+        s.load(nl)
+        w = s.add_window(synth.make_stimulus(cfg, nl.ppi_nets, seed=90), 0, cfg.t_end)
+        t = s.autotune()
+        ms = [c["ms"] for c in t["candidates"]]
+        assert len(ms) == 13
+        assert ms[0] == ms[1] == ms[2]
+        assert len(set(ms)) == 1 if late else len(set(ms)) > 1
+        if t["best"]["warp_mask"] == 0 and t["best"]["flags"] == 0:
+            assert t["best"]["seg_per_sm"] == 2048 and t["candidates"][9]["ms"] == ms[0]
+        assert not (t["best"]["flags"] == 1 and t["best"]["warp_mask"] == 0)
+        tuned = s.saif(w).copy()
+        s.run()
+        assert np.array_equal(tuned, s.saif(w))
