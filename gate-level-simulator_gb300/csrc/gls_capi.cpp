@@ -585,7 +585,7 @@ extern "C" int gls_load_netlist(gls_ctx *ctx, const gls_netlist *nl)
     ctx->seg_cap = std::max<uint32_t>(1u << 21, 8 * ctx->max_width + 64);
     if (ctx->lsc.empty()) ctx->lsc.push_back(new LevelScratch);
     for (LevelScratch *l : ctx->lsc) l->release();
-    CK(ctx->lsc[0]->ensure(ctx->max_width, ctx->seg_cap, ctx->scr_cap), "alloc level work space");
+    CK(ctx->lsc[0]->ensure(ctx->max_width, ctx->seg_cap, ctx->scr_cap, false), "alloc level work space");
     ctx->loaded = true;
     return GLS_OK;
 }
@@ -824,7 +824,7 @@ extern "C" int gls_add_window(gls_ctx *ctx, const gls_stimulus *st, uint64_t t_b
         want *= w->word_bytes() / 4;   // 32-bit words
         if (want > ctx->scr_cap) {
             ctx->scr_cap = want;
-            CK(ctx->lsc[0]->ensure(ctx->max_width, ctx->seg_cap, ctx->scr_cap), "alloc level scratch");
+            CK(ctx->lsc[0]->ensure(ctx->max_width, ctx->seg_cap, ctx->scr_cap, false), "alloc level scratch");
         }
     }
     // device buffers are filled when the window first runs
@@ -1180,14 +1180,20 @@ static int enqueue_window(gls_ctx *ctx, Window *w, uint32_t *launches)
     int rc = w->uploaded ? GLS_OK : upload_window(ctx, w);
     if (rc) return rc;
     w->saif_only = false;
+    const std::vector<GateThreads> threads = gate_blocks(ctx, 1, w->w64, gate_events_est(ctx, w));
+    {
+        const cudaError_t e = ctx->lsc[0]->ensure(ctx->max_width, ctx->seg_cap, ctx->scr_cap, threads.empty());
+        if (e != cudaSuccess)
+            return fail(ctx, GLS_ENOMEM, "level work space of %llu stack words / %u segments: %s",
+                        (unsigned long long)ctx->scr_cap, ctx->seg_cap, cudaGetErrorString(e));
+    }
     const WinDev d[2] = {make_windev(ctx, w, *ctx->lsc[0], 0), make_windev(ctx, w, *ctx->lsc[0], 1)};
     CK(w->dwin.ensure(sizeof d), "alloc window descriptor");
     CK(cudaMemcpyAsync(w->dwin.p, d, sizeof d, cudaMemcpyHostToDevice, ctx->stream), "upload window descriptor");
     const WinDev *dw[2] = {w->dwin.as<WinDev>(), w->dwin.as<WinDev>() + 1};
     const WinDev *hp[2] = {&d[0], &d[1]};
     launch_reset(dw[0], d[0], 1, d[0].n_stim, ctx->n_nets, (uint32_t)ctx->drv_level_start.size(), ctx->stream);
-    return enqueue_levels(ctx, dw, hp, 1, d[0].n_stim, true, launches, w->w64,
-                          gate_blocks(ctx, 1, w->w64, gate_events_est(ctx, w)));
+    return enqueue_levels(ctx, dw, hp, 1, d[0].n_stim, true, launches, w->w64, threads);
 }
 
 // Copies the flags and counters of windows [w0, w0 + n) to ctx->hsmall, behind
@@ -1274,7 +1280,7 @@ static int settle_window(gls_ctx *ctx, Window *w, RunAcc &acc, const unsigned lo
             ctx->scr_cap *= small_space ? 4 : 2;
         }
         {
-            const cudaError_t e = ctx->lsc[0]->ensure(ctx->max_width, ctx->seg_cap, ctx->scr_cap);
+            const cudaError_t e = ctx->lsc[0]->ensure(ctx->max_width, ctx->seg_cap, ctx->scr_cap, false);
             if (e != cudaSuccess)
                 return fail(ctx, GLS_ENOMEM, "grow level work space to %llu stack words / %u segments (flags 0x%x): %s",
                             (unsigned long long)ctx->scr_cap, ctx->seg_cap, err, cudaGetErrorString(e));
@@ -1391,6 +1397,31 @@ static uint32_t schedule_flags(const gls_ctx *ctx)
            ((ctx->sim_variant & 2u) ? GLS_SCHED_WIDE_LOADS : 0u) | (ctx->bal_weight > 0.f ? GLS_SCHED_LEARNED_BALANCE : 0u);
 }
 
+// The fan-in events of the gate outputs of windows [w0, w0 + nwin).
+static GateEvents wave_events(const gls_ctx *ctx, size_t w0, uint32_t nwin)
+{
+    GateEvents est;
+    for (uint32_t k = 0; k < nwin; ++k) {
+        const GateEvents e = gate_events_est(ctx, ctx->windows[w0 + k]);
+        est.mean += e.mean / nwin;
+        est.busiest = std::max(est.busiest, e.busiest);
+    }
+    return est;
+}
+
+// Whether a wave of nwin of the context's windows may need the segment
+// kernels' tables: decided for the quietest windows beside the busiest.
+static bool wave_tables(const gls_ctx *ctx, uint64_t nwin)
+{
+    GateEvents est;
+    for (size_t k = 0; k < ctx->windows.size(); ++k) {
+        const GateEvents e = gate_events_est(ctx, ctx->windows[k]);
+        est.mean = k ? std::min(est.mean, e.mean) : e.mean;
+        est.busiest = std::max(est.busiest, e.busiest);
+    }
+    return gate_blocks(ctx, (uint32_t)nwin, false, est).empty();
+}
+
 // Checks and buffers of a batched run; *B receives the windows per wave.
 static int batch_setup(gls_ctx *ctx, const gls_batch_opts &o, uint64_t *B)
 {
@@ -1405,20 +1436,21 @@ static int batch_setup(gls_ctx *ctx, const gls_batch_opts &o, uint64_t *B)
     // memory holds (each needs its pool, net tables and a level work space)
     uint64_t b = std::min<uint64_t>(std::max<size_t>(nw, 1), kMaxWave);
     if (o.max_wave) b = std::min<uint64_t>(b, o.max_wave);
+    const bool tables = wave_tables(ctx, b);
     if (o.saif_only) {
         size_t fr = 0, tot = 0;
         cudaMemGetInfo(&fr, &tot);
         fr += spare_bytes(ctx);
         uint64_t per = 0;
         for (Window *w : ctx->windows) per = std::max<uint64_t>(per, projected_cap(ctx, w) * w->word_bytes());
-        per += (uint64_t)ctx->n_nets * 56 + (uint64_t)(ctx->max_width + 1) * 32 +
-               (uint64_t)ctx->seg_cap * (sizeof(SegRec) + sizeof(CopyRec)) + ctx->scr_cap * 4;
+        per += (uint64_t)ctx->n_nets * 56 + (uint64_t)(ctx->max_width + 1) * 4 + ctx->scr_cap * 4;
+        if (tables) per += (uint64_t)(ctx->max_width + 1) * 48 + (uint64_t)ctx->seg_cap * (sizeof(SegRec) + sizeof(CopyRec));
         const uint64_t fit = std::max<uint64_t>(1, (uint64_t)(0.85 * (double)fr) / std::max<uint64_t>(per, 1));
         b = std::max<uint64_t>(1, std::min(b, fit));
     }
     while (ctx->lsc.size() < b) ctx->lsc.push_back(new LevelScratch);
     for (uint64_t k = 0; k < b; ++k)
-        CK(ctx->lsc[k]->ensure(ctx->max_width, ctx->seg_cap, ctx->scr_cap), "alloc level work spaces");
+        CK(ctx->lsc[k]->ensure(ctx->max_width, ctx->seg_cap, ctx->scr_cap, tables), "alloc level work spaces");
     // two descriptor sets: the per-gate-output tables of even and odd levels
     if (!ctx->hwave.ensure(2 * kMaxWave * sizeof(WinDev))) return fail(ctx, GLS_ENOMEM, "pinned wave descriptors");
     CK(ctx->dwave.ensure(2 * kMaxWave * sizeof(WinDev)), "alloc wave descriptors");
@@ -1438,18 +1470,6 @@ static uint64_t wave_length(const gls_ctx *ctx, size_t w0, uint64_t nwin)
     return nwin;
 }
 
-// The fan-in events of the gate outputs of windows [w0, w0 + nwin).
-static GateEvents wave_events(const gls_ctx *ctx, size_t w0, uint32_t nwin)
-{
-    GateEvents est;
-    for (uint32_t k = 0; k < nwin; ++k) {
-        const GateEvents e = gate_events_est(ctx, ctx->windows[w0 + k]);
-        est.mean += e.mean / nwin;
-        est.busiest = std::max(est.busiest, e.busiest);
-    }
-    return est;
-}
-
 // One wave: windows [w0, w0 + nwin) together; *ms receives its device time
 // (upload of new stimuli excluded, reruns of windows that outgrew a buffer
 // included in acc).
@@ -1458,8 +1478,10 @@ static int run_wave(gls_ctx *ctx, size_t w0, uint32_t nwin, const gls_batch_opts
 {
     WinDev *hw = ctx->hwave.as<WinDev>();
     uint32_t max_stim = 0;
+    const bool w64 = nwin == 1 && ctx->windows[w0]->w64;
+    const std::vector<GateThreads> threads = gate_blocks(ctx, nwin, w64, wave_events(ctx, w0, nwin));
     for (uint32_t k = 0; k < nwin; ++k)
-        CK(ctx->lsc[k]->ensure(ctx->max_width, ctx->seg_cap, ctx->scr_cap), "alloc level work spaces");
+        CK(ctx->lsc[k]->ensure(ctx->max_width, ctx->seg_cap, ctx->scr_cap, threads.empty()), "alloc level work spaces");
     for (uint32_t k = 0; k < nwin; ++k) {
         Window *w = ctx->windows[w0 + k];
         int rc = w->uploaded ? GLS_OK : upload_window(ctx, w);
@@ -1476,8 +1498,6 @@ static int run_wave(gls_ctx *ctx, size_t w0, uint32_t nwin, const gls_batch_opts
     const WinDev *dw[2] = {ctx->dwave.as<WinDev>(), ctx->dwave.as<WinDev>() + kMaxWave};
     const WinDev *hp[2] = {&hw[0], &hw[kMaxWave]};
     launch_reset(dw[0], hw[0], nwin, max_stim, ctx->n_nets, (uint32_t)ctx->drv_level_start.size(), ctx->stream);
-    const bool w64 = nwin == 1 && ctx->windows[w0]->w64;
-    const std::vector<GateThreads> threads = gate_blocks(ctx, nwin, w64, wave_events(ctx, w0, nwin));
     CK(cudaEventRecord(e0, ctx->stream), "event");
     if (o.use_graph && nwin > 1) {
         // one graph per wave shape; the descriptors it reads are rewritten per wave

@@ -140,34 +140,41 @@ struct PinBuf {   // page-locked host staging, reused across windows
     template <typename T> T *as() const { return static_cast<T *>(p); }
 };
 
-// One window's per-level work space: segment tables, slot offsets and the
-// segment stacks.  Sequential runs share set 0; a wave of windows run
+// One window's per-level work space: the segment stacks, the presize's
+// predictions, and, for runs through the segment kernels, slot offsets and
+// segment tables.  Sequential runs share set 0; a wave of windows run
 // together takes one set per window.
 struct LevelScratch {
-    DevBuf seg_base, slot, scr, res, pred, segs, copies, scratch;
+    DevBuf pred, scratch;
+    DevBuf seg_base, slot, scr, res, segs, copies;
     // the per-gate-output tables of odd levels: the next level's plan fills
     // one set while the previous level's copy still reads the other
     DevBuf seg_base1, slot1, scr1, res1;
     uint32_t seg_cap = 0;
     uint64_t scr_cap = 0;
-    uint32_t width = 0;
-    cudaError_t ensure(uint32_t w, uint32_t segs_need, uint64_t words_need)
+    uint32_t width = 0, table_width = 0;
+    // tables: a run through the segment kernels (48 bytes a gate output and 56
+    // a segment of at least 2^21: 117 MB that k_gate does not read)
+    cudaError_t ensure(uint32_t w, uint32_t segs_need, uint64_t words_need, bool tables)
     {
         cudaError_t e = cudaSuccess;
+        const size_t n = (size_t)w + 1;
         if (w > width) {
-            const size_t n = (size_t)w + 1;
+            e = pred.ensure(n * 4);
+            if (e == cudaSuccess) width = w;
+        }
+        if (tables && w > table_width) {
             if (e == cudaSuccess) e = seg_base.ensure(n * 4);
             if (e == cudaSuccess) e = slot.ensure(n * 8);
             if (e == cudaSuccess) e = scr.ensure(n * 8);
             if (e == cudaSuccess) e = res.ensure(n * 4);
-            if (e == cudaSuccess) e = pred.ensure(n * 4);
             if (e == cudaSuccess) e = seg_base1.ensure(n * 4);
             if (e == cudaSuccess) e = slot1.ensure(n * 8);
             if (e == cudaSuccess) e = scr1.ensure(n * 8);
             if (e == cudaSuccess) e = res1.ensure(n * 4);
-            if (e == cudaSuccess) width = w;
+            if (e == cudaSuccess) table_width = w;
         }
-        if (e == cudaSuccess && segs_need > seg_cap) {
+        if (e == cudaSuccess && tables && segs_need > seg_cap) {
             e = segs.ensure((size_t)segs_need * sizeof(gls::SegRec));
             if (e == cudaSuccess) e = copies.ensure((size_t)segs_need * sizeof(gls::CopyRec));
             if (e == cudaSuccess) seg_cap = segs_need;
@@ -185,7 +192,7 @@ struct LevelScratch {
         for (DevBuf *b : all) b->release();
         seg_cap = 0;
         scr_cap = 0;
-        width = 0;
+        width = table_width = 0;
     }
 };
 

@@ -200,3 +200,28 @@ def test_autotune_times_equal_schedules_once(late, design, gpu):
         tuned = s.saif(w).copy()
         s.run()
         assert np.array_equal(tuned, s.saif(w))
+
+
+def test_segment_tables_come_with_the_segment_kernels(design, gpu):
+    """Waves through the gate kernel alone hold no segment tables (117 MB a
+    window at least); a schedule that asks for the segment kernels brings them,
+    and going from one to the other changes no result."""
+    torch = pytest.importorskip("torch")
+    cfg, nl = design
+    sts = [synth.make_stimulus(cfg, nl.ppi_nets, seed=110 + k) for k in range(12)]
+    with Simulator() as s:
+        s.load(nl)
+        ids = [s.add_window(st, 0, cfg.t_end) for st in sts]
+        before = torch.cuda.mem_get_info()[0]
+        saif = []
+        for mask, batched in ((0, True), (7, True), (0, False), (2, False), (0, True)):
+            s.set_schedule(2048, mask, 0)
+            if batched:
+                s.run_batched()
+            else:
+                s.run()
+            if not saif:
+                assert before - torch.cuda.mem_get_info()[0] < 12 * 64 << 20
+            saif.append([s.saif(w).copy() for w in ids])
+        for other in saif[1:]:
+            assert all(np.array_equal(a, b) for a, b in zip(saif[0], other))
