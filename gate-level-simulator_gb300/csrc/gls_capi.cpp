@@ -496,8 +496,8 @@ extern "C" int gls_load_netlist(gls_ctx *ctx, const gls_netlist *nl)
     ctx->driven.assign(nl->n_nets, 0);
     ctx->ext_inputs.clear();
     for (uint32_t n = 0; n < nl->n_nets; ++n) {
-        ctx->driven[n] = drv_level_of_net[n] >= 0;
-        if (consumed[n] && !ctx->driven[n]) ctx->ext_inputs.push_back(n);
+        ctx->driven[n] = drv_level_of_net[n] >= 0 ? gls_ctx::kDriven : (consumed[n] ? gls_ctx::kReadOnly : 0);
+        if (ctx->driven[n] == gls_ctx::kReadOnly) ctx->ext_inputs.push_back(n);
     }
     if (h_arcs.empty()) h_arcs.push_back(ArcDev{0, 0, 0, 0});
     if (h_ndel.empty()) h_ndel.push_back(NetDelay{{kInf, kInf, kInf, kInf, kInf, kInf, kInf, kInf}});
@@ -673,21 +673,20 @@ extern "C" int gls_add_window(gls_ctx *ctx, const gls_stimulus *st, uint64_t t_b
     w->t_end = t_end;
     std::vector<uint8_t> seen(ctx->n_nets, 0);
     std::vector<uint64_t> at(st->n_nets + 1, 0);
+    uint64_t longest = 0;
     for (uint32_t k = 0; k < st->n_nets; ++k) {
         const uint32_t net = st->net[k];
         if (net >= ctx->n_nets) { ctx->spare.push_back(w); return fail(ctx, GLS_EINVAL, "stimulus net %u out of range", net); }
         if (seen[net]) { ctx->spare.push_back(w); return fail(ctx, GLS_EINVAL, "stimulus net %u given twice", net); }
-        if (ctx->driven[net]) { ctx->spare.push_back(w); return fail(ctx, GLS_EINVAL, "stimulus net %u is driven by a gate", net); }
+        if (ctx->driven[net] == gls_ctx::kDriven) { ctx->spare.push_back(w); return fail(ctx, GLS_EINVAL, "stimulus net %u is driven by a gate", net); }
         seen[net] = 1;
         if (st->ev_start[k + 1] < st->ev_start[k]) { ctx->spare.push_back(w); return fail(ctx, GLS_EINVAL, "stimulus ev_start not monotone"); }
-        at[k + 1] = at[k] + round4(st->ev_start[k + 1] - st->ev_start[k]);
+        const uint64_t words = round4(st->ev_start[k + 1] - st->ev_start[k]);
+        at[k + 1] = at[k] + words;
+        if (ctx->driven[net] == gls_ctx::kReadOnly) longest = std::max(longest, words);
     }
-    uint64_t longest = 0;
-    for (uint32_t net : ctx->ext_inputs) seen[net] |= 2;
-    for (uint32_t k = 0; k < st->n_nets; ++k)
-        if (seen[st->net[k]] & 2) longest = std::max(longest, at[k + 1] - at[k]);
     for (uint32_t net : ctx->ext_inputs)
-        if (!(seen[net] & 1)) { ctx->spare.push_back(w); return fail(ctx, GLS_EINVAL, "net %u is read by a gate but has no stimulus", net); }
+        if (!seen[net]) { ctx->spare.push_back(w); return fail(ctx, GLS_EINVAL, "net %u is read by a gate but has no stimulus", net); }
     const uint64_t total = at[st->n_nets];
     // validate and pack (time << 2 | value), each net on a 4-event boundary;
     // large stimuli are packed by several host threads.  32-bit words hold

@@ -255,7 +255,8 @@ struct gls_ctx {
     std::vector<uint32_t> cls_start;         // per level kClasses+1 entries: fan-in class ranges, level-relative
     uint32_t max_width = 0;
     uint64_t pins_total = 0;
-    std::vector<uint8_t> driven;             // net driven by a gate output
+    static constexpr uint8_t kDriven = 1, kReadOnly = 2;
+    std::vector<uint8_t> driven;             // per net: driven by a gate output, read by gates alone, or neither
     std::vector<uint32_t> ext_inputs;        // nets read by gates and driven by no gate
     DevBuf meta, arcs, ndel, lut, slut, fast;
     std::vector<LevelScratch *> lsc;         // level work spaces ([0]: sequential runs)
