@@ -139,14 +139,12 @@ static_assert(sense_of(kV0, kVX) == 1 && sense_of(kVX, kV0) == 2 && sense_of(kVX
 constexpr uint32_t kMaxDelay = kMaxTimeWide;
 constexpr uint32_t kNegTab = neg_table();
 
-template <class Wd>
-struct SegRecT {            // one time segment of one gate output
+struct SegRec {             // one time segment of one gate output
     uint32_t region;        // offset of the segment's stack inside the gate's scratch
     uint32_t cnt;           // entries on the segment's local stack
     uint32_t min_o;         // smallest candidate output time in the segment
-    Wd last;                // the stack's top entry (when cnt > 0): linking reads no scratch for it
+    uint32_t last;          // the stack's top entry (when cnt > 0): linking reads no scratch for it
 };
-using SegRec = SegRecT<uint32_t>;
 
 struct CopyRec {            // what k_copy does for one segment
     uint64_t src;           // scratch index of the first kept entry

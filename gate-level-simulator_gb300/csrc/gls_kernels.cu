@@ -360,7 +360,7 @@ __device__ __forceinline__ uint32_t sel4(const uint4 &q, uint32_t k)
 // the variant.
 constexpr uint32_t kSimBlock = 128;
 constexpr int kSimV256 = 1, kSimVWide = 2;
-template <int kV, int M> __host__ __device__ constexpr uint32_t sim_block()
+template <int kV> __host__ __device__ constexpr uint32_t sim_block()
 {
     return (kV & kSimV256) ? 256u : kSimBlock;
 }
@@ -456,7 +456,7 @@ struct Reader<1> {
     }
 };
 
-template <int M, class Wd, bool kWideChunk>
+template <int M, bool kWideChunk>
 __device__ void sim_segment(const WinDev &w, const LevelArgs &a, const DrvMeta &md, uint32_t s,
                             uint32_t S, uint32_t seg_id, uint64_t scr, const uint4 sl)
 {
@@ -465,7 +465,7 @@ __device__ void sim_segment(const WinDev &w, const LevelArgs &a, const DrvMeta &
     using RD = Reader<kRW>;
     using RC = typename RD::C;
     const RC *P = reinterpret_cast<const RC *>(w.pool);
-    const Wd *pw = reinterpret_cast<const Wd *>(w.pool);
+    const uint32_t *pw = w.pool;
     uint64_t off[M];
     uint32_t len[M];
     int piv = 0, sec = -1;   // the longest input list and the longest of the others
@@ -496,7 +496,7 @@ __device__ void sim_segment(const WinDev &w, const LevelArgs &a, const DrvMeta &
     uint32_t region = s, capn = 1;
     bool before = false;
     RD rd[M];
-    Wd hk[M];         // head word of every list with the value bits set: equal times compare equal
+    uint32_t hk[M];         // head word of every list with the value bits set: equal times compare equal
 #pragma unroll
     for (int j = 0; j < M; ++j) {
         uint32_t b = 0, e = 0;
@@ -515,18 +515,18 @@ __device__ void sim_segment(const WinDev &w, const LevelArgs &a, const DrvMeta &
     const uint8_t *lut = a.lut + md.lut_off;
     const NetDelay *nd = a.ndel + md.dt_off;
     const bool regular = md.flags & kFlagRegular;
-    Wd *ot = reinterpret_cast<Wd *>(w.scratch) + scr + region;
+    uint32_t *ot = w.scratch + scr + region;
     uint32_t cnt = 0;                 // stack size
-    Wd top = 0;                       // its top word
+    uint32_t top = 0;                       // its top word
     int popped_v = -1;
-    if (s == 0) { top = EvW<Wd>::word(0, kVX); ot[0] = top; cnt = 1; }
+    if (s == 0) { top = EvW<uint32_t>::word(0, kVX); ot[0] = top; cnt = 1; }
     uint32_t fprev = before ? (kSlut ? slut_get<M>(sl, curp) : lut[lut_index(curp, md)]) : kVX;
     uint32_t min_o = kInf;
     for (;;) {
-        Wd mk = hk[0] | 3u;
+        uint32_t mk = hk[0] | 3u;
 #pragma unroll
-        for (int j = 1; j < M; ++j) mk = min(mk, (Wd)(hk[j] | 3u));
-        if (mk == EvW<Wd>::kInfW) break;
+        for (int j = 1; j < M; ++j) mk = min(mk, hk[j] | 3u);
+        if (mk == EvW<uint32_t>::kInfW) break;
         const uint32_t lastp = curp;
         uint32_t chg = 0;
 #pragma unroll
@@ -546,7 +546,7 @@ __device__ void sim_segment(const WinDev &w, const LevelArgs &a, const DrvMeta &
                                    : select_delay(a.arcs + md.arc_off, md.n_arcs, chg, (int)so1 + 1, curp, lastp,
                                                   a.def_delay);
         const uint64_t o64 = (uint64_t)t + d;   // 64 bits: delays reach 2^32 - 2
-        if (o64 > EvW<Wd>::kMax) { atomicOr(w.err, kErrTime); break; }
+        if (o64 > EvW<uint32_t>::kMax) { atomicOr(w.err, kErrTime); break; }
         const uint32_t o = (uint32_t)o64;
         min_o = min(min_o, o);
         // inertial update, src/simulate.cpp:991-1009
@@ -558,16 +558,16 @@ __device__ void sim_segment(const WinDev &w, const LevelArgs &a, const DrvMeta &
         const int prevv = cnt > 0 ? (int)ev_val(top) : (s == 0 ? popped_v : -1);
         if (prevv != (int)F) {
             if (cnt >= capn) { atomicOr(w.err, kErrRegion); break; }
-            top = EvW<Wd>::word(o, F);
+            top = EvW<uint32_t>::word(o, F);
             ot[cnt++] = top;
         } else if (cnt == 0) {
             atomicOr(w.err, kErrEmptied);
             break;
         }
     }
-    SegRecT<Wd> r;
+    SegRec r;
     r.region = region; r.cnt = cnt; r.min_o = min_o; r.last = top;
-    reinterpret_cast<SegRecT<Wd> *>(w.segs)[seg_id] = r;
+    w.segs[seg_id] = r;
 }
 
 // One time segment of a gate output with at most three input nets, 32-bit
@@ -678,7 +678,7 @@ __device__ __forceinline__ uint32_t window_of(const uint32_t *s_pre, uint32_t nw
 // owns a contiguous share of the class's segments and its threads take the
 // next one from a shared counter as they finish, so long and short segments
 // balance inside the block.
-template <int M, bool kBatch, class Wd, int kV>
+template <int M, bool kBatch, int kV>
 #ifndef GLS_SIM2_BLOCKS
 #define GLS_SIM2_BLOCKS 8   // resident blocks per SM the 1- and 2-input gate kernels are compiled for
 #endif
@@ -688,11 +688,11 @@ template <int M, bool kBatch, class Wd, int kV>
 #ifndef GLS_SIM1_BLOCKS
 #define GLS_SIM1_BLOCKS GLS_SIM2_BLOCKS   // resident blocks per SM the 1-input gate kernel is compiled for
 #endif
-__global__ void __launch_bounds__(sim_block<kV, M>(), (M == 1 ? GLS_SIM1_BLOCKS : (M == 2 ? GLS_SIM2_BLOCKS : (M == 3 ? GLS_SIM3_BLOCKS : 4))) /
-                                                    (sim_block<kV, M>() / kSimBlock))
+__global__ void __launch_bounds__(sim_block<kV>(), (M == 1 ? GLS_SIM1_BLOCKS : (M == 2 ? GLS_SIM2_BLOCKS : (M == 3 ? GLS_SIM3_BLOCKS : 4))) /
+                                                    (sim_block<kV>() / kSimBlock))
     k_sim(const WinSet<kBatch> ws, LevelArgs a, uint32_t d0, uint32_t d1)
 {
-    constexpr bool kFast = M <= 3 && std::is_same<Wd, uint32_t>::value && !(kV & kSimVWide);
+    constexpr bool kFast = M <= 3 && !(kV & kSimVWide);
     __shared__ uint32_t s_next;
     __shared__ uint32_t s_pre[kBatch ? kMaxWave + 1 : 2];
     __shared__ uint32_t sm32[32];
@@ -766,7 +766,7 @@ __global__ void __launch_bounds__(sim_block<kV, M>(), (M == 1 ? GLS_SIM1_BLOCKS 
         } else {
             const DrvMeta md = a.meta[a.lo + i];
             const uint4 sl = M <= 3 ? __ldg(a.slut + a.lo + i) : make_uint4(0, 0, 0, 0);
-            sim_segment<M, Wd, (kV & kSimVWide) != 0>(w, a, md, g - sb, S, g, w.scr[i], sl);
+            sim_segment<M, (kV & kSimVWide) != 0>(w, a, md, g - sb, S, g, w.scr[i], sl);
         }
     }
 }
@@ -1271,7 +1271,7 @@ __device__ __forceinline__ void saif_add(unsigned long long acc[3], int cls, uns
 // pass B drops a segment's first entry when it repeats the last kept value
 // before it, places the segments back to back in the gate's pool slot and
 // hands each segment's copy to k_copy with the final event that precedes it.
-template <bool kBatch, class Wd>
+template <bool kBatch>
 #ifndef GLS_LINK_BLOCKS
 #define GLS_LINK_BLOCKS 1   // resident blocks per SM the link kernel is compiled for (1: no bound)
 #endif
@@ -1289,15 +1289,15 @@ __global__ void __launch_bounds__(256, GLS_LINK_BLOCKS) k_link(const WinSet<kBat
     const uint32_t sb = w.seg_base[i], se = w.seg_base[i + 1];
     const uint64_t slot = w.slot[i];
     const uint64_t scr = w.scr[i];
-    const Wd *sx = reinterpret_cast<const Wd *>(w.scratch) + scr;
-    const SegRecT<Wd> *segs = reinterpret_cast<const SegRecT<Wd> *>(w.segs);
+    const uint32_t *sx = w.scratch + scr;
+    const SegRec *segs = w.segs;
     const uint32_t out_net = a.meta[a.lo + i].out_net;
     // pass A (right to left)
     uint32_t carry_min = kInf;
     for (int64_t base = se; base > (int64_t)sb; base -= 32) {
         const int64_t s = base - 32 + lane;
         const bool valid = s >= (int64_t)sb;
-        SegRecT<Wd> r = {0, 0, kInf, 0};
+        SegRec r = {0, 0, kInf, 0};
         if (valid) r = segs[s];
         uint32_t x = r.min_o;
 #pragma unroll
@@ -1328,12 +1328,12 @@ __global__ void __launch_bounds__(256, GLS_LINK_BLOCKS) k_link(const WinSet<kBat
         const bool valid = s < se;
         uint32_t keep = 0, region = 0, firstv = 0, lastv = 0, lastt = 0;
         if (valid) {
-            const SegRecT<Wd> r = segs[s];
+            const SegRec r = segs[s];
             keep = w.copies[s].n;
             region = r.region;
             if (keep) {
                 firstv = ev_val(sx[region]);
-                const Wd lw = keep == r.cnt ? r.last : sx[region + keep - 1];
+                const uint32_t lw = keep == r.cnt ? r.last : sx[region + keep - 1];
                 lastv = ev_val(lw);
                 lastt = ev_time(lw);
             }
@@ -1442,7 +1442,7 @@ constexpr int kCopyUnroll = GLS_COPY_UNROLL;   // entries per lane loaded ahead 
 // level scratch into the pool and add their SAIF contributions to the gate
 // output's counters.  The next segment's record is loaded while the current
 // one is copied.
-template <bool kBatch, int W, class Wd>
+template <bool kBatch, int W>
 #ifndef GLS_COPY_BLOCKS
 #define GLS_COPY_BLOCKS 5   // resident blocks per SM the copy kernel is compiled for (48 registers)
 #endif
@@ -1499,13 +1499,12 @@ __global__ void __launch_bounds__(256, GLS_COPY_BLOCKS) k_copy(const WinSet<kBat
         const CopyRec nx = fetch(s + stride, nw);
         const WinDev &w = ws.get(cw);
         const bool live = s < nseg && c.n > 0;
-        using P = SaifP<Wd>;
-        const RelClampT<P> rc(w.t_begin, w.t_end);
-        P acc[3] = {0, 0, 0};
+        const RelClampT<uint32_t> rc(w.t_begin, w.t_end);
+        uint32_t acc[3] = {0, 0, 0};
         // c.cprev is a clamped absolute time: at most the largest event time
         // unless the window starts past every event (then it is t_begin,
         // relative 0)
-        P prev = (rc((uint32_t)min(c.cprev, (unsigned long long)EvW<Wd>::kMax)) << 2) | c.pclass;
+        uint32_t prev = (rc((uint32_t)min(c.cprev, (unsigned long long)EvW<uint32_t>::kMax)) << 2) | c.pclass;
         const uint32_t n = live ? c.n : 0;
         // groups of one warp may have different lengths: loop to the warp's longest
         uint32_t nmax = n;
@@ -1515,14 +1514,14 @@ __global__ void __launch_bounds__(256, GLS_COPY_BLOCKS) k_copy(const WinSet<kBat
         // kCopyUnroll loads per lane go out before the stores that follow
         // them: scratch and pool never overlap, and a segment's copy costs
         // one memory round trip per W * kCopyUnroll entries, not per W
-        const Wd *__restrict__ sp = reinterpret_cast<const Wd *>(w.scratch) + c.src;
-        Wd *__restrict__ dp = reinterpret_cast<Wd *>(w.pool) + dst;
+        const uint32_t *__restrict__ sp = w.scratch + c.src;
+        uint32_t *__restrict__ dp = w.pool + dst;
         for (uint32_t i0 = 0; i0 < nmax; i0 += W * kCopyUnroll) {
-            Wd wd[kCopyUnroll];
+            uint32_t wd[kCopyUnroll];
 #pragma unroll
             for (int u = 0; u < kCopyUnroll; ++u) {
                 const uint32_t i = i0 + u * W + sub;
-                wd[u] = i < n ? __ldcs(sp + i) : Wd(0);   // read once: stream it past L1
+                wd[u] = i < n ? __ldcs(sp + i) : 0u;   // read once: stream it past L1
             }
 #pragma unroll
             for (int u = 0; u < kCopyUnroll; ++u) {
@@ -1531,7 +1530,7 @@ __global__ void __launch_bounds__(256, GLS_COPY_BLOCKS) k_copy(const WinSet<kBat
                 const uint32_t i = ib + sub;
                 const bool v = i < n;
                 if (v) dp[i] = wd[u];
-                integrate_group<W, Wd, P>(rc, wd[u], v, ib < n ? n - ib : 1u, ib < n, prev, acc);
+                integrate_group<W>(rc, wd[u], v, ib < n ? n - ib : 1u, ib < n, prev, acc);
             }
         }
 #pragma unroll
@@ -1703,15 +1702,15 @@ void launch_plan(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelAr
 }
 
 // one block per resident slot of every SM
-template <class Wd, int kV, class WS>
+template <int kV, class WS>
 static void sim_thread(const WS &ws, const LevelArgs &a, int cls, uint32_t d0, uint32_t d1, int sm_count,
                        cudaStream_t st)
 {
     constexpr bool B = std::is_same<WS, WinSet<true>>::value;
     auto go = [&](auto mt, int per_sm) {   // per_sm: resident 128-thread blocks
         constexpr int M = decltype(mt)::value;
-        constexpr uint32_t bs = sim_block<kV, M>();
-        k_sim<M, B, Wd, kV><<<sm_count * per_sm / (bs / kSimBlock), bs, 0, st>>>(ws, a, d0, d1);
+        constexpr uint32_t bs = sim_block<kV>();
+        k_sim<M, B, kV><<<sm_count * per_sm / (bs / kSimBlock), bs, 0, st>>>(ws, a, d0, d1);
     };
     switch (cls) {
     case 0: go(std::integral_constant<int, 1>(), GLS_SIM1_BLOCKS); break;
@@ -1721,12 +1720,12 @@ static void sim_thread(const WS &ws, const LevelArgs &a, int cls, uint32_t d0, u
     }
 }
 
-template <class Wd, class WS>
+template <class WS>
 static void sim_kernels(const WS &ws, const LevelArgs &a, int cls, uint32_t d0, uint32_t d1, int sm_count,
                         cudaStream_t st)
 {
     constexpr bool B = std::is_same<WS, WinSet<true>>::value;
-    if (std::is_same<Wd, uint32_t>::value && ((a.warp_mask >> cls) & 1u)) {
+    if ((a.warp_mask >> cls) & 1u) {
         const int wgrid = sm_count * 8;
         switch (cls) {
         case 0: k_sim_warp<1, B><<<wgrid, 128, 0, st>>>(ws, a, d0, d1); return;
@@ -1735,21 +1734,18 @@ static void sim_kernels(const WS &ws, const LevelArgs &a, int cls, uint32_t d0, 
         default: break;
         }
     }
-    if constexpr (std::is_same<Wd, uint32_t>::value) {
-        switch (a.sim_variant) {
-        case 1: sim_thread<Wd, 1>(ws, a, cls, d0, d1, sm_count, st); return;
-        case 2: sim_thread<Wd, 2>(ws, a, cls, d0, d1, sm_count, st); return;
-        case 3: sim_thread<Wd, 3>(ws, a, cls, d0, d1, sm_count, st); return;
-        default: break;
-        }
+    switch (a.sim_variant) {
+    case 1: sim_thread<1>(ws, a, cls, d0, d1, sm_count, st); return;
+    case 2: sim_thread<2>(ws, a, cls, d0, d1, sm_count, st); return;
+    case 3: sim_thread<3>(ws, a, cls, d0, d1, sm_count, st); return;
+    default: sim_thread<0>(ws, a, cls, d0, d1, sm_count, st); return;
     }
-    sim_thread<Wd, 0>(ws, a, cls, d0, d1, sm_count, st);
 }
 
 void launch_sim(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelArgs &a, int cls, uint32_t d0, uint32_t d1,
                 int sm_count, cudaStream_t st)
 {
-    GLS_DISPATCH(h, dw, nwin, sim_kernels<uint32_t>(ws, a, cls, d0, d1, sm_count, st));
+    GLS_DISPATCH(h, dw, nwin, sim_kernels(ws, a, cls, d0, d1, sm_count, st));
 }
 
 void launch_link(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelArgs &a, uint32_t d0, uint32_t d1,
@@ -1758,17 +1754,17 @@ void launch_link(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelAr
     const uint64_t warps = (uint64_t)(d1 - d0) * nwin;
     if (!warps) return;
     const uint32_t blocks = (uint32_t)((warps * 32 + 255) / 256);
-    GLS_DISPATCH(h, dw, nwin, (k_link<decltype(ws)::kIsBatch, uint32_t><<<blocks, 256, 0, st>>>(ws, a, d0, d1)));
+    GLS_DISPATCH(h, dw, nwin, (k_link<decltype(ws)::kIsBatch><<<blocks, 256, 0, st>>>(ws, a, d0, d1)));
 }
 
 void launch_copy(const WinDev *dw, const WinDev &h, uint32_t nwin, const LevelArgs &a, uint32_t d0, uint32_t d1,
                  int sm_count, cudaStream_t st)
 {
     const int grid = sm_count * 8;
-    if (a.copy_lanes == 4) GLS_DISPATCH(h, dw, nwin, (k_copy<decltype(ws)::kIsBatch, 4, uint32_t><<<grid, 256, 0, st>>>(ws, a, d0, d1)));
-    else if (a.copy_lanes == 8) GLS_DISPATCH(h, dw, nwin, (k_copy<decltype(ws)::kIsBatch, 8, uint32_t><<<grid, 256, 0, st>>>(ws, a, d0, d1)));
-    else if (a.copy_lanes == 32) GLS_DISPATCH(h, dw, nwin, (k_copy<decltype(ws)::kIsBatch, 32, uint32_t><<<grid, 256, 0, st>>>(ws, a, d0, d1)));
-    else GLS_DISPATCH(h, dw, nwin, (k_copy<decltype(ws)::kIsBatch, 16, uint32_t><<<grid, 256, 0, st>>>(ws, a, d0, d1)));
+    if (a.copy_lanes == 4) GLS_DISPATCH(h, dw, nwin, (k_copy<decltype(ws)::kIsBatch, 4><<<grid, 256, 0, st>>>(ws, a, d0, d1)));
+    else if (a.copy_lanes == 8) GLS_DISPATCH(h, dw, nwin, (k_copy<decltype(ws)::kIsBatch, 8><<<grid, 256, 0, st>>>(ws, a, d0, d1)));
+    else if (a.copy_lanes == 32) GLS_DISPATCH(h, dw, nwin, (k_copy<decltype(ws)::kIsBatch, 32><<<grid, 256, 0, st>>>(ws, a, d0, d1)));
+    else GLS_DISPATCH(h, dw, nwin, (k_copy<decltype(ws)::kIsBatch, 16><<<grid, 256, 0, st>>>(ws, a, d0, d1)));
 }
 
 }  // namespace gls
