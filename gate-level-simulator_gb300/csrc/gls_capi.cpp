@@ -689,11 +689,9 @@ extern "C" int gls_add_window(gls_ctx *ctx, const gls_stimulus *st, uint64_t t_b
         if (!seen[net]) { ctx->spare.push_back(w); return fail(ctx, GLS_EINVAL, "net %u is read by a gate but has no stimulus", net); }
     const uint64_t total = at[st->n_nets];
     // validate and pack (time << 2 | value), each net on a 4-event boundary;
-    // large stimuli are packed by several host threads.  32-bit words hold
-    // times up to 2^30 - 2; a later time repacks the stimulus in 64-bit words.
+    // large stimuli are packed by several host threads
     std::atomic<int> bad(0);
     std::atomic<uint32_t> bad_net(0);
-    std::atomic<bool> long_times(false);
     // The loops carry no early exit so that the compiler vectorizes them; a
     // net's faults are reported in the order value, time range, time order.
     auto pack = [&](auto *hw, uint32_t k0, uint32_t k1) {
@@ -703,23 +701,20 @@ extern "C" int gls_add_window(gls_ctx *ctx, const gls_stimulus *st, uint64_t t_b
             const uint32_t *tt = st->time + a;
             const uint8_t *vv = st->value + a;
             Wd *o = hw + at[k];
-            uint32_t ev = 0, et = 0, ew = 0, eo = 0;
+            uint32_t ev = 0, et = 0, eo = 0;
             if (cnt) {   // one pass over the times: the order check reads the word before from cache
                 ev |= vv[0] > 3 ? 1u : 0u;
-                ew |= tt[0] > kMaxTime ? 1u : 0u;
                 et |= tt[0] > kMaxTimeWide ? 1u : 0u;
                 o[0] = ((Wd)tt[0] << 2) | (Wd)(vv[0] & 3u);
             }
             for (uint64_t e = 1; e < cnt; ++e) {
                 const uint32_t t = tt[e], v = vv[e];
                 ev |= v > 3 ? 1u : 0u;
-                ew |= t > kMaxTime ? 1u : 0u;
                 et |= t > kMaxTimeWide ? 1u : 0u;
                 eo |= t <= tt[e - 1] ? 1u : 0u;
                 o[e] = ((Wd)t << 2) | (Wd)(v & 3u);
             }
             for (uint64_t e = cnt; e < round4(cnt); ++e) o[e] = EvW<Wd>::kInfW;
-            if (ew) long_times = true;
             if (ev | et | eo) {
                 bad = ev ? 1 : (et ? 2 : 3);
                 bad_net = st->net[k];
@@ -727,8 +722,9 @@ extern "C" int gls_add_window(gls_ctx *ctx, const gls_stimulus *st, uint64_t t_b
             }
         }
     };
-    // times increase within a net, so its last one tells which words it needs
-    // (a net out of order is found by the pack)
+    // 32-bit words hold times up to 2^30 - 2.  Times increase within a net, so
+    // its last one tells which words it needs (a net out of order is refused by
+    // the pack, in words of either size)
     for (uint32_t k = 0; k < st->n_nets; ++k)
         if (st->ev_start[k + 1] > st->ev_start[k] && st->time[st->ev_start[k + 1] - 1] > kMaxTime) w->w64 = true;
     // several threads from about 2^17 events on: 110 us for any count up to
@@ -760,16 +756,12 @@ extern "C" int gls_add_window(gls_ctx *ctx, const gls_stimulus *st, uint64_t t_b
             pack(hw, 0, st->n_nets);
         }
     };
-    for (;;) {
-        if (!w->h_words.ensure(total * w->word_bytes())) {
-            ctx->spare.push_back(w);
-            return fail(ctx, GLS_ENOMEM, "pinned staging of %llu events", (unsigned long long)total);
-        }
-        if (w->w64) pack_all(w->h_words.as<WideWord>());
-        else pack_all(w->h_words.as<uint32_t>());
-        if (bad || w->w64 || !long_times) break;
-        w->w64 = true;   // a late time before a net's last one: the faults as 64-bit words have them
+    if (!w->h_words.ensure(total * w->word_bytes())) {
+        ctx->spare.push_back(w);
+        return fail(ctx, GLS_ENOMEM, "pinned staging of %llu events", (unsigned long long)total);
     }
+    if (w->w64) pack_all(w->h_words.as<WideWord>());
+    else pack_all(w->h_words.as<uint32_t>());
     if (bad) {
         ctx->spare.push_back(w);
         const int b = bad;

@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from gls import synth
-from gls.capi import Simulator
+from gls.capi import GlsError, Simulator
 from gls.netlist import Stimulus
 
 pytestmark = pytest.mark.gpu
@@ -44,3 +44,24 @@ def test_threads_are_made_when_they_pay(gpu):
         if len(sizes) > 5 and (os.cpu_count() or 1) > 1:
             assert sum(made[:5]) == 0 and max(made) > 0   # 1.0 M events alone, then the threads
     assert np.array_equal(results[0], results[1])
+
+
+@pytest.mark.parametrize("times,code,match", [
+    ([0, 2**31, 500], 1, "strictly increasing"),          # a late time before the last one
+    ([0, 700, 500, 2**31], 1, "strictly increasing"),     # out of order, the last one late
+    ([0, 700, 700], 1, "strictly increasing"),
+    ([0, 700, 2**32 - 1], None, "beyond the largest"),
+    ([0, 2**32 - 1, 5], None, "beyond the largest"),
+])
+def test_faulty_times_are_refused_in_words_of_either_size(times, code, match, gpu):
+    nl = synth.make_netlist(synth.scaled(synth.CONFIGS["c1"], cells=50, cycles=10, depth=2, ppi=8), seed=1)
+    nets = np.asarray(nl.ppi_nets, np.uint32)
+    lists = [times] + [[0, 100, 200]] * (len(nets) - 1)
+    start = np.cumsum([0] + [len(x) for x in lists]).astype(np.uint64)
+    t = np.concatenate([np.array(x, np.uint64) for x in lists]).astype(np.uint32)
+    v = np.concatenate([np.where(np.arange(len(x)) % 2, 3, 0) for x in lists]).astype(np.uint8)
+    with Simulator() as s:
+        s.load(nl)
+        with pytest.raises(GlsError, match=match) as e:
+            s.add_window(Stimulus(nets, start, t, v), 0, 2**32)
+        assert code is None or e.value.code == code
