@@ -5,7 +5,8 @@ import numpy as np
 import pytest
 
 from cases import stimulus
-from gls.capi import Simulator
+from gls import synth
+from gls.capi import MLP_PARAMS, Simulator
 from gls.cells import LIBRARY
 from gls.levelize import assemble, default_arcs
 from gpu_util import assert_same, gpu_run, simulator
@@ -140,3 +141,30 @@ def test_wave_in_the_largest_blocks(gpu, oracle_bin):
             lens = s.lengths(w)
             gw = {n: s.waveform(n, w) for n in range(nl.n_nets) if lens[n] != 2**32 - 1}
             assert_same(gw, s.saif(w), ow, osaif, f"window {w}")
+
+
+@pytest.mark.parametrize("threads", [32, 64, 128, 256, 512])
+@pytest.mark.parametrize("alloc", [0, 1, 2])
+def test_every_block_against_the_segment_kernels(alloc, threads, gpu):
+    """Every size and allocation mode with a pool that grows on the way; in the
+    learned one lists outgrow their predicted slots."""
+    cfg = synth.scaled(synth.CONFIGS["c1"], cells=900, cycles=2500, depth=12)
+    nl = synth.make_netlist(cfg, seed=15)
+    st = synth.make_stimulus(cfg, nl.ppi_nets, seed=16)
+    model = np.zeros(MLP_PARAMS, np.float32)
+    model[-1] = 3.0   # some 20 events a list
+    res = []
+    for env in ({"GLS_GATE": "0"}, {"GLS_GATE_THREADS": str(threads)}):
+        with simulator(env=env, alloc_mode=alloc, pool_events=200_000) as s:
+            if alloc == 2:
+                s.set_presize_model(model)
+            s.load(nl)
+            w = s.add_window(st, 300, cfg.t_end - 700)
+            s.run()
+            assert s.stats()["overflow_retries"] > 0
+            if alloc == 2:
+                assert s.stats()["presize_overflows"] > 0
+            res.append((s.saif(w), s.lengths(w), [s.waveform(int(n), w) for n in range(0, nl.n_nets, 29)]))
+    assert np.array_equal(res[0][0], res[1][0]) and np.array_equal(res[0][1], res[1][1])
+    for (t0, v0), (t1, v1) in zip(res[0][2], res[1][2]):
+        assert np.array_equal(t0, t1) and np.array_equal(v0, v1)
