@@ -1799,11 +1799,12 @@ extern "C" int gls_waveform(gls_ctx *ctx, uint32_t window, uint32_t net, uint32_
     cudaSetDevice(ctx->opts.device);
     const uint32_t wb = (uint32_t)w->word_bytes();
     const uint64_t want = (time || value) ? cap : 0;
-    // The length and a short list in one launch that writes page-locked memory
-    // (14 us at 1000 events, 37 us at 2^16; two copies for offset and length
-    // and one for the events 30 and 51 us); one block's stores fall behind a
-    // copy at about 2^18 events (107 us either way).
-    constexpr uint64_t kInline = 1u << 18;
+    // The length and a short list in one launch that writes page-locked memory;
+    // a longer list by a copy, which is as fast from about 2^17 events on and
+    // needs no staging.  A call from Python, launch / launch and copy / copies
+    // of offset, length and events: 1,000 events 18 / - / 50 us; 60,000 58 / - /
+    // 72; 262,000 152, the first time 311 / 143 / 141, the first time 185.
+    constexpr uint64_t kInline = 1u << 16;
     const uint64_t first = want > kInline ? 0 : want;
     if (!ctx->pin_out.ensure(16 + first * wb)) return fail(ctx, GLS_ENOMEM, "pinned staging for a waveform");
     launch_read_list(w->net_off.as<uint64_t>() + net, w->net_len.as<uint32_t>() + net, w->pool.p, w->pool.bytes, wb, first,

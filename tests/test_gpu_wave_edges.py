@@ -1,5 +1,7 @@
 """What waves of windows leave behind: windows whose pool a saif_only call
 gave back without running them."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -8,6 +10,7 @@ from gls import synth
 from gls.capi import GlsError, Simulator
 from gls.cells import LIBRARY
 from gls.levelize import assemble, default_arcs
+from gls.netlist import Stimulus
 
 pytestmark = pytest.mark.gpu
 
@@ -225,3 +228,34 @@ def test_segment_tables_come_with_the_segment_kernels(design, gpu):
             saif.append([s.saif(w).copy() for w in ids])
         for other in saif[1:]:
             assert all(np.array_equal(a, b) for a, b in zip(saif[0], other))
+
+
+@pytest.mark.parametrize("base", [0, 3_000_000_000])
+def test_waveforms_around_the_staged_length(base, gpu):
+    """Lists around 2^16 and 2^18 events, read with their length and by a copy,
+    whole and cut off, in both word sizes."""
+    c = LIBRARY["GEN_BUF_D1"]
+    sizes = [1, 1024, 1025, 65_535, 65_536, 65_537, 262_143, 262_144, 262_145]
+    k = len(sizes)
+    nl = assemble([(c.name, [j], [k + j], default_arcs(c, 3.0, 4.0)) for j in range(k)], n_nets=2 * k)
+    t = np.concatenate([base + 10 * np.arange(n, dtype=np.uint64) for n in sizes]).astype(np.uint32)
+    v = np.concatenate([np.where(np.arange(n) % 2, 3, 0) for n in sizes]).astype(np.uint8)
+    st = Stimulus(np.arange(k, dtype=np.uint32), np.cumsum([0] + sizes).astype(np.uint64), t, v)
+    with Simulator() as s:
+        s.load(nl)
+        w = s.add_window(st, base, base + 2_700_000)
+        s.run()
+        lens = s.lengths(w)
+        for j, n in enumerate(sizes):
+            a, b = int(st.ev_start[j]), int(st.ev_start[j + 1])
+            gt, gv = s.waveform(j, w)
+            assert np.array_equal(gt, t[a:b]) and np.array_equal(gv, v[a:b])
+            ot, ov = s.waveform(k + j, w)
+            assert len(ot) == lens[k + j] == n + 1
+            assert np.array_equal(ot[1:], t[a:b] + np.where(v[a:b] == 3, 3, 4)) and np.array_equal(ov[1:], v[a:b])
+            for cap in (65_535, 65_536, 65_537):   # a caller's shorter arrays
+                ct, cv, got = np.zeros(cap, np.uint32), np.zeros(cap, np.uint8), C.c_uint64()
+                assert s.lib.gls_waveform(s.h, w, j, ct.ctypes.data, cv.ctypes.data, cap, C.byref(got)) == 0
+                m = min(cap, n)
+                assert got.value == n and np.array_equal(ct[:m], t[a:a + m]) and np.array_equal(cv[:m], v[a:a + m])
+                assert not ct[m:].any()
