@@ -428,10 +428,11 @@ void touch_pages(std::initializer_list<std::pair<void *, size_t>> blocks)
     const size_t page = (size_t)std::max(4096l, sysconf(_SC_PAGESIZE));
     const unsigned n = (unsigned)std::min<size_t>(std::min(8u, std::max(1u, std::thread::hardware_concurrency())), total >> 20);
     if (n < 2) return;
-    auto part = [&](unsigned q) {
-        for (const auto &b : blocks)
-            for (size_t i = b.second / n * q / page * page, e = q + 1 == n ? b.second : b.second / n * (q + 1); i < e; i += page)
-                static_cast<volatile char *>(b.first)[i] = 0;
+    auto part = [&](unsigned q) {   // whole pages: no byte is written by two threads
+        for (const auto &b : blocks) {
+            const size_t step = b.second / n / page * page, e = q + 1 == n ? b.second : step * (q + 1);
+            for (size_t i = step * q; i < e; i += page) static_cast<volatile char *>(b.first)[i] = 0;
+        }
     };
     std::vector<std::thread> threads;
     try {
