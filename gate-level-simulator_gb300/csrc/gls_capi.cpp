@@ -299,41 +299,6 @@ extern "C" int gls_destroy(gls_ctx *ctx)
     return GLS_OK;
 }
 
-// A gate output's fast-step record; usable = 0 where the fast step does not
-// apply: more than three input nets, irregular arcs, some input nets with
-// arcs and some without, a delay of 2^16 - 1 or more, or a truth table that
-// gives X or Z for known inputs.
-static FastRec fast_rec(const DrvMeta &md, const uint4 &slut, const std::vector<NetDelay> &ndel, uint32_t def_delay)
-{
-    FastRec r{};
-    if (md.m < 1 || md.m > 3 || !(md.flags & kFlagRegular)) return r;
-    const uint32_t words[4] = {slut.x, slut.y, slut.z, slut.w};
-    for (uint32_t c = 0; c < (1u << md.m); ++c) {
-        uint32_t x = 0, bit = 0;
-        for (int j = 0; j < md.m; ++j)
-            if ((c >> j) & 1u) {
-                x |= 3u << (2 * j);
-                bit |= 1u << (2 * j);
-            }
-        const uint32_t v = (words[x >> 4] >> (2 * (x & 15u))) & 3u;
-        if (v != kV0 && v != kV1) return r;
-        if (v == kV1) r.tt |= 1u << bit;
-    }
-    int with_arcs = 0;
-    for (int j = 0; j < md.m; ++j) with_arcs += ndel[md.dt_off + j].d[0] != kInf;
-    if (with_arcs != 0 && with_arcs != md.m) return r;
-    for (int j = 0; j < md.m; ++j) {
-        for (int e = 0; e < 2; ++e) {
-            const uint32_t *d = &ndel[md.dt_off + j].d[e * 4];
-            const uint32_t rise = with_arcs ? d[0] : def_delay, fall = with_arcs ? d[1] : def_delay;
-            if (rise > kFastDelayMax || fall > kFastDelayMax) return r;
-            r.d[2 * j + e] = rise | fall << 16;
-        }
-    }
-    r.usable = 1;
-    return r;
-}
-
 extern "C" int gls_load_netlist(gls_ctx *ctx, const gls_netlist *nl)
 {
     if (!ctx || !nl) return GLS_EINVAL;
@@ -559,12 +524,6 @@ extern "C" int gls_load_netlist(gls_ctx *ctx, const gls_netlist *nl)
         }
         h_slut[d] = make_uint4(words[0], words[1], words[2], words[3]);
     }
-    // per gate output the record of the gate kernels' fast step
-    std::vector<FastRec> h_fast(h_meta.size(), FastRec{});
-    for (size_t d = 0; d < ctx->n_drv; ++d) h_fast[d] = fast_rec(h_meta[d], h_slut[d], h_ndel, ctx->def_delay);
-    CK(ctx->fast.ensure(h_fast.size() * sizeof(FastRec)), "alloc fast-step records");
-    CK(cudaMemcpy(ctx->fast.p, h_fast.data(), h_fast.size() * sizeof(FastRec), cudaMemcpyHostToDevice),
-       "upload fast-step records");
     CK(ctx->slut.ensure(h_slut.size() * sizeof(uint4)), "alloc slot truth tables");
     CK(cudaMemcpy(ctx->slut.p, h_slut.data(), h_slut.size() * sizeof(uint4), cudaMemcpyHostToDevice),
        "upload slot truth tables");
@@ -580,6 +539,10 @@ extern "C" int gls_load_netlist(gls_ctx *ctx, const gls_netlist *nl)
     CK(cudaMemcpy(ctx->ndel.p, h_ndel.data(), h_ndel.size() * sizeof(NetDelay), cudaMemcpyHostToDevice),
        "upload net delays");
     CK(cudaMemcpy(ctx->lut.p, h_lut.data(), h_lut.size(), cudaMemcpyHostToDevice), "upload lut");
+    CK(ctx->fast.ensure(h_meta.size() * sizeof(FastRec)), "alloc fast-step records");
+    launch_fast_recs(ctx->meta.as<DrvMeta>(), ctx->slut.as<uint4>(), ctx->ndel.as<NetDelay>(), ctx->n_drv, ctx->def_delay,
+                     ctx->fast.as<FastRec>());
+    CK(cudaStreamSynchronize(nullptr), "fast-step records");
     ctx_drop_graphs(ctx);   // they hold the previous netlist's tables
     free_spares(ctx);
     ctx->seg_cap = std::max<uint32_t>(1u << 21, 8 * ctx->max_width + 64);

@@ -224,6 +224,10 @@ constexpr uint32_t kMaxWave = 1024;
 // fan-in class of a gate output by its number of distinct input nets
 __host__ __device__ inline int fanin_class(int m) { return m <= 1 ? 0 : (m == 2 ? 1 : (m == 3 ? 2 : 3)); }
 
+// The fast-step records of n gate outputs, on the default stream, behind the
+// copies of their tables.
+void launch_fast_recs(const DrvMeta *meta, const uint4 *slut, const NetDelay *ndel, uint32_t n, uint32_t def_delay,
+                      FastRec *out);
 // A launch covers nwin windows: `h` is window 0's descriptor on the host
 // (used when nwin == 1), `dw` the device array of all nwin descriptors.
 // The windows' net tables, counts, counters and pool pointers as before a run.

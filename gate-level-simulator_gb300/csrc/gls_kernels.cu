@@ -1548,6 +1548,50 @@ __global__ void __launch_bounds__(256, GLS_COPY_BLOCKS) k_copy(const WinSet<kBat
     }
 }
 
+// ------------------------------------------------------- with a netlist
+// A gate output's fast-step record; usable = 0 where the fast step does not
+// apply: more than three input nets, irregular arcs, some input nets with
+// arcs and some without, a delay of 2^16 - 1 or more, or a truth table that
+// gives X or Z for known inputs.  (Made and uploaded by the host, the records
+// of 2 M gate outputs took 58 ms of a load.)
+__global__ void __launch_bounds__(256) k_fast_recs(const DrvMeta *__restrict__ meta, const uint4 *__restrict__ slut,
+                                                   const NetDelay *__restrict__ ndel, uint32_t n, uint32_t def_delay,
+                                                   FastRec *__restrict__ out)
+{
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const DrvMeta md = meta[i];
+    FastRec r = {};
+    if (md.m >= 1 && md.m <= 3 && (md.flags & kFlagRegular)) {
+        const uint4 t = slut[i];
+        const uint32_t words[4] = {t.x, t.y, t.z, t.w};
+        bool ok = true;
+        for (uint32_t c = 0; c < (1u << md.m); ++c) {
+            uint32_t x = 0, bit = 0;
+            for (int j = 0; j < md.m; ++j)
+                if ((c >> j) & 1u) {
+                    x |= 3u << (2 * j);
+                    bit |= 1u << (2 * j);
+                }
+            const uint32_t v = (words[x >> 4] >> (2 * (x & 15u))) & 3u;
+            ok &= v == kV0 || v == kV1;
+            if (v == kV1) r.tt |= 1u << bit;
+        }
+        int with_arcs = 0;
+        for (int j = 0; j < md.m; ++j) with_arcs += ndel[md.dt_off + j].d[0] != kInf;
+        ok &= with_arcs == 0 || with_arcs == md.m;
+        for (int j = 0; j < md.m; ++j)
+            for (int e = 0; e < 2; ++e) {
+                const uint32_t *d = &ndel[md.dt_off + j].d[e * 4];
+                const uint32_t rise = with_arcs ? d[0] : def_delay, fall = with_arcs ? d[1] : def_delay;
+                ok &= rise <= kFastDelayMax && fall <= kFastDelayMax;
+                r.d[2 * j + e] = rise | fall << 16;
+            }
+        r.usable = ok ? 1u : 0u;
+    }
+    out[i] = r;
+}
+
 // ------------------------------------------------------- before a run
 // A window's tables are rebuilt on the device from its stimulus' short ones
 // (net, length, offset per stimulus net): two launches for all windows of a
@@ -1672,6 +1716,12 @@ void launch_stim_saif(const WinDev *dw, const WinDev &h, uint32_t nwin, uint32_t
         return;
     }
     GLS_DISPATCH(h, dw, nwin, (k_stim_saif<decltype(ws)::kIsBatch, uint32_t><<<grid, 256, 0, st>>>(ws, n_nets)));
+}
+
+void launch_fast_recs(const DrvMeta *meta, const uint4 *slut, const NetDelay *ndel, uint32_t n, uint32_t def_delay,
+                      FastRec *out)
+{
+    if (n) k_fast_recs<<<(n + 255) / 256, 256>>>(meta, slut, ndel, n, def_delay, out);
 }
 
 void launch_reset(const WinDev *dw, const WinDev &h, uint32_t nwin, uint32_t max_stim, uint32_t n_nets, uint32_t n_levels,
