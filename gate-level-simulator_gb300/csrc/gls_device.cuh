@@ -411,12 +411,13 @@ struct ListReader<WideWord> {   // a list of up to 2^32 events: its end is a who
 // segment is a time (so no list needs an end position beyond its own end),
 // the entry below the stack top is kept so that an inertial pop rarely reads
 // the stack back, and the range check of output times is made once per
-// segment (a delay is below 2^16).  Measured against the walk with inner
-// branches and delay-table loads (sim_segment): the 3-input kernel of the
-// 100,000-cell, 6-level large-configuration case 460 -> 301 us and 350 -> 183
-// M warp instructions at 14 -> 25 active lanes, the 2-input one 320 -> 277 us
-// and 205 -> 119 M; the 2 M cell design over 5,000 cycles 97.2 -> 79.6 ms of
-// gate kernels.
+// segment (a delay is below 2^16).  What the fast step gave, in the kernels
+// with a thread per segment of a level (k_sim, which walks by it without a
+// step table, against sim_segment with inner branches and delay-table loads):
+// the 3-input kernel of the 100,000-cell, 6-level large-configuration case 460
+// -> 301 us and 350 -> 183 M warp instructions at 14 -> 25 active lanes, the
+// 2-input one 320 -> 277 us and 205 -> 119 M.  With the step table, in k_gate,
+// that case takes 4.2 warp instructions a fan-in event in all, at 28 lanes.
 //
 // kTab: `tab` is the shared address of the gate output's step table (see
 // step_entry; aligned to its size).  clean: from the segment's start on, all

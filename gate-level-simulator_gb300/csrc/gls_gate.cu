@@ -7,10 +7,11 @@
 // no segment tables and no launches in between.
 //
 // What bounds it: on wide levels issue (59 % of the cycles, the integer pipe
-// 58 %) by 32 warps an SM of 64 registers a thread, a quarter of whose time
+// 60 %) by 32 warps an SM of 64 registers a thread, a quarter of whose time
 // goes into waiting for the slowest warp of the block; on narrow levels the
 // chain of dependent steps of one gate output (its record, its lists' places,
-// the cut search, the walk).  Against plan, three classes of simulate, link
+// the cut search, the walk: 646 gate outputs of 1,600 events, little more than
+// a round of blocks, 25 us at 50 % issue).  Against plan, three classes of simulate, link
 // and copy kernels with one thread per segment of a level-wide segment list
 // (device ms): 2,000 cells over 1,000 cycles .95 -> .23; 37,501 cells, 3,333
 // cycles 3.97 -> 1.43; 200,000 cells, 10,000 cycles 20.1 -> 12.7; 2 M cells,
@@ -28,11 +29,12 @@ namespace gls {
 
 namespace {
 
-// threads per SM the kernels are compiled for.  kSix: the class of four to six
-// input nets, which walks by general steps in more registers (12 levels of
-// 3,000 such gate outputs of 140,000 events: 256 / 512 / 768 / 1,024 threads
-// 113 / 71 / 59 / 63 ms, the last with spills; of 100 such gate outputs of
-// 36,000 events 3.6 / 3.4 / 3.4 / 4.0).
+// Threads per SM the kernels are compiled for, in blocks of any size up to
+// that.  kSix: the class of four to six input nets, which walks by general
+// steps in more registers (12 levels of 3,000 such gate outputs of 140,000
+// events, in blocks of 256: 256 / 512 / 768 / 1,024 threads 113 / 71 / 59 / 63
+// ms, the last with spills).  How many threads a block has: see gate_block in
+// gls_capi.cpp.
 template <bool kSix, class Wd> __host__ __device__ constexpr uint32_t gate_resident()
 {
     return kSix ? (sizeof(Wd) == 4 ? 768u : 512u) : (sizeof(Wd) == 4 ? 1024u : 768u);
@@ -40,11 +42,11 @@ template <bool kSix, class Wd> __host__ __device__ constexpr uint32_t gate_resid
 
 // Shared memory is L1 lost: each kernel has only what it uses, the step table
 // (kTab) and the window's descriptor (kBatch), and behind the segments' words
-// what meets between the warps there are (WarpParts).  With 512 bytes before the segments' a 1,024-thread SM gets by
-// with 16 KB (one step of the split more: 2 M cells 68.7 instead of 68.3 ms,
-// 200,000 cells 13.1 instead of 12.9); one-warp blocks with 272 bytes instead
-// of 1,280: 8 windows of 200,000 cells 19.8 -> 19.5, 48 of 2,000 cells .89 ->
-// .87.
+// what meets between the warps there are (WarpParts).  With 512 bytes (432 now)
+// before the segments' a 1,024-thread SM gets by with 16 KB (one step of the
+// split more: 2 M cells 68.7 instead of 68.3 ms, 200,000 cells 13.1 instead of
+// 12.9); one-warp blocks with 272 bytes instead of 1,280: 8 windows of 200,000
+// cells 19.8 -> 19.5, 48 of 2,000 cells .89 -> .87.
 template <bool kTab> struct TabSmem { GateTab tab; };   // the gate output's tables
 template <> struct TabSmem<false> {};
 template <class Wd> struct WarpParts {   // an entry per warp, at the end of the dynamic shared memory

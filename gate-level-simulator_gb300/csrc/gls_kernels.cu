@@ -2,10 +2,11 @@
 //
 // The default schedule simulates a level in one launch of k_gate
 // (gls_gate.cu).  Here are the kernels beside it (stimulus SAIF, tables
-// before a run, waveforms read back) and the older form of a level, which the
+// before a run, waveforms read back) and the other form of a level, which
 // schedules with warp-per-segment classes, 256-thread blocks, wider loads or
-// learned balance, and the allocation-free entry point, take: four kinds of
-// launches,
+// learned balance, the allocation-free entry point, and runs with a few busy
+// gate outputs among very many quiet ones (gate_block in gls_capi.cpp) take:
+// four kinds of launches,
 //   k_plan     (1 CTA)   sizes every gate output's slot in the event pool and
 //                        its segment stacks in the level scratch, and splits
 //                        its fan-in timeline into time segments.

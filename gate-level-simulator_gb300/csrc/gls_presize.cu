@@ -431,9 +431,14 @@ void launch_presize(const PresizeArgs &a, bool tensor_cores, cudaStream_t st)
 // us, 3.7e-7; 64-bit atomics 116 us, 4.8e-8; eight copies 77 us, 5.8e-8; the
 // separate launches before 429 us, 2.5e-7).
 //
-// What bounds it: FP32 arithmetic, 114 kFLOP a row (8,192 rows: 14 us at the
-// peak rate).  Fifteen launches over activations in HBM, with 4 x 4 outputs a
-// thread, took 430 us a call.  Eight warps of eight rows each: a warp's lanes
+// What bounds it: latency at two warps a scheduler.  8,192 rows take 52 us of a
+// call of 78 (launches, read-back), 14 at the peak FP32 rate of their 114 kFLOP
+// each; the FMA pipe is busy 23 % of the cycles, issue 38 % of those with work,
+// and of 5.3 cycles between a warp's instructions 1.7 wait for memory and .6
+// for the queue of the atomics at the end.  254 registers a thread (the parts
+// of the gradient) leave no room for more warps.  Fifteen launches over
+// activations in HBM, with 4 x 4 outputs a thread, took 430 us a call.  Eight
+// warps of eight rows each: a warp's lanes
 // share the row operand (broadcast reads), 4 columns a lane make 32 FMAs for
 // every three 16-byte reads; row strides of 4 more floats than a multiple of
 // 32 keep the 16-byte reads down a column free of bank conflicts.

@@ -188,8 +188,8 @@ int gls_run(gls_ctx *ctx);
 typedef struct {
     uint32_t max_wave;   /* windows per wave (0: all, or as many as device memory holds with saif_only) */
     int use_graph;       /* 1: capture a wave's launches once as a CUDA graph and replay it for every wave */
-    int saif_only;       /* 1: free each window's event pool after its wave; SAIF counts and list lengths
-                            stay readable, gls_waveform does not */
+    int saif_only;       /* 1: free every window's event pool before the first wave and after its own; SAIF
+                            counts and list lengths stay readable, gls_waveform does not */
 } gls_batch_opts;
 int gls_run_batched(gls_ctx *ctx, const gls_batch_opts *opts);
 
@@ -203,7 +203,9 @@ int gls_run_batched(gls_ctx *ctx, const gls_batch_opts *opts);
  * candidates), and with GLS_ALLOC_LEARNED the learned balance of segments
  * (14).  Without warp-per-segment classes and flags other than class priority
  * a level is one launch with a block per gate output, which sizes its segments
- * itself: those candidates run alike.  Results never depend on the schedule. */
+ * itself (unless a few lists are very long among very many short ones): those
+ * candidates run alike, are timed once and share the time, and so do all for a
+ * window of 64-bit event words.  Results never depend on the schedule. */
 #define GLS_SCHED_CLASS_PRIORITY 1u   /* wider fan-in classes on higher-priority streams */
 #define GLS_SCHED_BLOCK256 2u         /* thread-per-segment gate kernels in blocks of 256 threads (else 128) */
 #define GLS_SCHED_WIDE_LOADS 4u       /* thread-per-segment gate kernels load 4 events at a time for 1- and
