@@ -774,8 +774,15 @@ extern "C" int gls_add_window(gls_ctx *ctx, const gls_stimulus *st, uint64_t t_b
         const double fan = std::max(1.0, (double)ctx->pins_total / std::max<uint32_t>(1, ctx->n_drv));
         const double grown = std::max(4.0, 1.0 + (double)(ctx->drv_level_start.size() - 1) / 20.0);
         const double per_event = grown * (1.0 + 1.0 / kGateMinSeg);
-        uint64_t want = (uint64_t)(per_event * avg * fan * ctx->max_width) + 16ull * ctx->max_width + 4096;
-        want *= w->word_bytes() / 4;   // 32-bit words
+        const double list = avg * fan * ctx->max_width;
+        const uint64_t rest = 16ull * ctx->max_width + 4096;
+        uint64_t want = ((uint64_t)(per_event * list) + rest) * (w->word_bytes() / 4);   // 32-bit words
+        if (want > ctx->scr_cap) {
+            // twice the stimulus' events where that much is not small
+            size_t fr = 0, tot = 0;
+            if (cudaMemGetInfo(&fr, &tot) == cudaSuccess) want = std::min<uint64_t>(want, fr / 64);
+            want = std::max(want, (uint64_t)(2.0 * list) + rest);
+        }
         if (want > ctx->scr_cap) {
             ctx->scr_cap = want;
             CK(ctx->lsc[0]->ensure(ctx->max_width, ctx->seg_cap, ctx->scr_cap, false), "alloc level scratch");

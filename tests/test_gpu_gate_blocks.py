@@ -65,6 +65,34 @@ def test_busy_gate_outputs_among_too_many_quiet_ones(gpu, oracle_bin):
     assert launches[0] > 4 and launches[1] == 2
 
 
+@pytest.mark.parametrize("use_graph", [False, True])
+@pytest.mark.parametrize("alloc", [0, 1, 2])
+def test_wave_of_busy_among_quiet(alloc, use_graph, gpu, oracle_bin):
+    """The same as a wave of windows, in every allocation mode, between waves
+    that take the gate kernel."""
+    n = 8_000
+    nl = level_of([("GEN_BUF_D1", [k]) for k in range(n + 3)])
+    quiet = {k: ticks(8) for k in range(n + 3)}
+    wins = [stimulus({**quiet, **{k: ticks(3_000 - 100 * w) for k in range(n, n + 3)}}) for w in range(3)]
+    model = np.zeros(MLP_PARAMS, np.float32)
+    model[-1] = 3.0
+    with Simulator(alloc_mode=alloc) as s:
+        if alloc == 2:
+            s.set_presize_model(model)
+        s.load(nl)
+        launches = []
+        for sts in ([stimulus(quiet)] * 3, wins, [stimulus(quiet)] * 3, wins):
+            s.clear_windows()
+            ids = [s.add_window(st, 0, 70_000) for st in sts]
+            s.run_batched(use_graph=use_graph)
+            launches.append(s.stats()["launches"])
+        assert launches[0] == launches[2] <= 3 and launches[1] == launches[3] > 4
+        for w, st in zip(ids, wins):
+            ow, osaif, _ = run_oracle(nl, st, 0, 70_000)
+            some = list(range(n - 2, n + 3)) + list(range(2 * n + 1, 2 * n + 6))
+            assert_same({k: s.waveform(k, w) for k in some}, s.saif(w), {k: ow[k] for k in some}, osaif, f"window {w}")
+
+
 def test_a_net_that_no_gate_reads_decides_nothing(gpu):
     """A long list that feeds no gate (a clock of registers alone) leaves the
     blocks as they are without it."""
