@@ -205,7 +205,6 @@ void ctx_drop_graphs(gls_ctx *ctx)
     ctx->graphs.clear();
 }
 
-// a window's large device buffers go; its SAIF counts, lengths and flags stay
 // a window's large device buffers go to the context's spares (saif_only);
 // its SAIF counts, lengths and flags stay
 static void release_window_pool(gls_ctx *ctx, Window *w)
@@ -765,10 +764,10 @@ extern "C" int gls_add_window(gls_ctx *ctx, const gls_stimulus *st, uint64_t t_b
     // Level scratch: the widest level's fan-in events, estimated from the
     // stimulus, and an entry more per segment.  A run that does not fit is lost
     // (the more the later the level), the space is small beside the pool.  Lists
-    // grow over the levels: the busiest level's were .98 to 3.94 times the
-    // stimulus' in 20 synthetic designs of 6 to 60 levels, 2.0 - 2.3 from 20 levels
-    // on, 2.9 from 47, 3.3 - 3.9 from 60.  First runs with room for 2 times took 17.0
-    // instead of 13.4 ms (200,000 cells, 60 levels).
+    // grow over the levels: in 20 synthetic designs the busiest level's were 1.2
+    // times the stimulus' at 6 levels, 1.7 - 2.3 at 15 to 30, 2.9 at 47, 3.3 - 3.9
+    // at 60.  First runs with room for 2 times took 17.0 instead of 13.4 ms
+    // (200,000 cells, 60 levels).
     {
         const double avg = st->n_nets ? (double)total / st->n_nets : 4.0;
         const double fan = std::max(1.0, (double)ctx->pins_total / std::max<uint32_t>(1, ctx->n_drv));

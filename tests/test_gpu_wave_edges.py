@@ -1,5 +1,6 @@
-"""What waves of windows leave behind: windows whose pool a saif_only call
-gave back without running them."""
+"""Edges of runs over several windows: windows whose pool a saif_only call gave
+back without running them, 64-bit windows among others, launch graphs and
+schedules that fit their windows, work spaces that grow, and lists read back."""
 import ctypes as C
 
 import numpy as np
